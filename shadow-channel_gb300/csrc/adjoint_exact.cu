@@ -252,42 +252,44 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
   for (int i = threadIdx.x; i < kTile; i += blockDim.x) exc[i] = 0;
   __syncthreads();
   if (KT <= kTRegs && blockDim.x == 16 * kTile) {
-    const int col = threadIdx.x % kTile, y0 = threadIdx.x / kTile;
+    const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
+    auto plane = [&](int k) { return y0 + 32 * (k >> 1) + (k & 1); };  // plane pairs, as quad_rhs_tc
     cpx vin[kTRegs];
     int emax = 0;
 #pragma unroll
     for (int k = 0; k < kTRegs; ++k) {
-      const int y = y0 + 16 * k;
-      vin[k] = (k < KT && y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
-      emax = max(emax, max((int)((__double_as_longlong(vin[k].re) >> 52) & 0x7FF),
-                           (int)((__double_as_longlong(vin[k].im) >> 52) & 0x7FF)));
+      const int y = plane(k);
+      vin[k] = (y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
+      emax = max(emax, max(exp_field(vin[k].re), exp_field(vin[k].im)));
     }
     if (emax) atomicMax(&exc[col], emax);
     __syncthreads();
     const int ex = exc[col] - 1022;
 #pragma unroll
-    for (int k = 0; k < kTRegs; ++k) {
-      if (k >= KT) break;
-      const int y = y0 + 16 * k;
-      digits_bf16(scaled56(vin[k].re, ex), dig + (size_t)(2 * col) * KS + y, 32 * KS);
-      digits_bf16(scaled56(vin[k].im, ex), dig + (size_t)(2 * col + 1) * KS + y, 32 * KS);
+    for (int k = 0; k < kTRegs; k += 2) {
+      const int y = plane(k);
+      if (y >= KT * 16) break;
+      uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
+      digits_pair(scaled56(vin[k].re, ex), scaled56(vin[k + 1].re, ex), d, 16 * KS);
+      digits_pair(scaled56(vin[k].im, ex), scaled56(vin[k + 1].im, ex), d + KS / 2, 16 * KS);
     }
   } else {
     for (int i = threadIdx.x; i < gsz.Q() * kTile; i += blockDim.x) {
       const int y = i / kTile, col = i - y * kTile;
       if (col >= nx) continue;
       const cpx v = input(y, col);
-      const int e = max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                        (int)((__double_as_longlong(v.im) >> 52) & 0x7FF));
+      const int e = max(exp_field(v.re), exp_field(v.im));
       if (e) atomicMax(&exc[col], e);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < KT * 16 * kTile; i += blockDim.x) {
-      const int y = i / kTile, col = i - y * kTile;
-      const cpx v = (y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
+    for (int i = threadIdx.x; i < KT * 8 * kTile; i += blockDim.x) {
+      const int y = 2 * (i / kTile), col = i % kTile;
+      const cpx v0 = (y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
+      const cpx v1 = (y + 1 < gsz.Q() && col < nx) ? input(y + 1, col) : cpx{0.0, 0.0};
       const int ex = exc[col] - 1022;
-      digits_bf16(scaled56(v.re, ex), dig + (size_t)(2 * col) * KS + y, 32 * KS);
-      digits_bf16(scaled56(v.im, ex), dig + (size_t)(2 * col + 1) * KS + y, 32 * KS);
+      uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
+      digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, 16 * KS);
+      digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, 16 * KS);
     }
   }
   __syncthreads();
@@ -295,17 +297,16 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
   const int NT = (2 * nx + 7) / 8, MTn = (N + 15) / 16;
   for (int item = warp; item < MTn * NT; item += blockDim.x >> 5) {
     const int mt = item / NT, nt = item - mt * NT;
-    const int col = nt * 4 + t, n = nt * 8 + gq;
-    const int ecol = exc[min(col, kTile - 1)] - 1022;
-    long long Hh[4], Ll[4];
-    tc_tile(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, dig, KS, (size_t)32 * KS, n, lane, t, Hh, Ll);
+    const int col = nt * 4 + t;
+    const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kFoldShift;
+    long long sums[4];
+    tc_tile(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const int row = mt * 16 + gq + 8 * rr;
       if (row >= N || col >= nx) continue;
-      const int e = TE[(size_t)b * gsz.R() + row] + ecol - 64;
-      const cpx val = {round_col(Hh[2 * rr], Ll[2 * rr], e, ecol + 1022),
-                       round_col(Hh[2 * rr + 1], Ll[2 * rr + 1], e, ecol + 1022)};
+      const int e = TE[(size_t)b * gsz.R() + row] + ecol;
+      const cpx val = {round_sum(sums[2 * rr], e), round_sum(sums[2 * rr + 1], e)};
       comb(row, col, val);
     }
   }
@@ -426,20 +427,22 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
     const int j = fb ? i - gsz.D() * kTile : i, row = j / kTile, col = j - row * kTile;
     if (col >= nx || col < xfirst) continue;
     const cpx v = (fb ? s.Fb : s.Fa)[row * kTile + col];
-    const int e = max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                      (int)((__double_as_longlong(v.im) >> 52) & 0x7FF));
+    const int e = max(exp_field(v.re), exp_field(v.im));
     if (e) atomicMax(&exa[(fb ? kTile : 0) + col], e);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * KTr * 16 * kTile; i += blockDim.x) {
-    const bool fb = i >= KTr * 16 * kTile;
-    const int j = fb ? i - KTr * 16 * kTile : i, row = j / kTile, col = j - row * kTile;
+  for (int i = threadIdx.x; i < 2 * KTr * 8 * kTile; i += blockDim.x) {
+    const bool fb = i >= KTr * 8 * kTile;
+    const int j = fb ? i - KTr * 8 * kTile : i, row = 2 * (j / kTile), col = j % kTile;
     const int N = fb ? gsz.R() : gsz.D();
-    const cpx v = (row < N && col < nx && col >= xfirst) ? (fb ? s.Fb : s.Fa)[row * kTile + col] : cpx{0.0, 0.0};
+    auto at = [&](int r) {
+      return (r < N && col < nx && col >= xfirst) ? (fb ? s.Fb : s.Fa)[r * kTile + col] : cpx{0.0, 0.0};
+    };
+    const cpx v0 = at(row), v1 = at(row + 1);
     const int ex = exa[(fb ? kTile : 0) + col] - 1022;
-    uint16_t* d = fb ? dB : dA;
-    digits_bf16(scaled56(v.re, ex), d + (size_t)(2 * col) * KS + row, 32 * KS);
-    digits_bf16(scaled56(v.im, ex), d + (size_t)(2 * col + 1) * KS + row, 32 * KS);
+    uint32_t* d = reinterpret_cast<uint32_t*>((fb ? dB : dA) + (size_t)(2 * col) * KS + row);
+    digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, 16 * KS);
+    digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, 16 * KS);
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
@@ -449,18 +452,18 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
   const double kz = g.Kz[z];
   for (int item = warp; item < MTq * NT; item += blockDim.x >> 5) {
     const int mt = item / NT, nt = item - mt * NT;
-    const int col = nt * 4 + t, n = nt * 8 + gq;
+    const int col = nt * 4 + t;
     double v[3][4];  // pa, qa, rb at (rows gq, gq + 8) x (Re, Im)
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const uint16_t* d = b < 2 ? dA : dB;
-      const int ecol = exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)] - 1022;
-      long long Hh[4], Ll[4];
-      tc_tile(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, d, KS, (size_t)32 * KS, n, lane, t, Hh, Ll);
+      const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + kFoldShift;
+      long long sums[4];
+      tc_tile(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int y = min(mt * 16 + gq + 8 * (r >> 1), gsz.Q() - 1);
-        v[b][r] = round_col(Hh[r], Ll[r], g.tcWTE[(size_t)b * gsz.Q() + y] + ecol - 64, ecol + 1022);
+        v[b][r] = round_sum(sums[r], g.tcWTE[(size_t)b * gsz.Q() + y] + ecol);
       }
     }
 #pragma unroll

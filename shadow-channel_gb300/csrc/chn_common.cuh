@@ -123,6 +123,7 @@ struct Grid {
   const int* tcXE;
   const int* tcZM;
   int tci;
+  int tcch;    // k-tiles per accumulation chunk of the transforms' tables (tc_common.cuh; 2 or 3)
   int tcminb;  // build of the tensor-core inverse (2..5: fields per pass, threads, blocks per SM; autotuned)
   // the same inverse on the fifth-generation tensor cores (phys_tc5.cu,
   // tcgen05.mma with tensor-memory accumulators): the two stages' digit

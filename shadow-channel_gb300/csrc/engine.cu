@@ -28,6 +28,7 @@
 #include "kernels.h"
 #include "sizes.cuh"
 #include "setup.h"
+#include "tc_common.cuh"
 
 namespace chn {
 
@@ -108,6 +109,12 @@ struct DevTables {
     *out = reinterpret_cast<const T*>(p);
     return true;
   }
+  // a digit table (two bf16 digits a word) as the fp16 digits the kernels read
+  bool up_digits(std::vector<uint32_t>& v, const uint32_t** out) {
+    for (uint32_t& w : v)
+      w = (uint32_t)half_bits_of_bf16_digit((uint16_t)w) | ((uint32_t)half_bits_of_bf16_digit((uint16_t)(w >> 16)) << 16);
+    return up(v, out);
+  }
   void release() {
     for (void* p : ptrs) cudaFree(p);
     ptrs.clear();
@@ -163,26 +170,31 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   if (!T.up(qs, &a) || !T.up(rs, &b)) return false;
   T.luQs = const_cast<double*>(a);
   T.luRs = const_cast<double*>(b);
+  bool tc_ok = false, tct_ok = false;
   {
     std::vector<uint32_t> frag, wfrag;
     std::vector<int> ex, wex;
     std::vector<uint32_t> btf, wtf;
     std::vector<int> bte, wte;
-    if (!build_adj_tc_tables(h, btf, bte, wtf, wte) || !T.up(btf, &g.tcBT) || !T.up(bte, &g.tcBTE) ||
-        !T.up(wtf, &g.tcWT) || !T.up(wte, &g.tcWTE))
-      return false;
-    if (!build_recon_tc_tables(h, frag, ex, wfrag, wex) || !T.up(frag, &g.tcA) || !T.up(ex, &g.tcE) ||
-        !T.up(wfrag, &g.tcW) || !T.up(wex, &g.tcWE))
+    // (a table whose level sums could leave the accumulators' exact range
+    // turns its kernels to FP64)
+    tc_ok = build_adj_tc_tables(h, btf, bte, wtf, wte) && build_recon_tc_tables(h, frag, ex, wfrag, wex);
+    if (!T.up_digits(btf, &g.tcBT) || !T.up(bte, &g.tcBTE) || !T.up_digits(wtf, &g.tcWT) || !T.up(wte, &g.tcWTE) ||
+        !T.up_digits(frag, &g.tcA) || !T.up(ex, &g.tcE) || !T.up_digits(wfrag, &g.tcW) || !T.up(wex, &g.tcWE))
       return false;
     std::vector<uint32_t> zf, xf;
     std::vector<int> ze, xe, zm;
-    if (!build_phys_tc_tables(h, zf, ze, xf, xe, zm) || !T.up(zf, &g.tcZ) || !T.up(ze, &g.tcZE) ||
-        !T.up(xf, &g.tcX) || !T.up(xe, &g.tcXE) || !T.up(zm, &g.tcZM))
+    const int ci = build_phys_tc_tables(h, zf, ze, xf, xe, zm);
+    if (!T.up_digits(zf, &g.tcZ) || !T.up(ze, &g.tcZE) || !T.up_digits(xf, &g.tcX) || !T.up(xe, &g.tcXE) ||
+        !T.up(zm, &g.tcZM))
       return false;
     std::vector<uint32_t> fxf, fzf, fuf;
     std::vector<int> fxe, fze, fue;
-    if (!build_fwd_tc_tables(h, fxf, fxe, fzf, fze, fuf, fue) || !T.up(fxf, &g.tcFX) || !T.up(fxe, &g.tcFXE) ||
-        !T.up(fzf, &g.tcFZ) || !T.up(fze, &g.tcFZE) || !T.up(fuf, &g.tcFXU) || !T.up(fue, &g.tcFXUE))
+    const int cf = build_fwd_tc_tables(h, fxf, fxe, fzf, fze, fuf, fue);
+    tct_ok = std::min(ci, cf) >= kChunkKT;
+    g.tcch = std::min(ci, cf);
+    if (!T.up_digits(fxf, &g.tcFX) || !T.up(fxe, &g.tcFXE) || !T.up_digits(fzf, &g.tcFZ) || !T.up(fze, &g.tcFZE) ||
+        !T.up_digits(fuf, &g.tcFXU) || !T.up(fue, &g.tcFXUE))
       return false;
   }
   // transforms: one block per plane where the plane fits the shared memory,
@@ -202,13 +214,13 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   }
   // reconstruction and quadratures on the tensor cores unless CHN_RECON_FP64=1 (or it does not fit)
   const char* fp64 = getenv("CHN_RECON_FP64");
-  g.tc = (!(fp64 && fp64[0] == '1') && recon_tc_smem_bytes(g) + 4096 <= (size_t)optin) ? 1 : 0;
+  g.tc = (tc_ok && !(fp64 && fp64[0] == '1') && recon_tc_smem_bytes(g) + 4096 <= (size_t)optin) ? 1 : 0;
   // inverse transforms on the tensor cores unless CHN_TRANSFORMS_FP64=1 (or they do not fit)
   const char* tfp64 = getenv("CHN_TRANSFORMS_FP64");
-  g.tci = (!(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
+  g.tci = (tct_ok && !(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
   g.fwdpb = 3;
   g.fxch = 8;
-  g.tcf = (!(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
+  g.tcf = (tct_ok && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
   // the kernels' builds compiled for the grid's sizes where it has them
   // (a batch's autotuner then times both); CHN_FIXED_SIZES=0 / 1 fixes it
   const bool spec = phys_tc_specialised(g);

@@ -22,6 +22,7 @@
 // (faithfully) rounded value of the exact sum of the 56-bit operands.  The
 // intermediate Z is rounded to FP64 in shared memory between the stages.  Same outputs,
 // CFL check and status bits as k_phys_inverse.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <type_traits>
@@ -118,16 +119,19 @@ bool phys_tc_matrices(const HostTables& h, std::vector<double>& Az, std::vector<
   return true;
 }
 
-bool build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std::vector<int>& zex,
+int build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std::vector<int>& zex,
                           std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap) {
   std::vector<double> Az, Ax;
   int zrows = 0, Kz = 0, xrows = 0, Kx = 0;
-  if (!phys_tc_matrices(h, Az, Ax, zmap, zrows, Kz, xrows, Kx)) return false;
+  if (!phys_tc_matrices(h, Az, Ax, zmap, zrows, Kz, xrows, Kx)) return 0;
   zfrag.clear(); zex.clear(); xfrag.clear(); xex.clear();
   // one table per stage with both classes in its K: a row's exponent covers
   // its even and odd parts, so their integer sums add exactly
-  return append_digit_table(Az.data(), zrows, Kz, (zrows + 15) / 16, Kz / 16, zfrag, zex) &&
-         append_digit_table(Ax.data(), xrows, Kx, (xrows + 15) / 16, Kx / 16, xfrag, xex);
+  const int cz = append_digit_table(Az.data(), zrows, Kz, (zrows + 15) / 16, Kz / 16, zfrag, zex);
+  const int cx = append_digit_table(Ax.data(), xrows, Kx, (xrows + 15) / 16, Kx / 16, xfrag, xex);
+  for (int e : zex)
+    if (e != kZRowExp) return 0;  // (every row holds a 1: exp(0) of kz = 0)
+  return std::min(cz, cx);
 }
 
 // forward transforms (channel/pass1.c:312-339): x stage Y[zp][kx] =
@@ -136,7 +140,7 @@ bool build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std
 // take an unscaled copy), z stage F[kz][kx] = sum_zp
 // Y[zp][kx] exp(-2 pi i zp(kz) zp/pz) for the Nz - 1 kept rows (rows 2kk,
 // 2kk+1; K = 2 pz with Re, Im of Y interleaved)
-bool build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
+int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
                          std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
                          std::vector<int>& uex) {
   const int pz = h.pz, px = h.px, Nz = h.Nz, X = h.X, Kk = Nz - 1;
@@ -162,9 +166,10 @@ bool build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std:
     }
   }
   xfrag.clear(); xex.clear(); zfrag.clear(); zex.clear(); ufrag.clear(); uex.clear();
-  return append_digit_table(Ax.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, xfrag, xex) &&
-         append_digit_table(Au.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, ufrag, uex) &&
-         append_digit_table(Az.data(), 2 * Kk, 2 * pz, (2 * Kk + 15) / 16, (2 * pz + 15) / 16, zfrag, zex);
+  const int cx = append_digit_table(Ax.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, xfrag, xex);
+  const int cu = append_digit_table(Au.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, ufrag, uex);
+  const int cz = append_digit_table(Az.data(), 2 * Kk, 2 * pz, (2 * Kk + 15) / 16, (2 * pz + 15) / 16, zfrag, zex);
+  return std::min(cx, std::min(cu, cz));
 }
 
 // ---------------------------------------------------------------------------
@@ -213,7 +218,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   int* exz = reinterpret_cast<int*>(p); p += (size_t)((d.NZ + 3) / 4 * 4) * sizeof(int);
   int* exx = reinterpret_cast<int*>(p); p += (size_t)((d.NX + 3) / 4 * 4) * sizeof(int);
   uint16_t* dig = reinterpret_cast<uint16_t*>(p); p += (phys_tc_dbuf_of(d) + 15) / 16 * 16;
-  cpx* Zb = reinterpret_cast<cpx*>(p);  // [fl][m][x]
+  cpx* Zb = reinterpret_cast<cpx*>(p);  // staged inputs, then [fl][m][x]: the z stage's folded sums
+  longlong2* Zs = reinterpret_cast<longlong2*>(Zb);
 
   const cpx* __restrict__ U = a.U.at(inst);
   double* __restrict__ P = a.P.at(inst);
@@ -224,6 +230,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
   constexpr int nwarp = NTHR >> 5;
   const int Kk = gsz.Nz() - 1;  // kept kz rows
+  const int chunk = gsz.tcch();
   bool nonfinite = false;
   for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
   __syncthreads();
@@ -245,8 +252,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
           const int z = kk < gsz.Nz() / 2 ? kk : kk + 1;
           const cpx v = field_value_qx(g, gsz.Q(), gsz.X(), U, f0 + fl, z, y, x);
           Fin[(size_t)n * Kk + kk] = v;
-          emax = max(emax, max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                               (int)((__double_as_longlong(v.im) >> 52) & 0x7FF)));
+          emax = max(emax, max(exp_field(v.re), exp_field(v.im)));
         }
         if (emax) atomicMax(&exz[n], emax);
       }
@@ -264,56 +270,55 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
         cpx v = {0.0, 0.0};
         if (kk >= 0 && n < nfb * gsz.X()) v = Fin[n * Kk + kk];
         const int ex = exz[n] - 1022;
-        digits_pair_bf16(scaled56(v.re, ex), scaled56(v.im, ex), dw + ((size_t)n * d.KSz) / 2 + w, zstride);
+        digits_pair(scaled56(v.re, ex), scaled56(v.im, ex), dw + ((size_t)n * d.KSz) / 2 + w, zstride);
       }
     }
     __syncthreads();
     {
-      // rows Re Z[m], Im Z[m] for m < pzh; E + O -> Z[m], E - O -> Z[m + pzh];
-      // the exponent of each value into its x-stage column (fl, m) (not the
-      // imaginary part of the kx = 0 bin, which c2r ignores)
+      // rows Re Z[m], Im Z[m] for m < pzh; E + O -> Z[m], E - O -> Z[m + pzh],
+      // kept as the folded 64-bit sums (scale 2^zsum_exp(column): the rows of
+      // this table share one exponent) that the x stage takes its digits
+      // from; the exponent of each value into its x-stage column (fl, m) (not
+      // the imaginary part of the kx = 0 bin, which c2r ignores)
       const int NT = (nfb * gsz.X() + 7) / 8;
       const size_t dstride = (size_t)((d.NZ + 7) / 8 * 8) * d.KSz;  // bf16 between digits
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
-        const int n = nt * 8 + gq;
-        long long HE[4], LE[4], HO[4], LO[4];
-        tc_tile_range(Az, mt, d.KTz, 0, d.KTzE, dig, d.KSz, dstride, n, lane, t, HE, LE);
-        tc_tile_range(Az, mt, d.KTz, d.KTzE, d.KTz, dig, d.KSz, dstride, n, lane, t, HO, LO);
+        long long TE[4], TO[4];
+        tc_tile_range(Az, mt, d.KTz, 0, d.KTzE, chunk, dig, d.KSz, dstride, nt * 8, lane, TE);
+        tc_tile_range(Az, mt, d.KTz, d.KTzE, d.KTz, chunk, dig, d.KSz, dstride, nt * 8, lane, TO);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int row = mt * 16 + gq + 8 * (r >> 1), col = nt * 8 + 2 * t + (r & 1);
           if (row >= 2 * d.pzh || col >= nfb * gsz.X()) continue;
-          const int e = g.tcZE[row] + exz[col] - 1022 - 64;
+          const int ce = exz[col];
           const bool im = row >= d.pzh;
           const int m = im ? row - d.pzh : row;
           int fl = 0, x = col;  // col = fl X + x, fl < FB
           while (x >= gsz.X()) { x -= gsz.X(); ++fl; }
           const bool counts = !(im && x == 0);
-          const double vp = round_col(HE[r] + HO[r], LE[r] + LO[r], e, exz[col]);
-          cpx& zp = Zb[((size_t)fl * gsz.pz() + m) * gsz.X() + x];
-          if (im) zp.im = vp;
-          else zp.re = vp;
-          const int ep = (int)((__double_as_longlong(vp) >> 52) & 0x7FF);
-          if (counts && ep) atomicMax(&exx[fl * gsz.pz() + m], ep);
+          const long long tp = TE[r] + TO[r];
+          longlong2& zp = Zs[((size_t)fl * gsz.pz() + m) * gsz.X() + x];
+          if (im) zp.y = tp;
+          else zp.x = tp;
+          const int ep = zsum_field(tp, ce);
+          if (counts && ep > 0) atomicMax(&exx[fl * gsz.pz() + m], ep);
           if (d.Rz == 2) {
-            const double vm = round_col(HE[r] - HO[r], LE[r] - LO[r], e, exz[col]);
-            cpx& zm = Zb[((size_t)fl * gsz.pz() + m + d.pzh) * gsz.X() + x];
-            if (im) zm.im = vm;
-            else zm.re = vm;
-            const int em = (int)((__double_as_longlong(vm) >> 52) & 0x7FF);
-            if (counts && em) atomicMax(&exx[fl * gsz.pz() + m + d.pzh], em);
+            const long long tm = TE[r] - TO[r];
+            longlong2& zm = Zs[((size_t)fl * gsz.pz() + m + d.pzh) * gsz.X() + x];
+            if (im) zm.y = tm;
+            else zm.x = tm;
+            const int em = zsum_field(tm, ce);
+            if (counts && em > 0) atomicMax(&exx[fl * gsz.pz() + m + d.pzh], em);
           }
         }
       }
     }
     __syncthreads();
     // ---- x stage, both fields: columns n = fl * pz + m, K words: Re, Im of
-    // Z[m][j] for the even j, then the odd j (Im of j = 0 unused).  The z
-    // stage's column exponents are cleared for the next pass.
+    // Z[m][j] for the even j, then the odd j (Im of j = 0 unused).
     const int ncx = nfb * gsz.pz();
     const size_t xstride = (size_t)((d.NX + 7) / 8 * 8) * d.KSx;
-    for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
     {
       uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
       const int npad = (ncx + 7) / 8 * 8, KW = d.KTx * 8, WE = d.KTxE * 8;
@@ -321,39 +326,40 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
       for (int i = threadIdx.x; i < npad * KW; i += NTHR, rc.next()) {
         const int n = rc.r, w = rc.c;
         const int j = w < WE ? (w < d.nxE ? d.Rx * w : -1) : (w - WE < d.nxO ? 2 * (w - WE) + 1 : -1);
-        cpx v = {0.0, 0.0};
-        if (j >= 0 && n < ncx) v = Zb[(size_t)n * gsz.X() + j];
-        if (j == 0) v.im = 0.0;
-        const int ex = exx[min(n, ncx - 1)] - 1022;
-        digits_pair_bf16(scaled56(v.re, ex), scaled56(v.im, ex), dw + ((size_t)n * d.KSx) / 2 + w, xstride / 2);
+        longlong2 v = make_longlong2(0, 0);
+        if (j >= 0 && n < ncx) {
+          v = Zs[(size_t)n * gsz.X() + j];
+          if (j == 0) v.y = 0;
+          int fl = 0, m = n;  // n = fl pz + m
+          while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
+          const int s = exx[n] - 1078 - zsum_exp(exz[fl * gsz.X() + j]);
+          v.x = scaled_sum(v.x, s);
+          v.y = scaled_sum(v.y, s);
+        }
+        digits_pair(v.x, v.y, dw + ((size_t)n * d.KSx) / 2 + w, xstride / 2);
       }
     }
     __syncthreads();
+    // the z stage's column exponents are cleared for the next pass
+    for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
     {
       // rows xp < pxh; E + O -> P[xp], E - O -> P[xp + pxh]
       const int NT = (ncx + 7) / 8;
       for (int item = warp; item < d.MTx * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
-        const int n = nt * 8 + gq;
-        long long HE[4], LE[4], HO[4], LO[4];
-        tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, dig, d.KSx, xstride, n, lane, t, HE, LE);
-        tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, dig, d.KSx, xstride, n, lane, t, HO, LO);
+        long long TE[4], TO[4];
+        tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE);
+        tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int xp = mt * 16 + gq + 8 * (r >> 1), col = nt * 8 + 2 * t + (r & 1);
           if (xp >= d.pxh || col >= ncx) continue;
           int fl = 0, m = col;  // col = fl pz + m, fl < FB
           while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
-          const int e = g.tcXE[xp] + exx[col] - 1022 - 64;
+          const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + kFoldShift;
           double* Pr = P + ((size_t)(f0 + fl) * gsz.Q() + y) * plane + (size_t)m * gsz.px();
-          const double vp = round_col(HE[r] + HO[r], LE[r] + LO[r], e, exx[col]);
-          Pr[xp] = vp;
-          nonfinite |= !finite_bits(vp);
-          if (d.Rx == 2) {
-            const double vm = round_col(HE[r] - HO[r], LE[r] - LO[r], e, exx[col]);
-            Pr[xp + d.pxh] = vm;
-            nonfinite |= !finite_bits(vm);
-          }
+          Pr[xp] = round_sum(TE[r] + TO[r], e, nonfinite);
+          if (d.Rx == 2) Pr[xp + d.pxh] = round_sum(TE[r] - TO[r], e, nonfinite);
         }
       }
     }
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     const size_t dx = (size_t)kDig * XCH * d.KSx * 2, dz = (size_t)kDig * d.Xp * d.KSz * 2;
     p += ((dx > dz ? dx : dz) + 15) / 16 * 16;
   }
-  double* stage3 = reinterpret_cast<double*>(p);  // [c][zp][xp] products; Y [zp][kx] (cpx) over plane c
+  double* stage3 = reinterpret_cast<double*>(p);  // [c][zp][xp] products; Y [zp][kx] (folded sums) over plane c
   p += ((size_t)pb * gsz.pz() * gsz.px() * sizeof(double) + 15) / 16 * 16;
   cpx* Fb = reinterpret_cast<cpx*>(p);  // [kk][kx]
   const size_t plane = (size_t)gsz.pz() * gsz.px(), fs = (size_t)gsz.Q() * plane;
@@ -493,11 +499,12 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
   constexpr int nwarp = kThreads >> 5;
   const int ncomp = mode >= 2 ? 6 : 3;
+  const int chunk = gsz.tcch();
   const size_t xstride = (size_t)XCH * d.KSx, zstride = (size_t)d.Xp * d.KSz;  // bf16 between digits
   for (int q = 0; q < ncomp; ++q) {
     const int c = q % pb;
     double* stage = stage3 + (size_t)c * plane;
-    cpx* Yb = reinterpret_cast<cpx*>(stage);
+    longlong2* Yb = reinterpret_cast<longlong2*>(stage);  // Re, Im of Y[zp][kx]: t 2^(AxE[2 kx (+ 1)] + ysum_exp(exx[zp]))
     int* exx = exx3 + c * exs;
     if (c == 0) {
       // ---- products of components q .. q+2 (each field loaded once per
@@ -515,7 +522,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
         for (int cc = 0; cc < PB; ++cc) {
           if (cc >= nc) break;
           stage3[(size_t)cc * plane + i] = v[cc];
-          const int e = (int)((__double_as_longlong(v[cc]) >> 52) & 0x7FF);
+          const int e = exp_field(v[cc]);
           if (e) atomicMax(&exx3[cc * exs + row], e);
         }
       };
@@ -530,53 +537,61 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     // ---- x stage: rows 2kx (+1), columns zp, in chunks of XCH columns; Y
     // into the staging region (Y row zp lies below stage row zp, 16 X < 8 px
     // bytes per row, so a chunk's outputs only cover rows already digitised)
+    // (the z stage's column exponents are cleared for this component first)
+    for (int i = threadIdx.x; i < gsz.X(); i += kThreads) exz[i] = 0;
     for (int zc = 0; zc < d.pzp; zc += XCH) {
       const int nch = min(XCH, d.pzp - zc);
-      FlatRC rcx(threadIdx.x, kThreads, d.KTx * 16);
-      for (int i = threadIdx.x; i < nch * (d.KTx * 16); i += kThreads, rcx.next()) {
-        const int n = zc + rcx.r, k = rcx.c;
-        const double v = (n < gsz.pz() && k < gsz.px()) ? stage[(size_t)n * gsz.px() + k] : 0.0;
-        digits_bf16(scaled56(v, exx[min(n, gsz.pz() - 1)] - 1022), dig + (size_t)rcx.r * d.KSx + k, xstride);
+      FlatRC rcx(threadIdx.x, kThreads, d.KTx * 8);
+      for (int i = threadIdx.x; i < nch * (d.KTx * 8); i += kThreads, rcx.next()) {
+        const int n = zc + rcx.r, k = 2 * rcx.c;
+        const double* src = stage + (size_t)n * gsz.px() + k;
+        const double v0 = (n < gsz.pz() && k < gsz.px()) ? src[0] : 0.0;
+        const double v1 = (n < gsz.pz() && k + 1 < gsz.px()) ? src[1] : 0.0;
+        const int ex = exx[min(n, gsz.pz() - 1)] - 1022;
+        digits_pair(scaled56(v0, ex), scaled56(v1, ex),
+                    reinterpret_cast<uint32_t*>(dig + (size_t)rcx.r * d.KSx + k), xstride / 2);
       }
       __syncthreads();
       const int NT = nch / 8;
       for (int item = warp; item < d.MTx * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
-        long long Hh[4], Ll[4];
-        tc_tile(Ax, mt, d.KTx, dig, d.KSx, xstride, nt * 8 + gq, lane, t, Hh, Ll);
+        long long T[4];
+        tc_tile(Ax, mt, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, T);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = mt * 16 + gq + 8 * (r >> 1), zp = zc + nt * 8 + 2 * t + (r & 1);
-          if (row >= 2 * gsz.X() || zp >= gsz.pz()) continue;
-          const double v = round_col(Hh[r], Ll[r], AxE[row] + exx[zp] - 1022 - 64, exx[zp]);
-          cpx& yv = Yb[(size_t)zp * gsz.X() + (row >> 1)];
-          if (row & 1) yv.im = v;
-          else yv.re = v;
+        for (int rr = 0; rr < 2; ++rr) {
+          const int row = mt * 16 + gq + 8 * rr;
+          if (row >= 2 * gsz.X()) continue;
+          const int er = AxE[row];
+          int ef = 0;  // the exponent field of this row's values, for the z stage's column
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int zp = zc + nt * 8 + 2 * t + c;
+            if (zp >= gsz.pz()) continue;
+            const long long tv = T[2 * rr + c];
+            longlong2& yv = Yb[(size_t)zp * gsz.X() + (row >> 1)];
+            if (row & 1) yv.y = tv;
+            else yv.x = tv;
+            ef = max(ef, sum_field(tv, er + ysum_exp(exx[zp]), exx[zp]));
+          }
+          if (ef > 0) atomicMax(&exz[row >> 1], ef);
         }
       }
       __syncthreads();
     }
     // ---- z stage inputs: columns kx, K = 2 pz (Re, Im of Y[zp][kx] interleaved)
-    for (int i = threadIdx.x; i < gsz.X(); i += kThreads) exz[i] = 0;
-    __syncthreads();
-    {
-      FlatRC rc(threadIdx.x, kThreads, gsz.X());
-      for (int i = threadIdx.x; i < gsz.pz() * gsz.X(); i += kThreads, rc.next()) {
-        const cpx v = Yb[i];
-        const int e = max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                          (int)((__double_as_longlong(v.im) >> 52) & 0x7FF));
-        if (e) atomicMax(&exz[rc.c], e);
-      }
-    }
-    __syncthreads();
     {
       uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
       FlatRC rc(threadIdx.x, kThreads, d.KTz * 8);
       for (int i = threadIdx.x; i < d.Xp * (d.KTz * 8); i += kThreads, rc.next()) {
         const int n = rc.r, zp = rc.c;
-        const cpx v = (n < gsz.X() && zp < gsz.pz()) ? Yb[(size_t)zp * gsz.X() + n] : cpx{0.0, 0.0};
-        const int ex = exz[min(n, gsz.X() - 1)] - 1022;
-        digits_pair_bf16(scaled56(v.re, ex), scaled56(v.im, ex), dw + ((size_t)n * d.KSz) / 2 + zp, zstride / 2);
+        longlong2 v = make_longlong2(0, 0);
+        if (n < gsz.X() && zp < gsz.pz()) {
+          v = Yb[(size_t)zp * gsz.X() + n];
+          const int s = exz[n] - 1078 - ysum_exp(exx[zp]);
+          v.x = scaled_sum(v.x, s - AxE[2 * n]);
+          v.y = scaled_sum(v.y, s - AxE[2 * n + 1]);
+        }
+        digits_pair(v.x, v.y, dw + ((size_t)n * d.KSz) / 2 + zp, zstride / 2);
       }
     }
     __syncthreads();
@@ -585,13 +600,13 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
       const int NT = d.Xp / 8;
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
-        long long Hh[4], Ll[4];
-        tc_tile(Az, mt, d.KTz, dig, d.KSz, zstride, nt * 8 + gq, lane, t, Hh, Ll);
+        long long T[4];
+        tc_tile(Az, mt, d.KTz, chunk, dig, d.KSz, zstride, nt * 8, lane, T);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int row = mt * 16 + gq + 8 * (r >> 1), kx = nt * 8 + 2 * t + (r & 1);
           if (row >= 2 * d.Kk || kx >= gsz.X()) continue;
-          const double v = round_col(Hh[r], Ll[r], g.tcFZE[row] + exz[kx] - 1022 - 64, exz[kx]);
+          const double v = round_sum(T[r], g.tcFZE[row] + col_exp(exz[kx]) - 64 + kFoldShift);
           cpx& fv = Fb[(size_t)(row >> 1) * gsz.X() + kx];
           if (row & 1) fv.im = v;
           else fv.re = v;

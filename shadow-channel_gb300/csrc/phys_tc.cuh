@@ -6,6 +6,7 @@
 
 #include "chn_common.cuh"
 #include "setup.h"
+#include "tc_common.cuh"
 
 namespace chn {
 
@@ -60,6 +61,20 @@ __host__ __device__ constexpr PhysTcDims phys_tc_dims_n(int Nz, int pz, int px, 
 __host__ __device__ inline PhysTcDims phys_tc_dims(const Grid& g, int fb = kFB) {
   return phys_tc_dims_n(g.Nz, g.pz, g.px, g.X, fb);
 }
+
+// the folded sums t of the z stage (every row of its table has the exponent
+// kZRowExp) of a column whose largest input exponent field is ce: the value is
+// t 2^zsum_exp(ce); zsum_field: its exponent field (<= 0 for zeros; 0x7FF where
+// the column held an infinity or a NaN)
+static constexpr int kZRowExp = 1;
+__device__ __forceinline__ int zsum_exp(int ce) { return kZRowExp + ce - 1022 - 64 + kFoldShift; }
+__device__ __forceinline__ int sum_field(long long t, int e, int ce) {
+  if (ce == 0x7FF) return 0x7FF;
+  return t == 0 ? 0 : max(sum_bits(t) + e + 1022, 1);
+}
+__device__ __forceinline__ int zsum_field(long long t, int ce) { return sum_field(t, zsum_exp(ce), ce); }
+// of the forward x stage, without its row's exponent
+__device__ __forceinline__ int ysum_exp(int ce) { return ce - 1022 - 64 + kFoldShift; }
 
 // the two stages' matrices (rows x K words of Re, Im) and the z stage's
 // K-word -> kept kz map

@@ -5,9 +5,9 @@
 // Same arithmetic as k_phys_inverse_tc (phys_tc.cu): the same DFT matrices,
 // row exponents and 56-bit column scaling, seven balanced base-256 digits
 // per operand, the even / odd (radix-2) split of each stage, level sums
-// l = i + k of digit products exact in FP32, folded exactly into 64-bit
-// integers and rounded once.  The integer sums do not depend on the order of
-// the products, so the outputs equal the mma.sync kernel's bit for bit.
+// l = i + k of digit products exact in FP32, folded into 64-bit integers by
+// the same rule and rounded once.  The integer sums do not depend on the order
+// of the products, so the outputs equal the mma.sync kernel's bit for bit.
 //
 // Layout of one tcgen05.mma (cta_group::1, kind::f16, M = 128, K = 16):
 //   A  the data digits: one row per data column of the stage (the z stage:
@@ -29,8 +29,7 @@
 // plane:
 //   z stage, all fields at once: stage the kept spectral rows, column
 //   exponents, digits of every k-tile; MMA the even-mode k-tiles, fold them
-//   into (H, L) pairs kept in the Z buffer (H in the slot of output m, L in
-//   that of m + pz/2: the two outputs the pair feeds); MMA the odd-mode
+//   into 64-bit sums kept in the Z buffer's slot of output m; MMA the odd-mode
 //   k-tiles into the same tensor memory and fold E + O -> Z[m],
 //   E - O -> Z[m + pz/2] in place, gathering the x stage's column exponents.
 //   x stage, in tiles of 128 columns: digits, even and odd k-tiles into two
@@ -124,8 +123,7 @@ static void append_umma_table(const double* M, int rows, int K, int Np, std::vec
     double mx = 0.0;
     for (int j = 0; j < K; ++j) mx = std::fmax(mx, std::fabs(M[(size_t)y * K + j]));
     if (mx == 0.0) continue;
-    int e = 0;
-    std::frexp(mx, &e);
+    const int e = digit_row_exponent(&M[(size_t)y * K], K);
     for (int j = 0; j < K; ++j) {
       int d[kDig];
       digits56(std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e)), d);
@@ -233,15 +231,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[N]) {
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-// exact (H, L) of seven FP32 level sums (levels at lv[0..6])
-__device__ __forceinline__ void fold7(const float (&lv)[kDig], long long& H, long long& L) {
-  int v[kDig];
-#pragma unroll
-  for (int l = 0; l < kDig; ++l) v[l] = __float2int_rn(lv[l]);
-  H = (long long)v[2] + (long long)v[1] * 256LL + (long long)v[0] * 65536LL;
-  L = (long long)v[6] + (long long)v[5] * 256LL + (long long)v[4] * 65536LL + (long long)v[3] * 16777216LL;
-}
-
 // One stage's MMAs over the k-tiles [k0, k1): data digits (A, blocks of
 // `ablk` bytes per (digit, k-tile), digit-major with KT k-tiles) against the
 // stacked table (B, k-tile blocks of 7 Np / 8 row groups) into the level
@@ -344,8 +333,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
           const int z = kk < g.Nz / 2 ? kk : kk + 1;
           const cpx v = field_value(g, U, f, z, y, x);
           Fin[(size_t)n * Kk + kk] = v;
-          emax = max(emax, max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                               (int)((__double_as_longlong(v.im) >> 52) & 0x7FF)));
+          emax = max(emax, max(exp_field(v.re), exp_field(v.im)));
         }
         if (emax) atomicMax(&exz[n], emax);
       }
@@ -386,8 +374,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
     const bool zwarp = 32 * q < t.ncz;
     const int nz = 32 * q + lane;
     const int rows_grp = t.NpZ / kT5Groups;  // a multiple of 4
-    // fold the even sums into (H, L) pairs in the Z buffer slots of the two
-    // outputs they feed
+    // fold the even sums into the Z buffer's slot of the first output they feed
     if (zwarp) {
       for (int r0 = grp * rows_grp; r0 < (grp + 1) * rows_grp; r0 += 4) {
         float lv[kDig][4];
@@ -403,14 +390,9 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             float c[kDig];
 #pragma unroll
             for (int l = 0; l < kDig; ++l) c[l] = lv[l][j];
-            long long H, L;
-            fold7(c, H, L);
             const bool im = r >= d.pzh;
             const int m = im ? r - d.pzh : r;
-            double* sp_ = reinterpret_cast<double*>(&Zb[((size_t)f * g.pz + m) * g.X + x]) + (im ? 1 : 0);
-            double* sm_ = reinterpret_cast<double*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x]) + (im ? 1 : 0);
-            *sp_ = __longlong_as_double(H);
-            *sm_ = __longlong_as_double(L);
+            reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x])[im ? 1 : 0] = fold_levels(c);
           }
         }
       }
@@ -443,23 +425,17 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             float c[kDig];
 #pragma unroll
             for (int l = 0; l < kDig; ++l) c[l] = lv[l][j];
-            long long HO, LO;
-            fold7(c, HO, LO);
             const bool im = r >= d.pzh;
             const int m = im ? r - d.pzh : r;
-            double* sp_ = reinterpret_cast<double*>(&Zb[((size_t)f * g.pz + m) * g.X + x]) + (im ? 1 : 0);
-            double* sm_ = reinterpret_cast<double*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x]) + (im ? 1 : 0);
-            const long long HE = __double_as_longlong(*sp_), LE = __double_as_longlong(*sm_);
-            const int e = g.tcZE[r] + ez - 1022 - 64;
-            const double vp = round_col(HE + HO, LE + LO, e, ez);
-            const double vm = round_col(HE - HO, LE - LO, e, ez);
-            *sp_ = vp;
-            *sm_ = vm;
+            long long* sp_ = reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x]) + (im ? 1 : 0);
+            long long* sm_ = reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x]) + (im ? 1 : 0);
+            const long long tE = *sp_, tO = fold_levels(c), tp = tE + tO, tq = tE - tO;
+            *sp_ = tp;
+            *sm_ = tq;
             if (!(im && x == 0)) {  // c2r ignores the imaginary part of the kx = 0 bin
-              const int ep = (int)((__double_as_longlong(vp) >> 52) & 0x7FF);
-              const int em = (int)((__double_as_longlong(vm) >> 52) & 0x7FF);
-              if (ep) atomicMax(&exx[f * g.pz + m], ep);
-              if (em) atomicMax(&exx[f * g.pz + m + d.pzh], em);
+              const int ep = zsum_field(tp, ez), em = zsum_field(tq, ez);
+              if (ep > 0) atomicMax(&exx[f * g.pz + m], ep);
+              if (em > 0) atomicMax(&exx[f * g.pz + m + d.pzh], em);
             }
           }
         }
@@ -478,18 +454,19 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
         const int rest = idx >> 5, ng = rest & 15, wg = rest >> 4;
         const int nl = ng * 8 + (idx & 7), w = wg * 4 + ((idx >> 3) & 3), n = c0 + nl;
         const int j = w < WE ? (w < d.nxE ? d.Rx * w : -1) : (w - WE < d.nxO ? 2 * (w - WE) + 1 : -1);
-        cpx v = {0.0, 0.0};
-        int ex = 0;
-        if (nl < nct) {
-          if (j >= 0) v = Zb[(size_t)n * g.X + j];
-          if (j == 0) v.im = 0.0;
-          ex = exx[n] - 1022;
+        longlong2 v = make_longlong2(0, 0);
+        if (nl < nct && j >= 0) {
+          v = reinterpret_cast<const longlong2*>(Zb)[(size_t)n * g.X + j];
+          if (j == 0) v.y = 0;
+          const int s = exx[n] - 1078 - zsum_exp(exz[n / g.pz * g.X + j]);
+          v.x = scaled_sum(v.x, s);
+          v.y = scaled_sum(v.y, s);
         }
         const int kt = w >> 3;
         uint32_t* dst = reinterpret_cast<uint32_t*>(areg + (size_t)kt * ablkx +
                                                     ((size_t)((nl >> 3) * 2 + ((w & 7) >> 2)) * 128) + (nl & 7) * 16 +
                                                     (w & 3) * 4);
-        digits_pair_bf16(scaled56(v.re, ex), scaled56(v.im, ex), dst, (size_t)d.KTx * ablkx / 4);
+        digits_pair_bf16(v.x, v.y, dst, (size_t)d.KTx * ablkx / 4);
       }
       fence_async_smem();
       __syncthreads();
@@ -527,15 +504,10 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
                 cE[l] = lvE[l][j];
                 cO[l] = lvO[l][j];
               }
-              long long HE, LE, HO, LO;
-              fold7(cE, HE, LE);
-              fold7(cO, HO, LO);
-              const int e = g.tcXE[xp] + ecol - 1022 - 64;
-              const double vp = round_col(HE + HO, LE + LO, e, ecol);
-              const double vm = round_col(HE - HO, LE - LO, e, ecol);
-              stage[(size_t)nl * t.stage_ld + xp] = vp;
-              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = vm;
-              nonfinite |= !finite_bits(vp) || !finite_bits(vm);
+              const long long tE = fold_levels(cE), tO = fold_levels(cO);
+              const int e = g.tcXE[xp] + col_exp(ecol) - 64 + kFoldShift;
+              stage[(size_t)nl * t.stage_ld + xp] = round_sum(tE + tO, e, nonfinite);
+              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = round_sum(tE - tO, e, nonfinite);
             }
           }
         }
@@ -606,6 +578,9 @@ static int s_t5_optin = 0;
 bool phys_tc5_fits(const Grid& g, int nf, int optin) {
   if (g.pz % 2 || g.px % 2 || nf < 1) return false;
   const T5Dims t = t5_dims(g, nf);
+  // (every class of modes in one chunk of the mma.sync kernel: the same folds)
+  const PhysTcDims& d = t.d;
+  if (max(max(d.KTzE, d.KTz - d.KTzE), max(d.KTxE, d.KTx - d.KTxE)) > g.tcch) return false;
   return t.ncz <= 128 && 7 * t.NpZ <= kT5Cols && 7 * t.NpX <= kT5XO && t5_smem_bytes(t) <= (size_t)optin;
 }
 

@@ -432,61 +432,63 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
     for (int i = threadIdx.x; i < kTile; i += NTHR) exc[i] = 0;
     __syncthreads();
     if (KT <= kQuadRegs && NTHR == 16 * kTile) {
-      // thread t holds column t % kTile, planes t / kTile + 16 k (k < KT):
-      // its inputs stay in registers from the exponent maximum to the digits
-      const int col = threadIdx.x % kTile, y0 = threadIdx.x / kTile;
+      // thread t holds column t % kTile and the plane pairs 2 (t / kTile) +
+      // 32 k, + 1 (entries 2 k, 2 k + 1): its inputs stay in registers from the
+      // exponent maximum to the digits, which pack two planes a word
+      const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
+      auto plane = [&](int k) { return y0 + 32 * (k >> 1) + (k & 1); };
       cpx vin[kQuadRegs];
       int emax = 0;
 #pragma unroll
       for (int k = 0; k < kQuadRegs; ++k) {
-        const int y = y0 + 16 * k;
-        vin[k] = (k < KT && y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
-        emax = max(emax, max((int)((__double_as_longlong(vin[k].re) >> 52) & 0x7FF),
-                             (int)((__double_as_longlong(vin[k].im) >> 52) & 0x7FF)));
+        const int y = plane(k);
+        vin[k] = (y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
+        emax = max(emax, max(exp_field(vin[k].re), exp_field(vin[k].im)));
       }
       if (emax) atomicMax(&exc[col], emax);
       __syncthreads();
       const int ex = exc[col] - 1022;
 #pragma unroll
-      for (int k = 0; k < kQuadRegs; ++k) {
-        if (k >= KT) break;
-        const int y = y0 + 16 * k;
-        digits_bf16(scaled56(vin[k].re, ex), dig + (size_t)(2 * col) * KS + y, NC * KS);
-        digits_bf16(scaled56(vin[k].im, ex), dig + (size_t)(2 * col + 1) * KS + y, NC * KS);
+      for (int k = 0; k < kQuadRegs; k += 2) {
+        const int y = plane(k);
+        if (y >= KT * 16) break;
+        uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
+        digits_pair(scaled56(vin[k].re, ex), scaled56(vin[k + 1].re, ex), d, kTile * KS);
+        digits_pair(scaled56(vin[k].im, ex), scaled56(vin[k + 1].im, ex), d + KS / 2, kTile * KS);
       }
     } else {
       for (int i = threadIdx.x; i < gsz.Q() * kTile; i += NTHR) {
         const int y = i / kTile, col = i - y * kTile;
         if (col >= nx) continue;
         const cpx v = input(q, y, col);
-        const int e = max((int)((__double_as_longlong(v.re) >> 52) & 0x7FF),
-                          (int)((__double_as_longlong(v.im) >> 52) & 0x7FF));
+        const int e = max(exp_field(v.re), exp_field(v.im));
         if (e) atomicMax(&exc[col], e);
       }
       __syncthreads();
-      for (int i = threadIdx.x; i < KT * 16 * kTile; i += NTHR) {
-        const int y = i / kTile, col = i - y * kTile;
-        const cpx v = (y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
+      for (int i = threadIdx.x; i < KT * 8 * kTile; i += NTHR) {
+        const int y = 2 * (i / kTile), col = i % kTile;
+        const cpx v0 = (y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
+        const cpx v1 = (y + 1 < gsz.Q() && col < nx) ? input(q, y + 1, col) : cpx{0.0, 0.0};
         const int ex = exc[col] - 1022;
-        digits_bf16(scaled56(v.re, ex), dig + (size_t)(2 * col) * KS + y, NC * KS);
-        digits_bf16(scaled56(v.im, ex), dig + (size_t)(2 * col + 1) * KS + y, NC * KS);
+        uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
+        digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, kTile * KS);
+        digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, kTile * KS);
       }
     }
     __syncthreads();
     const int MTn = (N + 15) / 16;
     for (int item = warp; item < MTn * NT; item += NTHR >> 5) {
       const int mt = item / NT, nt = item - mt * NT;
-      const int col = nt * 4 + t, n = nt * 8 + gq;
-      const int ecol = exc[min(col, kTile - 1)] - 1022;
-      long long Hh[4], Ll[4];
-      tc_tile_pf(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, KT, dig, KS, (size_t)NC * KS, n, lane, t, Hh, Ll);
+      const int col = nt * 4 + t;
+      const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kFoldShift;
+      long long T[4];
+      tc_tile<true>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = mt * 16 + gq + 8 * rr;
         if (row >= N || col >= nx) continue;
-        const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol - 64;
-        const cpx val = {round_col(Hh[2 * rr], Ll[2 * rr], e, ecol + 1022),
-                         round_col(Hh[2 * rr + 1], Ll[2 * rr + 1], e, ecol + 1022)};
+        const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol;
+        const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
         cpx& f = F[row * kTile + col];
         if (first) {
           f = val;

@@ -22,7 +22,9 @@
 // contraction to its own rounding.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -42,23 +44,54 @@ static constexpr int kReconRegs = 8;  // coefficient rows a thread keeps in regi
 // host: basis digit tables in mma A-fragment order
 // ---------------------------------------------------------------------------
 
-bool append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
+// the exponent of a row of K entries: |row| < 2^e, and the sum of the row's
+// 56-bit integers below 127 * 2^56, so that a folded sum over the whole row
+// fits 64 bits (only rows of more than 127 entries can need the second)
+int digit_row_exponent(const double* row, int K) {
+  double mx = 0.0, sum = 0.0;
+  for (int j = 0; j < K; ++j) {
+    mx = std::fmax(mx, std::fabs(row[j]));
+    sum += std::fabs(row[j]);
+  }
+  int e = 0;
+  std::frexp(mx, &e);
+  while (std::ldexp(sum, -e) >= 126.5) ++e;
+  return e;
+}
+
+int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
                         std::vector<int>& ex) {
   const size_t base = frag.size();
   frag.resize(base + (size_t)MT * KT * kDig * 32 * 4, 0u);
   const size_t ebase = ex.size();
   ex.resize(ebase + rows, -1022);
   std::vector<int> dig((size_t)rows * (KT * 16) * kDig, 0);
+  int chunk = kMaxChunkKT;
   for (int y = 0; y < rows; ++y) {
     double mx = 0.0;
     for (int j = 0; j < K; ++j) mx = std::fmax(mx, std::fabs(M[(size_t)y * K + j]));
     if (mx == 0.0) continue;
-    int e = 0;
-    std::frexp(mx, &e);  // |M[y][j]| < 2^e
+    const int e = digit_row_exponent(&M[(size_t)y * K], K);  // |M[y][j]| < 2^e
     ex[ebase + y] = e;
     for (int j = 0; j < K; ++j) {
       const long long x = std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e));
       digits56(x, &dig[((size_t)y * (KT * 16) + j) * kDig]);
+    }
+    // the largest level sum any data digits (|d_0| <= 256, the others <= 128)
+    // can reach over `chunk` consecutive k-tiles
+    for (int kt = 0; kt < KT && chunk > 0; ++kt) {
+      const int k1 = std::min(std::min(kt + chunk, KT) * 16, K);
+      long long used = 0;  // sum |digit i| of the window, i ascending
+      for (int l = 0; l < kDig; ++l) {
+        long long top = 0;
+        for (int j = kt * 16; j < k1; ++j) top += std::abs(dig[((size_t)y * (KT * 16) + j) * kDig + l]);
+        if (used * 128 + top * 256 > kLevelMax) {
+          --chunk;
+          --kt;  // this window again, one k-tile narrower
+          break;
+        }
+        used += top;
+      }
     }
   }
   auto at = [&](int y, int k, int i) -> uint16_t {
@@ -77,7 +110,7 @@ bool append_digit_table(const double* M, int rows, int K, int MT, int KT, std::v
           f[2] = (uint32_t)at(r0, k0 + 8, i) | ((uint32_t)at(r0, k0 + 9, i) << 16);
           f[3] = (uint32_t)at(r1, k0 + 8, i) | ((uint32_t)at(r1, k0 + 9, i) << 16);
         }
-  return true;
+  return chunk;
 }
 
 // the five bases [Q][D or R] (rows: planes) and the five weighted
@@ -86,10 +119,11 @@ bool build_recon_tc_tables(const HostTables& h, std::vector<uint32_t>& frag, std
                            std::vector<uint32_t>& wfrag, std::vector<int>& wex) {
   const int MT = (h.Q + 15) / 16, KT = (h.R + 15) / 16;
   const std::vector<double>* B[5] = {&h.Bq, &h.Bqp, &h.Bqpp, &h.Br, &h.Brp};
+  bool ok = true;
   frag.clear();
   ex.clear();
   for (int b = 0; b < 5; ++b)
-    if (!append_digit_table(B[b]->data(), h.Q, b < 3 ? h.D : h.R, MT, KT, frag, ex)) return false;
+    ok &= append_digit_table(B[b]->data(), h.Q, b < 3 ? h.D : h.R, MT, KT, frag, ex) >= kChunkKT;
   const int MTw = (h.R + 15) / 16, KTw = (h.Q + 15) / 16;
   const std::vector<double>* W[5] = {&h.Wq, &h.Wqp, &h.Wqpp, &h.Wr, &h.Wrp};
   wfrag.clear();
@@ -99,9 +133,9 @@ bool build_recon_tc_tables(const HostTables& h, std::vector<uint32_t>& frag, std
     std::vector<double> m((size_t)h.R * h.Q, 0.0);
     const int rows = b < 3 ? h.D : h.R;
     std::copy(W[b]->begin(), W[b]->begin() + (size_t)rows * h.Q, m.begin());
-    if (!append_digit_table(m.data(), h.R, h.Q, MTw, KTw, wfrag, wex)) return false;
+    ok &= append_digit_table(m.data(), h.R, h.Q, MTw, KTw, wfrag, wex) >= kChunkKT;
   }
-  return true;
+  return ok;
 }
 
 // the exact adjoint's tables: the bases transposed ([D or R][Q], rows
@@ -111,6 +145,7 @@ bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std
                          std::vector<uint32_t>& wtfrag, std::vector<int>& wtex) {
   const int MTw = (h.R + 15) / 16, KTq = (h.Q + 15) / 16;
   const std::vector<double>* B[5] = {&h.Bq, &h.Bqp, &h.Bqpp, &h.Br, &h.Brp};
+  bool ok = true;
   btfrag.clear();
   btex.clear();
   for (int b = 0; b < 5; ++b) {
@@ -118,7 +153,7 @@ bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std
     std::vector<double> m((size_t)h.R * h.Q, 0.0);
     for (int i = 0; i < cols; ++i)
       for (int y = 0; y < h.Q; ++y) m[(size_t)i * h.Q + y] = (*B[b])[(size_t)y * cols + i];
-    if (!append_digit_table(m.data(), h.R, h.Q, MTw, KTq, btfrag, btex)) return false;
+    ok &= append_digit_table(m.data(), h.R, h.Q, MTw, KTq, btfrag, btex) >= kChunkKT;
   }
   const std::vector<double>* W[3] = {&h.Wqp, &h.Wq, &h.Wr};  // [D or R][Q]
   wtfrag.clear();
@@ -128,9 +163,9 @@ bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std
     std::vector<double> m((size_t)h.Q * h.R, 0.0);
     for (int y = 0; y < h.Q; ++y)
       for (int i = 0; i < rows; ++i) m[(size_t)y * h.R + i] = (*W[b])[(size_t)i * h.Q + y];
-    if (!append_digit_table(m.data(), h.Q, h.R, KTq, MTw, wtfrag, wtex)) return false;
+    ok &= append_digit_table(m.data(), h.Q, h.R, KTq, MTw, wtfrag, wtex) >= kChunkKT;
   }
-  return true;
+  return ok;
 }
 
 // ---------------------------------------------------------------------------
@@ -178,18 +213,20 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
   __syncthreads();
   const int nent = 2 * (KT * 16) * TILE;
   if (KT <= kReconRegs && NTHR == 16 * TILE) {
-    // thread t holds column t % TILE, rows t / TILE + 16 k of both classes:
-    // its coefficients stay in registers from the exponent maxima to the digits
-    const int col = threadIdx.x % TILE, j0 = threadIdx.x / TILE;
+    // thread t holds column t % TILE and the row pairs 2 (t / TILE) + 32 k,
+    // + 1 of both classes (k < KT / 2; entry 2 k + p of vin): its coefficients
+    // stay in registers from the exponent maxima to the digits, which pack two
+    // rows a word
+    const int col = threadIdx.x % TILE, j0 = 2 * (threadIdx.x / TILE);
+    auto row = [&](int k) { return j0 + 32 * (k >> 1) + (k & 1); };
     cpx vin[2][kReconRegs];
     int emax[2] = {0, 0};
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls)
 #pragma unroll
       for (int k = 0; k < kReconRegs; ++k) {
-        vin[cls][k] = k < KT ? cval(cls, j0 + 16 * k, col) : cpx{0.0, 0.0};
-        emax[cls] = max(emax[cls], max((int)((__double_as_longlong(vin[cls][k].re) >> 52) & 0x7FF),
-                                       (int)((__double_as_longlong(vin[cls][k].im) >> 52) & 0x7FF)));
+        vin[cls][k] = k < (KT + 1) / 2 * 2 ? cval(cls, row(k), col) : cpx{0.0, 0.0};
+        emax[cls] = max(emax[cls], max(exp_field(vin[cls][k].re), exp_field(vin[cls][k].im)));
       }
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls)
@@ -199,30 +236,30 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
     for (int cls = 0; cls < 2; ++cls) {
       const int ex = exc[cls * TILE + col] - 1022;
 #pragma unroll
-      for (int k = 0; k < kReconRegs; ++k) {
-        if (k >= KT) break;
-        for (int p = 0; p < 2; ++p)  // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
-          digits_bf16(scaled56(p ? vin[cls][k].im : vin[cls][k].re, ex),
-                      dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col + p) * KS + j0 + 16 * k, (size_t)(2 * TILE) * KS);
+      for (int k = 0; k < kReconRegs; k += 2) {
+        if (k >= KT || row(k) >= KT * 16) break;
+        // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
+        uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col) * KS + row(k));
+        digits_pair(scaled56(vin[cls][k].re, ex), scaled56(vin[cls][k + 1].re, ex), d, (size_t)TILE * KS);
+        digits_pair(scaled56(vin[cls][k].im, ex), scaled56(vin[cls][k + 1].im, ex), d + KS / 2, (size_t)TILE * KS);
       }
     }
   } else {
     for (int i = threadIdx.x; i < nent; i += NTHR) {
       const int cls = i / ((KT * 16) * TILE), r = i - cls * (KT * 16) * TILE, j = r / TILE, col = r - j * TILE;
       const cpx v = cval(cls, j, col);
-      const int e1 = (int)((__double_as_longlong(v.re) >> 52) & 0x7FF);
-      const int e2 = (int)((__double_as_longlong(v.im) >> 52) & 0x7FF);
-      const int e = max(e1, e2);
+      const int e = max(exp_field(v.re), exp_field(v.im));
       if (e) atomicMax(&exc[cls * TILE + col], e);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nent; i += NTHR) {
-      const int cls = i / ((KT * 16) * TILE), r = i - cls * (KT * 16) * TILE, j = r / TILE, col = r - j * TILE;
-      const cpx v = cval(cls, j, col);
+    for (int i = threadIdx.x; i < nent / 2; i += NTHR) {
+      const int cls = i / ((KT * 8) * TILE), r = i - cls * (KT * 8) * TILE, j = 2 * (r / TILE), col = r % TILE;
+      const cpx v0 = cval(cls, j, col), v1 = cval(cls, j + 1, col);
       const int ex = exc[cls * TILE + col] - 1022;
-      for (int p = 0; p < 2; ++p)  // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
-        digits_bf16(scaled56(p ? v.im : v.re, ex), dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col + p) * KS + j,
-                    (size_t)(2 * TILE) * KS);
+      // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
+      uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col) * KS + j);
+      digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, (size_t)TILE * KS);
+      digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, (size_t)TILE * KS);
     }
   }
   __syncthreads();
@@ -236,26 +273,21 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
   for (int item = warp; item < MT * NT; item += NTHR >> 5) {
     const int mt = item / NT, nt = item - mt * NT;
     const int col = nt * 4 + t;  // this thread's complex column
-    const int n = nt * 8 + gq;   // the B-fragment column this thread loads
     cpx held[2];                 // Q' alpha, then Q'' alpha, at rows gq and gq + 8
     for (int ob = 0; ob < 5; ++ob) {
       const int b = order[ob], cls = b < 3 ? 0 : 1;
       const int KTb = ((cls == 0 ? gsz.D() : gsz.R()) + 15) / 16;
-      const int ecol = exc[cls * TILE + col] - 1022;
-      long long H[4], L[4];
-      if constexpr (MINB > 2)
-        tc_tile_range(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, dig + (size_t)cls * kDig * (2 * TILE) * KS,
-                      KS, (size_t)(2 * TILE) * KS, n, lane, t, H, L);
-      else
-        tc_tile_pf(A + (size_t)b * MT * KT * kDig * 32, mt, KT, KTb, dig + (size_t)cls * kDig * (2 * TILE) * KS, KS,
-                   (size_t)(2 * TILE) * KS, n, lane, t, H, L);
+      const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kFoldShift;
+      long long T[4];
+      tc_tile_range<(MINB <= 2)>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
+                                 dig + (size_t)cls * kDig * (2 * TILE) * KS, KS, (size_t)(2 * TILE) * KS, nt * 8, lane,
+                                 T);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int y = mt * 16 + gq + 8 * rr;
         if (y >= gsz.Q() || col >= nx || (meancol && col == 0)) continue;
-        const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol - 64;
-        const cpx val = {round_col(H[2 * rr], L[2 * rr], e, ecol + 1022),
-                         round_col(H[2 * rr + 1], L[2 * rr + 1], e, ecol + 1022)};
+        const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol;
+        const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
         const int x = x0 + col;
         cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
         const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];

@@ -19,6 +19,7 @@ struct SizesRT {
   __device__ int Qh() const { return g.Qh; }
   __device__ int R() const { return g.R; }
   __device__ int D() const { return g.D; }
+  __device__ int tcch() const { return g.tcch; }
 };
 
 // the sizes of an NX x NY x NZ grid (Nx, Ny, Nz as in c_init)
@@ -33,12 +34,13 @@ struct SizesCT {
   __host__ __device__ static constexpr int Qh() { return (3 * NY / 2 + 1) / 2; }
   __host__ __device__ static constexpr int R() { return NY - 2; }
   __host__ __device__ static constexpr int D() { return NY - 4; }
+  __host__ __device__ static constexpr int tcch() { return 3; }
 };
 
 template <class S>
 __host__ __device__ inline bool sizes_match(const Grid& g) {
   return g.Nz == S::Nz() && g.X == S::X() && g.pz == S::pz() && g.px == S::px() && g.Q == S::Q() &&
-         g.Qh == S::Qh() && g.R == S::R() && g.D == S::D();
+         g.Qh == S::Qh() && g.R == S::R() && g.D == S::D() && g.tcch >= S::tcch();
 }
 
 // the grids with specialised builds

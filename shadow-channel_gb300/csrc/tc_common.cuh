@@ -4,15 +4,24 @@
 //
 // An operand row or column is scaled by a power of two into an integer of 56
 // significant bits and written as seven balanced base-256 digits (the top
-// digit in [-256, 256], the others in [-128, 127]), each exact in bf16.
-// Digit products of level l = i + k accumulate in FP32 through mma.sync
-// m16n8k16; with at most 112 terms per chunk a level's partial sums stay
-// below 2^24, so FP32 holds them exactly.  Levels l < 7 are kept (the rest
-// lie below 2^-56 of the operands' scale), recombined exactly in 64-bit
-// integers and rounded once to FP64.
+// digit in [-256, 256], the others in [-128, 127]), each exact in fp16 (and
+// in the bf16 of the tcgen05 kernel).  Digit products of level l = i + k
+// accumulate in FP32 through mma.sync m16n8k16, exactly, in chunks of at most
+// two or three k-tiles.  Levels l < 7 are kept (the rest lie below 2^-56 of the
+// operands' scale), folded into one 64-bit integer per output (to 2^-56 of
+// that scale, a sixteenth of what the dropped levels leave) and rounded once
+// to FP64.
+//
+// What bounds these tiles is the work around the products: the digits, the
+// folds and the roundings.  Start values that make a level's integer readable
+// from the accumulator's bit pattern, levels combined in pairs in 32 bits, one
+// 64-bit sum instead of two and a rounding without a normalising shift take a
+// fold and rounding from about 45 instructions to 20, the packed fp16 digits
+// those of a pair of values from 39 to 17.
 #pragma once
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 #include <cstring>
@@ -23,7 +32,6 @@
 namespace chn {
 
 static constexpr int kDig = 7;      // base-256 digits per operand
-static constexpr int kChunkKT = 7;  // k-tiles per exact FP32 accumulation chunk (K <= 112)
 
 inline uint16_t bf16_bits_of_int(int d) {
   const float f = (float)d;  // |d| <= 256: exact in bf16, low 16 bits zero
@@ -42,68 +50,137 @@ inline void digits56(long long x, int* d) {
   d[0] = (int)x;
 }
 
-__device__ __forceinline__ void mma_bf16_16816(float* d, const uint4& a, uint32_t b0, uint32_t b1) {
+// fp16 bit pattern of an integer |d| <= 2048 held as a bf16 bit pattern (the
+// host tables): both formats hold every digit exactly
+inline uint16_t half_bits_of_bf16_digit(uint16_t b) {
+  const uint32_t u = (uint32_t)b << 16;
+  float f;
+  std::memcpy(&f, &u, 4);
+  const __half_raw r = __half_raw(__float2half_rn(f));
+  return r.x;
+}
+
+// Level accumulators start at 1.5 * 2^23 instead of 0: while a level sum
+// stays within +-2^22 the FP32 accumulator is 1.5 * 2^23 + sum exactly and
+// its bit pattern is kAccBits + sum, so the integer comes out without a
+// float-to-integer conversion.  The first product of a level takes the start
+// value as its C operand.  Level 6 starts 2^(kFoldShift - 1) higher, which
+// rounds the fold's shift to nearest.
+static constexpr uint32_t kAccBits = 0x4B400000u;
+// the folded sums' unit: 2^kFoldShift of level 6's
+static constexpr int kFoldShift = 8;
+// k-tiles per accumulation chunk: append_digit_table finds the most for which
+// every level sum stays within +-2^22 whatever the data (a digit of a table
+// averages 64 of 128 at most, so two k-tiles have a margin of two; three do
+// for most tables)
+static constexpr int kChunkKT = 2;     // the Legendre tables (FP64 kernels where a table allows fewer)
+static constexpr int kMaxChunkKT = 3;  // the transforms': Grid::tcch
+static constexpr long long kLevelMax = (1LL << 22) - (1LL << kFoldShift);
+
+__device__ __forceinline__ float acc_start(int l) {
+  return __uint_as_float(kAccBits + (l == kDig - 1 ? (1u << (kFoldShift - 1)) : 0u));
+}
+
+__device__ __forceinline__ void mma_f16_16816(float* d, const uint4& a, uint32_t b0, uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
 
-// the seven digits of v * 2^(56 - ex) from the bit pattern (integer ops only);
-// ex bounds the column: |v| < 2^ex
+// the same with a fresh accumulator c in every element
+__device__ __forceinline__ void mma_f16_16816_from(float* d, const uint4& a, uint32_t b0, uint32_t b1, float c) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%10,%10,%10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1), "f"(c));
+}
+
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr));
+}
+
+__device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr));
+}
+
+// biased exponent field of v
+__device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+
+// the exponent of a column whose largest biased exponent field is ce
+// (|v| < 2^col_exp); a column that held an infinity or a NaN (its digits
+// carry no meaning) gets one that round_sum turns into NaN
+static constexpr int kNanExp = 1 << 20;
+__device__ __forceinline__ int col_exp(int ce) { return ce == 0x7FF ? kNanExp : ce - 1022; }
+
+// v * 2^(56 - ex) as an integer, rounded half away from zero, from the bit
+// pattern (integer ops only); ex bounds the column: |v| < 2^ex
 __device__ __forceinline__ long long scaled56(double v, int ex) {
-  const long long bits = __double_as_longlong(v);
-  const int ef = (int)((bits >> 52) & 0x7FF);
-  if (ef == 0) return 0;  // zero (denormals are below every scale in use)
-  long long sig = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-  const int s = ef - 1019 - ex;  // <= 3
-  if (s >= 0) sig <<= s;
-  else if (s > -62) sig = (sig + (1LL << (-s - 1))) >> (-s);
-  else sig = 0;
-  return bits < 0 ? -sig : sig;
+  const int hi = __double2hiint(v);
+  const int ef = (hi >> 20) & 0x7FF;
+  const unsigned long long m =
+      (((unsigned long long)((hi & 0xFFFFF) | 0x100000) << 32) | (unsigned)__double2loint(v)) << 4;
+  long long x = (long long)(((m >> min(max(ex + 1022 - ef, 0), 63)) + 1) >> 1);
+  if (ef == 0) x = 0;  // zero (denormals are below every scale in use)
+  return hi < 0 ? -x : x;
 }
 
-// (H 2^32 + L) 2^e with one FP64 conversion: the sum is folded into one
-// int64 keeping at least 62 significant bits (|H| < 2^41, |L| < 2^50), the
-// conversion rounds it, and the power of two goes into the exponent field
-// with integer arithmetic.  Faithful (the folded-away low bits lie more
-// than 8 bits below the result's last place); the FP64 pipe sees one
-// conversion per value.
-__device__ __forceinline__ double round_fast(long long H, long long L, int e) {
-  const unsigned long long aH = (unsigned long long)(H < 0 ? -H : H);
-  const int sh = max(0, 34 - __clzll((long long)aH));  // |T| < 2^63
-  const long long T = (long long)((unsigned long long)H << (32 - sh)) + (L >> sh);
-  if (T == 0) return 0.0;
-  const double v = (double)T;
-  const long long bits = __double_as_longlong(v);
-  const int es = e + sh;
-  const int ex = (int)((bits >> 52) & 0x7FF) + es;
-  if (ex > 0 && ex < 2047) return __longlong_as_double(bits + ((long long)es << 52));
-  return scalbn(v, es);
+// a folded sum t (below) scaled by 2^-s, rounded half up
+__device__ __forceinline__ long long scaled_sum(long long t, int s) {
+  if (s > 0) return ((t >> min(s - 1, 62)) + 1) >> 1;
+  return t << min(-s, 63);
 }
 
-// round_fast for an output of a column whose largest biased exponent field
-// is ce: a column that held an infinity or a NaN (ce = 0x7FF; its digits
-// carry no meaning) gives NaN, as the FP64 sum would
-__device__ __forceinline__ double round_col(long long H, long long L, int e, int ce) {
-  return ce == 0x7FF ? __longlong_as_double(0x7FF8000000000000LL) : round_fast(H, L, e);
+// bits of |t|: |t| < 2^n (0 for t = 0; one's complement of a negative t,
+// which at most loses the step to an exact power of two)
+__device__ __forceinline__ int sum_bits(long long t) {
+  const unsigned long long a = (unsigned long long)(t < 0 ? -t : t);
+  return 64 - __clzll((long long)a);
+}
+
+// t * 2^e, rounded once: one FP64 conversion, the power of two added to the
+// exponent field.  Zeros, results outside the normal range and NaN columns
+// (e >= kNanExp / 2) take the multiplications below; bad is set for results
+// that are not finite.
+__device__ __forceinline__ double round_sum(long long t, int e, bool& bad) {
+  const double v = (double)t;
+  const int hi = __double2hiint(v);
+  const int ef = hi & 0x7FF00000;
+  if (ef != 0 && (unsigned)((ef >> 20) + e - 1) < 2046u) return __hiloint2double(hi + (e << 20), __double2loint(v));
+  if (e >= kNanExp / 2) {
+    bad = true;
+    return __longlong_as_double(0x7FF8000000000000LL);
+  }
+  const int h = e >> 1;
+  const double f0 = __hiloint2double((min(max(h, -1022), 1023) + 1023) << 20, 0);
+  const double f1 = __hiloint2double((min(max(e - h, -1022), 1023) + 1023) << 20, 0);
+  const double r = v * f0 * f1;
+  bad |= exp_field(r) == 0x7FF;
+  return r;
+}
+
+__device__ __forceinline__ double round_sum(long long t, int e) {
+  bool bad = false;
+  return round_sum(t, e, bad);
 }
 
 // x is neither infinite nor NaN (integer test on the exponent field)
-__device__ __forceinline__ bool finite_bits(double x) {
-  return ((__double_as_longlong(x) >> 52) & 0x7FF) != 0x7FF;
-}
+__device__ __forceinline__ bool finite_bits(double x) { return exp_field(x) != 0x7FF; }
 
 // Balanced digits without a carry chain: with B = sum_{i<6} 128 * 256^i,
 // x + B = sum_{q>=1} (d_q + 128) 256^(6-q) + d_0 256^6, so every lower digit
 // is an unsigned byte of x + B less 128 and the top digit (in [-256, 256])
-// its arithmetic shift by 48.  The digits come out as FP32 values without an
-// integer-to-float conversion: for 0 <= u < 2^23 the bit pattern
-// 0x4B000000 | u is the float 2^23 + u, so a byte b placed under that
-// exponent (one byte permute) less 2^23 + 128 is b - 128, exactly (one FP32
-// add); the top digit goes the same way through u = d_0 + 256.  Every digit
-// has at most 8 significant bits, so the float's upper half is its exact bf16.
+// its arithmetic shift by 48.  The digits come out as floats without an
+// integer-to-float conversion.  FP32 (the tcgen05 kernel's bf16 digits): for
+// 0 <= u < 2^23 the bit pattern 0x4B000000 | u is the float 2^23 + u, so a
+// byte b placed under that exponent (one byte permute) less 2^23 + 128 is
+// b - 128, exactly (one FP32 add); the top digit goes the same way through
+// u = d_0 + 256.  Every digit has at most 8 significant bits, so the float's
+// upper half is its exact bf16.
 __device__ __forceinline__ void balanced_digits_f32(long long x, float (&f)[kDig]) {
   const long long xb = x + 0x808080808080LL;
   const unsigned lo = (unsigned)xb, hi = (unsigned)(xb >> 32);
@@ -118,16 +195,8 @@ __device__ __forceinline__ void balanced_digits_f32(long long x, float (&f)[kDig
   f[0] = __uint_as_float((unsigned)(((int)hi >> 16) + (0x4B000000 + 256))) - 8388864.0f;  // 2^23 + 256
 }
 
-// seven balanced digits of x (|x| < 2^56) as bf16 bit patterns, most significant first
-__device__ __forceinline__ void digits_bf16(long long x, uint16_t* out, size_t stride) {
-  float f[kDig];
-  balanced_digits_f32(x, f);
-#pragma unroll
-  for (int q = 0; q < kDig; ++q) out[(size_t)q * stride] = (uint16_t)(__float_as_uint(f[q]) >> 16);
-}
-
-// the balanced digits of two values (re, im) packed per digit into one 32-bit
-// word (re in the low half): out[q * stride] for q = 0..6
+// the balanced digits of two values (re, im) as bf16 packed per digit into
+// one 32-bit word (re in the low half): out[q * stride] for q = 0..6
 __device__ __forceinline__ void digits_pair_bf16(long long xr, long long xi, uint32_t* out, size_t stride) {
   float fr[kDig], fi[kDig];
   balanced_digits_f32(xr, fr);
@@ -137,112 +206,130 @@ __device__ __forceinline__ void digits_pair_bf16(long long xr, long long xi, uin
     out[(size_t)q * stride] = __byte_perm(__float_as_uint(fr[q]), __float_as_uint(fi[q]), 0x7632);
 }
 
-// the exact level sums of one mma accumulator element added to (H, L): the
-// sum is (H 2^32 + L) 2^(e_row + e_col - 64) for operands scaled to 56-bit
-// integers.  Each level enters as a 32 x 32 -> 64-bit multiply-add onto the
-// running 64-bit sum (exact integer arithmetic: the order does not matter).
-__device__ __forceinline__ void fold_levels_add(const float (&acc)[kDig][4], int r, long long& H, long long& L) {
-  int lv[kDig];
+// The same as fp16, two values a word and two digits a permute (17 permutes
+// and packed adds for a pair where the bf16 form takes 39): a byte b under
+// the exponent of 1024 (0x6400 | b) is 1024 + b, less 1152 it is b - 128; the
+// top digit enters the 64-bit sum under 0x6500 (1024 + 256 + d_0).
+__device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t* out, size_t stride) {
+  constexpr long long kB = 0x6500808080808080LL;
+  const long long a = x0 + kB, b = x1 + kB;
+  const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+  constexpr uint32_t kE = 0x64646464u;
+  const uint32_t p65 = __byte_perm(al, bl, 0x5140), p43 = __byte_perm(al, bl, 0x7362), p21 = __byte_perm(ah, bh, 0x5140);
+  const uint32_t w[kDig] = {__byte_perm(ah, bh, 0x7632), __byte_perm(p21, kE, 0x4342), __byte_perm(p21, kE, 0x4140),
+                            __byte_perm(p43, kE, 0x4342), __byte_perm(p43, kE, 0x4140), __byte_perm(p65, kE, 0x4342),
+                            __byte_perm(p65, kE, 0x4140)};
 #pragma unroll
-  for (int l = 0; l < kDig; ++l) lv[l] = __float2int_rn(acc[l][r]);
-  H += (long long)lv[2];
-  H += (long long)lv[1] * 256LL;
-  H += (long long)lv[0] * 65536LL;
-  L += (long long)lv[6];
-  L += (long long)lv[5] * 256LL;
-  L += (long long)lv[4] * 65536LL;
-  L += (long long)lv[3] * 16777216LL;
+  for (int q = 0; q < kDig; ++q) {
+    const uint32_t off = q == 0 ? 0xE500E500u : 0xE480E480u;  // -1280, -1152
+    uint32_t r;
+    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(w[q]), "r"(off));
+    out[(size_t)q * stride] = r;
+  }
+}
+
+// Folds the level sums of one mma accumulator element (acc[l][r], levels
+// 0..6, started at acc_start) into t in units of 2^kFoldShift of level 6:
+// adjacent levels combine in 32 bits (|l + 256 l'| < 2^31), so a fold is seven
+// integer instructions.  The start values' bit patterns stay in: kFoldBias
+// per fold.
+__device__ __forceinline__ long long fold_raw(const float (&acc)[kDig][4], int r) {
+  auto bits = [&](int l) { return __float_as_uint(acc[l][r]); };
+  const uint32_t u56 = bits(6) + (bits(5) << 8), u34 = bits(4) + (bits(3) << 8), u12 = bits(2) + (bits(1) << 8);
+  unsigned long long t = u56 >> kFoldShift;
+  t += (unsigned long long)u34 * (1u << (16 - kFoldShift));
+  t += (unsigned long long)u12 * (1u << (32 - kFoldShift));
+  t += (unsigned long long)bits(0) << (48 - kFoldShift);
+  return (long long)t;
+}
+
+constexpr uint32_t kPairBits = kAccBits + (kAccBits << 8);  // of two combined start values (mod 2^32)
+constexpr unsigned long long kFoldBias =
+    (unsigned long long)(kPairBits >> kFoldShift) + ((unsigned long long)kPairBits << (16 - kFoldShift)) +
+    ((unsigned long long)kPairBits << (32 - kFoldShift)) + ((unsigned long long)kAccBits << (48 - kFoldShift));
+
+// the same fold of seven exact integer level sums (the tcgen05 kernel)
+__device__ __forceinline__ long long fold_levels(const float (&lv)[kDig]) {
+  int v[kDig];
+#pragma unroll
+  for (int l = 0; l < kDig; ++l) v[l] = __float2int_rn(lv[l]);
+  const int p56 = v[6] + v[5] * 256 + (1 << (kFoldShift - 1)), p34 = v[4] + v[3] * 256, p12 = v[2] + v[1] * 256;
+  return (long long)(p56 >> kFoldShift) + (long long)p34 * (1LL << (16 - kFoldShift)) +
+         (long long)p12 * (1LL << (32 - kFoldShift)) + (long long)v[0] * (1LL << (48 - kFoldShift));
 }
 
 // One exact digit GEMM tile of a fixed table A (fragment order
-// [mt][KT][7][32][4]) against the smem digits of column n, over the k-tiles
-// [k0, k1): FP32 level sums per chunk of at most 7 k-tiles (exact), folded
-// into the 64-bit integers H, L per accumulator element (exact across
-// chunks: |H| < 2^41, |L| < 2^50 per chunk); an empty range gives zeros
-__device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int mt, int KT, int k0, int k1,
-                                              const uint16_t* dig, size_t KS, size_t dstride, int n, int lane, int t,
-                                              long long (&H)[4], long long (&L)[4]) {
+// [mt][KT][7][32][4]) against the smem digits of the eight columns from n0
+// ([digit][column][KS], a digit plane every dstride), over the k-tiles
+// [k0, k1): exact level sums per chunk of at most `chunk` k-tiles, folded
+// into one 64-bit integer per accumulator element.  The sum is
+// t 2^(e_row + e_col - 64 + kFoldShift) for operands scaled to 56-bit
+// integers; an empty range gives zeros.  PF: the table fragments of k-tile
+// kt + 1 are loaded while kt's products run (tables that live in L2).
+template <bool PF = false>
+__device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int mt, int KT, int k0, int k1, int chunk,
+                                              const uint16_t* dig, size_t KS, size_t dstride, int n0, int lane,
+                                              long long (&T)[4]) {
 #pragma unroll
-  for (int r = 0; r < 4; ++r) { H[r] = 0; L[r] = 0; }
-  for (int kc = k0; kc < k1; kc += kChunkKT) {
+  for (int r = 0; r < 4; ++r) T[r] = 0;
+  const uint4* Am = A + (size_t)mt * KT * kDig * 32 + lane;
+  // ldmatrix rows: matrices 0, 1 the two k halves of a digit, 2, 3 of the next
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(dig) +
+                        (uint32_t)(((lane >> 4) * dstride + (n0 + (lane & 7)) * KS + ((lane >> 3) & 1) * 8) * 2);
+  const uint32_t dst2 = (uint32_t)(4 * dstride);  // bytes between digit pairs
+  uint4 an[kDig];
+  if (PF && k0 < k1) {
+#pragma unroll
+    for (int i = 0; i < kDig; ++i) an[i] = __ldg(Am + ((size_t)k0 * kDig + i) * 32);
+  }
+  for (int kc = k0; kc < k1; kc += chunk) {
     float acc[kDig][4];
+    const int kend = min(k1, kc + chunk);
+    auto tile = [&](int kt, bool first) {
+      uint4 af[kDig];
+      if (PF) {
+        const int kn = min(kt + 1, k1 - 1);
 #pragma unroll
-    for (int l = 0; l < kDig; ++l)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[l][r] = 0.f;
-    const int kend = min(k1, kc + kChunkKT);
-    for (int kt = kc; kt < kend; ++kt) {
-      const uint32_t* brow = reinterpret_cast<const uint32_t*>(dig + (size_t)n * KS + kt * 16);
-      uint32_t b0[kDig], b1[kDig];
-#pragma unroll
-      for (int k = 0; k < kDig; ++k) {
-        b0[k] = brow[(size_t)k * dstride / 2 + t];
-        b1[k] = brow[(size_t)k * dstride / 2 + t + 4];
+        for (int i = 0; i < kDig; ++i) {
+          af[i] = an[i];
+          an[i] = __ldg(Am + ((size_t)kn * kDig + i) * 32);
+        }
       }
+      uint32_t b0[kDig], b1[kDig];
+      const uint32_t row = base + (uint32_t)(kt * 32);
+#pragma unroll
+      for (int k = 0; k + 1 < kDig; k += 2) ldsm_x4(row + (k / 2) * dst2, b0[k], b1[k], b0[k + 1], b1[k + 1]);
+      ldsm_x2(row + (kDig / 2) * dst2, b0[kDig - 1], b1[kDig - 1]);
 #pragma unroll
       for (int i = 0; i < kDig; ++i) {
-        const uint4 af = __ldg(&A[(((size_t)mt * KT + kt) * kDig + i) * 32 + lane]);
+        const uint4 ai = PF ? af[i] : __ldg(Am + ((size_t)kt * kDig + i) * 32);
 #pragma unroll
-        for (int k = 0; k < kDig - i; ++k) mma_bf16_16816(acc[i + k], af, b0[k], b1[k]);
+        for (int k = 0; k < kDig - i; ++k) {
+          if (first && i == 0) mma_f16_16816_from(acc[k], ai, b0[k], b1[k], acc_start(k));
+          else mma_f16_16816(acc[i + k], ai, b0[k], b1[k]);
+        }
       }
-    }
+    };
+    tile(kc, true);
+    for (int kt = kc + 1; kt < kend; ++kt) tile(kt, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fold_levels_add(acc, r, H[r], L[r]);
+    for (int r = 0; r < 4; ++r) T[r] += fold_raw(acc, r) - (long long)kFoldBias;
   }
 }
 
-__device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, const uint16_t* dig, size_t KS,
-                                        size_t dstride, int n, int lane, int t, long long (&H)[4],
-                                        long long (&L)[4]) {
-  tc_tile_range(A, mt, KT, 0, KT, dig, KS, dstride, n, lane, t, H, L);
+template <bool PF = false>
+__device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
+                                        size_t KS, size_t dstride, int n0, int lane, long long (&T)[4]) {
+  tc_tile_range<PF>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T);
 }
 
-// The same tile over the k-tiles [0, k1) of a table with KT k-tiles per row
-// tile, with the table fragments of k-tile kt + 1 loaded while kt's products
-// run (for tables that live in L2)
-__device__ __forceinline__ void tc_tile_pf(const uint4* __restrict__ A, int mt, int KT, int k1, const uint16_t* dig,
-                                           size_t KS, size_t dstride, int n, int lane, int t, long long (&H)[4],
-                                           long long (&L)[4]) {
-#pragma unroll
-  for (int r = 0; r < 4; ++r) { H[r] = 0; L[r] = 0; }
-  const uint4* Am = A + (size_t)mt * KT * kDig * 32 + lane;
-  for (int kc = 0; kc < k1; kc += kChunkKT) {
-    float acc[kDig][4];
-#pragma unroll
-    for (int l = 0; l < kDig; ++l)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) acc[l][r] = 0.f;
-    const int kend = min(k1, kc + kChunkKT);
-    uint4 af[kDig];
-#pragma unroll
-    for (int i = 0; i < kDig; ++i) af[i] = __ldg(Am + ((size_t)kc * kDig + i) * 32);
-    for (int kt = kc; kt < kend; ++kt) {
-      const int kn = min(kt + 1, kend - 1);
-      uint4 an[kDig];
-#pragma unroll
-      for (int i = 0; i < kDig; ++i) an[i] = __ldg(Am + ((size_t)kn * kDig + i) * 32);
-      const uint32_t* brow = reinterpret_cast<const uint32_t*>(dig + (size_t)n * KS + kt * 16);
-      uint32_t b0[kDig], b1[kDig];
-#pragma unroll
-      for (int k = 0; k < kDig; ++k) {
-        b0[k] = brow[(size_t)k * dstride / 2 + t];
-        b1[k] = brow[(size_t)k * dstride / 2 + t + 4];
-      }
-#pragma unroll
-      for (int i = 0; i < kDig; ++i)
-#pragma unroll
-        for (int k = 0; k < kDig - i; ++k) mma_bf16_16816(acc[i + k], af[i], b0[k], b1[k]);
-#pragma unroll
-      for (int i = 0; i < kDig; ++i) af[i] = an[i];
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r) fold_levels_add(acc, r, H[r], L[r]);
-  }
-}
+// host: the exponent of a table row (its entries and their sum bounded)
+int digit_row_exponent(const double* row, int K);
 
 // host: digit table of a row-major matrix M[rows][K] in mma A-fragment order
-// [MT][KT][7][32 lanes][4] (appended to frag), row exponents appended to ex
-bool append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
+// [MT][KT][7][32 lanes][4] (appended to frag), row exponents appended to ex;
+// returns the k-tiles per chunk its level sums allow (0: none)
+int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
                         std::vector<int>& ex);
 
 }  // namespace chn
