@@ -246,6 +246,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // CHN_SOLVE_TILE=8 or 16 fixes it (and skips that timing)
   const char* stl = getenv("CHN_SOLVE_TILE");  // 16, 8 or 8/128 (8 columns, 128 threads)
   g.stile = (stl && atoi(stl) == 8) ? 8 : 16;
+  g.sfixed = (stl && stl[0]) ? 1 : 0;
   g.sthr = (g.stile == 8 && stl && strstr(stl, "/128")) ? 128 : 256;
   // the tensor-core reconstruction's build (recon_tc.cu): 0 until the
   // autotuner has timed 0, 1, 2; CHN_RECON_BUILD fixes it

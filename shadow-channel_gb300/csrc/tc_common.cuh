@@ -258,11 +258,42 @@ __device__ __forceinline__ long long fold_levels(const float (&lv)[kDig]) {
          (long long)p12 * (1LL << (32 - kFoldShift)) + (long long)v[0] * (1LL << (48 - kFoldShift));
 }
 
+// lane's ldmatrix address of the digits of the eight columns from n0
+// ([digit][column][KS], a digit plane every dstride): matrices 0, 1 are the
+// two k halves of a digit, 2, 3 of the next
+__device__ __forceinline__ uint32_t tc_row_addr(const uint16_t* dig, size_t KS, size_t dstride, int n0, int lane) {
+  return (uint32_t)__cvta_generic_to_shared(dig) +
+         (uint32_t)(((lane >> 4) * dstride + (n0 + (lane & 7)) * KS + ((lane >> 3) & 1) * 8) * 2);
+}
+
+// the 28 digit products of one k-tile (table fragments af, digits at row;
+// dst2 bytes between digit pairs), `first` of a chunk: on fresh accumulators
+__device__ __forceinline__ void tc_ktile(const uint4 (&af)[kDig], uint32_t row, uint32_t dst2, float (&acc)[kDig][4],
+                                         bool first) {
+  uint32_t b0[kDig], b1[kDig];
+#pragma unroll
+  for (int k = 0; k + 1 < kDig; k += 2) ldsm_x4(row + (k / 2) * dst2, b0[k], b1[k], b0[k + 1], b1[k + 1]);
+  ldsm_x2(row + (kDig / 2) * dst2, b0[kDig - 1], b1[kDig - 1]);
+#pragma unroll
+  for (int i = 0; i < kDig; ++i)
+#pragma unroll
+    for (int k = 0; k < kDig - i; ++k) {
+      if (first && i == 0) mma_f16_16816_from(acc[k], af[i], b0[k], b1[k], acc_start(k));
+      else mma_f16_16816(acc[i + k], af[i], b0[k], b1[k]);
+    }
+}
+
+__device__ __forceinline__ void tc_load_frags(uint4 (&af)[kDig], const uint4* __restrict__ A) {
+#pragma unroll
+  for (int i = 0; i < kDig; ++i) af[i] = __ldg(A + i * 32);
+}
+
+static constexpr int kFragStep = kDig * 32;  // uint4 between the k-tiles of a table
+
 // One exact digit GEMM tile of a fixed table A (fragment order
-// [mt][KT][7][32][4]) against the smem digits of the eight columns from n0
-// ([digit][column][KS], a digit plane every dstride), over the k-tiles
-// [k0, k1): exact level sums per chunk of at most `chunk` k-tiles, folded
-// into one 64-bit integer per accumulator element.  The sum is
+// [mt][KT][7][32][4]) against the smem digits of the eight columns from n0,
+// over the k-tiles [k0, k1): exact level sums per chunk of at most `chunk`
+// k-tiles, folded into one 64-bit integer per accumulator element.  The sum is
 // t 2^(e_row + e_col - 64 + kFoldShift) for operands scaled to 56-bit
 // integers; an empty range gives zeros.  PF: the table fragments of k-tile
 // kt + 1 are loaded while kt's products run (tables that live in L2).
@@ -272,43 +303,24 @@ __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int m
                                               long long (&T)[4]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) T[r] = 0;
-  const uint4* Am = A + (size_t)mt * KT * kDig * 32 + lane;
-  // ldmatrix rows: matrices 0, 1 the two k halves of a digit, 2, 3 of the next
-  const uint32_t base = (uint32_t)__cvta_generic_to_shared(dig) +
-                        (uint32_t)(((lane >> 4) * dstride + (n0 + (lane & 7)) * KS + ((lane >> 3) & 1) * 8) * 2);
-  const uint32_t dst2 = (uint32_t)(4 * dstride);  // bytes between digit pairs
+  const uint4* Am = A + (size_t)mt * KT * kFragStep + lane;
+  const uint32_t base = tc_row_addr(dig, KS, dstride, n0, lane);
+  const uint32_t dst2 = (uint32_t)(4 * dstride);
   uint4 an[kDig];
-  if (PF && k0 < k1) {
-#pragma unroll
-    for (int i = 0; i < kDig; ++i) an[i] = __ldg(Am + ((size_t)k0 * kDig + i) * 32);
-  }
+  if (PF && k0 < k1) tc_load_frags(an, Am + (size_t)k0 * kFragStep);
   for (int kc = k0; kc < k1; kc += chunk) {
     float acc[kDig][4];
     const int kend = min(k1, kc + chunk);
     auto tile = [&](int kt, bool first) {
       uint4 af[kDig];
       if (PF) {
-        const int kn = min(kt + 1, k1 - 1);
 #pragma unroll
-        for (int i = 0; i < kDig; ++i) {
-          af[i] = an[i];
-          an[i] = __ldg(Am + ((size_t)kn * kDig + i) * 32);
-        }
+        for (int i = 0; i < kDig; ++i) af[i] = an[i];
+        tc_load_frags(an, Am + (size_t)min(kt + 1, k1 - 1) * kFragStep);
+      } else {
+        tc_load_frags(af, Am + (size_t)kt * kFragStep);
       }
-      uint32_t b0[kDig], b1[kDig];
-      const uint32_t row = base + (uint32_t)(kt * 32);
-#pragma unroll
-      for (int k = 0; k + 1 < kDig; k += 2) ldsm_x4(row + (k / 2) * dst2, b0[k], b1[k], b0[k + 1], b1[k + 1]);
-      ldsm_x2(row + (kDig / 2) * dst2, b0[kDig - 1], b1[kDig - 1]);
-#pragma unroll
-      for (int i = 0; i < kDig; ++i) {
-        const uint4 ai = PF ? af[i] : __ldg(Am + ((size_t)kt * kDig + i) * 32);
-#pragma unroll
-        for (int k = 0; k < kDig - i; ++k) {
-          if (first && i == 0) mma_f16_16816_from(acc[k], ai, b0[k], b1[k], acc_start(k));
-          else mma_f16_16816(acc[i + k], ai, b0[k], b1[k]);
-        }
-      }
+      tc_ktile(af, base + (uint32_t)(kt * 32), dst2, acc, first);
     };
     tile(kc, true);
     for (int kt = kc + 1; kt < kend; ++kt) tile(kt, false);
@@ -321,6 +333,44 @@ template <bool PF = false>
 __device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
                                         size_t KS, size_t dstride, int n0, int lane, long long (&T)[4]) {
   tc_tile_range<PF>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T);
+}
+
+// The same whole tile as one of a sequence that a warp runs with few others
+// on its SM, where nothing else hides the tables' L2 latency: pf holds the
+// fragments of this tile's first two k-tiles on entry and of the next
+// tile's (at An; null: none) on exit, so two k-tiles are always in flight.
+// KT >= 2.
+struct FragPair {
+  uint4 f[2][kDig];
+};
+__device__ __forceinline__ void tc_stream_start(FragPair& pf, const uint4* __restrict__ Am) {
+  tc_load_frags(pf.f[0], Am);
+  tc_load_frags(pf.f[1], Am + kFragStep);
+}
+__device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __restrict__ Am, const uint4* __restrict__ An,
+                                               int KT, uint32_t base, uint32_t dst2, long long (&T)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) T[r] = 0;
+  if (An == nullptr) An = Am;  // the last tile: loads that nothing uses
+  for (int kc = 0; kc < KT; kc += kChunkKT) {
+    float acc[kDig][4];
+    auto tile = [&](int kt, bool first) {
+      uint4 af[kDig];
+#pragma unroll
+      for (int i = 0; i < kDig; ++i) {
+        af[i] = pf.f[0][i];
+        pf.f[0][i] = pf.f[1][i];
+      }
+      const int kn = kt + 2;
+      tc_load_frags(pf.f[1], kn < KT ? Am + (size_t)kn * kFragStep : An + (size_t)(kn - KT) * kFragStep);
+      tc_ktile(af, base + (uint32_t)(kt * 32), dst2, acc, first);
+    };
+    static_assert(kChunkKT == 2, "two k-tiles a chunk");
+    tile(kc, true);
+    if (kc + 1 < KT) tile(kc + 1, false);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) T[r] += fold_raw(acc, r) - (long long)kFoldBias;
+  }
 }
 
 // host: the exponent of a table row (its entries and their sum bounded)
