@@ -19,6 +19,7 @@
 // and the products kernel (k_products_adj with `exact`) takes H_bar's
 // physical fields to u_in_bar.
 #include "chn_common.cuh"
+#include "few_tile.cuh"
 #include "kernels.h"
 #include "sizes.cuh"
 #include "solve_common.cuh"
@@ -62,29 +63,88 @@ __device__ __forceinline__ cpx band_matvecT_row(const double* __restrict__ A, in
 // A^T y = b for one parity chain, A = L U the no-pivot factors of
 // channel/mvOps.c:29-91 (L unit lower in columns j < dl, U in dl..dl+du):
 // U^T w = b ascending, then L^T y = w descending; RD the reciprocal pivots
-// (the forward chain multiplies by them too)
-template <int W, int DL, int DU>
-__device__ void band_solveT_chain(const double* __restrict__ LU, const double* __restrict__ RD, int N, int par,
-                                  double* b, int bstride) {
-  for (int i = par; i < N; i += 2) {
-    double acc = b[i * bstride];
+// (the forward chain multiplies by them too).  The last results stay in
+// registers, the next rows' factors load meanwhile (as band_solve_chain).
+template <int W, int DL, int DU, bool GLOBAL>
+__device__ __forceinline__ void band_solveT_chain(const double* __restrict__ LU, const double* __restrict__ RD, int N,
+                                                  int par, double* b, int bstride) {
+  const int M = (N - par + 1) / 2;  // rows of this parity: i = par + 2 m
+  if (M <= 0) return;
+  constexpr int G = kChainRows;
+  {
+    double f[G][DU], v[G], p[G], x[DU];
+    auto load = [&](int m0) {
 #pragma unroll
-    for (int j = 1; j <= DU; ++j) {
-      const int m = i - 2 * j;
-      // row m of U holds column i when m >= 0 and j <= min(DU, (N - m + 1) / 2 - 1)
-      if (m >= 0 && j <= (N - m + 1) / 2 - 1) acc = fma(-__ldg(LU + (size_t)m * W + DL + j), b[m * bstride], acc);
+      for (int q = 0; q < G; ++q) {
+        const int m = min(m0 + q, M - 1), i = par + 2 * m;
+#pragma unroll
+        for (int j = 1; j <= DU; ++j)
+          f[q][j - 1] = band_load<GLOBAL>(LU + (size_t)(par + 2 * max(m - j, 0)) * W + DL + j);
+        p[q] = band_load<GLOBAL>(RD + i);
+        v[q] = b[i * bstride];
+      }
+    };
+#pragma unroll
+    for (int t = 0; t < DU; ++t) x[t] = 0.0;  // x[t]: the result t + 1 rows back
+    load(0);
+    for (int m0 = 0; m0 < M; m0 += G) {
+      double c[G][DU], w[G], r[G];
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+#pragma unroll
+        for (int j = 0; j < DU; ++j) c[q][j] = f[q][j];
+        w[q] = v[q];
+        r[q] = p[q];
+      }
+      load(m0 + G);
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        double acc = w[q];
+#pragma unroll
+        for (int j = DU - 1; j >= 0; --j) acc = fma(-c[q][j], x[j], acc);
+        acc *= r[q];
+#pragma unroll
+        for (int t = DU - 1; t > 0; --t) x[t] = x[t - 1];
+        x[0] = acc;
+        if (m0 + q < M) b[(par + 2 * (m0 + q)) * bstride] = acc;
+      }
     }
-    b[i * bstride] = acc * __ldg(RD + i);
   }
-  const int ilast = ((N - 1 - par) % 2 == 0) ? N - 1 : N - 2;
-  for (int i = ilast; i >= 0; i -= 2) {
-    double acc = b[i * bstride];
+  {
+    double f[G][DL], v[G], x[DL];
+    auto load = [&](int n0) {  // rows from the last one down
 #pragma unroll
-    for (int t = 1; t <= DL; ++t) {
-      const int m = i + 2 * t;
-      if (m < N && t <= m / 2) acc = fma(-__ldg(LU + (size_t)m * W + DL - t), b[m * bstride], acc);
+      for (int q = 0; q < G; ++q) {
+        const int m = max(M - 1 - (n0 + q), 0);
+#pragma unroll
+        for (int t = 1; t <= DL; ++t)
+          f[q][t - 1] = band_load<GLOBAL>(LU + (size_t)(par + 2 * min(m + t, M - 1)) * W + DL - t);
+        v[q] = b[(par + 2 * m) * bstride];
+      }
+    };
+#pragma unroll
+    for (int t = 0; t < DL; ++t) x[t] = 0.0;
+    load(0);
+    for (int n0 = 0; n0 < M; n0 += G) {
+      double c[G][DL], w[G];
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+#pragma unroll
+        for (int j = 0; j < DL; ++j) c[q][j] = f[q][j];
+        w[q] = v[q];
+      }
+      load(n0 + G);
+#pragma unroll
+      for (int q = 0; q < G; ++q) {
+        double acc = w[q];
+#pragma unroll
+        for (int t = DL - 1; t >= 0; --t) acc = fma(-c[q][t], x[t], acc);
+#pragma unroll
+        for (int t = DL - 1; t > 0; --t) x[t] = x[t - 1];
+        x[0] = acc;
+        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = acc;
+      }
     }
-    b[i * bstride] = acc;
   }
 }
 
@@ -94,8 +154,11 @@ struct SolveTSmem {
   cpx* rb;     // [R][kTile]
   cpx* Fa;     // [D][kTile] Recon^T alpha part, then F_bar alpha
   cpx* Fb;     // [R][kTile]
-  double* m0;  // mean mode: fa[R], fb[R], ca[R] (cpx), cb[R] (cpx)
+  // the FEW build's: digits (dig; hc unused), staged factors
+  uint16_t* dig;
+  double *luA, *luB, *rdA, *rdB;  // [tile][D][9], [tile][R][5], [tile][D], [tile][R]
 };
+
 
 // bytes of the tensor-core digits: Recon^T's [7][32][Q pad] (+ exponents),
 // Quad^T's two [7][32][R pad] (+ exponents)
@@ -113,8 +176,35 @@ __host__ __device__ inline size_t solveT_hc_elems(const Grid& g) {
 }
 
 static size_t solveT_smem_bytes(const Grid& g) {
-  size_t n = solveT_hc_elems(g) + (size_t)g.D * kTile + (size_t)g.R * kTile;
-  return n * sizeof(cpx) + (size_t)8 * g.R * sizeof(double);
+  return (solveT_hc_elems(g) + (size_t)g.D * kTile + (size_t)g.R * kTile) * sizeof(cpx);
+}
+
+// the FEW build's plan: digits (Recon^T's five inputs, then Quad^T's two),
+// right-hand sides, F, the tile's factors
+__host__ __device__ inline size_t solveT_few_dig_bytes(const Grid& g, int tile) {
+  const size_t rt = (size_t)5 * kDig * 2 * tile * ((g.Q + 15) / 16 * 16 + 8) * 2;
+  const size_t qt = (size_t)2 * kDig * 2 * tile * ((g.R + 15) / 16 * 16 + 8) * 2;
+  return ((rt > qt ? rt : qt) + 5 * tile * sizeof(int) + 15) / 16 * 16;
+}
+static size_t solveT_few_smem_bytes(const Grid& g, int tile) {
+  return solveT_few_dig_bytes(g, tile) + (size_t)tile * (3 * g.R + g.D) * sizeof(cpx) +
+         (size_t)tile * (10 * g.D + 6 * g.R) * sizeof(double);
+}
+template <int TT>
+__device__ inline SolveTSmem carve_solveT_few(const Grid& g, unsigned char* base) {
+  SolveTSmem s;
+  s.hc = nullptr;
+  s.dig = reinterpret_cast<uint16_t*>(base);
+  cpx* p = reinterpret_cast<cpx*>(base + solveT_few_dig_bytes(g, TT));
+  s.ra = p; p += (size_t)g.R * TT;
+  s.rb = p; p += (size_t)g.R * TT;
+  s.Fa = p; p += (size_t)g.D * TT;
+  s.Fb = p; p += (size_t)g.R * TT;
+  s.luA = reinterpret_cast<double*>(p);
+  s.luB = s.luA + (size_t)TT * g.D * 9;
+  s.rdA = s.luB + (size_t)TT * g.R * 5;
+  s.rdB = s.rdA + (size_t)TT * g.D;
+  return s;
 }
 
 __device__ inline SolveTSmem carve_solveT(const Grid& g, unsigned char* base) {
@@ -125,12 +215,18 @@ __device__ inline SolveTSmem carve_solveT(const Grid& g, unsigned char* base) {
   s.rb = p + (size_t)g.R * kTile;
   p += solveT_hc_elems(g);
   s.Fa = p; p += (size_t)g.D * kTile;
-  s.Fb = p; p += (size_t)g.R * kTile;
-  s.m0 = reinterpret_cast<double*>(p);
+  s.Fb = p;
   return s;
 }
 
-// Recon^T of the velocity cotangent of columns x0.. (not the mean mode):
+// the mean line's: R^T (u + i w) and R'^T (du + i dw), both real lines (its
+// imaginary parts never reach the fields); a non-finite one makes the input NaN
+__device__ __forceinline__ cpx recon_T_mean_input(const cpx& u, const cpx& w) {
+  const bool bad = exp_field(u.im) == 0x7FF || exp_field(w.im) == 0x7FF;
+  return cpx{bad ? u.im + w.im : u.re, w.re};
+}
+
+// Recon^T of the velocity cotangent of columns x0.. (the mean line: recon_T_mean_input):
 //   alpha_bar = Q^T v_bar - Q'^T Xp_bar + Q''^T dx_bar   (rows < D) -> s.Fa
 //   beta_bar  = R^T Zp_bar + R'^T dz_bar                 (rows < R) -> s.Fb
 // with Xp_bar = (i kx u_bar + i kz w_bar)/K2, Zp_bar = (i kz u_bar - i kx w_bar)/K2,
@@ -147,7 +243,7 @@ __device__ void recon_T_tile(const Grid& g, const cpx* __restrict__ Ub, int z, i
     for (int i = threadIdx.x; i < g.Qh * kTile; i += blockDim.x) {
       const int yp = i / kTile, l = i - yp * kTile;
       cpx* dst = s.hc + (size_t)i * 6;
-      if (l >= nx || l < xfirst) continue;
+      if (l >= nx) continue;
       const int x = x0 + l;
       const double ax = g.kxK2[(size_t)z * g.X + x], az = g.kzK2[(size_t)z * g.X + x];
       const int ya = yp, yb = g.Q - 1 - yp;
@@ -167,6 +263,10 @@ __device__ void recon_T_tile(const Grid& g, const cpx* __restrict__ Ub, int z, i
           in[side][0].im = fma(az, u.re, -ax * w.re);
           in[side][1].re = fma(ax, dw.im, -az * du.im);  // dz_bar = i(az du - ax dw)
           in[side][1].im = fma(az, du.re, -ax * dw.re);
+          if (l < xfirst) {
+            in[side][0] = recon_T_mean_input(u, w);
+            in[side][1] = recon_T_mean_input(du, dw);
+          }
         }
       }
       for (int q = 0; q < nin; ++q) {
@@ -182,7 +282,7 @@ __device__ void recon_T_tile(const Grid& g, const cpx* __restrict__ Ub, int z, i
       }
     }
     __syncthreads();
-    if (lx < nx && lx >= xfirst) {
+    if (lx < nx) {
       const int N = phase == 0 ? g.D : g.R;
       constexpr int MAXR = 4;
       for (int ib = grp; ib < N; ib += ngrp * MAXR) {
@@ -313,8 +413,18 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
   __syncthreads();
 }
 
+// the derived plane inputs of Recon^T: o[1] Xp_bar = i(ax u + az w), o[2]
+// dx_bar = -i(ax du + az dw), o[3] Zp_bar = i(az u - ax w), o[4] dz_bar =
+// i(az du - ax dw)
+__device__ __forceinline__ void recon_T_inputs(double ax, double az, const cpx& u, const cpx& w, const cpx& du,
+                                               const cpx& dw, cpx (&o)[5]) {
+  o[1] = cpx{-fma(ax, u.im, az * w.im), fma(ax, u.re, az * w.re)};
+  o[2] = cpx{fma(ax, du.im, az * dw.im), -fma(ax, du.re, az * dw.re)};
+  o[3] = cpx{fma(ax, w.im, -az * u.im), fma(az, u.re, -ax * w.re)};
+  o[4] = cpx{fma(ax, dw.im, -az * du.im), fma(az, du.re, -ax * dw.re)};
+}
+
 // Recon^T (as recon_T_tile) with its five contractions on the tensor cores
-// (the mean column, col < xfirst, gets zeros: it has its own rows)
 template <class S>
 __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ Ub, int z, int x0, int nx, int xfirst,
                            SolveTSmem& s) {
@@ -367,7 +477,7 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
   contract_planes_tc(
       g, gsz, T, g.tcBTE, 3, gsz.R(), nx,
       [&](int y, int col) {
-        if (col < xfirst) return cpx{0.0, 0.0};
+        if (col < xfirst) return recon_T_mean_input(at(0, y, col), at(2, y, col));
         double ax, az;
         axz(col, ax, az);
         const cpx u = at(0, y, col), w = at(2, y, col);
@@ -377,7 +487,7 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
   contract_planes_tc(
       g, gsz, T, g.tcBTE, 4, gsz.R(), nx,
       [&](int y, int col) {
-        if (col < xfirst) return cpx{0.0, 0.0};
+        if (col < xfirst) return recon_T_mean_input(at(3, y, col), at(4, y, col));
         double ax, az;
         axz(col, ax, az);
         const cpx du = at(3, y, col), dw = at(4, y, col);
@@ -391,25 +501,24 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
       dig, exc);
 }
 
-// Recon^T of the mean mode, row i (transpose of channel/initAlphaBeta2.c:25-68):
-// a_bar = R^T u_bar + R'^T du_bar, b_bar = R^T w_bar + R'^T dw_bar
-__device__ __forceinline__ void recon_T_mean_row(const Grid& g, const cpx* __restrict__ Ub, int i, cpx& a, cpx& b) {
-  const size_t cs = (size_t)g.Q * g.X;
-  double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-  for (int y = 0; y < g.Q; ++y) {
-    const double r = __ldg(g.Br + (size_t)y * g.R + i), rp = __ldg(g.Brp + (size_t)y * g.R + i);
-    const cpx u = Ub[0 * cs + (size_t)y * g.X], w = Ub[2 * cs + (size_t)y * g.X];
-    const cpx du = Ub[3 * cs + (size_t)y * g.X], dw = Ub[4 * cs + (size_t)y * g.X];
-    ar = fma(r, u.re, fma(rp, du.re, ar));
-    ai = fma(r, u.im, fma(rp, du.im, ai));
-    br = fma(r, w.re, fma(rp, dw.re, br));
-    bi = fma(r, w.im, fma(rp, dw.im, bi));
-  }
-  a = cpx{ar, ai};
-  b = cpx{br, bi};
+// Hz, Hx, Hy of one plane and column from pa = Qpw^T Fa, qa = Qw^T Fa, rb =
+// Rw^T Fb, its roundings fixed (the builds agree bit for bit):
+// Hx = -i kx pa - i kz rb, Hz = -i kz pa + i kx rb, Hy = -K2 qa, times scl
+__device__ __forceinline__ void quad_T_combine(double kx, double kz, double k2, double scl, const cpx& pa, const cpx& qa,
+                                               const cpx& rb, cpx* out, size_t cs) {
+  out[0] = cpx{scl * fma(kz, pa.im, __dmul_rn(-kx, rb.im)), scl * fma(kx, rb.re, __dmul_rn(-kz, pa.re))};
+  out[cs] = cpx{scl * fma(kx, pa.im, __dmul_rn(kz, rb.im)), -scl * fma(kx, pa.re, __dmul_rn(kz, rb.re))};
+  out[2 * cs] = cpx{__dmul_rn(-scl, k2) * qa.re, __dmul_rn(-scl, k2) * qa.im};
 }
 
-// H_bar = Quad^T(F_bar) on the tensor cores for the columns [xfirst, nx):
+// the mean line's: Hx.re = Rw^T fa, Hz.re = Rw^T fb, rb = Rw^T (fa + i fb)
+__device__ __forceinline__ void quad_T_mean(double scl, const cpx& rb, cpx* out, size_t cs) {
+  out[0] = cpx{scl * rb.im, 0.0};
+  out[cs] = cpx{scl * rb.re, 0.0};
+  out[2 * cs] = cpx{0.0, 0.0};
+}
+
+// H_bar = Quad^T(F_bar) on the tensor cores for the columns [0, nx):
 // per plane y the contractions over the modes pa = Qpw^T Fa, qa = Qw^T Fa,
 // rb = Rw^T Fb as GEMMs (rows: planes), then the combination of the FP64
 // loop in k_solve_T (the mean column keeps that loop)
@@ -425,7 +534,7 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
   for (int i = threadIdx.x; i < (gsz.D() + gsz.R()) * kTile; i += blockDim.x) {
     const bool fb = i >= gsz.D() * kTile;
     const int j = fb ? i - gsz.D() * kTile : i, row = j / kTile, col = j - row * kTile;
-    if (col >= nx || col < xfirst) continue;
+    if (col >= nx || (col < xfirst && !fb)) continue;
     const cpx v = (fb ? s.Fb : s.Fa)[row * kTile + col];
     const int e = max(exp_field(v.re), exp_field(v.im));
     if (e) atomicMax(&exa[(fb ? kTile : 0) + col], e);
@@ -436,7 +545,7 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
     const int j = fb ? i - KTr * 8 * kTile : i, row = 2 * (j / kTile), col = j % kTile;
     const int N = fb ? gsz.R() : gsz.D();
     auto at = [&](int r) {
-      return (r < N && col < nx && col >= xfirst) ? (fb ? s.Fb : s.Fa)[r * kTile + col] : cpx{0.0, 0.0};
+      return (r < N && col < nx && (col >= xfirst || fb)) ? (fb ? s.Fb : s.Fa)[r * kTile + col] : cpx{0.0, 0.0};
     };
     const cpx v0 = at(row), v1 = at(row + 1);
     const int ex = exa[(fb ? kTile : 0) + col] - 1022;
@@ -469,41 +578,156 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const int y = mt * 16 + gq + 8 * rr;
-      if (y >= gsz.Q() || col >= nx || col < xfirst) continue;
+      if (y >= gsz.Q() || col >= nx) continue;
       const int x = x0 + col;
-      const double kx = g.Kx[x], k2 = g.K2[(size_t)z * gsz.X() + x];
-      const double scl = x == 0 ? g.norm : 0.5 * g.norm;
-      const cpx pa = {v[0][2 * rr], v[0][2 * rr + 1]}, qa = {v[1][2 * rr], v[1][2 * rr + 1]};
-      const cpx rb = {v[2][2 * rr], v[2][2 * rr + 1]};
-      cpx hx, hy, hz;
-      hx.re = scl * (kx * pa.im + kz * rb.im);  // -i kx pa - i kz rb
-      hx.im = -scl * (kx * pa.re + kz * rb.re);
-      hz.re = scl * (kz * pa.im - kx * rb.im);  // -i kz pa + i kx rb
-      hz.im = scl * (kx * rb.re - kz * pa.re);
-      hy.re = -scl * k2 * qa.re;
-      hy.im = -scl * k2 * qa.im;
-      cpx* out = Hb + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
-      out[0] = hz;
-      out[cs] = hx;
-      out[2 * cs] = hy;
+      if (col < xfirst) {
+        quad_T_mean(g.norm, cpx{v[2][2 * rr], v[2][2 * rr + 1]}, Hb + (size_t)y * gsz.X(), cs);
+        continue;
+      }
+      quad_T_combine(g.Kx[x], kz, g.K2[(size_t)z * gsz.X() + x], x == 0 ? g.norm : 0.5 * g.norm,
+                     cpx{v[0][2 * rr], v[0][2 * rr + 1]}, cpx{v[1][2 * rr], v[1][2 * rr + 1]},
+                     cpx{v[2][2 * rr], v[2][2 * rr + 1]}, Hb + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x, cs);
     }
   }
 }
 
-// S: the sizes (SizesRT, or SizesCT for a specialised grid)
-template <bool MULTI, class S>
-__global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__ Grid g0, SolveTArgs a) {
-  const int ntx = (g0.X + kTile - 1) / kTile;
+// quad_T_tc for launches with few blocks: a 4-column tile, a warp per 16
+// planes, its three tables' k-tiles as one stream.  KP: row pairs of Fa or Fb
+// a thread holds (R <= 64 KP).
+template <int KP, class S>
+__device__ __forceinline__ void quad_T_few(const Grid& g, const S& gsz, int z, int x0, int nx, int xfirst, SolveTSmem& s,
+                                           cpx* __restrict__ Hb) {
+  constexpr int TT = 4, NTHR = 256, NC = 2 * TT;
+  const int KTr = (gsz.R() + 15) / 16, MTq = (gsz.Q() + 15) / 16;
+  const size_t KS = (size_t)KTr * 16 + 8;
+  int* exc = reinterpret_cast<int*>(s.dig + (size_t)2 * kDig * NC * KS);  // [2][TT]
+  if (threadIdx.x < 2 * TT) exc[threadIdx.x] = 0;
+  __syncthreads();
+  {
+    // threads [0, 128) take Fa, the rest Fb; row pairs 2 (t / TT) + 64 k
+    const int cls = threadIdx.x >> 7, col = threadIdx.x % TT, j0 = 2 * ((threadIdx.x & 127) / TT);
+    const int N = cls ? gsz.R() : gsz.D();
+    const cpx* F = cls ? s.Fb : s.Fa;
+    const bool on = col < nx && (col >= xfirst || cls);
+    cpx v[KP][2];
+    int e = 0;
+#pragma unroll
+    for (int k = 0; k < KP; ++k)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int j = j0 + p + 64 * k;
+        v[k][p] = (on && j < N) ? F[j * TT + col] : cpx{0.0, 0.0};
+        e = max(e, max(exp_field(v[k][p].re), exp_field(v[k][p].im)));
+      }
+#pragma unroll
+    for (int o = 16; o >= TT; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if ((threadIdx.x & 31) < TT) atomicMax(&exc[cls * TT + col], e);
+    __syncthreads();
+    const int ex = exc[cls * TT + col] - 1022;
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int j = j0 + 64 * k;
+      if (j >= KTr * 16) break;
+      uint32_t* d = reinterpret_cast<uint32_t*>(s.dig + ((size_t)cls * kDig * NC + 2 * col) * KS + j);
+      digits_pair(scaled56(v[k][0].re, ex), scaled56(v[k][1].re, ex), d, NC * KS / 2);
+      digits_pair(scaled56(v[k][0].im, ex), scaled56(v[k][1].im, ex), d + KS / 2, NC * KS / 2);
+    }
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
+  const uint4* __restrict__ W = reinterpret_cast<const uint4*>(g.tcWT) + lane;
+  const size_t cs = (size_t)gsz.Q() * gsz.X();
+  const int x = x0 + min(t, nx - 1);
+  auto table = [&](int mt, int b) { return W + ((size_t)b * MTq + mt) * KTr * kFragStep; };
+  FragPair pf;
+  if (warp < MTq) tc_stream_start(pf, table(warp, 0));
+  for (int mt = warp; mt < MTq; mt += NTHR / 32) {
+    cpx v[3][2];  // pa, qa, rb at rows gq, gq + 8
+#pragma unroll
+    for (int b = 0; b < 3; ++b) {
+      const int cls = b < 2 ? 0 : 1, nm = mt + NTHR / 32;
+      long long T[4];
+      tc_tile_stream(pf, table(mt, b), b < 2 ? table(mt, b + 1) : (nm < MTq ? table(nm, 0) : nullptr), KTr,
+                     tc_row_addr(s.dig + (size_t)cls * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
+                     (uint32_t)(4 * NC * KS), T);
+      const int ecol = col_exp(exc[cls * TT + t]) - 64 + kFoldShift;
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int e = g.tcWTE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
+        v[b][rr] = cpx{round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
+      }
+    }
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const int y = mt * 16 + gq + 8 * rr;
+      if (y >= gsz.Q() || t >= nx) continue;
+      if (t < xfirst) quad_T_mean(g.norm, v[2][rr], Hb + (size_t)y * gsz.X(), cs);
+      else quad_T_combine(g.Kx[x], g.Kz[z], g.K2[(size_t)z * gsz.X() + x], x == 0 ? g.norm : 0.5 * g.norm, v[0][rr], v[1][rr],
+                     v[2][rr], Hb + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x, cs);
+    }
+  }
+}
+
+// Recon^T (as recon_T_tc) for launches with few blocks
+template <int KP, class S>
+__device__ __forceinline__ void recon_T_few(const Grid& g, const S& gsz, const cpx* __restrict__ Ub, int z, int x0,
+                                            int nx, int xfirst, SolveTSmem& s) {
+  constexpr int TT = 4, NTHR = 256;
+  const size_t cs = (size_t)gsz.Q() * gsz.X();
+  const int col = threadIdx.x % TT, x = x0 + min(col, nx - 1);
+  const cpx* Uc = Ub + (size_t)z * 5 * cs + x;
+  const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
+  few_contract<TT, NTHR, KP>(
+      gsz, g.tcBT, g.tcBTE, true, nx, s.dig,
+      [&](int y, cpx (&o)[5]) {
+        const cpx* b = Uc + (size_t)y * gsz.X();
+        if (col < xfirst) {
+          o[3] = recon_T_mean_input(b[0], b[2 * cs]);
+          o[4] = recon_T_mean_input(b[3 * cs], b[4 * cs]);
+          return;
+        }
+        recon_T_inputs(ax, az, b[0], b[2 * cs], b[3 * cs], b[4 * cs], o);
+        o[0] = b[cs];
+      },
+      [](int q) { return q; },
+      [](int q, const cpx& f, const cpx& v) {
+        if (q == 1) return cpx{f.re - v.re, f.im - v.im};
+        return cpx{f.re + v.re, f.im + v.im};
+      },
+      s.Fa, s.Fb);
+}
+
+// Block z ntx + tx: kx tile tx of line z; the mean line is column 0 of the
+// kz = 0 line's first tile, its parts as Re and Im of the beta class (as in
+// k_solve).  S: the sizes (SizesRT, or SizesCT for a specialised grid); TT kx
+// columns per block; FEW (the row and plane pairs a thread holds): the build
+// for launches with few blocks (TT 4)
+template <bool MULTI, class S, int TT = kTile, int FEW = 0>
+__global__ void __launch_bounds__(kThreads, FEW ? 1 : 2) k_solve_T(const __grid_constant__ Grid g0, SolveTArgs a) {
+  const int ntx = (g0.X + TT - 1) / TT;
   const int z = blockIdx.x / ntx, tx = blockIdx.x - z * ntx;
   const int inst = blockIdx.y;
   CHN_INSTANCE_GRID(g0, a.grids, inst);
   const S gsz(g);
-  if (z >= gsz.Nz() || tx * kTile >= gsz.X()) return;
+  if (z >= gsz.Nz() || tx * TT >= gsz.X()) return;
   if (blocked_t(a.status, a.sdiv, inst)) return;
-  const int x0 = tx * kTile;
-  const int nx = min(kTile, gsz.X() - x0);
+  const int x0 = tx * TT;
+  const int nx = min(TT, gsz.X() - x0);
   cpx* __restrict__ Cc = a.Cc.at(inst);
   auto cidx = [&](int v, int r, int x) { return (((size_t)z * 2 + v) * gsz.R() + r) * gsz.X() + x; };
+  extern __shared__ __align__(16) unsigned char smem[];
+  // deterministic block sum of the Re parts into this block's slot
+  __shared__ double gred[kThreads / 32];
+  auto add_re_part = [&](double v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) gred[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += gred[w];
+      a.gacc[(long long)inst * a.gstride + 1 + blockIdx.x] += t;
+    }
+  };
   if (z == gsz.Nz() / 2) {
     // the tangent zeroes this line every substage (channel/channel.c:460-467)
     if (!a.final_only)
@@ -513,36 +737,40 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__
       }
     return;
   }
-  extern __shared__ __align__(16) unsigned char smem[];
-  SolveTSmem s = carve_solveT(g, smem);
   const cpx* __restrict__ Ub = a.Ub.at(inst);
   const int xfirst = (z == 0 && x0 == 0) ? 1 : 0;
-  if (g.tc) recon_T_tc(g, gsz, Ub, z, x0, nx, xfirst, s);
-  else recon_T_tile(g, Ub, z, x0, nx, xfirst, s);
+  SolveTSmem s;
+  if constexpr (FEW) {
+    s = carve_solveT_few<TT>(g, smem);
+    if (!a.final_only)
+      stage_factors<kThreads>(g, gsz, ((size_t)a.k * gsz.Nz() + z) * gsz.X() + x0, nx, s.luA, s.luB, s.rdA, s.rdB);
+    recon_T_few<FEW>(g, gsz, Ub, z, x0, nx, xfirst, s);
+  } else {
+    s = carve_solveT(g, smem);
+    if (g.tc) recon_T_tc(g, gsz, Ub, z, x0, nx, xfirst, s);
+    else recon_T_tile(g, Ub, z, x0, nx, xfirst, s);
+  }
   if (a.final_only) {
     // the sweep's start state: IU = Recon(IC), so IC_bar += Recon^T(IU_bar)
-    for (int i = threadIdx.x; i < gsz.R() * kTile; i += blockDim.x) {
-      const int r = i / kTile, l = i - r * kTile;
-      if (l >= nx || l < xfirst) continue;
+    for (int i = threadIdx.x; i < gsz.R() * TT; i += blockDim.x) {
+      const int r = i / TT, l = i - r * TT;
+      if (l >= nx) continue;
       const int x = x0 + l;
+      if (l < xfirst) {  // real lines: R^T u_bar + R'^T du_bar to alpha, of w_bar to beta
+        const cpx f = s.Fb[r * TT];
+        Cc[cidx(0, r, 0)].re += f.re;
+        Cc[cidx(1, r, 0)].re += f.im;
+        continue;
+      }
       if (r < gsz.D()) {
-        const cpx f = s.Fa[r * kTile + l];
+        const cpx f = s.Fa[r * TT + l];
         Cc[cidx(0, r, x)].re += f.re;
         Cc[cidx(0, r, x)].im += f.im;
       }
-      const cpx f = s.Fb[r * kTile + l];
+      const cpx f = s.Fb[r * TT + l];
       Cc[cidx(1, r, x)].re += f.re;
       Cc[cidx(1, r, x)].im += f.im;
     }
-    if (xfirst == 1)
-      for (int i = threadIdx.x; i < gsz.R(); i += blockDim.x) {
-        cpx ma, mb;
-        recon_T_mean_row(g, Ub, i, ma, mb);
-        Cc[cidx(0, i, 0)].re += ma.re;
-        Cc[cidx(0, i, 0)].im += ma.im;
-        Cc[cidx(1, i, 0)].re += mb.re;
-        Cc[cidx(1, i, 0)].im += mb.im;
-      }
     return;
   }
   const int k = a.k;
@@ -553,22 +781,40 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__
   const int bidx = k;
   const int aidx_next = (k == 0) ? 1 : 0;  // a[1] = -1/2, a[2] = 1/3
   // x_bar = Recon^T part + E_{k+1}^T c_out_bar (or c_out_bar); F_bar = dt d_{k+1} c_out_bar
-  for (int i = threadIdx.x; i < gsz.R() * kTile; i += blockDim.x) {
-    const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
+  for (int i = threadIdx.x; i < gsz.R() * TT; i += blockDim.x) {
+    const int r = i / TT, l = i - r * TT;
+    if (l >= nx) continue;
     const int x = x0 + l;
     const size_t zx = (size_t)z * gsz.X() + x;
     cpx xa, xb;
+    if (l < xfirst) {
+      const cpx rec = s.Fb[r * TT], coa = Cc[cidx(0, r, 0)], cob = Cc[cidx(1, r, 0)];
+      xa = coa;
+      xb = cob;
+      if (k < 2) {
+        const double* E = g.ex0 + (size_t)aidx_next * gsz.R() * 5;
+        xa = band_matvecT_row(E, 5, 2, 2, gsz.R(), Cc + cidx(0, 0, 0), gsz.X(), r);
+        xb = band_matvecT_row(E, 5, 2, 2, gsz.R(), Cc + cidx(1, 0, 0), gsz.X(), r);
+        s.Fb[r * TT] = cpx{dt * dnext * coa.re, dt * dnext * cob.re};  // the mean right-hand side is real
+      } else {
+        s.Fb[r * TT] = cpx{0.0, 0.0};
+      }
+      xa.re += rec.re;
+      xb.re += rec.im;
+      s.ra[r * TT] = xa;
+      s.rb[r * TT] = xb;
+      continue;
+    }
     if (r < gsz.D()) {
-      const cpx rec = s.Fa[r * kTile + l];
+      const cpx rec = s.Fa[r * TT + l];
       const cpx co = Cc[cidx(0, r, x)];
       if (k < 2) {
         const double* E = g.exA + ((size_t)aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.D() * 9;
         xa = band_matvecT_row(E, 9, 4, 4, gsz.D(), Cc + cidx(0, 0, x), gsz.X(), r);
-        s.Fa[r * kTile + l] = cpx{dt * dnext * co.re, dt * dnext * co.im};
+        s.Fa[r * TT + l] = cpx{dt * dnext * co.re, dt * dnext * co.im};
       } else {
         xa = co;
-        s.Fa[r * kTile + l] = cpx{0.0, 0.0};
+        s.Fa[r * TT + l] = cpx{0.0, 0.0};
       }
       xa.re += rec.re;
       xa.im += rec.im;
@@ -576,193 +822,151 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__
       xa = Cc[cidx(0, r, x)];  // alpha rows >= Ny-4 ride along unchanged
     }
     {
-      const cpx rec = s.Fb[r * kTile + l];
+      const cpx rec = s.Fb[r * TT + l];
       const cpx co = Cc[cidx(1, r, x)];
       if (k < 2) {
         const double* E = g.exB + ((size_t)aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.R() * 5;
         xb = band_matvecT_row(E, 5, 2, 2, gsz.R(), Cc + cidx(1, 0, x), gsz.X(), r);
-        s.Fb[r * kTile + l] = cpx{dt * dnext * co.re, dt * dnext * co.im};
+        s.Fb[r * TT + l] = cpx{dt * dnext * co.re, dt * dnext * co.im};
       } else {
         xb = co;
-        s.Fb[r * kTile + l] = cpx{0.0, 0.0};
+        s.Fb[r * TT + l] = cpx{0.0, 0.0};
       }
       xb.re += rec.re;
       xb.im += rec.im;
     }
-    s.ra[r * kTile + l] = xa;
-    s.rb[r * kTile + l] = xb;
+    s.ra[r * TT + l] = xa;
+    s.rb[r * TT + l] = xb;
   }
   __syncthreads();
-  // L^{-T}: per column 4 chains for alpha, 4 for beta (parity x re/im)
-  if (threadIdx.x < 8 * kTile) {
-    // threads [0, 4 kTile) run the alpha chains, [4 kTile, 8 kTile) the beta
-    // ones: a warp holds one system (no divergence between the two bands)
-    const int l = (threadIdx.x % (4 * kTile)) / 4, ch = 4 * (threadIdx.x / (4 * kTile)) + threadIdx.x % 4;
-    if (l < nx && l >= xfirst) {
-      const size_t zx = (size_t)z * gsz.X() + x0 + l;
-      const int par = ch & 1, part = (ch >> 1) & 1;
-      if (ch < 4)
-        band_solveT_chain<9, 4, 4>(g.luA + ((size_t)bidx * gsz.Nz() * gsz.X() + zx) * gsz.D() * 9,
-                                   g.rdA + ((size_t)bidx * gsz.Nz() * gsz.X() + zx) * gsz.D(), gsz.D(), par,
-                                   reinterpret_cast<double*>(s.ra + l) + part, 2 * kTile);
+  const bool want_g = a.gacc != nullptr;
+  if (xfirst) {
+    // the mean line's flux correction x = xs - 0.5 add (rwsum . xs.re),
+    // transposed: xs_bar.re = x_bar.re - 0.5 rwsum (add . x_bar.re); warp 0
+    if (threadIdx.x < 32) {
+      double part = 0.0;
+      for (int i = threadIdx.x; i < gsz.R(); i += 32) part = fma(g.add0[i], s.ra[i * TT].re, part);
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      // the forced tangent adds 0.5 * 2.0 * add to this line's real part
+      // (channel/increproject0.c:209-214): its cotangent is <add, x_bar.re>
+      if (want_g && threadIdx.x == 0) a.gacc[(long long)inst * a.gstride] += part;
+      for (int i = threadIdx.x; i < gsz.R(); i += 32) s.ra[i * TT].re = fma(-0.5 * part, g.rwsum[i], s.ra[i * TT].re);
+    }
+    __syncthreads();
+  }
+  // L^{-T}: per column 4 chains for alpha, 4 for beta (parity x re/im), the
+  // alpha chains in threads [0, 4 TT), the beta ones from a warp boundary, the
+  // mean line's from the next
+  constexpr int kHalf = 4 * TT < 32 ? 32 : 4 * TT;
+  if (xfirst && (int)threadIdx.x >= 2 * kHalf) {
+    const int t = (int)threadIdx.x - 2 * kHalf;
+    if (t < 8)
+      band_solveT_chain<5, 2, 2, true>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), t & 1,
+                                       reinterpret_cast<double*>(t < 4 ? s.ra : s.rb) + ((t >> 1) & 1), 2 * TT);
+  } else {
+    const bool beta = (int)threadIdx.x >= kHalf;
+    const int t = beta ? (int)threadIdx.x - kHalf : (int)threadIdx.x, l = t / 4, par = t & 1, part = (t >> 1) & 1;
+    if (t < 4 * TT && l < nx && l >= xfirst) {
+      const size_t sys = ((size_t)bidx * gsz.Nz() + z) * gsz.X() + x0 + l;
+      if (!beta)
+        band_solveT_chain<9, 4, 4, !FEW>(FEW ? s.luA + (size_t)l * gsz.D() * 9 : g.luA + sys * gsz.D() * 9,
+                                         FEW ? s.rdA + (size_t)l * gsz.D() : g.rdA + sys * gsz.D(), gsz.D(), par,
+                                         reinterpret_cast<double*>(s.ra + l) + part, 2 * TT);
       else
-        band_solveT_chain<5, 2, 2>(g.luB + ((size_t)bidx * gsz.Nz() * gsz.X() + zx) * gsz.R() * 5,
-                                   g.rdB + ((size_t)bidx * gsz.Nz() * gsz.X() + zx) * gsz.R(), gsz.R(), par,
-                                   reinterpret_cast<double*>(s.rb + l) + part, 2 * kTile);
+        band_solveT_chain<5, 2, 2, !FEW>(FEW ? s.luB + (size_t)l * gsz.R() * 5 : g.luB + sys * gsz.R() * 5,
+                                         FEW ? s.rdB + (size_t)l * gsz.R() : g.rdB + sys * gsz.R(), gsz.R(), par,
+                                         reinterpret_cast<double*>(s.rb + l) + part, 2 * TT);
     }
   }
   __syncthreads();
   // dJ/dRe: <c2_bar, f_Re> of this block's columns (the forcing of
   // recon_solve.cu's kind 3 rebuilt from the stored primal states)
-  const bool want_g = a.gacc != nullptr;
-  const cpx* xk = nullptr;
-  double ft1 = 0.0, gpart = 0.0;
+  double gpart = 0.0;
   const double re2 = g.re * g.re;
   const double akf = k == 1 ? -1. / 2 : 1. / 3.;                  // forward a_k
   const double bkf = k == 0 ? 1. / 6 : (k == 1 ? 2. / 3 : 0.0);  // forward b_k
   if (want_g) {
     const int xs = a.xslot.slot();
-    xk = a.Xf + (long long)inst * a.xstride + (long long)xs * a.xslot.stride;
-    if (a.Ftr) ft1 = a.Ftr[(long long)inst * a.ftr_stride + xs + 1];
+    const cpx* xk = a.Xf + (long long)inst * a.xstride + (long long)xs * a.xslot.stride;
+    const double ft1 = a.Ftr ? a.Ftr[(long long)inst * a.ftr_stride + xs + 1] : 0.0;
     const size_t csz = coef_size(g);
-    for (int i = threadIdx.x; i < gsz.R() * kTile; i += blockDim.x) {
-      const int r = i / kTile, l = i - r * kTile;
-      if (l >= nx || l < xfirst) continue;
+    for (int i = threadIdx.x; i < gsz.R() * TT; i += blockDim.x) {
+      const int r = i / TT, l = i - r * TT;
+      if (l >= nx) continue;
       const int x = x0 + l;
+      if (l < xfirst) {
+        // D0 = -Rps on the primal's solved mean flow before its flux
+        // correction, MC[3n + k + 1] - 0.5 flux_t add
+        const cpx p0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(0, 0, 0), gsz.X(), r);
+        cpx p1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(0, 0, 0), gsz.X(), r);
+        p1.re -= 0.5 * ft1 * rps_row_real(g, g.add0, r);
+        const cpx q0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(1, 0, 0), gsz.X(), r);
+        const cpx q1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(1, 0, 0), gsz.X(), r);
+        const cpx c2a = s.ra[r * TT], c2b = s.rb[r * TT];
+        gpart += re2 * dt * (c2a.re * (akf * p0.re + bkf * p1.re) + c2a.im * (akf * p0.im + bkf * p1.im));
+        gpart += re2 * dt * (c2b.re * (akf * q0.re + bkf * q1.re) + c2b.im * (akf * q0.im + bkf * q1.im));
+        continue;
+      }
       const double k2 = g.K2[(size_t)z * gsz.X() + x];
       if (r < gsz.D()) {
         const cpx d0 = visc_v_row(g, k2, xk + cidx(0, 0, x), gsz.X(), r);
         const cpx d1 = visc_v_row(g, k2, xk + csz + cidx(0, 0, x), gsz.X(), r);
-        const cpx c2 = s.ra[r * kTile + l];
+        const cpx c2 = s.ra[r * TT + l];
         gpart -= re2 * dt * (c2.re * (akf * d0.re + bkf * d1.re) + c2.im * (akf * d0.im + bkf * d1.im));
       }
       const cpx d0 = visc_g_row(g, k2, xk + cidx(1, 0, x), gsz.X(), r);
       const cpx d1 = visc_g_row(g, k2, xk + csz + cidx(1, 0, x), gsz.X(), r);
-      const cpx c2 = s.rb[r * kTile + l];
+      const cpx c2 = s.rb[r * TT + l];
       gpart += re2 * dt * (c2.re * (akf * d0.re + bkf * d1.re) + c2.im * (akf * d0.im + bkf * d1.im));
     }
   }
   // F_bar += dt c_k c2_bar; c_in_bar = E_0^T c2_bar (k == 0) or c2_bar
-  for (int i = threadIdx.x; i < gsz.R() * kTile; i += blockDim.x) {
-    const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
+  for (int i = threadIdx.x; i < gsz.R() * TT; i += blockDim.x) {
+    const int r = i / TT, l = i - r * TT;
+    if (l >= nx) continue;
     const int x = x0 + l;
     const size_t zx = (size_t)z * gsz.X() + x;
+    if (l < xfirst) {
+      const cpx c2a = s.ra[r * TT], c2b = s.rb[r * TT];
+      cpx& f = s.Fb[r * TT];
+      f = cpx{fma(dt * ck, c2a.re, f.re), fma(dt * ck, c2b.re, f.im)};
+      Cc[cidx(0, r, 0)] = k == 0 ? band_matvecT_row(g.ex0, 5, 2, 2, gsz.R(), s.ra, TT, r) : c2a;
+      Cc[cidx(1, r, 0)] = k == 0 ? band_matvecT_row(g.ex0, 5, 2, 2, gsz.R(), s.rb, TT, r) : c2b;
+      continue;
+    }
     if (r < gsz.D()) {
-      const cpx c2 = s.ra[r * kTile + l];
-      s.Fa[r * kTile + l].re += dt * ck * c2.re;
-      s.Fa[r * kTile + l].im += dt * ck * c2.im;
-      Cc[cidx(0, r, x)] = k == 0 ? band_matvecT_row(g.exA + zx * gsz.D() * 9, 9, 4, 4, gsz.D(), s.ra + l, kTile, r) : c2;
+      const cpx c2 = s.ra[r * TT + l];
+      s.Fa[r * TT + l].re += dt * ck * c2.re;
+      s.Fa[r * TT + l].im += dt * ck * c2.im;
+      Cc[cidx(0, r, x)] = k == 0 ? band_matvecT_row(g.exA + zx * gsz.D() * 9, 9, 4, 4, gsz.D(), s.ra + l, TT, r) : c2;
     } else {
-      Cc[cidx(0, r, x)] = s.ra[r * kTile + l];
+      Cc[cidx(0, r, x)] = s.ra[r * TT + l];
     }
-    const cpx c2 = s.rb[r * kTile + l];
-    s.Fb[r * kTile + l].re += dt * ck * c2.re;
-    s.Fb[r * kTile + l].im += dt * ck * c2.im;
-    Cc[cidx(1, r, x)] = k == 0 ? band_matvecT_row(g.exB + zx * gsz.R() * 5, 5, 2, 2, gsz.R(), s.rb + l, kTile, r) : c2;
-  }
-  // mean mode (transpose of channel/increproject0.c with the homogeneous
-  // flux correction), warp 0
-  if (xfirst == 1 && threadIdx.x < 32) {
-    double* fa = s.m0;
-    double* fb = s.m0 + gsz.R();
-    cpx* ca = reinterpret_cast<cpx*>(s.m0 + 2 * gsz.R());
-    cpx* cb = ca + gsz.R();
-    const int lane = threadIdx.x;
-    const double* Enext = g.ex0 + (size_t)aidx_next * gsz.R() * 5;
-    for (int i = lane; i < gsz.R(); i += 32) {
-      cpx ma, mb;
-      recon_T_mean_row(g, Ub, i, ma, mb);
-      const cpx coa = Cc[cidx(0, i, 0)], cob = Cc[cidx(1, i, 0)];
-      cpx xa, xb;
-      if (k < 2) {
-        xa = band_matvecT_row(Enext, 5, 2, 2, gsz.R(), Cc + cidx(0, 0, 0), gsz.X(), i);
-        xb = band_matvecT_row(Enext, 5, 2, 2, gsz.R(), Cc + cidx(1, 0, 0), gsz.X(), i);
-        fa[i] = dt * dnext * coa.re;  // the mean right-hand side is real
-        fb[i] = dt * dnext * cob.re;
-      } else {
-        xa = coa;
-        xb = cob;
-        fa[i] = 0.0;
-        fb[i] = 0.0;
-      }
-      ca[i] = cpx{xa.re + ma.re, xa.im + ma.im};
-      cb[i] = cpx{xb.re + mb.re, xb.im + mb.im};
-    }
-    __syncwarp();
-    // flux correction x = xs - 0.5 add (rwsum . xs.re), transposed:
-    // xs_bar.re = x_bar.re - 0.5 rwsum (add . x_bar.re)
-    double part = 0.0;
-    for (int i = lane; i < gsz.R(); i += 32) part = fma(g.add0[i], ca[i].re, part);
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    // the forced tangent adds 0.5 * 2.0 * add to this line's real part
-    // (channel/increproject0.c:209-214): its cotangent is <add, x_bar.re>
-    if (want_g && lane == 0) a.gacc[(long long)inst * a.gstride] += part;
-    __syncwarp();
-    for (int i = lane; i < gsz.R(); i += 32) ca[i].re = fma(-0.5 * part, g.rwsum[i], ca[i].re);
-    __syncwarp();
-    if (lane < 8) {
-      const int par = lane & 1, pt = (lane >> 1) & 1;
-      band_solveT_chain<5, 2, 2>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), par,
-                                 reinterpret_cast<double*>(lane < 4 ? ca : cb) + pt, 2);
-    }
-    __syncwarp();
-    if (want_g) {
-      // the mean lines' Re forcing: D0 = -Rps on the primal's solved mean flow
-      // before its flux correction, MC[3n + k + 1] - 0.5 flux_t add
-      const size_t csz = coef_size(g);
-      double mp = 0.0;
-      for (int i = lane; i < gsz.R(); i += 32) {
-        const cpx p0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(0, 0, 0), gsz.X(), i);
-        cpx p1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(0, 0, 0), gsz.X(), i);
-        p1.re -= 0.5 * ft1 * rps_row_real(g, g.add0, i);
-        const cpx q0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(1, 0, 0), gsz.X(), i);
-        const cpx q1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(1, 0, 0), gsz.X(), i);
-        mp += re2 * dt * (ca[i].re * (akf * p0.re + bkf * p1.re) + ca[i].im * (akf * p0.im + bkf * p1.im));
-        mp += re2 * dt * (cb[i].re * (akf * q0.re + bkf * q1.re) + cb[i].im * (akf * q0.im + bkf * q1.im));
-      }
-      gpart += mp;  // lane partials; the block reduction below adds every thread's
-    }
-    for (int i = lane; i < gsz.R(); i += 32) {
-      fa[i] = fma(dt * ck, ca[i].re, fa[i]);
-      fb[i] = fma(dt * ck, cb[i].re, fb[i]);
-      if (k == 0) {
-        Cc[cidx(0, i, 0)] = band_matvecT_row(g.ex0, 5, 2, 2, gsz.R(), ca, 1, i);
-        Cc[cidx(1, i, 0)] = band_matvecT_row(g.ex0, 5, 2, 2, gsz.R(), cb, 1, i);
-      } else {
-        Cc[cidx(0, i, 0)] = ca[i];
-        Cc[cidx(1, i, 0)] = cb[i];
-      }
-    }
+    const cpx c2 = s.rb[r * TT + l];
+    s.Fb[r * TT + l].re += dt * ck * c2.re;
+    s.Fb[r * TT + l].im += dt * ck * c2.im;
+    Cc[cidx(1, r, x)] = k == 0 ? band_matvecT_row(g.exB + zx * gsz.R() * 5, 5, 2, 2, gsz.R(), s.rb + l, TT, r) : c2;
   }
   __syncthreads();
-  if (want_g) {
-    // deterministic block sum of the Re parts into this block's slot
-    __shared__ double gred[kThreads / 32];
-    double v = gpart;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) gred[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += gred[w];
-      a.gacc[(long long)inst * a.gstride + 1 + blockIdx.x] += t;
-    }
-  }
+  if (want_g) add_re_part(gpart);
   // H_bar = Quad^T(F_bar) (transpose of channel/project.c:97-115, 177-191):
   //   Hx_bar = -i kx Qpw^T Fa_bar - i kz Rw^T Fb_bar
   //   Hz_bar = -i kz Qpw^T Fa_bar + i kx Rw^T Fb_bar,  Hy_bar = -K2 Qw^T Fa_bar
-  // mean mode: Hx_bar.re = Rw^T fa_bar, Hz_bar.re = Rw^T fb_bar.  Scaled for
-  // the inverse transform that follows: the forward transform's 1/(px pz),
+  // Scaled for the inverse transform that follows: the forward transform's 1/(px pz),
   // halved off the kx = 0 column (the transpose of the real-to-complex x
   // transform).  Plane pairs (y, -y) share the sums: weights of even type
   // (Qw, Rw) give E + O / E - O, of odd type (Qpw) E + O / O - E.
-  if (g.tc) quad_T_tc(g, gsz, z, x0, nx, xfirst, s, a.Hb.at(inst));
-  const int lx = threadIdx.x % kTile, grp = threadIdx.x / kTile, ngrp = blockDim.x / kTile;
+  if constexpr (FEW) {
+    quad_T_few<FEW>(g, gsz, z, x0, nx, xfirst, s, a.Hb.at(inst));
+    return;
+  }
+  if (g.tc) {
+    quad_T_tc(g, gsz, z, x0, nx, xfirst, s, a.Hb.at(inst));
+    return;
+  }
+  const int lx = threadIdx.x % TT, grp = threadIdx.x / TT, ngrp = blockDim.x / TT;
   if (lx >= nx) return;
-  if (g.tc && lx >= xfirst) return;  // the tensor cores took every column but the mean one
   const int x = x0 + lx;
-  const bool mean = (z == 0 && x == 0);
   const double kx = g.Kx[x], kz = g.Kz[z], k2 = g.K2[(size_t)z * gsz.X() + x];
   const double scl = x == 0 ? g.norm : 0.5 * g.norm;
   cpx* __restrict__ Hb = a.Hb.at(inst);
@@ -771,41 +975,27 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__
     const int y1 = yp, y2 = gsz.Q() - 1 - yp;
     // E/O sums over even/odd rows: [0] Qpw^T Fa, [1] Qw^T Fa, [2] Rw^T Fb
     double er[3] = {0, 0, 0}, ei[3] = {0, 0, 0}, orr[3] = {0, 0, 0}, oi[3] = {0, 0, 0};
-    if (!mean) {
+    {
       int i = 0;
       for (; i + 1 < gsz.D(); i += 2) {
-        const cpx f0 = s.Fa[i * kTile + lx], f1 = s.Fa[(i + 1) * kTile + lx];
+        const cpx f0 = s.Fa[i * TT + lx], f1 = s.Fa[(i + 1) * TT + lx];
         cfma_t(__ldg(g.Wqp + (size_t)i * gsz.Q() + yp), f0, er[0], ei[0]);
         cfma_t(__ldg(g.Wqp + (size_t)(i + 1) * gsz.Q() + yp), f1, orr[0], oi[0]);
         cfma_t(__ldg(g.Wq + (size_t)i * gsz.Q() + yp), f0, er[1], ei[1]);
         cfma_t(__ldg(g.Wq + (size_t)(i + 1) * gsz.Q() + yp), f1, orr[1], oi[1]);
       }
       if (i < gsz.D()) {
-        const cpx f0 = s.Fa[i * kTile + lx];
+        const cpx f0 = s.Fa[i * TT + lx];
         cfma_t(__ldg(g.Wqp + (size_t)i * gsz.Q() + yp), f0, er[0], ei[0]);
         cfma_t(__ldg(g.Wq + (size_t)i * gsz.Q() + yp), f0, er[1], ei[1]);
       }
       i = 0;
       for (; i + 1 < gsz.R(); i += 2) {
-        const cpx f0 = s.Fb[i * kTile + lx], f1 = s.Fb[(i + 1) * kTile + lx];
+        const cpx f0 = s.Fb[i * TT + lx], f1 = s.Fb[(i + 1) * TT + lx];
         cfma_t(__ldg(g.Wr + (size_t)i * gsz.Q() + yp), f0, er[2], ei[2]);
         cfma_t(__ldg(g.Wr + (size_t)(i + 1) * gsz.Q() + yp), f1, orr[2], oi[2]);
       }
-      if (i < gsz.R()) cfma_t(__ldg(g.Wr + (size_t)i * gsz.Q() + yp), s.Fb[i * kTile + lx], er[2], ei[2]);
-    } else {
-      const double* fa = s.m0;
-      const double* fb = s.m0 + gsz.R();
-      // [0] Rw^T fa, [2] Rw^T fb (real)
-      for (int i = 0; i < gsz.R(); ++i) {
-        const double w = __ldg(g.Wr + (size_t)i * gsz.Q() + yp);
-        if (i & 1) {
-          orr[0] = fma(w, fa[i], orr[0]);
-          orr[2] = fma(w, fb[i], orr[2]);
-        } else {
-          er[0] = fma(w, fa[i], er[0]);
-          er[2] = fma(w, fb[i], er[2]);
-        }
-      }
+      if (i < gsz.R()) cfma_t(__ldg(g.Wr + (size_t)i * gsz.Q() + yp), s.Fb[i * TT + lx], er[2], ei[2]);
     }
     for (int side = 0; side < 2; ++side) {
       if (side == 1 && y2 == y1) break;
@@ -817,24 +1007,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_solve_T(const __grid_constant__
         else { r.re = orr[c] - er[c]; r.im = oi[c] - ei[c]; }
         return r;
       };
-      cpx hx, hy, hz;
-      if (mean) {
-        hx = cpx{val(0, false).re * scl, 0.0};
-        hz = cpx{val(2, false).re * scl, 0.0};
-        hy = cpx{0.0, 0.0};
-      } else {
-        const cpx pa = val(0, true), qa = val(1, false), rb = val(2, false);
-        hx.re = scl * (kx * pa.im + kz * rb.im);    // -i kx pa - i kz rb
-        hx.im = -scl * (kx * pa.re + kz * rb.re);
-        hz.re = scl * (kz * pa.im - kx * rb.im);    // -i kz pa + i kx rb
-        hz.im = scl * (kx * rb.re - kz * pa.re);
-        hy.re = -scl * k2 * qa.re;
-        hy.im = -scl * k2 * qa.im;
-      }
-      cpx* out = Hb + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
-      out[0] = hz;
-      out[cs] = hx;
-      out[2 * cs] = hy;
+      if (lx < xfirst) quad_T_mean(scl, val(2, false), Hb + (size_t)y * gsz.X(), cs);
+      else
+        quad_T_combine(kx, kz, k2, scl, val(0, true), val(1, false), val(2, false),
+                     Hb + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x, cs);
     }
   }
 }
@@ -866,23 +1042,47 @@ cudaError_t launch_add_source(const Grid& g, Batch<const cpx> src, Batch<cpx> ca
   return cudaGetLastError();
 }
 
+static int s_solveT_optin = 0;
+
+// launches of at most kFewTiles 4-column tiles take the FEW build (where
+// CHN_SOLVE_TILE does not ask for a tile)
+static bool solveT_few(const Grid& g, const SolveTArgs& a) {
+  if (a.grids || !g.tc || g.sfixed || g.R <= 16 || g.R > 128 || g.Q > 256) return false;
+  if ((long long)g.Nz * ((g.X + 3) / 4) * a.ninst > kFewTiles) return false;
+  return solveT_few_smem_bytes(g, 4) + 1024 <= (size_t)s_solveT_optin;
+}
+
 cudaError_t launch_solve_T(const Grid& g, const SolveTArgs& a, cudaStream_t st) {
   if (a.ninst <= 0) return cudaSuccess;
-  const int ntx = (g.X + kTile - 1) / kTile;
+  if (solveT_few(g, a)) {
+    const dim3 grid(g.Nz * ((g.X + 3) / 4), a.ninst);
+    const size_t sm = solveT_few_smem_bytes(g, 4);
+    if (sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
+    else if (sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
+    else if (g.Q <= 128 && g.R <= 64) k_solve_T<false, SizesRT, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
+    else k_solve_T<false, SizesRT, 4, 2><<<grid, kThreads, sm, st>>>(g, a);
+    return cudaGetLastError();
+  }
+  const dim3 grid(g.Nz * ((g.X + kTile - 1) / kTile), a.ninst);
   const size_t sm = solveT_smem_bytes(g);
   const bool fx = (g.fixed & FIXED_SOLVE) && !a.grids;  // the solve's fixed-size choice covers its transpose
-  if (a.grids) k_solve_T<true, SizesRT><<<dim3(g.Nz * ntx, a.ninst), kThreads, sm, st>>>(g, a);
-  else if (fx && sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32><<<dim3(g.Nz * ntx, a.ninst), kThreads, sm, st>>>(g, a);
-  else if (fx && sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16><<<dim3(g.Nz * ntx, a.ninst), kThreads, sm, st>>>(g, a);
-  else k_solve_T<false, SizesRT><<<dim3(g.Nz * ntx, a.ninst), kThreads, sm, st>>>(g, a);
+  if (a.grids) k_solve_T<true, SizesRT><<<grid, kThreads, sm, st>>>(g, a);
+  else if (fx && sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32><<<grid, kThreads, sm, st>>>(g, a);
+  else if (fx && sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16><<<grid, kThreads, sm, st>>>(g, a);
+  else k_solve_T<false, SizesRT><<<grid, kThreads, sm, st>>>(g, a);
   return cudaGetLastError();
 }
 
 void prepare_solve_T(int optin) {
+  s_solveT_optin = optin;
   allow_max_smem(k_solve_T<false, SizesRT>, optin);
   allow_max_smem(k_solve_T<true, SizesRT>, optin);
   allow_max_smem(k_solve_T<false, Sizes32>, optin);
   allow_max_smem(k_solve_T<false, Sizes16>, optin);
+  allow_max_smem(k_solve_T<false, SizesRT, 4, 1>, optin);
+  allow_max_smem(k_solve_T<false, SizesRT, 4, 2>, optin);
+  allow_max_smem(k_solve_T<false, Sizes32, 4, 1>, optin);
+  allow_max_smem(k_solve_T<false, Sizes16, 4, 1>, optin);
 }
 
 }  // namespace chn

@@ -110,6 +110,7 @@ struct Grid {
   int stile;
   int sthr;
   int sfixed;  // CHN_SOLVE_TILE asked for the tile: no build of fewer columns in its place
+  int rfixed;  // CHN_RECON_BUILD likewise
   int rbuild;  // tensor-core reconstruction: 0 = 16 columns, 256 threads; 1 = 8 columns, 128 threads;
                // 2 = 16 columns at 3 blocks per SM (autotuned)
   // inverse transforms as DFT GEMMs on the tensor cores (phys_tc.cu), each

@@ -251,6 +251,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // the tensor-core reconstruction's build (recon_tc.cu): 0 until the
   // autotuner has timed 0, 1, 2; CHN_RECON_BUILD fixes it
   const char* rbe = getenv("CHN_RECON_BUILD");
+  g.rfixed = (rbe && rbe[0]) ? 1 : 0;
   g.rbuild = (rbe && rbe[0] >= '0' && rbe[0] <= '2' && rbe[1] == 0) ? rbe[0] - '0' : 0;
   // the inverse on tcgen05 where it fits: a candidate of the autotuner
   // (bit-identical results); CHN_INVERSE_TC5=1 forces it, =0 leaves it out
@@ -385,7 +386,7 @@ struct Work {
            alloc_grad(g);
   }
   bool alloc_grad(const Grid& g) {
-    gstride = 1 + g.Nz * ((g.X + 15) / 16);  // the solve's blocks: kz lines x 16-column tiles
+    gstride = 1 + g.Nz * ((g.X + 3) / 4);  // the transposed solve's blocks: kz lines x tiles of 4 columns or more
     return alloc(&gacc, (size_t)nseg * gstride);
   }
   // split transforms (required where a plane exceeds a block's shared

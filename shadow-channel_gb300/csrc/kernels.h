@@ -145,6 +145,11 @@ struct DdtArgs {
   const Grid* grids;        // uneven batch: grid of each segment (its sizes, weights and dt)
 };
 
+// 4-column tiles (kz lines x kx tiles x instances) up to which a launch of the
+// reconstruction, the solve or its transpose runs its build for few blocks:
+// two per SM
+constexpr int kFewTiles = 2 * 152;
+
 void prepare_kernels(const Grid& g);  // function attributes; call once, outside graph capture
 
 cudaError_t launch_recon(const Grid& g, const ReconArgs& a, cudaStream_t st);

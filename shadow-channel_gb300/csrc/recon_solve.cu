@@ -13,12 +13,11 @@
 // (-1)^(n+1), so for the plane pair (y, -y) a contraction splits into an
 // even-index sum E and an odd-index sum O with values E +- O.  This halves
 // the FP64 multiply-adds of every quadrature and reconstruction.
-#include <algorithm>
-
 #include "chn_common.cuh"
 #include "kernels.h"
 #include "solve_common.cuh"
 #include "sizes.cuh"
+#include "few_tile.cuh"
 #include "tc_common.cuh"
 
 namespace chn {
@@ -239,13 +238,9 @@ __host__ __device__ inline size_t solve_hc_elems(const Grid& g) {
   return tc > hc ? tc : hc;
 }
 
-// doubles of shared memory the mean line's block needs
-__host__ __device__ inline size_t solve_mean_elems(const Grid& g) { return (size_t)6 * g.R + 4 * (size_t)g.Q; }
-
 template <int kTile>
 size_t solve_smem_bytes_t(const Grid& g) {
-  const size_t n = (solve_hc_elems<kTile>(g) + (size_t)g.D * kTile + (size_t)g.R * kTile) * sizeof(cpx);
-  return std::max(n, solve_mean_elems(g) * sizeof(double));
+  return (solve_hc_elems<kTile>(g) + (size_t)g.D * kTile + (size_t)g.R * kTile) * sizeof(cpx);
 }
 
 // the widest tile's (the fit check of a grid)
@@ -270,9 +265,8 @@ __host__ __device__ inline size_t solve_few_dig_bytes(const Grid& g, int tile, b
   return ((size_t)(adj ? 5 : 3) * kDig * 2 * tile * solve_tc_kstride(g) * 2 + 5 * tile * sizeof(int) + 15) / 16 * 16;
 }
 inline size_t solve_few_smem_bytes(const Grid& g, int tile, bool adj) {
-  const size_t n = solve_few_dig_bytes(g, tile, adj) + (size_t)tile * (3 * g.R + g.D) * sizeof(cpx) +
-                   (size_t)tile * (10 * g.D + 6 * g.R) * sizeof(double);
-  return std::max(n, solve_mean_elems(g) * sizeof(double));
+  return solve_few_dig_bytes(g, tile, adj) + (size_t)tile * (3 * g.R + g.D) * sizeof(cpx) +
+         (size_t)tile * (10 * g.D + 6 * g.R) * sizeof(double);
 }
 template <int kTile>
 __device__ inline SolveSmem carve_solve_few(const Grid& g, unsigned char* base, bool adj) {
@@ -291,25 +285,8 @@ __device__ inline SolveSmem carve_solve_few(const Grid& g, unsigned char* base, 
   return s;
 }
 
-__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-               : "memory");
-}
-
-// the factors of the tile's columns (contiguous per kind, from system sys0
-// on) into shared memory, in the background of the quadratures; the caller's
-// quad_rhs_few waits for the copies
-template <int kTile, int NTHR, class S>
-__device__ __forceinline__ void stage_factors(const Grid& g, const S& gsz, size_t sys0, int nx, const SolveSmem& s) {
-  auto copy = [&](double* dst, const double* src, int n) {
-    for (int i = threadIdx.x; i < n; i += NTHR) copy8_async(dst + i, src + i);
-  };
-  copy(s.luA, g.luA + sys0 * gsz.D() * 9, nx * gsz.D() * 9);
-  copy(s.luB, g.luB + sys0 * gsz.R() * 5, nx * gsz.R() * 5);
-  copy(s.rdA, g.rdA + sys0 * gsz.D(), nx * gsz.D());
-  copy(s.rdB, g.rdB + sys0 * gsz.R(), nx * gsz.R());
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
+// the mean line's stand-ins for G and Sb (its two real quadratures as Re, Im)
+__device__ __forceinline__ cpx mean_input(const cpx& u, const cpx& v, double sign) { return cpx{u.re, sign * v.re}; }
 
 // Quadrature right-hand side for columns x0..x0+nx-1 of line z from terms H:
 //   Fa = Qpw . i(kx Hx + kz Hz) - K2 Qw . Hy  [+ Qppw . -i(kz Sx - kx Sz)]
@@ -348,12 +325,15 @@ __device__ void quad_rhs(const Grid& g, const cpx* __restrict__ H, int z, int x0
             in[side][2].im = -kz * sx.re + kx * sz.re;
           }
         } else {
+          const bool mean = z == 0 && x == 0;
           in[side][0].re = -kz * hx.im + kx * hz.im;   // G = i(kz Hx - kx Hz)
           in[side][0].im = kz * hx.re - kx * hz.re;
+          if (mean) in[side][0] = mean_input(hx, hz, 1.0);
           if (adj) {
             const cpx sx = Hz_[3 * cs + (size_t)y * g.X + x], sz = Hz_[4 * cs + (size_t)y * g.X + x];
             in[side][1].re = -kz * sz.im - kx * sx.im;  // Sb = i(kz Sz + kx Sx)
             in[side][1].im = kz * sz.re + kx * sx.re;
+            if (mean) in[side][1] = mean_input(sz, sx, -1.0);
           }
         }
       }
@@ -463,6 +443,7 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
     const int x = x0 + col;
     const double kx = g.Kx[x];
     const cpx* b = Hz_ + (size_t)y * gsz.X() + x;
+    if (q >= 3 && z == 0 && x == 0) return q == 3 ? mean_input(b[cs], b[0], 1.0) : mean_input(b[4 * cs], b[3 * cs], -1.0);
     switch (q) {
       case 0: return imul_sum(kx, b[cs], kz, b[0]);
       case 1: return b[2 * cs];
@@ -561,226 +542,37 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
 }
 
 
-// quad_rhs_tc for launches with few blocks, where a block has its SM almost
-// to itself and latency counts: every input of the 4-column tile is loaded,
-// digitised and contracted at once (one pass of loads, three barriers), a warp
-// per 16 rows of Fa or of Fb runs its tables' k-tiles as one stream with two
-// in flight.  32x65x32, one instance: 62k -> 12k cycles a block (the adjoint
-// 102k -> 17k); KP: plane pairs a thread holds (Q <= KP 2 NTHR / kTile).
+// quad_rhs_tc for launches with few blocks (few_contract)
 template <int kTile, int NTHR, int KP, class S>
 __device__ void quad_rhs_few(const Grid& g, const S& gsz, const cpx* __restrict__ H, int z, int x0, int nx, bool adj,
                              SolveSmem& s) {
-  static_assert(kTile == 4, "one 8-column digit tile");
-  constexpr int NC = 2 * kTile;
-  const int KT = (gsz.Q() + 15) / 16, MTw = (gsz.R() + 15) / 16;
-  const size_t KS = (size_t)KT * 16 + 8;
-  const int nin = adj ? 5 : 3;
-  // inputs in table order of use: 0 P, 1 Hy, 2 Sa (alpha), 3 G, 4 Sb (beta); without the
-  // adjoint's two: 0 P, 1 Hy, 2 G
-  const int iG = adj ? 3 : 2;
-  int* exc = reinterpret_cast<int*>(s.dig + (size_t)nin * kDig * NC * KS);  // [nin][kTile]
-  for (int i = threadIdx.x; i < nin * kTile; i += NTHR) exc[i] = 0;
-  __syncthreads();
-  const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
-  constexpr int kStep = 2 * (NTHR / kTile);
-  cpx v[KP][2][5];
-  {
-    const int x = x0 + min(col, nx - 1);
-    const double kx = g.Kx[x], kz = g.Kz[z];
-    const size_t cs = (size_t)gsz.Q() * gsz.X();
-    const cpx* Hc = H + (size_t)z * 5 * cs + x;
-    int e[5] = {0, 0, 0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < KP; ++k)
-#pragma unroll
-      for (int p = 0; p < 2; ++p) {
-        const int y = y0 + p + k * kStep;
-        const cpx zero = {0.0, 0.0};
-        cpx hz = zero, hx = zero, hy = zero, sx = zero, sz = zero;
-        if (y < gsz.Q() && col < nx) {
-          const cpx* b = Hc + (size_t)y * gsz.X();
-          hz = b[0];
-          hx = b[cs];
-          hy = b[2 * cs];
-          if (adj) {
-            sx = b[3 * cs];
-            sz = b[4 * cs];
-          }
+  const int col = threadIdx.x % kTile, x = x0 + min(col, nx - 1);
+  const double kx = g.Kx[x], kz = g.Kz[z];
+  const size_t cs = (size_t)gsz.Q() * gsz.X();
+  const cpx* Hc = H + (size_t)z * 5 * cs + x;
+  const bool mean = z == 0 && x == 0;
+  const int lx = x0 + min((int)(threadIdx.x & 3), nx - 1);
+  const double k2 = g.K2[(size_t)z * gsz.X() + lx];  // of this lane's output column
+  few_contract<kTile, NTHR, KP>(
+      gsz, g.tcW, g.tcWE, adj, nx, s.dig,
+      [&](int y, cpx (&o)[5]) {
+        const cpx* b = Hc + (size_t)y * gsz.X();
+        const cpx hz = b[0], hx = b[cs];
+        o[0] = imul_sum(kx, hx, kz, hz);   // P
+        o[1] = b[2 * cs];                  // Hy
+        o[3] = mean ? mean_input(hx, hz, 1.0) : imul_sum(kz, hx, -kx, hz);  // G
+        if (adj) {
+          const cpx sx = b[3 * cs], sz = b[4 * cs];
+          o[2] = imul_sum(-kz, sx, kx, sz);                                   // Sa
+          o[4] = mean ? mean_input(sz, sx, -1.0) : imul_sum(kz, sz, kx, sx);  // Sb
         }
-        cpx* o = v[k][p];
-        o[0] = imul_sum(kx, hx, kz, hz);
-        o[1] = hy;
-        o[2] = imul_sum(-kz, sx, kx, sz);
-        o[3] = imul_sum(kz, hx, -kx, hz);
-        o[4] = imul_sum(kz, sz, kx, sx);
-#pragma unroll
-        for (int q = 0; q < 5; ++q) e[q] = max(e[q], max(exp_field(o[q].re), exp_field(o[q].im)));
-      }
-    // lanes of a column lie kTile apart
-#pragma unroll
-    for (int q = 0; q < 5; ++q)
-#pragma unroll
-      for (int o = 16; o >= kTile; o >>= 1) e[q] = max(e[q], __shfl_xor_sync(0xffffffffu, e[q], o));
-    if ((threadIdx.x & 31) < kTile) {
-      atomicMax(&exc[0 * kTile + col], e[0]);
-      atomicMax(&exc[1 * kTile + col], e[1]);
-      atomicMax(&exc[iG * kTile + col], e[3]);
-      if (adj) {
-        atomicMax(&exc[2 * kTile + col], e[2]);
-        atomicMax(&exc[4 * kTile + col], e[4]);
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 5; ++q) {
-    if (!adj && (q == 2 || q == 4)) continue;
-    const int slot = (!adj && q == 3) ? 2 : q;
-    const int ex = exc[slot * kTile + col] - 1022;
-#pragma unroll
-    for (int k = 0; k < KP; ++k) {
-      const int y = y0 + k * kStep;
-      if (y >= KT * 16) break;
-      uint32_t* d = reinterpret_cast<uint32_t*>(s.dig + ((size_t)slot * kDig * NC + 2 * col) * KS + y);
-      digits_pair(scaled56(v[k][0][q].re, ex), scaled56(v[k][1][q].re, ex), d, NC * KS / 2);
-      digits_pair(scaled56(v[k][0][q].im, ex), scaled56(v[k][1][q].im, ex), d + KS / 2, NC * KS / 2);
-    }
-  }
-  asm volatile("cp.async.wait_all;\n" ::: "memory");  // the staged factors too
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
-  const uint4* __restrict__ W = reinterpret_cast<const uint4*>(g.tcW) + lane;
-  for (int item = warp; item < 2 * MTw; item += NTHR / 32) {
-    const bool toA = item < MTw;
-    const int mt = toA ? item : item - MTw, N = toA ? gsz.D() : gsz.R();
-    const int n = toA ? (adj ? 3 : 2) : (adj ? 2 : 1);
-    // weight tables: Qpw 1, Qw 0, Qppw 2; Rw 3, Rpw 4
-    auto table = [&](int q) { return W + ((size_t)(toA ? (q == 0 ? 1 : (q == 1 ? 0 : 2)) : 3 + q) * MTw + mt) * KT * kFragStep; };
-    cpx f[2];
-    const double k2 = g.K2[(size_t)z * gsz.X() + x0 + min(t, nx - 1)];
-    FragPair pf;
-    tc_stream_start(pf, table(0));
-    for (int q = 0; q < n; ++q) {
-      const int slot = toA ? q : iG + q, w = toA ? (q == 0 ? 1 : (q == 1 ? 0 : 2)) : 3 + q;
-      long long T[4];
-      tc_tile_stream(pf, table(q), q + 1 < n ? table(q + 1) : nullptr, KT,
-                     tc_row_addr(s.dig + (size_t)slot * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
-                     (uint32_t)(4 * NC * KS), T);
-      const int ecol = col_exp(exc[slot * kTile + t]) - 64 + kFoldShift;
-#pragma unroll
-      for (int rr = 0; rr < 2; ++rr) {
-        const int row = min(mt * 16 + gq + 8 * rr, N - 1);
-        const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol;
-        const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
-        if (q == 0) f[rr] = val;
-        else if (toA && q == 1) f[rr] = cpx{fma(-k2, val.re, f[rr].re), fma(-k2, val.im, f[rr].im)};
-        else f[rr] = cpx{f[rr].re + val.re, f[rr].im + val.im};
-      }
-    }
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      const int row = mt * 16 + gq + 8 * rr;
-      if (row < N && t < nx) (toA ? s.Fa : s.Fb)[row * kTile + t] = f[rr];
-    }
-  }
-  __syncthreads();
-}
-
-// One elimination chain (fixed parity, real or imaginary part) of the
-// no-pivot every-other-diagonal LU solve (channel/mvOps.c:29-91); W, DL, DU
-// the band layout (width, lower, upper), RD the reciprocal pivots; entries
-// outside the matrix are zero.  The last DL or DU results stay in registers
-// and the multiply-adds run from the oldest to the newest, so a row waits for
-// one multiply-add (and the pivot's product) of the row before it.  The
-// factors of the next kChainRows rows load while a group's rows run (GLOBAL:
-// from global memory; else they are staged in shared memory): 32x65x32, one
-// instance, 36k -> 9k cycles of a block's 260k.
-static constexpr int kChainRows = 4;
-
-template <bool GLOBAL>
-__device__ __forceinline__ double band_load(const double* p) {
-  return GLOBAL ? __ldg(p) : *p;
-}
-
-template <int W, int DL, int DU, bool GLOBAL>
-__device__ __forceinline__ void band_solve_chain(const double* __restrict__ LU, const double* __restrict__ RD, int N,
-                                                 int par, double* b, int bstride) {
-  const int M = (N - par + 1) / 2;  // rows of this parity: i = par + 2 m
-  if (M <= 0) return;
-  constexpr int G = kChainRows;
-  {
-    double f[G][DL], v[G], x[DL];
-    auto load = [&](int m0) {
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        const int i = par + 2 * min(m0 + q, M - 1);
-#pragma unroll
-        for (int j = 0; j < DL; ++j) f[q][j] = band_load<GLOBAL>(LU + (size_t)i * W + j);
-        v[q] = b[i * bstride];
-      }
-    };
-#pragma unroll
-    for (int t = 0; t < DL; ++t) x[t] = 0.0;  // x[t]: the result t + 1 rows back
-    load(0);
-    for (int m0 = 0; m0 < M; m0 += G) {
-      double c[G][DL], w[G];
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-#pragma unroll
-        for (int j = 0; j < DL; ++j) c[q][j] = f[q][j];
-        w[q] = v[q];
-      }
-      load(m0 + G);
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        double acc = w[q];
-#pragma unroll
-        for (int j = 0; j < DL; ++j) acc = fma(-c[q][j], x[DL - 1 - j], acc);
-#pragma unroll
-        for (int t = DL - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (m0 + q < M) b[(par + 2 * (m0 + q)) * bstride] = acc;
-      }
-    }
-  }
-  {
-    double f[G][DU], v[G], p[G], x[DU];
-    auto load = [&](int n0) {  // rows from the last one down
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        const int i = par + 2 * max(M - 1 - (n0 + q), 0);
-#pragma unroll
-        for (int j = 0; j < DU; ++j) f[q][j] = band_load<GLOBAL>(LU + (size_t)i * W + DL + 1 + j);
-        p[q] = band_load<GLOBAL>(RD + i);
-        v[q] = b[i * bstride];
-      }
-    };
-#pragma unroll
-    for (int t = 0; t < DU; ++t) x[t] = 0.0;
-    load(0);
-    for (int n0 = 0; n0 < M; n0 += G) {
-      double c[G][DU], w[G], r[G];
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-#pragma unroll
-        for (int j = 0; j < DU; ++j) c[q][j] = f[q][j];
-        w[q] = v[q];
-        r[q] = p[q];
-      }
-      load(n0 + G);
-#pragma unroll
-      for (int q = 0; q < G; ++q) {
-        double acc = w[q];
-#pragma unroll
-        for (int j = DU - 1; j >= 0; --j) acc = fma(-c[q][j], x[j], acc);
-        acc *= r[q];
-#pragma unroll
-        for (int t = DU - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = acc;
-      }
-    }
-  }
+      },
+      [](int q) { return q == 0 ? 1 : (q == 1 ? 0 : q); },  // Qpw P, Qw Hy, Qppw Sa, Rw G, Rpw Sb
+      [&](int q, const cpx& f, const cpx& v) {
+        if (q == 1) return cpx{fma(-k2, v.re, f.re), fma(-k2, v.im, f.im)};
+        return cpx{f.re + v.re, f.im + v.im};
+      },
+      s.Fa, s.Fb);
 }
 
 // the banded solves of a tile: per column 4 chains for alpha, 4 for beta
@@ -791,6 +583,13 @@ template <int kTile, bool GLOBAL, class S>
 __device__ __forceinline__ void solve_chains(const Grid& g, const S& gsz, int bidx, int z, int x0, int nx, int xfirst,
                                              const SolveSmem& s) {
   constexpr int kHalf = 4 * kTile < 32 ? 32 : 4 * kTile;
+  if (xfirst && (int)threadIdx.x >= 2 * kHalf) {  // the mean line's two, in a warp of their own
+    const int t = (int)threadIdx.x - 2 * kHalf;
+    if (t < 8)
+      band_solve_chain<5, 2, 2, true>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), t & 1,
+                                      reinterpret_cast<double*>(t < 4 ? s.ra : s.rb) + ((t >> 1) & 1), 2 * kTile);
+    return;
+  }
   const bool beta = (int)threadIdx.x >= kHalf;
   const int t = beta ? (int)threadIdx.x - kHalf : (int)threadIdx.x, l = t / 4, par = t & 1, part = (t >> 1) & 1;
   if (t >= 4 * kTile || l >= nx || l < xfirst) return;
@@ -805,177 +604,20 @@ __device__ __forceinline__ void solve_chains(const Grid& g, const S& gsz, int bi
                                       reinterpret_cast<double*>(s.rb + l) + part, 2 * kTile);
 }
 
-// The (kx, kz) = (0, 0) line of one substage (channel/project0.c,
-// increproject0.c, adjproject0.c) in a block of its own: its quadratures, a
-// warp per row (they took one warp of the kz = 0 tile's block 115k cycles,
-// more than that tile's own work), its chains, the flux correction and the
-// next right-hand side.  Same arguments as the tiles' blocks.
-template <int NTHR, class S>
-__device__ void solve_mean(const Grid& g, const S& gsz, const SolveArgs& a, int inst, const RKc& rk, int mean_mode,
-                           cpx* __restrict__ Cc, cpx* __restrict__ So, cpx* Tst, int tslot, int fkind, const cpx* xk,
-                           double ft1, double* sm) {
-  const int R = gsz.R(), Q = gsz.Q(), X = gsz.X();
-  const size_t csz = coef_size(g);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* fa = sm;                                 // [R]
-  double* fb = sm + R;                             // [R]
-  cpx* ca = reinterpret_cast<cpx*>(sm + 2 * R);    // [R]
-  cpx* cb = ca + R;                                // [R]
-  double* hv = sm + 6 * R;                         // [4][Q] Hx, Hz, Sz, Sx of the line
-  __shared__ double flux_part;
-  const bool adj = a.adjoint != 0;
-  const double dt = g.dt, re2 = g.re * g.re;
-  const double ak = a.k == 1 ? -1. / 2 : 1. / 3.;
-  auto cidx = [&](int v, int r) { return ((size_t)v * R + r) * X; };
-  // fa = Rw Hx [+ Rpw Sz], fb = Rw Hz [- Rpw Sx] (real parts)
-  auto quad = [&](const cpx* __restrict__ H) {
-    const size_t cs = (size_t)Q * X;
-    for (int y = threadIdx.x; y < Q; y += NTHR) {
-      hv[y] = H[cs + (size_t)y * X].re;
-      hv[Q + y] = H[(size_t)y * X].re;
-      if (adj) {
-        hv[2 * Q + y] = H[4 * cs + (size_t)y * X].re;
-        hv[3 * Q + y] = H[3 * cs + (size_t)y * X].re;
-      }
-    }
-    __syncthreads();
-    for (int i = warp; i < R; i += NTHR / 32) {
-      double sa = 0.0, sb = 0.0;
-      for (int y = lane; y < Q; y += 32) {
-        const double rw = __ldg(g.Wr + (size_t)i * Q + y);
-        sa = fma(rw, hv[y], sa);
-        sb = fma(rw, hv[Q + y], sb);
-        if (adj) {
-          const double rpw = __ldg(g.Wrp + (size_t)i * Q + y);
-          sa = fma(rpw, hv[2 * Q + y], sa);
-          sb = fma(-rpw, hv[3 * Q + y], sb);
-        }
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      }
-      if (lane == 0) {
-        fa[i] = sa;
-        fb[i] = sb;
-      }
-    }
-    __syncthreads();
-  };
-  auto chains = [&](int bidx) {  // ca, cb <- the mean system's solution
-    if (threadIdx.x < 8) {
-      const int par = threadIdx.x & 1, part = (threadIdx.x >> 1) & 1;
-      band_solve_chain<5, 2, 2, true>(g.lu0 + (size_t)bidx * R * 5, g.rd0 + (size_t)bidx * R, R, par,
-                                      reinterpret_cast<double*>(threadIdx.x < 4 ? ca : cb) + part, 2);
-    }
-    __syncthreads();
-  };
-  if (fkind == 2 && a.k == 0) {
-    // tangent_forcing0.c:31-41 on MC[3n+1], Rs^-1, IC += dt f (increproject0.c:45-90)
-    const cpx* x1 = xk + csz;
-    for (int i = threadIdx.x; i < R; i += NTHR) {
-      const cpx p = band_matvec_row(g.Rps, 5, 2, 2, R, x1 + cidx(0, 0), X, i);
-      const cpx q = band_matvec_row(g.Rps, 5, 2, 2, R, x1 + cidx(1, 0), X, i);
-      ca[i] = cpx{re2 * p.re, re2 * p.im};
-      cb[i] = cpx{re2 * q.re, re2 * q.im};
-    }
-    __syncthreads();
-    chains(2);
-    for (int i = threadIdx.x; i < R; i += NTHR) {
-      Cc[cidx(0, i)].re += dt * ca[i].re;
-      Cc[cidx(0, i)].im += dt * ca[i].im;
-      Cc[cidx(1, i)].re += dt * cb[i].re;
-      Cc[cidx(1, i)].im += dt * cb[i].im;
-    }
-    __syncthreads();
-  }
-  quad(a.H.at(inst));
-  for (int i = threadIdx.x; i < R; i += NTHR) {
-    cpx va, vb;
-    if (a.k == 0) {
-      const double* E = g.ex0 + (size_t)rk.aidx0 * R * 5;
-      va = band_matvec_row(E, 5, 2, 2, R, Cc + cidx(0, 0), X, i);
-      vb = band_matvec_row(E, 5, 2, 2, R, Cc + cidx(1, 0), X, i);
-    } else {
-      va = Cc[cidx(0, i)];
-      vb = Cc[cidx(1, i)];
-    }
-    va.re += dt * rk.c * fa[i];
-    vb.re += dt * rk.c * fb[i];
-    if (fkind == 3) {
-      // D0 = -Rps; the implicit term acts on the primal's solved mean flow
-      // before its flux correction: MC[3n+k+1] - 0.5 flux_t add
-      const cpx p0 = band_matvec_row(g.Rps, 5, 2, 2, R, xk + cidx(0, 0), X, i);
-      cpx p1 = band_matvec_row(g.Rps, 5, 2, 2, R, xk + csz + cidx(0, 0), X, i);
-      p1.re -= 0.5 * ft1 * rps_row_real(g, g.add0, i);
-      const cpx q0 = band_matvec_row(g.Rps, 5, 2, 2, R, xk + cidx(1, 0), X, i);
-      const cpx q1 = band_matvec_row(g.Rps, 5, 2, 2, R, xk + csz + cidx(1, 0), X, i);
-      va.re += re2 * dt * ak * p0.re;
-      va.im += re2 * dt * ak * p0.im;
-      va.re += re2 * dt * rk.b * p1.re;
-      va.im += re2 * dt * rk.b * p1.im;
-      vb.re += re2 * dt * ak * q0.re;
-      vb.im += re2 * dt * ak * q0.im;
-      vb.re += re2 * dt * rk.b * q1.re;
-      vb.im += re2 * dt * rk.b * q1.im;
-    }
-    ca[i] = va;
-    cb[i] = vb;
-  }
-  __syncthreads();
-  chains(rk.bidx);
-  // constant mass flux: a += 0.5 * flux_t * add (channel/project0.c:153-168)
-  if (warp == 0) {
-    double part = 0.0;
-    for (int i = lane; i < R; i += 32) part = fma(g.rwsum[i], ca[i].re, part);
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) flux_part = part;
-  }
-  __syncthreads();
-  double flux_t;
-  if (mean_mode == MEAN_PRIMAL) flux_t = g.flux - flux_part;
-  else if (mean_mode == MEAN_TAN_FORCED) flux_t = 2.0 - flux_part;
-  else flux_t = -flux_part;
-  const double* add = g.add0 + (size_t)(adj ? 1 + rk.bidx : 0) * R;
-  if (mean_mode == MEAN_PRIMAL && a.Fts && Tst && threadIdx.x == 0)
-    a.Fts[(long long)(inst / a.tdiv) * a.fts_stride + tslot] = flux_t;
-  for (int i = threadIdx.x; i < R; i += NTHR) {
-    const cpx va = {ca[i].re + flux_t * add[i] * 0.5, ca[i].im};
-    ca[i] = va;
-    So[cidx(0, i)] = va;
-    So[cidx(1, i)] = cb[i];
-    if (Tst) {
-      Tst[cidx(0, i)] = va;
-      Tst[cidx(1, i)] = cb[i];
-    }
-    if (a.k == 2) {
-      Cc[cidx(0, i)] = va;
-      Cc[cidx(1, i)] = cb[i];
-    }
-  }
-  if (a.k == 2) return;
-  __syncthreads();
-  if (adj) quad(a.Hprev.at(inst));  // from the previous-stage terms (channel/adjproject0.c:254-294)
-  const double* E = g.ex0 + (size_t)rk.aidx_next * R * 5;
-  for (int i = threadIdx.x; i < R; i += NTHR) {
-    cpx va = band_matvec_row(E, 5, 2, 2, R, ca, 1, i);
-    cpx vb = band_matvec_row(E, 5, 2, 2, R, cb, 1, i);
-    va.re += dt * rk.dnext * fa[i];
-    vb.re += dt * rk.dnext * fb[i];
-    Cc[cidx(0, i)] = va;
-    Cc[cidx(1, i)] = vb;
-  }
-}
+// The (kx, kz) = (0, 0) line (channel/project0.c, increproject0.c,
+// adjproject0.c) is column 0 of the kz = 0 line's first tile: two real systems
+// of the R basis (alpha and beta hold u and w), whose quadratures fa = Rw Hx
+// [+ Rpw Sz] and fb = Rw Hz [- Rpw Sx] come out of the tile's beta contraction
+// as Re and Im of Fb's column 0 (mean_input); they took one warp 115k cycles of
+// the tile's block, more than the rest of it.
 
-// Block 0 of an instance: the mean line; block 1 + z ntx + tx: kx tile tx of
-// line z.  S: the sizes (SizesRT, or SizesCT for a specialised grid); NTHR
+// Block z ntx + tx: kx tile tx of line z.  S: the sizes (SizesRT, or SizesCT for a specialised grid); NTHR
 // threads (256, or 128 with the 8-column tile), MINB blocks per SM; FEW: the
 // build for launches with few blocks (quad_rhs_few, staged factors)
 template <bool MULTI, int kTile, class S, int NTHR = kThreads, int MINB = 2, int FEW = 0>
 __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Grid g0, SolveArgs a) {
   const int ntx = (g0.X + kTile - 1) / kTile;
-  const bool mean_block = blockIdx.x == 0;
-  const int z = mean_block ? 0 : (blockIdx.x - 1) / ntx, tx = mean_block ? 0 : (int)(blockIdx.x - 1) - z * ntx;
+  const int z = blockIdx.x / ntx, tx = blockIdx.x - z * ntx;
   const int inst = blockIdx.y;
   CHN_INSTANCE_GRID(g0, a.grids, inst);
   const S gsz(g);
@@ -1025,15 +667,11 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
       if (a.Ftr) ft1 = a.Ftr[(long long)(inst / a.xdiv) * a.ftr_stride + xs + 1];
     }
   }
-  if (mean_block) {
-    solve_mean<NTHR>(g, gsz, a, inst, rk, mean_mode, Cc, So, Tst, tslot, fkind, xk, ft1, reinterpret_cast<double*>(smem));
-    return;
-  }
   const cpx* __restrict__ H = a.H.at(inst);
   SolveSmem s;
   if constexpr (FEW) {
     s = carve_solve_few<kTile>(g, smem, adj);
-    stage_factors<kTile, NTHR>(g, gsz, (size_t)rk.bidx * gsz.Nz() * gsz.X() + (size_t)z * gsz.X() + x0, nx, s);
+    stage_factors<NTHR>(g, gsz, (size_t)rk.bidx * gsz.Nz() * gsz.X() + (size_t)z * gsz.X() + x0, nx, s.luA, s.luB, s.rdA, s.rdB);
     quad_rhs_few<kTile, NTHR, FEW>(g, gsz, H, z, x0, nx, adj, s);
   } else {
     s = carve_solve<kTile>(g, smem);
@@ -1048,8 +686,15 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
     const cpx* x1 = xk + csz;
     for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
       const int r = i / kTile, l = i - r * kTile;
-      if (l >= nx || l < xfirst) continue;
+      if (l >= nx) continue;
       const int x = x0 + l;
+      if (l < xfirst) {  // tangent_forcing0.c:31-41
+        const cpx p = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), x1 + cidx(0, 0, 0), gsz.X(), r);
+        const cpx q = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), x1 + cidx(1, 0, 0), gsz.X(), r);
+        s.ra[r * kTile] = cpx{re2 * p.re, re2 * p.im};
+        s.rb[r * kTile] = cpx{re2 * q.re, re2 * q.im};
+        continue;
+      }
       const double k2 = g.K2[(size_t)z * gsz.X() + x];
       if (r < gsz.D()) {
         const cpx v = visc_v_row(g, k2, x1 + cidx(0, 0, x), gsz.X(), r);
@@ -1063,9 +708,9 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
     __syncthreads();
     for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
       const int r = i / kTile, l = i - r * kTile;
-      if (l >= nx || l < xfirst) continue;
+      if (l >= nx) continue;
       const int x = x0 + l;
-      if (r < gsz.D()) {
+      if (r < gsz.D() || l < xfirst) {
         const cpx f = s.ra[r * kTile + l];
         Cc[cidx(0, r, x)].re += dt * f.re;
         Cc[cidx(0, r, x)].im += dt * f.im;
@@ -1079,10 +724,43 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
   // right-hand sides (channel/project.c:60-81, 125-130, 143-163, 202-207)
   for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
     const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
+    if (l >= nx) continue;
     const int x = x0 + l;
     const size_t zx = (size_t)z * gsz.X() + x;
     cpx va, vb;
+    if (l < xfirst) {
+      if (a.k == 0) {
+        const double* E = g.ex0 + (size_t)rk.aidx0 * gsz.R() * 5;
+        va = band_matvec_row(E, 5, 2, 2, gsz.R(), Cc + cidx(0, 0, 0), gsz.X(), r);
+        vb = band_matvec_row(E, 5, 2, 2, gsz.R(), Cc + cidx(1, 0, 0), gsz.X(), r);
+      } else {
+        va = Cc[cidx(0, r, 0)];
+        vb = Cc[cidx(1, r, 0)];
+      }
+      const cpx f = s.Fb[r * kTile];
+      va.re += dt * rk.c * f.re;
+      vb.re += dt * rk.c * f.im;
+      if (fkind == 3) {
+        // D0 = -Rps; the implicit term acts on the primal's solved mean flow
+        // before its flux correction: MC[3n+k+1] - 0.5 flux_t add
+        const cpx p0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(0, 0, 0), gsz.X(), r);
+        cpx p1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(0, 0, 0), gsz.X(), r);
+        p1.re -= 0.5 * ft1 * rps_row_real(g, g.add0, r);
+        const cpx q0 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + cidx(1, 0, 0), gsz.X(), r);
+        const cpx q1 = band_matvec_row(g.Rps, 5, 2, 2, gsz.R(), xk + csz + cidx(1, 0, 0), gsz.X(), r);
+        va.re += re2 * dt * ak * p0.re;
+        va.im += re2 * dt * ak * p0.im;
+        va.re += re2 * dt * rk.b * p1.re;
+        va.im += re2 * dt * rk.b * p1.im;
+        vb.re += re2 * dt * ak * q0.re;
+        vb.im += re2 * dt * ak * q0.im;
+        vb.re += re2 * dt * rk.b * q1.re;
+        vb.im += re2 * dt * rk.b * q1.im;
+      }
+      s.ra[r * kTile] = va;
+      s.rb[r * kTile] = vb;
+      continue;
+    }
     if (r < gsz.D()) {
       if (a.k == 0) {
         const double* E = g.exA + ((size_t)rk.aidx0 * gsz.Nz() * gsz.X() + zx) * gsz.D() * 9;
@@ -1129,10 +807,30 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
   __syncthreads();
   solve_chains<kTile, !FEW>(g, gsz, rk.bidx, z, x0, nx, xfirst, s);
   __syncthreads();
+  if (xfirst) {
+    // constant mass flux: a += 0.5 * flux_t * add (channel/project0.c:153-168), warp 0
+    if (threadIdx.x < 32) {
+      double part = 0.0;
+      for (int i = threadIdx.x; i < gsz.R(); i += 32) part = fma(g.rwsum[i], s.ra[i * kTile].re, part);
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      double flux_t;
+      if (mean_mode == MEAN_PRIMAL) flux_t = g.flux - part;
+      else if (mean_mode == MEAN_TAN_FORCED) flux_t = 2.0 - part;
+      else flux_t = -part;
+      const double* add = g.add0 + (size_t)(adj ? 1 + rk.bidx : 0) * gsz.R();
+      if (mean_mode == MEAN_PRIMAL && a.Fts && Tst && threadIdx.x == 0)
+        a.Fts[(long long)(inst / a.tdiv) * a.fts_stride + tslot] = flux_t;
+      for (int i = threadIdx.x; i < gsz.R(); i += 32) {
+        double& v = s.ra[i * kTile].re;
+        v = v + flux_t * add[i] * 0.5;
+      }
+    }
+    __syncthreads();
+  }
   // state rows: alpha from the solve (rows >= Ny-4 carried), beta from the solve
   for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
     const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
+    if (l >= nx) continue;
     const int x = x0 + l;
     const cpx va = s.ra[r * kTile + l], vb = s.rb[r * kTile + l];
     So[cidx(0, r, x)] = va;
@@ -1147,7 +845,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
     // the carried array is the state after the last substage
     for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
       const int r = i / kTile, l = i - r * kTile;
-      if (l >= nx || l < xfirst) continue;
+      if (l >= nx) continue;
       const int x = x0 + l;
       Cc[cidx(0, r, x)] = So[cidx(0, r, x)];
       Cc[cidx(1, r, x)] = So[cidx(1, r, x)];
@@ -1168,57 +866,52 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
     __syncthreads();
   }
   // the solved state of this tile (So) is still in ra, rb unless the
-  // adjoint's second quadrature overwrote them (they share its digit
-  // buffer); the results go to Fa, Fb (each element read and written by one
-  // thread)
+  // adjoint's second quadrature overwrote them (they share its digit buffer)
   for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
     const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
+    if (l >= nx) continue;
     const int x = x0 + l;
     const size_t zx = (size_t)z * gsz.X() + x;
     const cpx* ya = adj ? So + cidx(0, 0, x) : s.ra + l;
     const cpx* yb = adj ? So + cidx(1, 0, x) : s.rb + l;
     const int ys = adj ? gsz.X() : kTile;
-    if (r < gsz.D()) {
-      const double* E = g.exA + ((size_t)rk.aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.D() * 9;
-      cpx va = band_matvec_row_t<9, 4, 4>(E, gsz.D(), ya, ys, r);
-      const cpx f = s.Fa[r * kTile + l];
-      va.re += dt * rk.dnext * f.re;
-      va.im += dt * rk.dnext * f.im;
-      s.Fa[r * kTile + l] = va;
-    }
-    const double* E = g.exB + ((size_t)rk.aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.R() * 5;
-    cpx vb = band_matvec_row_t<5, 2, 2>(E, gsz.R(), yb, ys, r);
+    const bool mean = l < xfirst;
     const cpx f = s.Fb[r * kTile + l];
-    vb.re += dt * rk.dnext * f.re;
-    vb.im += dt * rk.dnext * f.im;
-    s.Fb[r * kTile + l] = vb;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
-    const int r = i / kTile, l = i - r * kTile;
-    if (l >= nx || l < xfirst) continue;
-    const int x = x0 + l;
-    Cc[cidx(0, r, x)] = r < gsz.D() ? s.Fa[r * kTile + l] : So[cidx(0, r, x)];  // rows >= Ny-4 carried
-    Cc[cidx(1, r, x)] = s.Fb[r * kTile + l];
+    cpx va = ya[r * ys];  // alpha rows >= Ny-4 carried
+    if (mean) {
+      va = band_matvec_row_t<5, 2, 2>(g.ex0 + (size_t)rk.aidx_next * gsz.R() * 5, gsz.R(), ya, ys, r);
+      va.re += dt * rk.dnext * f.re;
+    } else if (r < gsz.D()) {
+      const double* E = g.exA + ((size_t)rk.aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.D() * 9;
+      va = band_matvec_row_t<9, 4, 4>(E, gsz.D(), ya, ys, r);
+      const cpx fa = s.Fa[r * kTile + l];
+      va.re += dt * rk.dnext * fa.re;
+      va.im += dt * rk.dnext * fa.im;
+    }
+    const double* E = mean ? g.ex0 + (size_t)rk.aidx_next * gsz.R() * 5
+                           : g.exB + ((size_t)rk.aidx_next * gsz.Nz() * gsz.X() + zx) * gsz.R() * 5;
+    cpx vb = band_matvec_row_t<5, 2, 2>(E, gsz.R(), yb, ys, r);
+    vb.re += dt * rk.dnext * (mean ? f.im : f.re);
+    if (!mean) vb.im += dt * rk.dnext * f.im;
+    Cc[cidx(0, r, x)] = va;
+    Cc[cidx(1, r, x)] = vb;
   }
 }
 
 // The build for few blocks (4-column tiles, one block per SM): where its
-// blocks are at most kFewWaves per SM, CHN_SOLVE_TILE does not ask for a tile
+// tiles are at most kFewTiles, CHN_SOLVE_TILE does not ask for a tile
 // and the grid's tables and shared memory allow it.
 static int s_solve_optin = 0;
-static constexpr int kFewBlocks = 2 * 152;
 static bool solve_few(const Grid& g, const SolveArgs& a) {
   if (a.grids || !g.tc || g.sfixed || g.Q <= 16 || g.Q > 256) return false;  // (a stream takes two k-tiles or more)
-  if ((long long)g.Nz * ((g.X + 3) / 4) * a.ninst > kFewBlocks) return false;
+  if ((long long)g.Nz * ((g.X + 3) / 4) * a.ninst > kFewTiles) return false;
   return solve_few_smem_bytes(g, 4, a.adjoint != 0) + 1024 <= (size_t)s_solve_optin;
 }
 
 template <int T, class S, int NTHR = kThreads, int MINB = 2>
 static void launch_solve_t(const Grid& g, const SolveArgs& a, cudaStream_t st) {
   const int ntx = (g.X + T - 1) / T;
-  const dim3 grid(1 + g.Nz * ntx, a.ninst);
+  const dim3 grid(g.Nz * ntx, a.ninst);
   if (a.grids) k_solve<true, T, SizesRT, NTHR, MINB><<<grid, NTHR, solve_smem_bytes_t<T>(g), st>>>(g, a);
   else k_solve<false, T, S, NTHR, MINB><<<grid, NTHR, solve_smem_bytes_t<T>(g), st>>>(g, a);
 }
@@ -1237,7 +930,7 @@ static void launch_solve_s(const Grid& g, const SolveArgs& a, cudaStream_t st) {
 cudaError_t launch_solve(const Grid& g, const SolveArgs& a, cudaStream_t st) {
   if (a.ninst <= 0) return cudaSuccess;
   if (solve_few(g, a)) {
-    const dim3 grid(1 + g.Nz * ((g.X + 3) / 4), a.ninst);
+    const dim3 grid(g.Nz * ((g.X + 3) / 4), a.ninst);
     const size_t sm = solve_few_smem_bytes(g, 4, a.adjoint != 0);
     if (g.Q <= 128 && sizes_match<Sizes32>(g)) k_solve<false, 4, Sizes32, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
     else if (g.Q <= 128 && sizes_match<Sizes16>(g)) k_solve<false, 4, Sizes16, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);

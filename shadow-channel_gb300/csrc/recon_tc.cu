@@ -17,8 +17,7 @@
 //   - levels l < 7 are kept (the rest lie below 2^-56 of the operands'
 //     scale), recombined exactly in 64-bit integers and rounded once to FP64
 //     by one fma.
-// Only the rounding, the K-algebra and the (kx, kz) = (0, 0) mean mode
-// (computed directly) use the FP64 pipe.  Results agree with the FP64
+// Only the rounding and the K-algebra use the FP64 pipe.  Results agree with the FP64
 // contraction to its own rounding.
 #include <cuda_bf16.h>
 
@@ -182,7 +181,31 @@ size_t recon_tc_smem_bytes(const Grid& g, int tile) {
 
 size_t recon_tc_smem_bytes(const Grid& g) { return recon_tc_smem_bytes(g, kTile); }
 
-// S: the sizes (SizesRT, or SizesCT for a specialised grid); TILE kx
+// The (kx, kz) = (0, 0) column (channel/initAlphaBeta2.c:25-68) is real: u = R a,
+// du = R' a, v = 0, w = R b, dw = R' b with a, b the real parts of alpha and
+// beta (a complex-to-real transform ignores the imaginary parts).  Its two
+// systems are Re and Im of the beta class's column 0: the contractions with R
+// and R' give (u, w) and (du, dw).  A non-finite imaginary part makes the
+// column NaN.
+__device__ __forceinline__ cpx mean_coefficients(const cpx& al, const cpx& be, int& e) {
+  e = max(e, max(exp_field(al.re), exp_field(be.re)));
+  if (exp_field(al.im) == 0x7FF || exp_field(be.im) == 0x7FF) e = 0x7FF;
+  return cpx{al.re, be.re};
+}
+
+// u, w and du/dy, dw/dy of a column from f = -Q' alpha, g = R beta and Q''
+// alpha, R' beta: u = (kx Im f + kz Im g)/K2 - i (kx Re f + kz Re g)/K2 etc.
+__device__ __forceinline__ void recon_velocity(double ax, double az, const cpx& qp, const cpx& gg, cpx& u, cpx& w) {
+  const cpx f = {-qp.re, -qp.im};
+  u = cpx{fma(ax, f.im, az * gg.im), -fma(ax, f.re, az * gg.re)};
+  w = cpx{fma(-ax, gg.im, az * f.im), fma(ax, gg.re, -az * f.re)};
+}
+__device__ __forceinline__ void recon_derivative(double ax, double az, const cpx& qpp, const cpx& rp, cpx& du, cpx& dw) {
+  du = cpx{fma(-ax, qpp.im, az * rp.im), fma(ax, qpp.re, -az * rp.re)};
+  dw = cpx{-fma(ax, rp.im, az * qpp.im), fma(ax, rp.re, az * qpp.re)};
+}
+
+// Block z ntx + tx: kx tile tx of line z.  S: the sizes (SizesRT, or SizesCT for a specialised grid); TILE kx
 // columns per block (2 TILE real digit columns) in NTHR = 16 TILE threads
 template <bool MULTI, class S, int TILE = kTile, int NTHR = kThreads, int MINB = 2>
 __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__ Grid g0, ReconArgs a) {
@@ -203,10 +226,17 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
   int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * (2 * TILE) * KS * sizeof(uint16_t));  // [cls][TILE]
   const cpx* __restrict__ C = a.C.at(inst);
   if (a.slot.stride) C += (long long)a.slot.slot() * a.slot.stride;
-  auto cval = [&](int cls, int j, int col) -> cpx {
+  // coefficient (class, row, column), its exponent field joined into e
+  auto cval = [&](int cls, int j, int col, int& e) -> cpx {
     const int K = cls == 0 ? gsz.D() : gsz.R();
-    if (j >= K || col >= nx || (meancol && col == 0)) return cpx{0.0, 0.0};
-    return C[(((size_t)z * 2 + cls) * gsz.R() + j) * gsz.X() + x0 + col];
+    if (j >= K || col >= nx) return cpx{0.0, 0.0};
+    const cpx* p = C + (((size_t)z * 2 + cls) * gsz.R() + j) * gsz.X() + x0 + col;
+    if (meancol && col == 0) {
+      if (cls == 0) return cpx{0.0, 0.0};
+      return mean_coefficients(*(p - (size_t)gsz.R() * gsz.X()), *p, e);
+    }
+    e = max(e, max(exp_field(p->re), exp_field(p->im)));
+    return *p;
   };
   // column exponents: |c| < 2^exc over the column's real and imaginary parts
   for (int i = threadIdx.x; i < 2 * TILE; i += NTHR) exc[i] = 0;
@@ -225,8 +255,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
     for (int cls = 0; cls < 2; ++cls)
 #pragma unroll
       for (int k = 0; k < kReconRegs; ++k) {
-        vin[cls][k] = k < (KT + 1) / 2 * 2 ? cval(cls, row(k), col) : cpx{0.0, 0.0};
-        emax[cls] = max(emax[cls], max(exp_field(vin[cls][k].re), exp_field(vin[cls][k].im)));
+        vin[cls][k] = k < (KT + 1) / 2 * 2 ? cval(cls, row(k), col, emax[cls]) : cpx{0.0, 0.0};
       }
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls)
@@ -247,14 +276,15 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
   } else {
     for (int i = threadIdx.x; i < nent; i += NTHR) {
       const int cls = i / ((KT * 16) * TILE), r = i - cls * (KT * 16) * TILE, j = r / TILE, col = r - j * TILE;
-      const cpx v = cval(cls, j, col);
-      const int e = max(exp_field(v.re), exp_field(v.im));
+      int e = 0;
+      cval(cls, j, col, e);
       if (e) atomicMax(&exc[cls * TILE + col], e);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nent / 2; i += NTHR) {
       const int cls = i / ((KT * 8) * TILE), r = i - cls * (KT * 8) * TILE, j = 2 * (r / TILE), col = r % TILE;
-      const cpx v0 = cval(cls, j, col), v1 = cval(cls, j + 1, col);
+      int e = 0;
+      const cpx v0 = cval(cls, j, col, e), v1 = cval(cls, j + 1, col, e);
       const int ex = exc[cls * TILE + col] - 1022;
       // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col) * KS + j);
@@ -285,7 +315,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int y = mt * 16 + gq + 8 * rr;
-        if (y >= gsz.Q() || col >= nx || (meancol && col == 0)) continue;
+        if (y >= gsz.Q() || col >= nx) continue;
+        const bool mean = meancol && col == 0;
         const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol;
         const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
         const int x = x0 + col;
@@ -295,38 +326,120 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
           out[cs] = val;  // v = Q alpha
         } else if (b == 1 || b == 2) {
           held[rr] = val;
+        } else if (mean) {
+          out[b == 3 ? 0 : 3 * cs] = cpx{val.re, 0.0};
+          out[b == 3 ? 2 * cs : 4 * cs] = cpx{val.im, 0.0};
         } else if (b == 3) {
-          // u = (kx Im f + kz Im g)/K2 - i (kx Re f + kz Re g)/K2 etc., f = -Q' alpha
-          const cpx f = {-held[rr].re, -held[rr].im}, gg = val;
-          out[0] = cpx{fma(ax, f.im, az * gg.im), -fma(ax, f.re, az * gg.re)};
-          out[2 * cs] = cpx{fma(-ax, gg.im, az * f.im), fma(ax, gg.re, -az * f.re)};
+          recon_velocity(ax, az, held[rr], val, out[0], out[2 * cs]);
         } else {
-          const cpx qpp = held[rr], rp = val;
-          out[3 * cs] = cpx{fma(-ax, qpp.im, az * rp.im), fma(ax, qpp.re, -az * rp.re)};
-          out[4 * cs] = cpx{-fma(ax, rp.im, az * qpp.im), fma(ax, rp.re, az * qpp.re)};
+          recon_derivative(ax, az, held[rr], val, out[3 * cs], out[4 * cs]);
         }
       }
     }
   }
-  if (meancol) {
-    // (kx, kz) = (0, 0): u = R a, du = R' a, v = 0, w = R b, dw = R' b
-    // (channel/initAlphaBeta2.c:25-68), direct FP64
-    for (int y = threadIdx.x; y < gsz.Q(); y += NTHR) {
-      double ur = 0, ui = 0, dur = 0, dui = 0, wr = 0, wi = 0, dwr = 0, dwi = 0;
-      for (int j = 0; j < gsz.R(); ++j) {
-        const double r = __ldg(g.Br + (size_t)y * gsz.R() + j), rp = __ldg(g.Brp + (size_t)y * gsz.R() + j);
-        const cpx al = C[((size_t)0 * gsz.R() + j) * gsz.X()], be = C[((size_t)1 * gsz.R() + j) * gsz.X()];
-        ur = fma(r, al.re, ur); ui = fma(r, al.im, ui);
-        dur = fma(rp, al.re, dur); dui = fma(rp, al.im, dui);
-        wr = fma(r, be.re, wr); wi = fma(r, be.im, wi);
-        dwr = fma(rp, be.re, dwr); dwi = fma(rp, be.im, dwi);
+}
+
+// The reconstruction for launches with few blocks, where a block has its SM
+// almost to itself: 4-column tiles (one 8-column digit tile), a warp per
+// (16 planes, output group) -- u and w, du/dy and dw/dy, v -- whose tables'
+// k-tiles run as one stream with two in flight.  KP: row pairs of a class a
+// thread holds (R <= 64 KP).
+template <class S, int KP>
+__global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Grid g, ReconArgs a) {
+  constexpr int TILE = 4, NTHR = 256, NC = 2 * TILE;
+  const S gsz(g);
+  const int ntx = (gsz.X() + TILE - 1) / TILE;
+  const int z = blockIdx.x / ntx, tx = blockIdx.x - z * ntx;
+  const int inst = blockIdx.y;
+  if (z == gsz.Nz() / 2) return;  // never read (channel/pass1.c:51-85 skips it)
+  if (a.status != nullptr && (a.status[inst / a.sdiv] & ST_CFL) != 0) return;
+  const cpx* __restrict__ C = a.C.at(inst);
+  if (a.slot.stride) C += (long long)a.slot.slot() * a.slot.stride;
+  cpx* __restrict__ U = a.U.at(inst);
+  const int x0 = tx * TILE, nx = min(TILE, gsz.X() - x0);
+  const bool meancol = z == 0 && x0 == 0;
+  const int KT = (gsz.R() + 15) / 16, KS = recon_tc_kstride(KT), MT = (gsz.Q() + 15) / 16;
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint16_t* dig = reinterpret_cast<uint16_t*>(smem);  // [cls][digit][n 2 TILE][KS]
+  int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * NC * KS * sizeof(uint16_t));  // [cls][TILE]
+  if (threadIdx.x < 2 * TILE) exc[threadIdx.x] = 0;
+  __syncthreads();
+  {
+    // threads [0, 128) the alpha rows, the rest the beta ones; row pairs 2 (t / TILE) + 64 k
+    const int cls = threadIdx.x >> 7, col = threadIdx.x % TILE, j0 = 2 * ((threadIdx.x & 127) / TILE);
+    const int K = cls == 0 ? gsz.D() : gsz.R();
+    const bool mean = meancol && col == 0, on = col < nx && !(mean && cls == 0);
+    const cpx* src = C + ((size_t)(z * 2 + cls) * gsz.R()) * gsz.X() + x0 + col;
+    cpx v[KP][2];
+    int e = 0;
+#pragma unroll
+    for (int k = 0; k < KP; ++k)
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int j = j0 + p + 64 * k;
+        v[k][p] = (on && j < K) ? src[(size_t)j * gsz.X()] : cpx{0.0, 0.0};
+        if (mean && on && j < K) v[k][p] = mean_coefficients(src[((ptrdiff_t)j - gsz.R()) * gsz.X()], v[k][p], e);
+        else e = max(e, max(exp_field(v[k][p].re), exp_field(v[k][p].im)));
       }
-      cpx* out = U + (size_t)y * gsz.X();
-      out[0] = cpx{ur, ui};
-      out[cs] = cpx{0.0, 0.0};
-      out[2 * cs] = cpx{wr, wi};
-      out[3 * cs] = cpx{dur, dui};
-      out[4 * cs] = cpx{dwr, dwi};
+#pragma unroll
+    for (int o = 16; o >= TILE; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if ((threadIdx.x & 31) < TILE) atomicMax(&exc[cls * TILE + col], e);
+    __syncthreads();
+    const int ex = exc[cls * TILE + col] - 1022;
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+      const int j = j0 + 64 * k;
+      if (j >= KT * 16) break;
+      uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * NC + 2 * col) * KS + j);
+      digits_pair(scaled56(v[k][0].re, ex), scaled56(v[k][1].re, ex), d, (size_t)NC * KS / 2);
+      digits_pair(scaled56(v[k][0].im, ex), scaled56(v[k][1].im, ex), d + KS / 2, (size_t)NC * KS / 2);
+    }
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
+  const uint4* __restrict__ A = reinterpret_cast<const uint4*>(g.tcA) + lane;
+  const size_t cs = (size_t)gsz.Q() * gsz.X();
+  const int x = x0 + min(t, nx - 1);
+  const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
+  const uint32_t base0 = tc_row_addr(dig, KS, (size_t)NC * KS, 0, lane);
+  const uint32_t cls_bytes = (uint32_t)(2 * kDig * NC * KS);
+  // items: (Q', R) of every row tile, (Q'', R'), then Q
+  const int nit = 3 * MT;
+  auto table = [&](int item, int part) {
+    const int grp = item / MT, mt = item - grp * MT, b = grp == 0 ? (part ? 3 : 1) : (grp == 1 ? (part ? 4 : 2) : 0);
+    return A + ((size_t)b * MT + mt) * KT * kFragStep;
+  };
+  FragPair pf;
+  if (warp < nit) tc_stream_start(pf, table(warp, 0));
+  for (int item = warp; item < nit; item += NTHR / 32) {
+    const int grp = item / MT, mt = item - grp * MT, nxt = item + NTHR / 32;
+    const int nparts = grp < 2 ? 2 : 1;
+    cpx val[2][2];
+    for (int part = 0; part < nparts; ++part) {
+      const int b = grp == 0 ? (part ? 3 : 1) : (grp == 1 ? (part ? 4 : 2) : 0), cls = b < 3 ? 0 : 1;
+      const uint4* next = part + 1 < nparts ? table(item, 1) : (nxt < nit ? table(nxt, 0) : nullptr);
+      long long T[4];
+      tc_tile_stream(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T);
+      const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kFoldShift;
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {
+        const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
+        const cpx v = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
+        if (part) val[1][rr] = v;
+        else val[0][rr] = v;
+      }
+    }
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const int y = mt * 16 + gq + 8 * rr;
+      if (y >= gsz.Q() || t >= nx) continue;
+      cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
+      if (meancol && t == 0 && grp < 2) {
+        out[grp == 0 ? 0 : 3 * cs] = cpx{val[1][rr].re, 0.0};
+        out[grp == 0 ? 2 * cs : 4 * cs] = cpx{val[1][rr].im, 0.0};
+      } else if (grp == 0) recon_velocity(ax, az, val[0][rr], val[1][rr], out[0], out[2 * cs]);
+      else if (grp == 1) recon_derivative(ax, az, val[0][rr], val[1][rr], out[3 * cs], out[4 * cs]);
+      else out[cs] = val[0][rr];
     }
   }
 }
@@ -353,8 +466,20 @@ static void launch_recon_sizes(const Grid& g, const ReconArgs& a, cudaStream_t s
   else k_recon_tc<false, S><<<dim3(g.Nz * ntx, a.ninst), kThreads, sm, st>>>(g, a);
 }
 
-// Grid::fixed & FIXED_RECON: the build compiled for the grid's sizes
+// Grid::fixed & FIXED_RECON: the build compiled for the grid's sizes; launches
+// of at most kFewTiles 4-column tiles (two waves of one block per SM) take
+// k_recon_few, unless CHN_RECON_BUILD asked for a build
 cudaError_t launch_recon_tc(const Grid& g, const ReconArgs& a, cudaStream_t st) {
+  const int ntf = g.Nz * ((g.X + 3) / 4);
+  if (!a.grids && !g.rfixed && g.R > 16 && g.R <= 128 && (long long)ntf * a.ninst <= kFewTiles) {
+    const dim3 grid(ntf, a.ninst);
+    const size_t sm = recon_tc_smem_bytes(g, 4);
+    if (sizes_match<Sizes32>(g)) k_recon_few<Sizes32, 1><<<grid, 256, sm, st>>>(g, a);
+    else if (sizes_match<Sizes16>(g)) k_recon_few<Sizes16, 1><<<grid, 256, sm, st>>>(g, a);
+    else if (g.R <= 64) k_recon_few<SizesRT, 1><<<grid, 256, sm, st>>>(g, a);
+    else k_recon_few<SizesRT, 2><<<grid, 256, sm, st>>>(g, a);
+    return cudaGetLastError();
+  }
   const bool fx = (g.fixed & FIXED_RECON) && !a.grids;
   if (fx && sizes_match<Sizes32>(g)) launch_recon_sizes<Sizes32>(g, a, st);
   else if (fx && sizes_match<Sizes16>(g)) launch_recon_sizes<Sizes16>(g, a, st);
@@ -363,6 +488,10 @@ cudaError_t launch_recon_tc(const Grid& g, const ReconArgs& a, cudaStream_t st) 
 }
 
 void prepare_recon_tc(int optin) {
+  allow_max_smem(k_recon_few<Sizes32, 1>, optin);
+  allow_max_smem(k_recon_few<Sizes16, 1>, optin);
+  allow_max_smem(k_recon_few<SizesRT, 1>, optin);
+  allow_max_smem(k_recon_few<SizesRT, 2>, optin);
   allow_max_smem(k_recon_tc<false, SizesRT>, optin);
   allow_max_smem(k_recon_tc<true, SizesRT>, optin);
   allow_max_smem(k_recon_tc<false, Sizes32>, optin);
