@@ -18,6 +18,8 @@
 //   H_bar = Quad^T(F_bar)  (written pre-scaled for the inverse transform),
 // and the products kernel (k_products_adj with `exact`) takes H_bar's
 // physical fields to u_in_bar.
+#include <type_traits>
+
 #include "chn_common.cuh"
 #include "few_tile.cuh"
 #include "kernels.h"
@@ -63,86 +65,80 @@ __device__ __forceinline__ cpx band_matvecT_row(const double* __restrict__ A, in
 // A^T y = b for one parity chain, A = L U the no-pivot factors of
 // channel/mvOps.c:29-91 (L unit lower in columns j < dl, U in dl..dl+du):
 // U^T w = b ascending, then L^T y = w descending; RD the reciprocal pivots
-// (the forward chain multiplies by them too).  The last results stay in
-// registers, the next rows' factors load meanwhile (as band_solve_chain).
-template <int W, int DL, int DU, bool GLOBAL>
+// (the forward chain multiplies by them too).  As band_solve_chain.
+template <int W, int DL, int DU>
 __device__ __forceinline__ void band_solveT_chain(const double* __restrict__ LU, const double* __restrict__ RD, int N,
-                                                  int par, double* b, int bstride) {
+                                   int par, double* b, int bstride) {
   const int M = (N - par + 1) / 2;  // rows of this parity: i = par + 2 m
   if (M <= 0) return;
   constexpr int G = kChainRows;
   {
-    double f[G][DU], v[G], p[G], x[DU];
-    auto load = [&](int m0) {
+    // f[q][t]: what the result of row n0 + q subtracts from the row t + 1 further on
+    double f[G][DU], v[G], p[G], acc[DU];
+    auto load = [&](int n0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        const int m = min(m0 + q, M - 1), i = par + 2 * m;
+        const int m = min(n0 + q, M - 1);
 #pragma unroll
-        for (int j = 1; j <= DU; ++j)
-          f[q][j - 1] = band_load<GLOBAL>(LU + (size_t)(par + 2 * max(m - j, 0)) * W + DL + j);
-        p[q] = band_load<GLOBAL>(RD + i);
-        v[q] = b[i * bstride];
+        for (int t = 1; t <= DU; ++t) f[q][t - 1] = __ldg(LU + (size_t)(par + 2 * m) * W + DL + t);
+        p[q] = __ldg(RD + par + 2 * m);
+        v[q] = b[(par + 2 * min(m + DU, M - 1)) * bstride];
       }
     };
 #pragma unroll
-    for (int t = 0; t < DU; ++t) x[t] = 0.0;  // x[t]: the result t + 1 rows back
+    for (int t = 0; t < DU; ++t) acc[t] = b[(par + 2 * min(t, M - 1)) * bstride];
     load(0);
-    for (int m0 = 0; m0 < M; m0 += G) {
+    for (int n0 = 0; n0 < M; n0 += G) {
       double c[G][DU], w[G], r[G];
 #pragma unroll
       for (int q = 0; q < G; ++q) {
 #pragma unroll
-        for (int j = 0; j < DU; ++j) c[q][j] = f[q][j];
+        for (int t = 0; t < DU; ++t) c[q][t] = f[q][t];
         w[q] = v[q];
         r[q] = p[q];
       }
-      load(m0 + G);
+      load(n0 + G);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        double acc = w[q];
+        const double x = acc[0] * r[q];
 #pragma unroll
-        for (int j = DU - 1; j >= 0; --j) acc = fma(-c[q][j], x[j], acc);
-        acc *= r[q];
-#pragma unroll
-        for (int t = DU - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (m0 + q < M) b[(par + 2 * (m0 + q)) * bstride] = acc;
+        for (int t = 0; t + 1 < DU; ++t) acc[t] = fma(-c[q][t], x, acc[t + 1]);
+        acc[DU - 1] = fma(-c[q][DU - 1], x, w[q]);
+        if (n0 + q < M) b[(par + 2 * (n0 + q)) * bstride] = x;
       }
     }
   }
   {
-    double f[G][DL], v[G], x[DL];
-    auto load = [&](int n0) {  // rows from the last one down
+    // f[q][t]: what the result of row n0 + q subtracts from the row t + 1 further on
+    double f[G][DL], v[G], acc[DL];
+    auto load = [&](int n0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) {
         const int m = max(M - 1 - (n0 + q), 0);
 #pragma unroll
-        for (int t = 1; t <= DL; ++t)
-          f[q][t - 1] = band_load<GLOBAL>(LU + (size_t)(par + 2 * min(m + t, M - 1)) * W + DL - t);
-        v[q] = b[(par + 2 * m) * bstride];
+        for (int t = 1; t <= DL; ++t) f[q][t - 1] = __ldg(LU + (size_t)(par + 2 * m) * W + DL - t);
+        v[q] = b[(par + 2 * max(m - DL, 0)) * bstride];
       }
     };
 #pragma unroll
-    for (int t = 0; t < DL; ++t) x[t] = 0.0;
+    for (int t = 0; t < DL; ++t) acc[t] = b[(par + 2 * max(M - 1 - t, 0)) * bstride];
     load(0);
     for (int n0 = 0; n0 < M; n0 += G) {
       double c[G][DL], w[G];
 #pragma unroll
       for (int q = 0; q < G; ++q) {
 #pragma unroll
-        for (int j = 0; j < DL; ++j) c[q][j] = f[q][j];
+        for (int t = 0; t < DL; ++t) c[q][t] = f[q][t];
         w[q] = v[q];
       }
       load(n0 + G);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        double acc = w[q];
+        const double x = acc[0];
 #pragma unroll
-        for (int t = DL - 1; t >= 0; --t) acc = fma(-c[q][t], x[t], acc);
-#pragma unroll
-        for (int t = DL - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = acc;
+        for (int t = 0; t + 1 < DL; ++t) acc[t] = fma(-c[q][t], x, acc[t + 1]);
+        acc[DL - 1] = fma(-c[q][DL - 1], x, w[q]);
+        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = x;
       }
     }
   }
@@ -697,6 +693,40 @@ __device__ __forceinline__ void recon_T_few(const Grid& g, const S& gsz, const c
       s.Fa, s.Fb);
 }
 
+// the chains of a few-block tile (as solve_chains_few): U^T then L^T
+template <int TT, class S>
+__device__ __forceinline__ void solveT_chains_few(const Grid& g, const S& gsz, int bidx, int nx, int xfirst,
+                                                  const SolveTSmem& s) {
+  static_assert(TT == 4, "the thread map");
+  const int tid = threadIdx.x;
+  auto run = [&](auto nl, const double* LU, const double* RD, int W, int N, int par, bool on, double* b) {
+    constexpr int NL = decltype(nl)::value;
+    const int M = max((N - par + 1) / 2, 1), steps = (N + 1) / 2, l = tid & (NL - 1);
+    double* bp = b + (N > par ? par * 2 * TT : 0);
+    on = on && N > par;
+    chain_sweep<NL, false, true>(M, steps, l, on, bp, 4 * TT,
+                                 [&](int m, int t) { return LU[(size_t)(par + 2 * m) * W + NL + t]; },
+                                 [&](int m) { return RD[par + 2 * m]; });
+    __syncwarp();
+    chain_sweep<NL, true, false>(M, steps, l, on, bp, 4 * TT,
+                                 [&](int m, int t) { return LU[(size_t)(par + 2 * m) * W + NL - t]; },
+                                 [](int) { return 1.0; });
+  };
+  if (tid < 64) {
+    const int ch = tid / 4, l = ch / 4, lc = min(l, nx - 1);
+    run(std::integral_constant<int, 4>(), s.luA + (size_t)lc * gsz.D() * 9, s.rdA + (size_t)lc * gsz.D(), 9, gsz.D(),
+        ch & 1, l < nx && l >= xfirst, reinterpret_cast<double*>(s.ra + lc) + ((ch >> 1) & 1));
+  } else if (tid < 96) {
+    const int ch = (tid - 64) / 2, l = ch / 4, lc = min(l, nx - 1);
+    run(std::integral_constant<int, 2>(), s.luB + (size_t)lc * gsz.R() * 5, s.rdB + (size_t)lc * gsz.R(), 5, gsz.R(),
+        ch & 1, l < nx && l >= xfirst, reinterpret_cast<double*>(s.rb + lc) + ((ch >> 1) & 1));
+  } else if (tid < 128 && xfirst) {
+    const int ch = ((tid - 96) / 2) & 7;
+    run(std::integral_constant<int, 2>(), g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), 5, gsz.R(),
+        ch & 1, tid < 112, reinterpret_cast<double*>(ch < 4 ? s.ra : s.rb) + ((ch >> 1) & 1));
+  }
+}
+
 // Block z ntx + tx: kx tile tx of line z; the mean line is column 0 of the
 // kz = 0 line's first tile, its parts as Re and Im of the beta class (as in
 // k_solve).  S: the sizes (SizesRT, or SizesCT for a specialised grid); TT kx
@@ -854,28 +884,26 @@ __global__ void __launch_bounds__(kThreads, FEW ? 1 : 2) k_solve_T(const __grid_
     }
     __syncthreads();
   }
-  // L^{-T}: per column 4 chains for alpha, 4 for beta (parity x re/im), the
-  // alpha chains in threads [0, 4 TT), the beta ones from a warp boundary, the
-  // mean line's from the next
-  constexpr int kHalf = 4 * TT < 32 ? 32 : 4 * TT;
-  if (xfirst && (int)threadIdx.x >= 2 * kHalf) {
-    const int t = (int)threadIdx.x - 2 * kHalf;
-    if (t < 8)
-      band_solveT_chain<5, 2, 2, true>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), t & 1,
-                                       reinterpret_cast<double*>(t < 4 ? s.ra : s.rb) + ((t >> 1) & 1), 2 * TT);
+  if constexpr (FEW) {
+    solveT_chains_few<TT>(g, gsz, bidx, nx, xfirst, s);
   } else {
-    const bool beta = (int)threadIdx.x >= kHalf;
-    const int t = beta ? (int)threadIdx.x - kHalf : (int)threadIdx.x, l = t / 4, par = t & 1, part = (t >> 1) & 1;
-    if (t < 4 * TT && l < nx && l >= xfirst) {
+    // L^{-T}: per column 4 chains for alpha, 4 for beta (parity x re/im), the
+    // alpha chains in threads [0, 4 TT), the beta ones from a warp boundary, the
+    // mean line's from the next
+    constexpr int kHalf = 4 * TT;
+    const int sec = (int)threadIdx.x / kHalf, t = (int)threadIdx.x - sec * kHalf, l = t / 4;
+    const int par = t & 1, part = (t >> 1) & 1;
+    if (sec < 2 && l < nx && l >= xfirst) {
       const size_t sys = ((size_t)bidx * gsz.Nz() + z) * gsz.X() + x0 + l;
-      if (!beta)
-        band_solveT_chain<9, 4, 4, !FEW>(FEW ? s.luA + (size_t)l * gsz.D() * 9 : g.luA + sys * gsz.D() * 9,
-                                         FEW ? s.rdA + (size_t)l * gsz.D() : g.rdA + sys * gsz.D(), gsz.D(), par,
-                                         reinterpret_cast<double*>(s.ra + l) + part, 2 * TT);
+      if (sec == 0)
+        band_solveT_chain<9, 4, 4>(g.luA + sys * gsz.D() * 9, g.rdA + sys * gsz.D(), gsz.D(), par,
+                                   reinterpret_cast<double*>(s.ra + l) + part, 2 * TT);
       else
-        band_solveT_chain<5, 2, 2, !FEW>(FEW ? s.luB + (size_t)l * gsz.R() * 5 : g.luB + sys * gsz.R() * 5,
-                                         FEW ? s.rdB + (size_t)l * gsz.R() : g.rdB + sys * gsz.R(), gsz.R(), par,
-                                         reinterpret_cast<double*>(s.rb + l) + part, 2 * TT);
+        band_solveT_chain<5, 2, 2>(g.luB + sys * gsz.R() * 5, g.rdB + sys * gsz.R(), gsz.R(), par,
+                                   reinterpret_cast<double*>(s.rb + l) + part, 2 * TT);
+    } else if (sec == 2 && xfirst && t < 8) {
+      band_solveT_chain<5, 2, 2>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), par,
+                                 reinterpret_cast<double*>(t < 4 ? s.ra : s.rb) + part, 2 * TT);
     }
   }
   __syncthreads();

@@ -30,7 +30,49 @@ __device__ __forceinline__ void stage_factors(const Grid& g, const S& gsz, size_
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// bf16-table contractions over the planes of a 4-column tile, all inputs at
+// One sweep over the M rows of an elimination chain by a group of NL lanes
+// (NL: the band's reach), rows ascending or (DOWN) descending.  An FP64 warp
+// instruction occupies its scheduler's FP64 unit for some 70 cycles however
+// few lanes are active, so a lane per chain waits for every multiply-add of
+// every row (279 a chain of the alpha band at 32x65x32: 23k cycles); here lane
+// l of the group owns the rows congruent to l, a row's result goes to the
+// group by shuffles and ONE multiply-add updates the next NL rows (8k).
+// coef(m, t): what row m's result subtracts from the row t further on; scale(m):
+// the pivot's reciprocal (SCALE).  steps: the longest chain's rows of the warp
+// (every lane takes part in every shuffle); on: the group's stores.
+template <int NL, bool DOWN, bool SCALE, class Coef, class Scale>
+__device__ __forceinline__ void chain_sweep(int M, int steps, int l, bool on, double* b, int bstride, Coef coef,
+                                            Scale scale) {
+  auto row = [&](int n) { return min(max(DOWN ? M - 1 - n : n, 0), M - 1); };
+  double acc = b[row(l) * bstride];
+  double cf[NL], nb = 0.0, sc = 0.0;
+  auto load = [&](int n0) {  // the group's values for steps n0 .. n0 + NL - 1
+#pragma unroll
+    for (int s = 0; s < NL; ++s) cf[s] = coef(row(n0 + s), NL - ((s - l) & (NL - 1)));
+    nb = b[row(n0 + l + NL) * bstride];
+    if (SCALE) sc = scale(row(n0 + l));
+  };
+  load(0);
+  for (int n0 = 0; n0 < steps; n0 += NL) {
+    double c[NL];
+#pragma unroll
+    for (int s = 0; s < NL; ++s) c[s] = cf[s];
+    const double bn = nb, rs = sc;
+    load(n0 + NL);
+#pragma unroll
+    for (int s = 0; s < NL; ++s) {
+      const double v = SCALE ? acc * rs : acc;
+      const double x = __shfl_sync(0xffffffffu, v, s, NL);
+      if (l == s) {
+        if (on && n0 + s < M) b[row(n0 + s) * bstride] = x;
+        acc = bn;
+      }
+      acc = fma(-c[s], x, acc);
+    }
+  }
+}
+
+// Digit-table contractions over the planes of a 4-column tile, all inputs at
 // once: load(y, o) gives the thread's column's inputs o[0..4] at plane y (o[2]
 // and o[4] only with `all`); table w(q) of input q (digit tables Wt
 // [5][ceil(R/16)][KT][7][32][4], exponents WE [5][R]); inputs 0..2 sum into Fa

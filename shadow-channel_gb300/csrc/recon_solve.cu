@@ -13,6 +13,8 @@
 // (-1)^(n+1), so for the plane pair (y, -y) a contraction splits into an
 // even-index sum E and an odd-index sum O with values E +- O.  This halves
 // the FP64 multiply-adds of every quadrature and reconstruction.
+#include <type_traits>
+
 #include "chn_common.cuh"
 #include "kernels.h"
 #include "solve_common.cuh"
@@ -578,15 +580,15 @@ __device__ void quad_rhs_few(const Grid& g, const S& gsz, const cpx* __restrict_
 // the banded solves of a tile: per column 4 chains for alpha, 4 for beta
 // (parity x re/im), threads [0, 4 kTile) the alpha chains, as many from a
 // warp boundary the beta ones: a warp holds one system (no divergence between
-// the two bands).  GLOBAL: factors from global memory, else the staged ones.
-template <int kTile, bool GLOBAL, class S>
+// the two bands).
+template <int kTile, class S>
 __device__ __forceinline__ void solve_chains(const Grid& g, const S& gsz, int bidx, int z, int x0, int nx, int xfirst,
                                              const SolveSmem& s) {
   constexpr int kHalf = 4 * kTile < 32 ? 32 : 4 * kTile;
   if (xfirst && (int)threadIdx.x >= 2 * kHalf) {  // the mean line's two, in a warp of their own
     const int t = (int)threadIdx.x - 2 * kHalf;
     if (t < 8)
-      band_solve_chain<5, 2, 2, true>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), t & 1,
+      band_solve_chain<5, 2, 2>(g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), gsz.R(), t & 1,
                                       reinterpret_cast<double*>(t < 4 ? s.ra : s.rb) + ((t >> 1) & 1), 2 * kTile);
     return;
   }
@@ -595,13 +597,44 @@ __device__ __forceinline__ void solve_chains(const Grid& g, const S& gsz, int bi
   if (t >= 4 * kTile || l >= nx || l < xfirst) return;
   const size_t sys = ((size_t)bidx * gsz.Nz() + z) * gsz.X() + x0 + l;
   if (!beta)
-    band_solve_chain<9, 4, 4, GLOBAL>(GLOBAL ? g.luA + sys * gsz.D() * 9 : s.luA + (size_t)l * gsz.D() * 9,
-                                      GLOBAL ? g.rdA + sys * gsz.D() : s.rdA + (size_t)l * gsz.D(), gsz.D(), par,
-                                      reinterpret_cast<double*>(s.ra + l) + part, 2 * kTile);
+    band_solve_chain<9, 4, 4>(g.luA + sys * gsz.D() * 9, g.rdA + sys * gsz.D(), gsz.D(), par,
+                              reinterpret_cast<double*>(s.ra + l) + part, 2 * kTile);
   else
-    band_solve_chain<5, 2, 2, GLOBAL>(GLOBAL ? g.luB + sys * gsz.R() * 5 : s.luB + (size_t)l * gsz.R() * 5,
-                                      GLOBAL ? g.rdB + sys * gsz.R() : s.rdB + (size_t)l * gsz.R(), gsz.R(), par,
-                                      reinterpret_cast<double*>(s.rb + l) + part, 2 * kTile);
+    band_solve_chain<5, 2, 2>(g.luB + sys * gsz.R() * 5, g.rdB + sys * gsz.R(), gsz.R(), par,
+                              reinterpret_cast<double*>(s.rb + l) + part, 2 * kTile);
+}
+
+// the same for the few-block build: chains of four lanes (alpha, warps 0 and
+// 1) and of two (beta, warp 2; the mean line's, warp 3), the factors staged
+template <int kTile, class S>
+__device__ __forceinline__ void solve_chains_few(const Grid& g, const S& gsz, int bidx, int nx, int xfirst,
+                                                 const SolveSmem& s) {
+  static_assert(kTile == 4, "the thread map");
+  const int tid = threadIdx.x;
+  auto run = [&](auto nl, const double* LU, const double* RD, int W, int N, int par, bool on, double* b) {
+    constexpr int NL = decltype(nl)::value;
+    const int M = max((N - par + 1) / 2, 1), steps = (N + 1) / 2, l = tid & (NL - 1);
+    double* bp = b + (N > par ? par * 2 * kTile : 0);
+    on = on && N > par;
+    chain_sweep<NL, false, false>(M, steps, l, on, bp, 4 * kTile, [&](int m, int t) {
+      return LU[(size_t)(par + 2 * min(m + t, M - 1)) * W + NL - t]; }, [](int) { return 1.0; });
+    __syncwarp();
+    chain_sweep<NL, true, true>(M, steps, l, on, bp, 4 * kTile, [&](int m, int t) {
+      return LU[(size_t)(par + 2 * max(m - t, 0)) * W + NL + t]; }, [&](int m) { return RD[par + 2 * m]; });
+  };
+  if (tid < 64) {
+    const int ch = tid / 4, l = ch / 4, lc = min(l, nx - 1);
+    run(std::integral_constant<int, 4>(), s.luA + (size_t)lc * gsz.D() * 9, s.rdA + (size_t)lc * gsz.D(), 9, gsz.D(),
+        ch & 1, l < nx && l >= xfirst, reinterpret_cast<double*>(s.ra + lc) + ((ch >> 1) & 1));
+  } else if (tid < 96) {
+    const int ch = (tid - 64) / 2, l = ch / 4, lc = min(l, nx - 1);
+    run(std::integral_constant<int, 2>(), s.luB + (size_t)lc * gsz.R() * 5, s.rdB + (size_t)lc * gsz.R(), 5, gsz.R(),
+        ch & 1, l < nx && l >= xfirst, reinterpret_cast<double*>(s.rb + lc) + ((ch >> 1) & 1));
+  } else if (tid < 128 && xfirst) {
+    const int ch = ((tid - 96) / 2) & 7;
+    run(std::integral_constant<int, 2>(), g.lu0 + (size_t)bidx * gsz.R() * 5, g.rd0 + (size_t)bidx * gsz.R(), 5, gsz.R(),
+        ch & 1, tid < 112, reinterpret_cast<double*>(ch < 4 ? s.ra : s.rb) + ((ch >> 1) & 1));
+  }
 }
 
 // The (kx, kz) = (0, 0) line (channel/project0.c, increproject0.c,
@@ -704,7 +737,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
       s.rb[r * kTile + l] = cpx{re2 * w.re, re2 * w.im};
     }
     __syncthreads();
-    solve_chains<kTile, true>(g, gsz, 2, z, x0, nx, xfirst, s);  // mass matrices: the b = 0 factors
+    solve_chains<kTile>(g, gsz, 2, z, x0, nx, xfirst, s);  // mass matrices: the b = 0 factors
     __syncthreads();
     for (int i = threadIdx.x; i < gsz.R() * kTile; i += NTHR) {
       const int r = i / kTile, l = i - r * kTile;
@@ -805,7 +838,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_solve(const __grid_constant__ Gr
     s.rb[r * kTile + l] = vb;
   }
   __syncthreads();
-  solve_chains<kTile, !FEW>(g, gsz, rk.bidx, z, x0, nx, xfirst, s);
+  if constexpr (FEW) solve_chains_few<kTile>(g, gsz, rk.bidx, nx, xfirst, s);
+  else solve_chains<kTile>(g, gsz, rk.bidx, z, x0, nx, xfirst, s);
   __syncthreads();
   if (xfirst) {
     // constant mass flux: a += 0.5 * flux_t * add (channel/project0.c:153-168), warp 0

@@ -51,96 +51,87 @@ __device__ __forceinline__ cpx band_matvec_row(const double* __restrict__ A, int
 
 // One elimination chain (fixed parity, real or imaginary part) of the
 // no-pivot every-other-diagonal LU solve (channel/mvOps.c:29-91); W, DL, DU
-// the band layout (width, lower, upper), RD the reciprocal pivots; entries
-// outside the matrix are zero.  The last DL or DU results stay in registers
-// and the multiply-adds run from the oldest to the newest, so a row waits for
-// one multiply-add (and the pivot's product) of the row before it.  The
-// factors of the next kChainRows rows load while a group's rows run (GLOBAL:
-// from global memory; else they are staged in shared memory): 32x65x32, one
-// instance, 36k -> 9k cycles of a block's 260k.
+// the band layout (width, lower, upper), RD the reciprocal pivots.  Each
+// result is subtracted at once from the next DL or DU rows' running values,
+// which stay in registers (the same order per row as the reference's forward
+// elimination); rows past the end subtract into values nothing reads.  The
+// factors of the next kChainRows rows load while a group's rows run: 36k -> 23k
+// cycles at 32x65x32, the FP64 unit's time for the chain's 279 operations.
 static constexpr int kChainRows = 4;
 
-template <bool GLOBAL>
-__device__ __forceinline__ double band_load(const double* p) {
-  return GLOBAL ? __ldg(p) : *p;
-}
-
-template <int W, int DL, int DU, bool GLOBAL>
+template <int W, int DL, int DU>
 __device__ __forceinline__ void band_solve_chain(const double* __restrict__ LU, const double* __restrict__ RD, int N,
-                                                 int par, double* b, int bstride) {
+                                   int par, double* b, int bstride) {
   const int M = (N - par + 1) / 2;  // rows of this parity: i = par + 2 m
   if (M <= 0) return;
   constexpr int G = kChainRows;
   {
-    double f[G][DL], v[G], x[DL];
-    auto load = [&](int m0) {
+    // f[q][t]: what the result of row n0 + q subtracts from the row t + 1 further on
+    double f[G][DL], v[G], acc[DL];
+    auto load = [&](int n0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        const int i = par + 2 * min(m0 + q, M - 1);
+        const int m = min(n0 + q, M - 1);
 #pragma unroll
-        for (int j = 0; j < DL; ++j) f[q][j] = band_load<GLOBAL>(LU + (size_t)i * W + j);
-        v[q] = b[i * bstride];
+        for (int t = 1; t <= DL; ++t) f[q][t - 1] = __ldg(LU + (size_t)(par + 2 * min(m + t, M - 1)) * W + DL - t);
+        v[q] = b[(par + 2 * min(m + DL, M - 1)) * bstride];
       }
     };
 #pragma unroll
-    for (int t = 0; t < DL; ++t) x[t] = 0.0;  // x[t]: the result t + 1 rows back
+    for (int t = 0; t < DL; ++t) acc[t] = b[(par + 2 * min(t, M - 1)) * bstride];
     load(0);
-    for (int m0 = 0; m0 < M; m0 += G) {
+    for (int n0 = 0; n0 < M; n0 += G) {
       double c[G][DL], w[G];
 #pragma unroll
       for (int q = 0; q < G; ++q) {
 #pragma unroll
-        for (int j = 0; j < DL; ++j) c[q][j] = f[q][j];
+        for (int t = 0; t < DL; ++t) c[q][t] = f[q][t];
         w[q] = v[q];
       }
-      load(m0 + G);
+      load(n0 + G);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        double acc = w[q];
+        const double x = acc[0];
 #pragma unroll
-        for (int j = 0; j < DL; ++j) acc = fma(-c[q][j], x[DL - 1 - j], acc);
-#pragma unroll
-        for (int t = DL - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (m0 + q < M) b[(par + 2 * (m0 + q)) * bstride] = acc;
+        for (int t = 0; t + 1 < DL; ++t) acc[t] = fma(-c[q][t], x, acc[t + 1]);
+        acc[DL - 1] = fma(-c[q][DL - 1], x, w[q]);
+        if (n0 + q < M) b[(par + 2 * (n0 + q)) * bstride] = x;
       }
     }
   }
   {
-    double f[G][DU], v[G], p[G], x[DU];
-    auto load = [&](int n0) {  // rows from the last one down
+    // f[q][t]: what the result of row n0 + q subtracts from the row t + 1 further on
+    double f[G][DU], v[G], p[G], acc[DU];
+    auto load = [&](int n0) {
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        const int i = par + 2 * max(M - 1 - (n0 + q), 0);
+        const int m = max(M - 1 - (n0 + q), 0);
 #pragma unroll
-        for (int j = 0; j < DU; ++j) f[q][j] = band_load<GLOBAL>(LU + (size_t)i * W + DL + 1 + j);
-        p[q] = band_load<GLOBAL>(RD + i);
-        v[q] = b[i * bstride];
+        for (int t = 1; t <= DU; ++t) f[q][t - 1] = __ldg(LU + (size_t)(par + 2 * max(m - t, 0)) * W + DL + t);
+        p[q] = __ldg(RD + par + 2 * m);
+        v[q] = b[(par + 2 * max(m - DU, 0)) * bstride];
       }
     };
 #pragma unroll
-    for (int t = 0; t < DU; ++t) x[t] = 0.0;
+    for (int t = 0; t < DU; ++t) acc[t] = b[(par + 2 * max(M - 1 - t, 0)) * bstride];
     load(0);
     for (int n0 = 0; n0 < M; n0 += G) {
       double c[G][DU], w[G], r[G];
 #pragma unroll
       for (int q = 0; q < G; ++q) {
 #pragma unroll
-        for (int j = 0; j < DU; ++j) c[q][j] = f[q][j];
+        for (int t = 0; t < DU; ++t) c[q][t] = f[q][t];
         w[q] = v[q];
         r[q] = p[q];
       }
       load(n0 + G);
 #pragma unroll
       for (int q = 0; q < G; ++q) {
-        double acc = w[q];
+        const double x = acc[0] * r[q];
 #pragma unroll
-        for (int j = DU - 1; j >= 0; --j) acc = fma(-c[q][j], x[j], acc);
-        acc *= r[q];
-#pragma unroll
-        for (int t = DU - 1; t > 0; --t) x[t] = x[t - 1];
-        x[0] = acc;
-        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = acc;
+        for (int t = 0; t + 1 < DU; ++t) acc[t] = fma(-c[q][t], x, acc[t + 1]);
+        acc[DU - 1] = fma(-c[q][DU - 1], x, w[q]);
+        if (n0 + q < M) b[(par + 2 * (M - 1 - (n0 + q))) * bstride] = x;
       }
     }
   }
