@@ -228,12 +228,12 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   const bool fixed_on = (fx && fx[0]) ? fx[0] == '1' : spec;
   g.fixed = fixed_on ? (FIXED_PRODUCTS | FIXED_RECON | FIXED_SOLVE) : 0;
   // the inverse's build (phys_tc.cu) until a batch's autotuner has timed
-  // them: two fields per pass (the single trajectory's plane count gives a
-  // block per plane), compiled for the grid's sizes where it has them;
+  // them: one field per block, compiled for the grid's sizes where it has
+  // them;
   // CHN_INVERSE_BUILD=2..7 fixes it (and skips that timing)
   const char* ib = getenv("CHN_INVERSE_BUILD");
   const int ibv = ib ? atoi(ib) : 0;
-  g.tcminb = (ibv >= 2 && ibv <= 12) ? ibv : (spec ? 7 : 2);
+  g.tcminb = (ibv >= 2 && ibv <= 12) ? ibv : (spec ? 11 : 4);
   // the adjoint products' planes per pass: 1 until the autotuner has timed
   // 1 and 3; CHN_ADJ_PRODUCTS_PER_PASS=1 or 3 fixes it
   const char* apb = getenv("CHN_ADJ_PRODUCTS_PER_PASS");
@@ -844,7 +844,8 @@ static bool enqueue_adjoint_step(Engine& e, Work& w, double strength_dt, bool ca
     a.pslot = scur;
     a.H = mb(w.Up, w.usz);
     // the two passes read the same adjoint fields and write apart: branches
-    const bool conc = k < 2 && chains_concurrent(e);
+    // (not where they would share the scratch array)
+    const bool conc = k < 2 && chains_concurrent(e) && products_groups(g, a, 2) == 1;
     if (conc && !fork_to(e, st, e.st2, 0)) return false;
     LK(launch_products_adj(g, a, st));
     if (k < 2) {

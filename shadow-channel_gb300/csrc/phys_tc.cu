@@ -203,6 +203,36 @@ __host__ __device__ constexpr size_t phys_tc_dbuf_of(const PhysTcDims& d) {
              : (size_t)kDig * ((d.NX + 7) / 8 * 8) * d.KSx * 2;
 }
 
+// block maximum of the CFL field of plane y (channel/pass1.c:116-138), from
+// the written velocity fields
+template <int NTHR>
+__device__ __forceinline__ void plane_cfl(const Grid& g, const PhysArgs& a, const double* P, int inst, int y, int Q,
+                                          int plane) {
+  __shared__ double red[NTHR];
+  double mx = 0.0;
+  const double* Pu = P + (size_t)y * plane;
+  const size_t fs = (size_t)Q * plane;
+  const double c2 = g.cfl2[y];
+  for (int i = threadIdx.x; i < plane; i += NTHR)
+    mx = fmax(mx, fabs(Pu[i]) * g.cfl1 + fabs(Pu[fs + i]) * c2 + fabs(Pu[2 * fs + i]) * g.cfl3);
+  red[threadIdx.x] = mx;
+  __syncthreads();
+  constexpr int P2 = NTHR >= 256 ? 256 : (NTHR >= 128 ? 128 : 64);  // largest power of 2 <= NTHR
+  if (P2 < NTHR && threadIdx.x < NTHR - P2) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + P2]);
+  if (P2 < NTHR) __syncthreads();
+  for (int w = P2 / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    const double c = red[0] * g.dt;
+    if (a.cflmax)
+      atomicMax(reinterpret_cast<unsigned long long*>(&a.cflmax[inst / a.sdiv]),
+                (unsigned long long)__double_as_longlong(c));
+    if (c >= 2.8) atomicOr(&a.status[inst / a.sdiv], ST_CFL);
+  }
+}
+
 // FB fields per pass, NTHR threads, MINB blocks per SM (the register
 // budget), S the sizes (SizesRT, or SizesCT for a specialised grid)
 template <bool MULTI, int MINB, int FB, int NTHR, class S>
@@ -232,10 +262,13 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   const int Kk = gsz.Nz() - 1;  // kept kz rows
   const int chunk = gsz.tcch();
   bool nonfinite = false;
+  // this block's fields: all of them, or one of gridDim.z groups
+  const int fper = (a.nfields + gridDim.z - 1) / gridDim.z, fbeg = blockIdx.z * fper;
+  const int fend = min(a.nfields, fbeg + fper);
   for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
   __syncthreads();
-  for (int f0 = 0; f0 < a.nfields; f0 += FB) {
-    const int nfb = min(FB, a.nfields - f0);
+  for (int f0 = fbeg; f0 < fend; f0 += FB) {
+    const int nfb = min(FB, fend - f0);
     // ---- z stage: columns n = fl * X + x.  The inputs are staged in the Z
     // buffer (free until the z stage writes it: X (Nz - 1) <= pz X values per
     // field); each thread keeps one column (consecutive threads: consecutive
@@ -366,33 +399,17 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
     __syncthreads();
   }
   if (nonfinite && a.status) atomicOr(&a.status[inst / a.sdiv], ST_NONFINITE);
-  if (a.cfl_check) {
-    // block max of the CFL field (channel/pass1.c:116-138), from the written
-    // velocity fields (this block's own stores)
-    __shared__ double red[NTHR];
-    double mx = 0.0;
-    const double* Pu = P + (size_t)y * plane;
-    const size_t fs = (size_t)gsz.Q() * plane;
-    const double c2 = g.cfl2[y];
-    for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += NTHR)
-      mx = fmax(mx, fabs(Pu[i]) * g.cfl1 + fabs(Pu[fs + i]) * c2 + fabs(Pu[2 * fs + i]) * g.cfl3);
-    red[threadIdx.x] = mx;
-    __syncthreads();
-    constexpr int P2 = NTHR >= 256 ? 256 : (NTHR >= 128 ? 128 : 64);  // largest power of 2 <= NTHR
-    if (P2 < NTHR && threadIdx.x < NTHR - P2) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + P2]);
-    if (P2 < NTHR) __syncthreads();
-    for (int w = P2 / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const double c = red[0] * g.dt;
-      if (a.cflmax)
-        atomicMax(reinterpret_cast<unsigned long long*>(&a.cflmax[inst / a.sdiv]),
-                  (unsigned long long)__double_as_longlong(c));
-      if (c >= 2.8) atomicOr(&a.status[inst / a.sdiv], ST_CFL);
-    }
-  }
+  // (with the fields in groups, k_cfl follows)
+  if (a.cfl_check && gridDim.z == 1) plane_cfl<NTHR>(g, a, P, inst, y, gsz.Q(), gsz.pz() * gsz.px());
+}
+
+// The CFL check of a launch whose fields ran in groups, one block per plane
+__global__ void __launch_bounds__(kThreads) k_cfl(const __grid_constant__ Grid g, PhysArgs a) {
+  const int inst = blockIdx.y, y = blockIdx.x;
+  if (a.skip_blocked && blocked(a.status, a.sdiv, inst)) return;
+  double* __restrict__ P = a.P.at(inst);
+  if (a.pslot.stride) P += (long long)a.pslot.slot() * a.pslot.stride;
+  plane_cfl<kThreads>(g, a, P, inst, y, g.Q, g.pz * g.px);
 }
 
 // ---------------------------------------------------------------------------
@@ -498,11 +515,13 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
   const uint4* __restrict__ Az = reinterpret_cast<const uint4*>(g.tcFZ);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
   constexpr int nwarp = kThreads >> 5;
-  const int ncomp = mode >= 2 ? 6 : 3;
+  // this block's components: all of them, or one of gridDim.z groups
+  const int nall = mode >= 2 ? 6 : 3, qper = (nall + gridDim.z - 1) / gridDim.z, qbeg = blockIdx.z * qper;
+  const int ncomp = min(nall, qbeg + qper);
   const int chunk = gsz.tcch();
-  const size_t xstride = (size_t)XCH * d.KSx, zstride = (size_t)d.Xp * d.KSz;  // bf16 between digits
-  for (int q = 0; q < ncomp; ++q) {
-    const int c = q % pb;
+  const size_t xstride = (size_t)XCH * d.KSx, zstride = (size_t)d.Xp * d.KSz;  // 16-bit words between digits
+  for (int q = qbeg; q < ncomp; ++q) {
+    const int c = (q - qbeg) % pb;
     double* stage = stage3 + (size_t)c * plane;
     longlong2* Yb = reinterpret_cast<longlong2*>(stage);  // Re, Im of Y[zp][kx]: t 2^(AxE[2 kx (+ 1)] + ysum_exp(exx[zp]))
     int* exx = exx3 + c * exs;
@@ -620,10 +639,28 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
       const int kk = rco.r, x = rco.c;
       const int z = kk < gsz.Nz() / 2 ? kk : kk + 1;
       if (mode < 2) H[(((size_t)z * 5 + q) * gsz.Q() + y) * gsz.X() + x] = Fb[i];
+      else if (gridDim.z > 1) a.tmp[((((size_t)inst * 6 + q) * gsz.Nz() + z) * gsz.Q() + y) * gsz.X() + x] = Fb[i];
       else assemble_stage(g, mode == 3, H, z, y, x, q, Fb[i]);
     }
     __syncthreads();
   }
+}
+
+// the adjoint modes' output slots from the six components' spectra of a
+// launch that ran them in groups (k_products_tc, gridDim.z > 1)
+__global__ void __launch_bounds__(kThreads) k_assemble(const __grid_constant__ Grid g, ProdArgs a, int exact) {
+  const int inst = blockIdx.y, z = blockIdx.z < g.Nz / 2 ? blockIdx.z : blockIdx.z + 1;
+  if (blocked(a.status, a.sdiv, inst)) return;
+  cpx* __restrict__ H = a.H.at(inst);
+  const int i = blockIdx.x * kThreads + threadIdx.x;
+  if (i >= g.Q * g.X) return;
+  const cpx* F = a.tmp + (((size_t)inst * 6) * g.Nz + z) * g.Q * g.X + i;
+  cpx v[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) v[q] = F[(size_t)q * g.Nz * g.Q * g.X];
+  const int y = i / g.X, x = i - y * g.X;
+#pragma unroll
+  for (int q = 0; q < 6; ++q) assemble_stage(g, exact != 0, H, z, y, x, q, v[q]);
 }
 
 // The forward products' shared-memory plan: product planes per pass of the
@@ -674,9 +711,34 @@ static void launch_products_b3(const Grid& g, const ProdArgs& a, int mode, cudaS
   k_products_tc<false, 2, S, 3><<<grid, kThreads, sm, st>>>(g, a, mode);
 }
 
+// The products' launches of few planes likewise: one component per block, the
+// adjoint modes through the scratch array and k_assemble.  Forward modes up to
+// 4 planes per SM (one instance at 32x65x32 40 -> 25 us, 8 of 16x33x16 39 -> 31;
+// 8 of 48x97x48, 7.6 per SM, 699 -> 726), adjoint modes up to 3 (76 -> 41, 64 ->
+// 53; 4 of 48x97x48, 3.8 per SM, 685 -> 719).
+int products_groups(const Grid& g, const ProdArgs& a, int mode) {
+  const long long planes = (long long)g.Q * a.ninst;
+  if (a.grids) return 1;
+  if (mode < 2) return planes <= 4 * 152 ? 3 : 1;
+  return planes <= 3 * 152 && a.tmp && a.ninst <= a.tmp_inst ? 6 : 1;
+}
+
 // Grid::fixed & FIXED_PRODUCTS: the build compiled for the grid's sizes
 // (32x65x32, 16x33x16; single-grid batches), else the run-time sizes
 cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st) {
+  const int groups = products_groups(g, a, mode);
+  if (groups > 1) {
+    const FwdTcDims d = fwd_tc_dims(g);
+    const dim3 grid(g.Q, a.ninst, groups);
+    const int xch = g.fxch < d.pzp ? g.fxch : d.pzp;
+    const size_t sm = fwd_tc_smem_bytes(g, 1, xch);
+    if (xch == d.pzp && sizes_match<Sizes32>(g)) k_products_tc<false, 1, Sizes32><<<grid, kThreads, sm, st>>>(g, a, mode);
+    else if (xch == d.pzp && sizes_match<Sizes16>(g)) k_products_tc<false, 1, Sizes16><<<grid, kThreads, sm, st>>>(g, a, mode);
+    else k_products_tc<false, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
+    if (mode >= 2)
+      k_assemble<<<dim3((g.Q * g.X + kThreads - 1) / kThreads, a.ninst, g.Nz - 1), kThreads, 0, st>>>(g, a, mode == 3);
+    return cudaGetLastError();
+  }
   if (g.prodb == 1 && !a.grids) {
     const bool fx = (g.fixed & FIXED_PRODUCTS) != 0;
     if (fx && sizes_match<Sizes32>(g)) launch_products_b3<Sizes32>(g, a, mode, st);
@@ -698,6 +760,15 @@ bool phys_tc_fits(const Grid& g, int optin) {
   return kFB * g.X <= kThreads && phys_tc_smem_bytes(g, true, kFB) + 4096 <= (size_t)optin;
 }
 
+// Launches of few planes run a plane's fields in blocks of their own, FB
+// fields each, instead of one after another: up to kGroupPlanes planes (5 per
+// SM).  One instance at 32x65x32: 49 -> 23 us in one-field blocks, 10 of
+// 28x43x18 (4.2 per SM) 127 -> 105; 24 of 16x33x16 (7.7 per SM) 77 -> 84.
+static constexpr long long kGroupPlanes = 5 * 152;
+static int inverse_groups(const Grid& g, const PhysArgs& a, int fb) {
+  return !a.grids && (long long)g.Q * a.ninst <= kGroupPlanes ? (a.nfields + fb - 1) / fb : 1;
+}
+
 // Builds of the kernel (Grid::tcminb; the autotuner times them, the results
 // are identical): fields per pass, threads, blocks per SM (the register
 // budget) and the sizes, run-time (RT) or compiled for the grid (CT):
@@ -712,7 +783,8 @@ bool phys_tc_fits(const Grid& g, int optin) {
 // need fewer registers (96 at 5 blocks of 128 threads without spills).
 template <bool MULTI>
 static void launch_inverse_build(const Grid& g, const PhysArgs& a, cudaStream_t st) {
-  const dim3 grid(g.Q, a.ninst);
+  const int fb = (g.tcminb == 4 || g.tcminb == 5 || g.tcminb == 8) ? 1 : 2;
+  const dim3 grid(g.Q, a.ninst, inverse_groups(g, a, fb));
   const bool cfl = a.cfl_check != 0;
   const size_t s2 = phys_tc_smem_bytes(g, cfl, 2), s1 = phys_tc_smem_bytes(g, cfl, 1);
   using RT = SizesRT;
@@ -741,7 +813,7 @@ static bool inverse_ct_build(int b) { return b == 6 || b == 7 || b >= 9; }
 
 template <class S>
 static void launch_inverse_ct(const Grid& g, const PhysArgs& a, cudaStream_t st) {
-  const dim3 grid(g.Q, a.ninst);
+  const dim3 grid(g.Q, a.ninst, inverse_groups(g, a, g.tcminb == 7 ? 2 : 1));
   const bool cfl = a.cfl_check != 0;
   const size_t s1 = phys_tc_smem_bytes(g, cfl, 1);
   switch (g.tcminb) {
@@ -766,6 +838,7 @@ cudaError_t launch_phys_inverse_tc(const Grid& g, const PhysArgs& a, cudaStream_
     if (a.grids) launch_inverse_build<true>(gr, a, st);
     else launch_inverse_build<false>(gr, a, st);
   }
+  if (a.cfl_check && inverse_groups(g, a, 1) > 1) k_cfl<<<dim3(g.Q, a.ninst), kThreads, 0, st>>>(g, a);
   return cudaGetLastError();
 }
 
