@@ -221,6 +221,8 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   g.fwdpb = 3;
   g.fxch = 8;
   g.tcf = (tct_ok && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
+  // and as split tensor-core passes where a plane does not fit one block
+  g.tcs = (tct_ok && !(tfp64 && tfp64[0] == '1') && !(force && force[0] == '1') && phys_tcs_fits(g, optin)) ? 1 : 0;
   // the kernels' builds compiled for the grid's sizes where it has them
   // (a batch's autotuner then times both); CHN_FIXED_SIZES=0 / 1 fixes it
   const bool spec = phys_tc_specialised(g);
@@ -1148,6 +1150,7 @@ static bool autotune_transforms(Engine& e, Work& w) {
   const char* force = getenv("CHN_SPLIT_TRANSFORMS");
   if (force && force[0] == '1') return true;
   Grid& g = e.T.g;
+  if (g.tcs && !w.gdev && !(g.tci && g.tcf)) return true;  // (no choice among the split tensor-core passes)
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));

@@ -170,6 +170,15 @@ int tc5_take_error();
 // products + forward transforms as digit GEMMs (mode 0 primal, 1 tangent, 2 adjoint, 3 exact transpose)
 cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st);
 bool fwd_tc_fits(const Grid& g, int optin);
+// the same transforms as z and x passes through PhysArgs::tmp / ProdArgs::tmp, for
+// planes that do not fit one block (phys_tcs.cu; single-grid launches)
+bool phys_tcs_fits(const Grid& g, int optin);
+cudaError_t launch_phys_inverse_tcs(const Grid& g, const PhysArgs& a, cudaStream_t st);
+cudaError_t launch_products_tcs(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st);
+// pieces the two share: the CFL check from the written fields, the adjoint
+// modes' assembly of instances inst0 .. inst0 + n - 1 from the scratch array
+void launch_cfl(const Grid& g, const PhysArgs& a, cudaStream_t st);
+void launch_assemble(const Grid& g, const ProdArgs& a, bool exact, int inst0, int n, cudaStream_t st);
 // blocks a plane's products are divided among (> 1 in the adjoint modes: through ProdArgs::tmp)
 int products_groups(const Grid& g, const ProdArgs& a, int mode);
 // the forward products' shared-memory plan (planes per pass, x-stage columns per chunk)

@@ -353,6 +353,7 @@ cudaError_t launch_phys_inverse(const Grid& g, const PhysArgs& a, cudaStream_t s
   // the autotuner's choice among the bit-identical FFT variants)
   if (g.tc5 && !a.grids) return launch_phys_inverse_tc5(g, a, st);  // fits every nfields once 6 fit
   if (g.tci) return launch_phys_inverse_tc(g, a, st);
+  if (g.tcs && !a.grids && a.tmp && a.tmp_inst > 0) return launch_phys_inverse_tcs(g, a, st);
   if (g.split) return kSplit[split_index(g)].inverse(g, a, st);
   const size_t sm = phys_smem_bytes(g, a.cfl_check != 0);
   CHN_LAUNCH_FUSED(k_phys_inverse, dim3(g.Q, a.ninst), sm, st, g, a);
@@ -362,6 +363,7 @@ cudaError_t launch_phys_inverse(const Grid& g, const PhysArgs& a, cudaStream_t s
 cudaError_t launch_products_fwd(const Grid& g, const ProdArgs& a, cudaStream_t st) {
   if (a.ninst <= 0) return cudaSuccess;
   if (g.tcf) return launch_products_tc(g, a, a.Pt.base ? 1 : 0, st);
+  if (g.tcs && !a.grids && a.tmp && a.tmp_inst > 0) return launch_products_tcs(g, a, a.Pt.base ? 1 : 0, st);
   if (g.split) return kSplit[split_index(g)].products(g, a, a.Pt.base ? 1 : 0, st);
   const size_t sm = phys_smem_bytes(g, false);
   CHN_LAUNCH_FUSED(k_products_fwd, dim3(g.Q, a.ninst), sm, st, g, a);
@@ -371,6 +373,7 @@ cudaError_t launch_products_fwd(const Grid& g, const ProdArgs& a, cudaStream_t s
 cudaError_t launch_products_adj(const Grid& g, const ProdArgs& a, cudaStream_t st) {
   if (a.ninst <= 0) return cudaSuccess;
   if (g.tcf) return launch_products_tc(g, a, a.exact ? 3 : 2, st);
+  if (g.tcs && !a.grids && a.tmp && a.tmp_inst > 0) return launch_products_tcs(g, a, a.exact ? 3 : 2, st);
   if (g.split) return kSplit[split_index(g)].products(g, a, a.exact ? 3 : 2, st);
   const size_t sm = prod_adj_smem_bytes(g);
   CHN_LAUNCH_FUSED(k_products_adj, dim3(g.Q, a.ninst), sm, st, g, a);
@@ -382,6 +385,7 @@ void prepare_solve_T(int optin);
 void prepare_recon_tc(int optin);
 void prepare_phys_tc(int optin);
 void prepare_phys_tc5(int optin);
+void prepare_phys_tcs(int optin);
 
 // Every kernel may use up to the device's opt-in shared memory per block: the
 // single-grid engine and an uneven batch (sized for its largest grid) share
@@ -408,6 +412,7 @@ void prepare_kernels(const Grid& g) {
   prepare_recon_tc(optin);
   prepare_phys_tc(optin);
   prepare_phys_tc5(optin);
+  prepare_phys_tcs(optin);
 }
 
 }  // namespace chn

@@ -403,7 +403,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   if (a.cfl_check && gridDim.z == 1) plane_cfl<NTHR>(g, a, P, inst, y, gsz.Q(), gsz.pz() * gsz.px());
 }
 
-// The CFL check of a launch whose fields ran in groups, one block per plane
+// The CFL check of a launch whose fields ran in blocks of their own (or in
+// split passes), one block per plane
 __global__ void __launch_bounds__(kThreads) k_cfl(const __grid_constant__ Grid g, PhysArgs a) {
   const int inst = blockIdx.y, y = blockIdx.x;
   if (a.skip_blocked && blocked(a.status, a.sdiv, inst)) return;
@@ -639,28 +640,36 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
       const int kk = rco.r, x = rco.c;
       const int z = kk < gsz.Nz() / 2 ? kk : kk + 1;
       if (mode < 2) H[(((size_t)z * 5 + q) * gsz.Q() + y) * gsz.X() + x] = Fb[i];
-      else if (gridDim.z > 1) a.tmp[((((size_t)inst * 6 + q) * gsz.Nz() + z) * gsz.Q() + y) * gsz.X() + x] = Fb[i];
+      else if (gridDim.z > 1) a.tmp[((((size_t)inst * 6 + q) * gsz.Q() + y) * gsz.pz() + kk) * gsz.X() + x] = Fb[i];
       else assemble_stage(g, mode == 3, H, z, y, x, q, Fb[i]);
     }
     __syncthreads();
   }
 }
 
-// the adjoint modes' output slots from the six components' spectra of a
-// launch that ran them in groups (k_products_tc, gridDim.z > 1)
-__global__ void __launch_bounds__(kThreads) k_assemble(const __grid_constant__ Grid g, ProdArgs a, int exact) {
-  const int inst = blockIdx.y, z = blockIdx.z < g.Nz / 2 ? blockIdx.z : blockIdx.z + 1;
+// the adjoint modes' output slots from the six components' spectra in the
+// scratch array [local instance][6][Q][pz][X] (kept rows first): launches that
+// ran the components in blocks of their own, and the split passes
+__global__ void __launch_bounds__(kThreads) k_assemble(const __grid_constant__ Grid g, ProdArgs a, int exact, int inst0) {
+  const int il = blockIdx.y, inst = inst0 + il, kk = blockIdx.z, z = kk < g.Nz / 2 ? kk : kk + 1;
   if (blocked(a.status, a.sdiv, inst)) return;
   cpx* __restrict__ H = a.H.at(inst);
   const int i = blockIdx.x * kThreads + threadIdx.x;
   if (i >= g.Q * g.X) return;
-  const cpx* F = a.tmp + (((size_t)inst * 6) * g.Nz + z) * g.Q * g.X + i;
+  const int y = i / g.X, x = i - y * g.X;
   cpx v[6];
 #pragma unroll
-  for (int q = 0; q < 6; ++q) v[q] = F[(size_t)q * g.Nz * g.Q * g.X];
-  const int y = i / g.X, x = i - y * g.X;
+  for (int q = 0; q < 6; ++q) v[q] = a.tmp[((((size_t)il * 6 + q) * g.Q + y) * g.pz + kk) * g.X + x];
 #pragma unroll
   for (int q = 0; q < 6; ++q) assemble_stage(g, exact != 0, H, z, y, x, q, v[q]);
+}
+
+void launch_assemble(const Grid& g, const ProdArgs& a, bool exact, int inst0, int n, cudaStream_t st) {
+  k_assemble<<<dim3((g.Q * g.X + kThreads - 1) / kThreads, n, g.Nz - 1), kThreads, 0, st>>>(g, a, exact, inst0);
+}
+
+void launch_cfl(const Grid& g, const PhysArgs& a, cudaStream_t st) {
+  k_cfl<<<dim3(g.Q, a.ninst), kThreads, 0, st>>>(g, a);
 }
 
 // The forward products' shared-memory plan: product planes per pass of the
@@ -735,8 +744,7 @@ cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaS
     if (xch == d.pzp && sizes_match<Sizes32>(g)) k_products_tc<false, 1, Sizes32><<<grid, kThreads, sm, st>>>(g, a, mode);
     else if (xch == d.pzp && sizes_match<Sizes16>(g)) k_products_tc<false, 1, Sizes16><<<grid, kThreads, sm, st>>>(g, a, mode);
     else k_products_tc<false, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
-    if (mode >= 2)
-      k_assemble<<<dim3((g.Q * g.X + kThreads - 1) / kThreads, a.ninst, g.Nz - 1), kThreads, 0, st>>>(g, a, mode == 3);
+    if (mode >= 2) launch_assemble(g, a, mode == 3, 0, a.ninst, st);
     return cudaGetLastError();
   }
   if (g.prodb == 1 && !a.grids) {
@@ -838,7 +846,7 @@ cudaError_t launch_phys_inverse_tc(const Grid& g, const PhysArgs& a, cudaStream_
     if (a.grids) launch_inverse_build<true>(gr, a, st);
     else launch_inverse_build<false>(gr, a, st);
   }
-  if (a.cfl_check && inverse_groups(g, a, 1) > 1) k_cfl<<<dim3(g.Q, a.ninst), kThreads, 0, st>>>(g, a);
+  if (a.cfl_check && inverse_groups(g, a, 1) > 1) launch_cfl(g, a, st);
   return cudaGetLastError();
 }
 
