@@ -190,9 +190,8 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
       return false;
     std::vector<uint32_t> fxf, fzf, fuf;
     std::vector<int> fxe, fze, fue;
-    const int cf = build_fwd_tc_tables(h, fxf, fxe, fzf, fze, fuf, fue);
-    tct_ok = std::min(ci, cf) >= kChunkKT;
-    g.tcch = std::min(ci, cf);
+    tct_ok = ci >= kChunkKT && build_fwd_split_tables(h, fxf, fxe, fzf, fze, fuf, fue) >= kChunkKT;
+    g.tcch = ci;
     if (!T.up_digits(fxf, &g.tcFX) || !T.up(fxe, &g.tcFXE) || !T.up_digits(fzf, &g.tcFZ) || !T.up(fze, &g.tcFZE) ||
         !T.up_digits(fuf, &g.tcFXU) || !T.up(fue, &g.tcFXUE))
       return false;
@@ -265,9 +264,9 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
     if (!build_phys_tc5_tables(h, zt, xt) || !T.up(zt, &g.t5Z) || !T.up(xt, &g.t5X)) return false;
     g.tc5 = (t5 && t5[0] == '1') ? 1 : 0;
   }
-  if (solve_smem_bytes(g) > (size_t)optin || recon_smem_bytes(g) > (size_t)optin) {
+  if (solve_smem_limit(g) > (size_t)optin || recon_smem_bytes(g) > (size_t)optin) {
     set_error(1, "grid %dx%dx%d: the implicit solve needs %zu bytes of shared memory per block, the device has %d",
-              Nx, Ny, Nz, solve_smem_bytes(g), optin);
+              Nx, Ny, Nz, solve_smem_limit(g), optin);
     return false;
   }
   prepare_kernels(g);
@@ -2642,7 +2641,7 @@ int c_multi_init(int n, const int* Nx, const int* Ny, const int* Nz, const doubl
   gmax.split = (!fused_transforms_fit(gmax, optin) || (force && force[0] == '1')) ? 1 : 0;
   if (!phys_tc_fits(gmax, optin)) gmax.tci = 0;
   if (!fwd_tc_plan(gmax, optin, gmax.fwdpb, gmax.fxch)) gmax.tcf = 0;
-  if (solve_smem_bytes(gmax) > (size_t)optin) {
+  if (solve_smem_limit(gmax) > (size_t)optin) {
     set_error(1, "c_multi_init: the largest grid needs more shared memory than the device has");
     c_multi_destroy();
     return 1;

@@ -206,6 +206,7 @@ size_t recon_smem_bytes(const Grid& g);
 size_t phys_smem_bytes(const Grid& g, bool with_cfl);
 size_t prod_adj_smem_bytes(const Grid& g);
 size_t solve_smem_bytes(const Grid& g);
+size_t solve_smem_limit(const Grid& g);
 
 // flow[d][xp][y][zp] <- P[d][y][zp][xp]
 cudaError_t launch_flow_out(const Grid& g, const double* P, double* flow, cudaStream_t st);

@@ -172,6 +172,55 @@ int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::
   return std::min(cx, std::min(cu, cz));
 }
 
+// The same stages split radix-2 (decimation in frequency) as the kernels run
+// them: per class the rows 2 e + part of the e-th kept output of that parity
+// over the first half of the inputs (the class's own sums or differences), the
+// classes' row tiles and exponents one after another.  Returns the k-tiles per
+// chunk the tables allow.
+int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
+                           std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
+                           std::vector<int>& uex) {
+  const int pz = h.pz, px = h.px, Nz = h.Nz, X = h.X;
+  const FwdTcDims d = fwd_tc_dims_n(Nz, X, pz, px);
+  const double norm = 1.0 / ((3. * h.Nx / 2.) * (3. * h.Nz / 2.));
+  xfrag.clear(); xex.clear(); zfrag.clear(); zex.clear(); ufrag.clear(); uex.clear();
+  int chunk = kMaxChunkKT;
+  for (int c = 0; c < 2; ++c) {
+    const int n = c ? d.nxO : d.nxE;
+    std::vector<double> Ax((size_t)2 * n * d.pxh), Au((size_t)2 * n * d.pxh);
+    for (int e = 0; e < n; ++e)
+      for (int xp = 0; xp < d.pxh; ++xp) {
+        const int idx = (int)(((long long)(2 * e + c) * xp) % px);
+        for (int part = 0; part < 2; ++part) {  // cos, -sin
+          Au[(size_t)(2 * e + part) * d.pxh + xp] = h.twx[2 * idx + part];
+          Ax[(size_t)(2 * e + part) * d.pxh + xp] = h.twx[2 * idx + part] * norm;
+        }
+      }
+    chunk = std::min(chunk, append_digit_table(Ax.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, xfrag, xex, 512));
+    chunk = std::min(chunk, append_digit_table(Au.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, ufrag, uex, 512));
+  }
+  for (int c = 0; c < d.Rz; ++c) {
+    std::vector<int> kk;
+    z_class_modes(Nz, pz, c, kk);
+    const int n = (int)kk.size(), K = 2 * d.pzh;
+    if (n != (c ? d.nzO : d.nzE)) return 0;
+    std::vector<double> Az((size_t)2 * n * K);
+    for (int e = 0; e < n; ++e) {
+      const int zo = kk[e] < Nz / 2 ? kk[e] : kk[e] + 1 + Nz / 2;  // padded output row
+      for (int zp = 0; zp < d.pzh; ++zp) {
+        const int idx = (int)(((long long)zo * zp) % pz);
+        const double cs = h.twz[2 * idx], ms = h.twz[2 * idx + 1];  // cos, -sin
+        Az[(size_t)(2 * e) * K + 2 * zp] = cs;
+        Az[(size_t)(2 * e) * K + 2 * zp + 1] = -ms;
+        Az[(size_t)(2 * e + 1) * K + 2 * zp] = ms;
+        Az[(size_t)(2 * e + 1) * K + 2 * zp + 1] = cs;
+      }
+    }
+    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, 512));
+  }
+  return chunk;
+}
+
 // ---------------------------------------------------------------------------
 // shared-memory plan
 // ---------------------------------------------------------------------------
@@ -419,33 +468,14 @@ __global__ void __launch_bounds__(kThreads) k_cfl(const __grid_constant__ Grid g
 
 static constexpr int kPB = 3;  // products computed per pass over the plane
 
-struct FwdTcDims {
-  int KTx, KTz, MTx, MTz, KSx, KSz, pzp, Xp, Kk;
-};
-
-__host__ __device__ constexpr FwdTcDims fwd_tc_dims_n(int Nz, int X, int pz, int px) {
-  FwdTcDims d{};
-  d.Kk = Nz - 1;
-  d.KTx = (px + 15) / 16;
-  d.KTz = (2 * pz + 15) / 16;
-  d.MTx = (2 * X + 15) / 16;
-  d.MTz = (2 * d.Kk + 15) / 16;
-  d.KSx = d.KTx * 16 + 8;
-  d.KSz = d.KTz * 16 + 8;
-  d.pzp = (pz + 7) / 8 * 8;
-  d.Xp = (X + 7) / 8 * 8;
-  return d;
-}
-
-__host__ __device__ inline FwdTcDims fwd_tc_dims(const Grid& g) { return fwd_tc_dims_n(g.Nz, g.X, g.pz, g.px); }
-
 // shared memory of a products block: pb product planes, x-stage digits of
-// xch columns (a chunk), z-stage digits, exponents, the z-stage outputs
+// xch columns (a chunk), z-stage digits, exponents (px is even: a plane is
+// whole 16-byte words)
 __host__ __device__ constexpr size_t fwd_tc_smem_n(int Nz, int X, int pz, int px, int pb, int xch) {
   const FwdTcDims d = fwd_tc_dims_n(Nz, X, pz, px);
   const size_t dx = (size_t)kDig * xch * d.KSx * 2, dz = (size_t)kDig * d.Xp * d.KSz * 2;
   return (size_t)(pb * ((pz + 3) / 4 * 4) + (X + 3) / 4 * 4) * sizeof(int) + ((dx > dz ? dx : dz) + 15) / 16 * 16 +
-         ((size_t)pb * pz * px * sizeof(double) + 15) / 16 * 16 + (size_t)d.Kk * X * sizeof(cpx);
+         (size_t)pb * pz * px * sizeof(double);
 }
 
 // the widest x-stage chunk (a multiple of 8 columns) with which minb blocks
@@ -502,9 +532,9 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     const size_t dx = (size_t)kDig * XCH * d.KSx * 2, dz = (size_t)kDig * d.Xp * d.KSz * 2;
     p += ((dx > dz ? dx : dz) + 15) / 16 * 16;
   }
-  double* stage3 = reinterpret_cast<double*>(p);  // [c][zp][xp] products; Y [zp][kx] (folded sums) over plane c
-  p += ((size_t)pb * gsz.pz() * gsz.px() * sizeof(double) + 15) / 16 * 16;
-  cpx* Fb = reinterpret_cast<cpx*>(p);  // [kk][kx]
+  // [c][zp][xp] products; over plane c Y [zp][kx] (folded sums), then the z
+  // stage's outputs Fb [kk][kx] (less than half a plane)
+  double* stage3 = reinterpret_cast<double*>(p);
   const size_t plane = (size_t)gsz.pz() * gsz.px(), fs = (size_t)gsz.Q() * plane;
   const double* __restrict__ Pp = a.Pp.base + (long long)(inst / a.pdiv) * a.Pp.stride + (size_t)y * plane +
                                   (a.pslot.stride ? (long long)a.pslot.slot() * a.pslot.stride : 0LL);
@@ -519,12 +549,12 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
   // this block's components: all of them, or one of gridDim.z groups
   const int nall = mode >= 2 ? 6 : 3, qper = (nall + gridDim.z - 1) / gridDim.z, qbeg = blockIdx.z * qper;
   const int ncomp = min(nall, qbeg + qper);
-  const int chunk = gsz.tcch();
   const size_t xstride = (size_t)XCH * d.KSx, zstride = (size_t)d.Xp * d.KSz;  // 16-bit words between digits
   for (int q = qbeg; q < ncomp; ++q) {
     const int c = (q - qbeg) % pb;
     double* stage = stage3 + (size_t)c * plane;
     longlong2* Yb = reinterpret_cast<longlong2*>(stage);  // Re, Im of Y[zp][kx]: t 2^(AxE[2 kx (+ 1)] + ysum_exp(exx[zp]))
+    cpx* Fb = reinterpret_cast<cpx*>(stage);
     int* exx = exx3 + c * exs;
     if (c == 0) {
       // ---- products of components q .. q+2 (each field loaded once per
@@ -554,82 +584,89 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
       }
       __syncthreads();
     }
-    // ---- x stage: rows 2kx (+1), columns zp, in chunks of XCH columns; Y
+    // ---- x stage: columns zp, in chunks of XCH columns; Y
     // into the staging region (Y row zp lies below stage row zp, 16 X < 8 px
     // bytes per row, so a chunk's outputs only cover rows already digitised)
     // (the z stage's column exponents are cleared for this component first)
     for (int i = threadIdx.x; i < gsz.X(); i += kThreads) exz[i] = 0;
     for (int zc = 0; zc < d.pzp; zc += XCH) {
       const int nch = min(XCH, d.pzp - zc);
-      FlatRC rcx(threadIdx.x, kThreads, d.KTx * 8);
-      for (int i = threadIdx.x; i < nch * (d.KTx * 8); i += kThreads, rcx.next()) {
-        const int n = zc + rcx.r, k = 2 * rcx.c;
-        const double* src = stage + (size_t)n * gsz.px() + k;
-        const double v0 = (n < gsz.pz() && k < gsz.px()) ? src[0] : 0.0;
-        const double v1 = (n < gsz.pz() && k + 1 < gsz.px()) ? src[1] : 0.0;
-        const int ex = exx[min(n, gsz.pz() - 1)] - 1022;
-        digits_pair(scaled56(v0, ex), scaled56(v1, ex),
-                    reinterpret_cast<uint32_t*>(dig + (size_t)rcx.r * d.KSx + k), xstride / 2);
+      FlatRC rcx(threadIdx.x, kThreads, d.KTxc * 8);
+      for (int i = threadIdx.x; i < nch * (d.KTxc * 8); i += kThreads, rcx.next()) {
+        const int n = zc + rcx.r;
+        fwd_x_digits(d, stage + (size_t)n * gsz.px(), 2 * rcx.c, n < gsz.pz(), exx[min(n, gsz.pz() - 1)] - 1022,
+                     reinterpret_cast<uint32_t*>(dig + (size_t)rcx.r * d.KSx), xstride / 2);
       }
       __syncthreads();
       const int NT = nch / 8;
       for (int item = warp; item < d.MTx * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
-        tc_tile(Ax, mt, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, T);
+        tc_tile(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, xstride, nt * 8, lane, T);
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
-          const int row = mt * 16 + gq + 8 * rr;
-          if (row >= 2 * gsz.X()) continue;
-          const int er = AxE[row];
+          FwdRow row;
+          if (!fwd_row(mt, gq + 8 * rr, d.MTxE, d.nxE, d.nxO, row)) continue;
+          const int kx = 2 * row.e + row.cls, er = AxE[2 * (row.cls * d.nxE + row.e) + row.part];
           int ef = 0;  // the exponent field of this row's values, for the z stage's column
 #pragma unroll
           for (int c = 0; c < 2; ++c) {
             const int zp = zc + nt * 8 + 2 * t + c;
             if (zp >= gsz.pz()) continue;
             const long long tv = T[2 * rr + c];
-            longlong2& yv = Yb[(size_t)zp * gsz.X() + (row >> 1)];
-            if (row & 1) yv.y = tv;
+            longlong2& yv = Yb[(size_t)zp * gsz.X() + kx];
+            if (row.part) yv.y = tv;
             else yv.x = tv;
             ef = max(ef, sum_field(tv, er + ysum_exp(exx[zp]), exx[zp]));
           }
-          if (ef > 0) atomicMax(&exz[row >> 1], ef);
+          if (ef > 0) atomicMax(&exz[kx], ef);
         }
       }
       __syncthreads();
     }
-    // ---- z stage inputs: columns kx, K = 2 pz (Re, Im of Y[zp][kx] interleaved)
+    // ---- z stage inputs: columns kx (Re, Im of Y[zp][kx] interleaved)
     {
       uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
-      FlatRC rc(threadIdx.x, kThreads, d.KTz * 8);
-      for (int i = threadIdx.x; i < d.Xp * (d.KTz * 8); i += kThreads, rc.next()) {
+      FlatRC rc(threadIdx.x, kThreads, d.KTzc * 8);
+      for (int i = threadIdx.x; i < d.Xp * (d.KTzc * 8); i += kThreads, rc.next()) {
         const int n = rc.r, zp = rc.c;
-        longlong2 v = make_longlong2(0, 0);
-        if (n < gsz.X() && zp < gsz.pz()) {
-          v = Yb[(size_t)zp * gsz.X() + n];
-          const int s = exz[n] - 1078 - ysum_exp(exx[zp]);
-          v.x = scaled_sum(v.x, s - AxE[2 * n]);
-          v.y = scaled_sum(v.y, s - AxE[2 * n + 1]);
+        longlong2 u = make_longlong2(0, 0), v = u;
+        if (n < gsz.X() && zp < d.pzh) {
+          const int2 er = *reinterpret_cast<const int2*>(AxE + 2 * ((n & 1) * d.nxE + (n >> 1)));
+          auto input = [&](int z) {
+            longlong2 w = Yb[(size_t)z * gsz.X() + n];
+            const int s = exz[n] - 1078 - ysum_exp(exx[z]);
+            w.x = scaled_sum(w.x, s - er.x);
+            w.y = scaled_sum(w.y, s - er.y);
+            return w;
+          };
+          u = input(zp);
+          if (d.Rz == 2) v = input(zp + d.pzh);
         }
-        digits_pair(v.x, v.y, dw + ((size_t)n * d.KSz) / 2 + zp, zstride / 2);
+        fwd_z_digits(d, zp, u, v, dw + ((size_t)n * d.KSz) / 2, zstride / 2);
       }
     }
     __syncthreads();
-    // ---- z stage: rows 2kk (+1), columns kx -> Fb
+    // ---- z stage: columns kx -> Fb
     {
       const int NT = d.Xp / 8;
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
-        tc_tile(Az, mt, d.KTz, chunk, dig, d.KSz, zstride, nt * 8, lane, T);
+        tc_tile(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, zstride, nt * 8, lane, T);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int row = mt * 16 + gq + 8 * (r >> 1), kx = nt * 8 + 2 * t + (r & 1);
-          if (row >= 2 * d.Kk || kx >= gsz.X()) continue;
-          const double v = round_sum(T[r], g.tcFZE[row] + col_exp(exz[kx]) - 64 + kFoldShift);
-          cpx& fv = Fb[(size_t)(row >> 1) * gsz.X() + kx];
-          if (row & 1) fv.im = v;
-          else fv.re = v;
+        for (int rr = 0; rr < 2; ++rr) {
+          FwdRow row;
+          if (!fwd_row(mt, gq + 8 * rr, d.MTzE, d.nzE, d.nzO, row)) continue;
+          const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + kFoldShift;
+          const int kk = fwd_z_mode(gsz.Nz(), d.Rz, row.cls, row.e);
+#pragma unroll
+          for (int c2 = 0; c2 < 2; ++c2) {
+            const int kx = nt * 8 + 2 * t + c2;
+            if (kx >= gsz.X()) continue;
+            reinterpret_cast<double*>(Fb + (size_t)kk * gsz.X() + kx)[row.part] =
+                round_sum(T[2 * rr + c2], er + col_exp(exz[kx]));
+          }
         }
       }
     }
@@ -676,7 +713,7 @@ void launch_cfl(const Grid& g, const PhysArgs& a, cudaStream_t st) {
 // forward modes (kPB, else one) and x-stage columns per chunk (the widest
 // multiple of 8), the first that lets two blocks share an SM; false if none
 // does (the FFT kernels then run).  48x97x48: one plane per pass, chunks of
-// 24 columns, 111 KB per block.
+// 48 columns, 112 KB per block.
 bool fwd_tc_plan(const Grid& g, int optin, int& pb, int& xch) {
   const FwdTcDims d = fwd_tc_dims(g);
   const int pbs[2] = {kPB, 1};

@@ -8,7 +8,8 @@
 // digit products, 28 a k-tile, run on the tensor cores and leave the FP64 unit
 // the products and one conversion an output.  One instance at 128x129x128,
 // six fields inverse / three products forward / six adjoint:
-// TIMINGS.
+// 2.66 / 1.55 / 3.07 ms with the FFT passes, 1.52 / 0.87 / 1.50 here (the
+// forward passes 1.21 / 2.22 before they were split radix-2).
 #include <algorithm>
 
 #include "chn_common.cuh"
@@ -178,22 +179,8 @@ __global__ void __launch_bounds__(kThreads, 3) k_x_inv_tc(const __grid_constant_
 // products and forward transforms
 // ---------------------------------------------------------------------------
 
-struct FwdDims {
-  int KTx, KTz, MTx, MTz, KSx, KSz;
-};
-__host__ __device__ inline FwdDims fwd_dims(const Grid& g) {
-  FwdDims d;
-  d.KTx = (g.px + 15) / 16;
-  d.KTz = (2 * g.pz + 15) / 16;
-  d.MTx = (2 * g.X + 15) / 16;
-  d.MTz = (2 * (g.Nz - 1) + 15) / 16;
-  d.KSx = d.KTx * 16 + 8;
-  d.KSz = d.KTz * 16 + 8;
-  return d;
-}
-
 static size_t x_fwd_smem(const Grid& g) {
-  const FwdDims d = fwd_dims(g);
+  const FwdTcDims d = fwd_tc_dims(g);
   return (size_t)kDig * kCols * d.KSx * 2 + (size_t)kCols * g.px * sizeof(double) + kCols * sizeof(int);
 }
 
@@ -202,11 +189,10 @@ static size_t x_fwd_smem(const Grid& g) {
 __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant__ Grid g, ProdArgs a, int mode, int inst0,
                                                           cpx* T) {
   const int y = blockIdx.x, il = blockIdx.y, inst = inst0 + il;
-  const int ncomp = mode >= 2 ? 6 : 3, nzc = (g.pz + kCols - 1) / kCols;
+  const int ncomp = mode >= 2 ? 6 : 3;
   const int q = blockIdx.z % ncomp, z0 = (blockIdx.z / ncomp) * kCols;  // components of the same rows side by side
   if (blocked(a.status, a.sdiv, inst)) return;
-  (void)nzc;
-  const FwdDims d = fwd_dims(g);
+  const FwdTcDims d = fwd_tc_dims(g);
   const int nz = min(kCols, g.pz - z0);
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* dig = reinterpret_cast<uint16_t*>(smem);
@@ -232,15 +218,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant_
   __syncthreads();
   const size_t dstride = (size_t)kCols * d.KSx;
   {
-    FlatRC rc(threadIdx.x, kThreads, d.KTx * 8);
-    for (int i = threadIdx.x; i < kCols * (d.KTx * 8); i += kThreads, rc.next()) {
-      const int n = rc.r, k = 2 * rc.c;
-      const double* src = st + (size_t)n * g.px + k;
-      const double v0 = k < g.px ? src[0] : 0.0, v1 = k + 1 < g.px ? src[1] : 0.0;
-      const int ex = exx[n] - 1022;
-      digits_pair(scaled56(v0, ex), scaled56(v1, ex), reinterpret_cast<uint32_t*>(dig + (size_t)n * d.KSx + k),
-                  dstride / 2);
-    }
+    FlatRC rc(threadIdx.x, kThreads, d.KTxc * 8);
+    for (int i = threadIdx.x; i < kCols * (d.KTxc * 8); i += kThreads, rc.next())
+      fwd_x_digits(d, st + (size_t)rc.r * g.px, 2 * rc.c, true, exx[rc.r] - 1022,
+                   reinterpret_cast<uint32_t*>(dig + (size_t)rc.r * d.KSx), dstride / 2);
   }
   __syncthreads();
   const uint4* __restrict__ Ax = reinterpret_cast<const uint4*>(mode == 3 ? g.tcFXU : g.tcFX);
@@ -250,19 +231,24 @@ __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant_
   for (int item = warp; item < d.MTx * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
-    tc_tile<true>(Ax, mt, d.KTx, g.tcch, dig, d.KSx, dstride, nt * 8, lane, S);
+    tc_tile<true>(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, dstride, nt * 8, lane, S);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
-      if (row >= 2 * g.X || n >= nz) continue;
-      reinterpret_cast<double*>(Tp + (size_t)n * g.X + (row >> 1))[row & 1] =
-          round_sum(S[r], AxE[row] + col_exp(exx[n]) - 64 + kFoldShift);
+    for (int rr = 0; rr < 2; ++rr) {
+      FwdRow row;
+      if (!fwd_row(mt, gq + 8 * rr, d.MTxE, d.nxE, d.nxO, row)) continue;
+      const int kx = 2 * row.e + row.cls, er = AxE[2 * (row.cls * d.nxE + row.e) + row.part] - 64 + kFoldShift;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int n = nt * 8 + 2 * t + c;
+        if (n >= nz) continue;
+        reinterpret_cast<double*>(Tp + (size_t)n * g.X + kx)[row.part] = round_sum(S[2 * rr + c], er + col_exp(exx[n]));
+      }
     }
   }
 }
 
 static size_t z_fwd_smem(const Grid& g) {
-  const FwdDims d = fwd_dims(g);
+  const FwdTcDims d = fwd_tc_dims(g);
   return (size_t)kDig * kCols * d.KSz * 2 + kCols * sizeof(int);
 }
 
@@ -275,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_fwd_tc(const __grid_constant_
   const int ncomp = mode >= 2 ? 6 : 3, nxc = (g.X + kCols - 1) / kCols;
   const int q = blockIdx.z / nxc, x0 = (blockIdx.z - q * nxc) * kCols;
   if (blocked(a.status, a.sdiv, inst)) return;
-  const FwdDims d = fwd_dims(g);
+  const FwdTcDims d = fwd_tc_dims(g);
   const int nx = min(kCols, g.X - x0);
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* dig = reinterpret_cast<uint16_t*>(smem);
@@ -298,31 +284,38 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_fwd_tc(const __grid_constant_
   __syncthreads();
   const size_t dstride = (size_t)kCols * d.KSz;
   {
-    const int KW = d.KTz * 8;
+    const int KW = d.KTzc * 8;
     uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
     for (int i = threadIdx.x; i < kCols * KW; i += kThreads) {
-      const int n = (i & 7) + 8 * ((i >> 5) & 1), zp = ((i >> 3) & 3) + 4 * (i >> 6);
-      const cpx v = (n < nx && zp < g.pz) ? Tc[(size_t)zp * g.X + n] : cpx{0.0, 0.0};
-      const int ex = exz[n] - 1022;
-      digits_pair(scaled56(v.re, ex), scaled56(v.im, ex), dw + (size_t)n * d.KSz / 2 + zp, dstride / 2);
+      const int n = (i & 7) + 8 * ((i >> 5) & 1), zp = ((i >> 3) & 3) + 4 * (i >> 6), ex = exz[n] - 1022;
+      auto input = [&](int z) {
+        const cpx v = (n < nx && zp < d.pzh) ? Tc[(size_t)z * g.X + n] : cpx{0.0, 0.0};
+        return make_longlong2(scaled56(v.re, ex), scaled56(v.im, ex));
+      };
+      const longlong2 u = input(zp), v = d.Rz == 2 ? input(zp + d.pzh) : u;
+      fwd_z_digits(d, zp, u, v, dw + (size_t)n * d.KSz / 2, dstride / 2);
     }
   }
   __syncthreads();
   const uint4* __restrict__ Az = reinterpret_cast<const uint4*>(g.tcFZ);
   cpx* __restrict__ H = a.H.at(inst);
-  const int NT = (nx + 7) / 8, Kk = g.Nz - 1;
+  const int NT = (nx + 7) / 8;
   for (int item = warp; item < d.MTz * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
-    tc_tile<true>(Az, mt, d.KTz, g.tcch, dig, d.KSz, dstride, nt * 8, lane, S);
+    tc_tile<true>(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, dstride, nt * 8, lane, S);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
-      if (row >= 2 * Kk || n >= nx) continue;
-      const double v = round_sum(S[r], g.tcFZE[row] + col_exp(exz[n]) - 64 + kFoldShift);
-      const int kk = row >> 1, z = kk < g.Nz / 2 ? kk : kk + 1;
-      cpx* out = mode < 2 ? H + (((size_t)z * 5 + q) * g.Q + y) * g.X + x0 + n : Tc + (size_t)kk * g.X + n;
-      reinterpret_cast<double*>(out)[row & 1] = v;
+    for (int rr = 0; rr < 2; ++rr) {
+      FwdRow row;
+      if (!fwd_row(mt, gq + 8 * rr, d.MTzE, d.nzE, d.nzO, row)) continue;
+      const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + kFoldShift;
+      const int kk = fwd_z_mode(g.Nz, d.Rz, row.cls, row.e), z = kk < g.Nz / 2 ? kk : kk + 1;
+      cpx* out = mode < 2 ? H + (((size_t)z * 5 + q) * g.Q + y) * g.X + x0 : Tc + (size_t)kk * g.X;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int n = nt * 8 + 2 * t + c;
+        if (n < nx) reinterpret_cast<double*>(out + n)[row.part] = round_sum(S[2 * rr + c], er + col_exp(exz[n]));
+      }
     }
   }
 }

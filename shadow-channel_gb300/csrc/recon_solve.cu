@@ -247,6 +247,10 @@ size_t solve_smem_bytes_t(const Grid& g) {
 
 // the widest tile's (the fit check of a grid)
 size_t solve_smem_bytes(const Grid& g) { return solve_smem_bytes_t<16>(g); }
+// what a grid is accepted by: eight doubles per coefficient row above the
+// blocks' plan (the mean line's own arrays, when it had some), so that the
+// range of Ny (up to 179) stays
+size_t solve_smem_limit(const Grid& g) { return solve_smem_bytes(g) + (size_t)8 * g.R * sizeof(double); }
 
 template <int kTile>
 __device__ inline SolveSmem carve_solve(const Grid& g, unsigned char* base) {

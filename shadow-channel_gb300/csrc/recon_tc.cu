@@ -45,8 +45,10 @@ static constexpr int kReconRegs = 8;  // coefficient rows a thread keeps in regi
 
 // the exponent of a row of K entries: |row| < 2^e, and the sum of the row's
 // 56-bit integers below 127 * 2^56, so that a folded sum over the whole row
-// fits 64 bits (only rows of more than 127 entries can need the second)
-int digit_row_exponent(const double* row, int K) {
+// fits 64 bits (only rows of more than 127 entries can need the second); top:
+// the largest top digit of the data, 256, or 512 for the sums and differences
+// of two 56-bit integers (half the row's sum then)
+int digit_row_exponent(const double* row, int K, int top) {
   double mx = 0.0, sum = 0.0;
   for (int j = 0; j < K; ++j) {
     mx = std::fmax(mx, std::fabs(row[j]));
@@ -54,12 +56,12 @@ int digit_row_exponent(const double* row, int K) {
   }
   int e = 0;
   std::frexp(mx, &e);
-  while (std::ldexp(sum, -e) >= 126.5) ++e;
+  while (std::ldexp(sum, -e) >= 126.5 * 256 / top) ++e;
   return e;
 }
 
 int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
-                        std::vector<int>& ex) {
+                        std::vector<int>& ex, int top) {
   const size_t base = frag.size();
   frag.resize(base + (size_t)MT * KT * kDig * 32 * 4, 0u);
   const size_t ebase = ex.size();
@@ -70,26 +72,26 @@ int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::ve
     double mx = 0.0;
     for (int j = 0; j < K; ++j) mx = std::fmax(mx, std::fabs(M[(size_t)y * K + j]));
     if (mx == 0.0) continue;
-    const int e = digit_row_exponent(&M[(size_t)y * K], K);  // |M[y][j]| < 2^e
+    const int e = digit_row_exponent(&M[(size_t)y * K], K, top);  // |M[y][j]| < 2^e
     ex[ebase + y] = e;
     for (int j = 0; j < K; ++j) {
       const long long x = std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e));
       digits56(x, &dig[((size_t)y * (KT * 16) + j) * kDig]);
     }
-    // the largest level sum any data digits (|d_0| <= 256, the others <= 128)
+    // the largest level sum any data digits (|d_0| <= top, the others <= 128)
     // can reach over `chunk` consecutive k-tiles
     for (int kt = 0; kt < KT && chunk > 0; ++kt) {
       const int k1 = std::min(std::min(kt + chunk, KT) * 16, K);
       long long used = 0;  // sum |digit i| of the window, i ascending
       for (int l = 0; l < kDig; ++l) {
-        long long top = 0;
-        for (int j = kt * 16; j < k1; ++j) top += std::abs(dig[((size_t)y * (KT * 16) + j) * kDig + l]);
-        if (used * 128 + top * 256 > kLevelMax) {
+        long long last = 0;
+        for (int j = kt * 16; j < k1; ++j) last += std::abs(dig[((size_t)y * (KT * 16) + j) * kDig + l]);
+        if (used * 128 + last * top > kLevelMax) {
           --chunk;
           --kt;  // this window again, one k-tile narrower
           break;
         }
-        used += top;
+        used += last;
       }
     }
   }

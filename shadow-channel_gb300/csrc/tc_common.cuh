@@ -210,8 +210,11 @@ __device__ __forceinline__ void digits_pair_bf16(long long xr, long long xi, uin
 // and packed adds for a pair where the bf16 form takes 39): a byte b under
 // the exponent of 1024 (0x6400 | b) is 1024 + b, less 1152 it is b - 128; the
 // top digit enters the 64-bit sum under 0x6500 (1024 + 256 + d_0).
+// WIDE: |x| up to 2^57 (the sum or difference of two 56-bit integers), the top
+// digit in [-512, 512] under 0x6600 (1536 + d_0).
+template <bool WIDE = false>
 __device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t* out, size_t stride) {
-  constexpr long long kB = 0x6500808080808080LL;
+  constexpr long long kB = WIDE ? 0x6600808080808080LL : 0x6500808080808080LL;
   const long long a = x0 + kB, b = x1 + kB;
   const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
   constexpr uint32_t kE = 0x64646464u;
@@ -221,7 +224,7 @@ __device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t
                             __byte_perm(p65, kE, 0x4140)};
 #pragma unroll
   for (int q = 0; q < kDig; ++q) {
-    const uint32_t off = q == 0 ? 0xE500E500u : 0xE480E480u;  // -1280, -1152
+    const uint32_t off = q == 0 ? (WIDE ? 0xE600E600u : 0xE500E500u) : 0xE480E480u;  // -1536 or -1280, -1152
     uint32_t r;
     asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(r) : "r"(w[q]), "r"(off));
     out[(size_t)q * stride] = r;
@@ -374,12 +377,12 @@ __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __rest
 }
 
 // host: the exponent of a table row (its entries and their sum bounded)
-int digit_row_exponent(const double* row, int K);
+int digit_row_exponent(const double* row, int K, int top = 256);
 
 // host: digit table of a row-major matrix M[rows][K] in mma A-fragment order
 // [MT][KT][7][32 lanes][4] (appended to frag), row exponents appended to ex;
 // returns the k-tiles per chunk its level sums allow (0: none)
 int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
-                        std::vector<int>& ex);
+                        std::vector<int>& ex, int top = 256);
 
 }  // namespace chn
