@@ -243,17 +243,20 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // 1 (two planes per pass at 3 blocks per SM); CHN_PRODUCTS_BUILD fixes it
   const char* pbe = getenv("CHN_PRODUCTS_BUILD");
   g.prodb = (pbe && pbe[0] == '1' && pbe[1] == 0) ? 1 : 0;
-  // the solve's block tile: 16 until the autotuner has timed both;
+  // the solve's block tile: 8 until the autotuner has timed both (a single
+  // trajectory past the few-block builds: 128x129x128 0.80 -> 0.53 ms, 64x65x64
+  // 0.073 -> 0.064; 16 columns leave the last wave of blocks half empty);
   // CHN_SOLVE_TILE=8 or 16 fixes it (and skips that timing)
   const char* stl = getenv("CHN_SOLVE_TILE");  // 16, 8 or 8/128 (8 columns, 128 threads)
-  g.stile = (stl && atoi(stl) == 8) ? 8 : 16;
+  g.stile = (stl && stl[0] && atoi(stl) != 8) ? 16 : 8;
   g.sfixed = (stl && stl[0]) ? 1 : 0;
   g.sthr = (g.stile == 8 && stl && strstr(stl, "/128")) ? 128 : 256;
-  // the tensor-core reconstruction's build (recon_tc.cu): 0 until the
-  // autotuner has timed 0, 1, 2; CHN_RECON_BUILD fixes it
+  // the tensor-core reconstruction's build (recon_tc.cu): 1 (128x129x128 0.60 ->
+  // 0.50 ms against build 0, 64x65x64 0.058 -> 0.056) until the autotuner has
+  // timed 0, 1, 2; CHN_RECON_BUILD fixes it
   const char* rbe = getenv("CHN_RECON_BUILD");
   g.rfixed = (rbe && rbe[0]) ? 1 : 0;
-  g.rbuild = (rbe && rbe[0] >= '0' && rbe[0] <= '2' && rbe[1] == 0) ? rbe[0] - '0' : 0;
+  g.rbuild = (rbe && rbe[0] >= '0' && rbe[0] <= '2' && rbe[1] == 0) ? rbe[0] - '0' : (g.rfixed ? 0 : 1);
   // the inverse on tcgen05 where it fits: a candidate of the autotuner
   // (bit-identical results); CHN_INVERSE_TC5=1 forces it, =0 leaves it out
   const char* t5 = getenv("CHN_INVERSE_TC5");
