@@ -759,14 +759,14 @@ static void launch_products_b3(const Grid& g, const ProdArgs& a, int mode, cudaS
 
 // The products' launches of few planes likewise: one component per block, the
 // adjoint modes through the scratch array and k_assemble.  Forward modes up to
-// 4 planes per SM (one instance at 32x65x32 40 -> 25 us, 8 of 16x33x16 39 -> 31;
-// 8 of 48x97x48, 7.6 per SM, 699 -> 726), adjoint modes up to 3 (76 -> 41, 64 ->
-// 53; 4 of 48x97x48, 3.8 per SM, 685 -> 719).
+// 3 planes per SM (one instance at 32x65x32 40 -> 25 us), adjoint modes up to 2
+// (76 -> 41); alone they gain up to 4 and 3 (8 of 16x33x16 39 -> 31, 64 -> 53),
+// but not beside the tangents' launches (the limits below: inverse_groups).
 int products_groups(const Grid& g, const ProdArgs& a, int mode) {
   const long long planes = (long long)g.Q * a.ninst;
   if (a.grids) return 1;
-  if (mode < 2) return planes <= 4 * 152 ? 3 : 1;
-  return planes <= 3 * 152 && a.tmp && a.ninst <= a.tmp_inst ? 6 : 1;
+  if (mode < 2) return planes <= 3 * 152 ? 3 : 1;
+  return planes <= 2 * 152 && a.tmp && a.ninst <= a.tmp_inst ? 6 : 1;
 }
 
 // Grid::fixed & FIXED_PRODUCTS: the build compiled for the grid's sizes
@@ -806,10 +806,13 @@ bool phys_tc_fits(const Grid& g, int optin) {
 }
 
 // Launches of few planes run a plane's fields in blocks of their own, FB
-// fields each, instead of one after another: up to kGroupPlanes planes (5 per
-// SM).  One instance at 32x65x32: 49 -> 23 us in one-field blocks, 10 of
-// 28x43x18 (4.2 per SM) 127 -> 105; 24 of 16x33x16 (7.7 per SM) 77 -> 84.
-static constexpr long long kGroupPlanes = 5 * 152;
+// fields each, instead of one after another: up to kGroupPlanes planes (3 per
+// SM).  One instance at 32x65x32: 49 -> 23 us in one-field blocks.  Launches of
+// more planes share the chip with another stream's: with limits of 5, 4 and 3
+// per SM (inverse, forward, adjoint products) an adjoint chain of 25 segments at
+// 16x33x16 takes 5.01 ms, with 3, 3, 2 4.72, with 2, 2, 1 4.83; 6 segments of
+// 28x43x18 8.83, 8.63, 8.97.
+static constexpr long long kGroupPlanes = 3 * 152;
 static int inverse_groups(const Grid& g, const PhysArgs& a, int fb) {
   return !a.grids && (long long)g.Q * a.ninst <= kGroupPlanes ? (a.nfields + fb - 1) / fb : 1;
 }
