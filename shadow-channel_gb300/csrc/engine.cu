@@ -242,7 +242,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // the products' build (phys_tc.cu): 0 until the autotuner has timed 0 and
   // 1 (two planes per pass at 3 blocks per SM); CHN_PRODUCTS_BUILD fixes it
   const char* pbe = getenv("CHN_PRODUCTS_BUILD");
-  g.prodb = (pbe && pbe[0] == '1' && pbe[1] == 0) ? 1 : 0;
+  g.prodb = (pbe && pbe[0] == '1' && pbe[1] == 0) ? 3 : 0;
   // the solve's block tile: 8 until the autotuner has timed both (a single
   // trajectory past the few-block builds: 128x129x128 0.80 -> 0.53 ms, 64x65x64
   // 0.073 -> 0.064; 16 columns leave the last wave of blocks half empty);
@@ -1251,7 +1251,7 @@ static bool autotune_transforms(Engine& e, Work& w) {
   g.tvar = best->tvar;
   g.tcminb = best->minb;
   g.tc5 = best->tc5;
-  char buf[160];
+  char buf[240];
   g_tune_report = "{";
   const bool tcv = g.tci && g.tcf;
   for (const Cand& c : cands) {
@@ -1426,7 +1426,7 @@ static bool autotune_fixed(Engine& e, Work& w) {
   const int saved = g.fixed;
   bool ok = true;
   std::string rep;
-  char buf[160];
+  char buf[240];
   for (const Part& pt : parts) {
     if (!do_fixed) break;
     float ms[2] = {0.f, 0.f};
@@ -1473,25 +1473,30 @@ static bool autotune_fixed(Engine& e, Work& w) {
     }
   }
   // the products' build: three planes per pass at 2 blocks per SM (the
-  // plan) against two planes at 3 blocks
+  // plan) against two planes at 3 blocks, forward and adjoint apart (12
+  // segments at 16x33x16: 0.107 / 0.094 ms forward, 0.062 / 0.076 adjoint)
   const char* pbe = getenv("CHN_PRODUCTS_BUILD");
   if (ok && g.tcf && !w.gdev && !(pbe && pbe[0])) {
     const int saved_b = g.prodb;
-    float ms[2] = {0.f, 0.f};
-    for (int c = 0; c < 2 && ok; ++c) {
-      g.prodb = c;
-      ok = enqueue(FIXED_PRODUCTS);  // warm-up
+    float ms[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [forward, adjoint][build]
+    for (int c = 0; c < 4 && ok; ++c) {
+      const bool adj = c >= 2;
+      auto launch = [&]() { return (adj ? launch_products_adj(g, b, e.st) : launch_products_fwd(g, f, e.st)) == cudaSuccess; };
+      g.prodb = c % 2 ? 3 : 0;
+      ok = launch();  // warm-up
       ok = ok && cudaEventRecord(t0, e.st) == cudaSuccess;
-      for (int k = 0; k < 3 && ok; ++k) ok = enqueue(FIXED_PRODUCTS);
+      for (int k = 0; k < 3 && ok; ++k) ok = launch();
       ok = ok && cudaEventRecord(t1, e.st) == cudaSuccess && cudaEventSynchronize(t1) == cudaSuccess;
-      if (ok) cudaEventElapsedTime(&ms[c], t0, t1);
-      ms[c] /= 3;
+      if (ok) cudaEventElapsedTime(&ms[adj][c % 2], t0, t1);
+      ms[adj][c % 2] /= 3;
     }
     if (ok) {
       g_launches += 16;
-      g.prodb = ms[1] < ms[0] ? 1 : 0;
-      snprintf(buf, sizeof(buf), "\"products_b0\": %.4f, \"products_b1\": %.4f, \"products_build\": %d", ms[0], ms[1],
-               g.prodb);
+      const int fb = ms[0][1] < ms[0][0] ? 1 : 0, ab = ms[1][1] < ms[1][0] ? 1 : 0;
+      g.prodb = fb | 2 * ab;
+      snprintf(buf, sizeof(buf),
+               "\"products_b0\": %.4f, \"products_b1\": %.4f, \"products_build\": %d, \"products_adj_b0\": %.4f, "
+               "\"products_adj_b1\": %.4f, \"products_adj_build\": %d", ms[0][0], ms[0][1], fb, ms[1][0], ms[1][1], ab);
       if (!rep.empty()) rep += ", ";
       rep += buf;
     } else {

@@ -748,7 +748,7 @@ static void launch_products_sizes(const Grid& g, const ProdArgs& a, int mode, cu
   }
 }
 
-// Grid::prodb 1 (single-grid batches): two product planes per pass at 3
+// Grid::prodb's bit (single-grid batches): two product planes per pass at 3
 // blocks per SM (80 registers), the x stage in the chunks that fit
 template <class S>
 static void launch_products_b3(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st) {
@@ -784,7 +784,7 @@ cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaS
     if (mode >= 2) launch_assemble(g, a, mode == 3, 0, a.ninst, st);
     return cudaGetLastError();
   }
-  if (g.prodb == 1 && !a.grids) {
+  if ((g.prodb & (mode < 2 ? 1 : 2)) && !a.grids) {
     const bool fx = (g.fixed & FIXED_PRODUCTS) != 0;
     if (fx && sizes_match<Sizes32>(g)) launch_products_b3<Sizes32>(g, a, mode, st);
     else if (fx && sizes_match<Sizes16>(g)) launch_products_b3<Sizes16>(g, a, mode, st);
@@ -809,8 +809,8 @@ bool phys_tc_fits(const Grid& g, int optin) {
 // fields each, instead of one after another: up to kGroupPlanes planes (3 per
 // SM).  One instance at 32x65x32: 49 -> 23 us in one-field blocks.  Launches of
 // more planes share the chip with another stream's: with limits of 5, 4 and 3
-// per SM (inverse, forward, adjoint products) an adjoint chain of 25 segments at
-// 16x33x16 takes 5.01 ms, with 3, 3, 2 4.72, with 2, 2, 1 4.83; 6 segments of
+// per SM (inverse, forward, adjoint products) eight segments' adjoint chain at
+// 16x33x16 takes 5.01 ms, with 3, 3, 2 4.72, with 2, 2, 1 4.83; five of
 // 28x43x18 8.83, 8.63, 8.97.
 static constexpr long long kGroupPlanes = 3 * 152;
 static int inverse_groups(const Grid& g, const PhysArgs& a, int fb) {
