@@ -225,32 +225,50 @@ int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, st
 // shared-memory plan
 // ---------------------------------------------------------------------------
 
-__host__ __device__ inline size_t phys_tc_dbuf_bytes(const Grid& g, int fb) {
+// the digits (z, then x of xch columns)
+__host__ __device__ constexpr size_t phys_tc_dbuf(const PhysTcDims& d, int xch) {
+  const size_t z = (size_t)kDig * ((d.NZ + 7) / 8 * 8) * d.KSz * 2, x = (size_t)kDig * xch * d.KSx * 2;
+  return ((z > x ? z : x) + 15) / 16 * 16;
+}
+// the exponents of both stages' columns, and the Z intermediate
+__host__ __device__ constexpr size_t phys_tc_rest(const PhysTcDims& d, int pz, int X, int fb) {
+  return (size_t)((d.NZ + 3) / 4 * 4 + (d.NX + 3) / 4 * 4) * sizeof(int) + (size_t)fb * pz * X * sizeof(cpx);
+}
+__host__ __device__ constexpr int phys_tc_all_columns(const PhysTcDims& d) { return (d.NX + 7) / 8 * 8; }
+
+size_t phys_tc_smem_bytes(const Grid& g, int fb, int xch) {
   const PhysTcDims d = phys_tc_dims(g, fb);
-  const size_t z = (size_t)kDig * ((d.NZ + 7) / 8 * 8) * d.KSz * 2, x = (size_t)kDig * ((d.NX + 7) / 8 * 8) * d.KSx * 2;
-  return (z > x ? z : x + 0);
+  return phys_tc_dbuf(d, xch) + phys_tc_rest(d, g.pz, g.X, fb);
+}
+static size_t phys_tc_smem_bytes(const Grid& g, int fb) {
+  return phys_tc_smem_bytes(g, fb, phys_tc_all_columns(phys_tc_dims(g, fb)));
 }
 
-size_t phys_tc_smem_bytes(const Grid& g, bool with_cfl, int fb) {
-  const PhysTcDims d = phys_tc_dims(g, fb);
-  size_t b = 0;
-  b += (size_t)((d.NZ + 3) / 4 * 4) * sizeof(int);            // z-stage column exponents
-  b += (size_t)((d.NX + 3) / 4 * 4) * sizeof(int);            // x-stage column exponents
-  b += (phys_tc_dbuf_bytes(g, fb) + 15) / 16 * 16;             // digits (z, then x)
-  b += (size_t)fb * g.pz * g.X * sizeof(cpx);                  // Z intermediate
-  (void)with_cfl;  // the CFL number is read back from the written fields
-  return b;
+// The x stage takes its columns in chunks where all of them at once would
+// leave fewer than minb blocks an SM (1 KB reserved and 3 KB declared per
+// block): the largest chunk (a multiple of 8) that lets the most blocks, up to
+// minb, share one.  48x97x48, one field: all 72 columns 101 KB, 2 blocks; 40
+// and 32, 68 KB, 3 (12 instances 1.66 -> 1.23 ms: the kernel waits on latency,
+// and 8 warps an SM did not cover it).
+static size_t phys_tc_smem_chunked(const Grid& g, int fb, int minb) {
+  const int all = phys_tc_all_columns(phys_tc_dims(g, fb));
+  for (int nb = minb; nb > 1; --nb)
+    for (int c = all; c >= 16; c -= 8)
+      if (nb * (phys_tc_smem_bytes(g, fb, c) + 4096) <= 233472) return phys_tc_smem_bytes(g, fb, c);
+  return phys_tc_smem_bytes(g, fb);
+}
+// the chunk that smem bytes of a launch hold for a grid (a launch of several
+// grids is sized by the largest), the columns shared evenly
+__device__ __forceinline__ int phys_tc_xch(const PhysTcDims& d, int pz, int X, int fb, size_t smem) {
+  const int all = phys_tc_all_columns(d);
+  const int fit = min(all, (int)((smem - phys_tc_rest(d, pz, X, fb)) / ((size_t)kDig * d.KSx * 2)) / 8 * 8);
+  const int n = (all + fit - 1) / fit;
+  return ((all + n - 1) / n + 7) / 8 * 8;
 }
 
 // ---------------------------------------------------------------------------
 // kernel
 // ---------------------------------------------------------------------------
-
-__host__ __device__ constexpr size_t phys_tc_dbuf_of(const PhysTcDims& d) {
-  return (size_t)kDig * ((d.NZ + 7) / 8 * 8) * d.KSz * 2 > (size_t)kDig * ((d.NX + 7) / 8 * 8) * d.KSx * 2
-             ? (size_t)kDig * ((d.NZ + 7) / 8 * 8) * d.KSz * 2
-             : (size_t)kDig * ((d.NX + 7) / 8 * 8) * d.KSx * 2;
-}
 
 // block maximum of the CFL field of plane y (channel/pass1.c:116-138), from
 // the written velocity fields
@@ -296,7 +314,14 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   unsigned char* p = smem;
   int* exz = reinterpret_cast<int*>(p); p += (size_t)((d.NZ + 3) / 4 * 4) * sizeof(int);
   int* exx = reinterpret_cast<int*>(p); p += (size_t)((d.NX + 3) / 4 * 4) * sizeof(int);
-  uint16_t* dig = reinterpret_cast<uint16_t*>(p); p += (phys_tc_dbuf_of(d) + 15) / 16 * 16;
+  // x-stage columns per chunk: all of them in the fixed-size builds
+  int XCH = phys_tc_all_columns(d);
+  if constexpr (std::is_same<S, SizesRT>::value) {
+    uint32_t dyn;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    XCH = phys_tc_xch(d, gsz.pz(), gsz.X(), FB, dyn);
+  }
+  uint16_t* dig = reinterpret_cast<uint16_t*>(p); p += phys_tc_dbuf(d, XCH);
   cpx* Zb = reinterpret_cast<cpx*>(p);  // staged inputs, then [fl][m][x]: the z stage's folded sums
   longlong2* Zs = reinterpret_cast<longlong2*>(Zb);
 
@@ -400,52 +425,56 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
     // ---- x stage, both fields: columns n = fl * pz + m, K words: Re, Im of
     // Z[m][j] for the even j, then the odd j (Im of j = 0 unused).
     const int ncx = nfb * gsz.pz();
-    const size_t xstride = (size_t)((d.NX + 7) / 8 * 8) * d.KSx;
-    {
-      uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
-      const int npad = (ncx + 7) / 8 * 8, KW = d.KTx * 8, WE = d.KTxE * 8;
-      FlatRC rc(threadIdx.x, NTHR, KW);
-      for (int i = threadIdx.x; i < npad * KW; i += NTHR, rc.next()) {
-        const int n = rc.r, w = rc.c;
-        const int j = w < WE ? (w < d.nxE ? d.Rx * w : -1) : (w - WE < d.nxO ? 2 * (w - WE) + 1 : -1);
-        longlong2 v = make_longlong2(0, 0);
-        if (j >= 0 && n < ncx) {
-          v = Zs[(size_t)n * gsz.X() + j];
-          if (j == 0) v.y = 0;
-          int fl = 0, m = n;  // n = fl pz + m
-          while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
-          const int s = exx[n] - 1078 - zsum_exp(exz[fl * gsz.X() + j]);
-          v.x = scaled_sum(v.x, s);
-          v.y = scaled_sum(v.y, s);
+    const size_t xstride = (size_t)XCH * d.KSx;
+    for (int n0 = 0; n0 < ncx; n0 += XCH) {
+      const int nch = min(XCH, (ncx - n0 + 7) / 8 * 8);
+      {
+        uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
+        const int KW = d.KTx * 8, WE = d.KTxE * 8;
+        FlatRC rc(threadIdx.x, NTHR, KW);
+        for (int i = threadIdx.x; i < nch * KW; i += NTHR, rc.next()) {
+          const int n = n0 + rc.r, w = rc.c;
+          const int j = w < WE ? (w < d.nxE ? d.Rx * w : -1) : (w - WE < d.nxO ? 2 * (w - WE) + 1 : -1);
+          longlong2 v = make_longlong2(0, 0);
+          if (j >= 0 && n < ncx) {
+            v = Zs[(size_t)n * gsz.X() + j];
+            if (j == 0) v.y = 0;
+            int fl = 0, m = n;  // n = fl pz + m
+            while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
+            const int s = exx[n] - 1078 - zsum_exp(exz[fl * gsz.X() + j]);
+            v.x = scaled_sum(v.x, s);
+            v.y = scaled_sum(v.y, s);
+          }
+          digits_pair(v.x, v.y, dw + ((size_t)rc.r * d.KSx) / 2 + w, xstride / 2);
         }
-        digits_pair(v.x, v.y, dw + ((size_t)n * d.KSx) / 2 + w, xstride / 2);
       }
-    }
-    __syncthreads();
-    // the z stage's column exponents are cleared for the next pass
-    for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
-    {
-      // rows xp < pxh; E + O -> P[xp], E - O -> P[xp + pxh]
-      const int NT = (ncx + 7) / 8;
-      for (int item = warp; item < d.MTx * NT; item += nwarp) {
-        const int mt = item / NT, nt = item - mt * NT;
-        long long TE[4], TO[4];
-        tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE);
-        tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO);
+      __syncthreads();
+      // the z stage's column exponents are cleared for the next pass
+      if (n0 + XCH >= ncx)
+        for (int i = threadIdx.x; i < d.NZ; i += NTHR) exz[i] = 0;
+      {
+        // rows xp < pxh; E + O -> P[xp], E - O -> P[xp + pxh]
+        const int NT = nch / 8;
+        for (int item = warp; item < d.MTx * NT; item += nwarp) {
+          const int mt = item / NT, nt = item - mt * NT;
+          long long TE[4], TO[4];
+          tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE);
+          tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const int xp = mt * 16 + gq + 8 * (r >> 1), col = nt * 8 + 2 * t + (r & 1);
-          if (xp >= d.pxh || col >= ncx) continue;
-          int fl = 0, m = col;  // col = fl pz + m, fl < FB
-          while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
-          const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + kFoldShift;
-          double* Pr = P + ((size_t)(f0 + fl) * gsz.Q() + y) * plane + (size_t)m * gsz.px();
-          Pr[xp] = round_sum(TE[r] + TO[r], e, nonfinite);
-          if (d.Rx == 2) Pr[xp + d.pxh] = round_sum(TE[r] - TO[r], e, nonfinite);
+          for (int r = 0; r < 4; ++r) {
+            const int xp = mt * 16 + gq + 8 * (r >> 1), col = n0 + nt * 8 + 2 * t + (r & 1);
+            if (xp >= d.pxh || col >= ncx) continue;
+            int fl = 0, m = col;  // col = fl pz + m, fl < FB
+            while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
+            const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + kFoldShift;
+            double* Pr = P + ((size_t)(f0 + fl) * gsz.Q() + y) * plane + (size_t)m * gsz.px();
+            Pr[xp] = round_sum(TE[r] + TO[r], e, nonfinite);
+            if (d.Rx == 2) Pr[xp + d.pxh] = round_sum(TE[r] - TO[r], e, nonfinite);
+          }
         }
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
   if (nonfinite && a.status) atomicOr(&a.status[inst / a.sdiv], ST_NONFINITE);
   // (with the fields in groups, k_cfl follows)
@@ -802,7 +831,7 @@ bool phys_tc_fits(const Grid& g, int optin) {
   // the kernel's static shared memory (reduction, staged grid) is below 4 KB;
   // the input staging keeps one thread per z-stage column (the widest build's
   // plan; the one-field builds need less)
-  return kFB * g.X <= kThreads && phys_tc_smem_bytes(g, true, kFB) + 4096 <= (size_t)optin;
+  return kFB * g.X <= kThreads && phys_tc_smem_bytes(g, kFB) + 4096 <= (size_t)optin;
 }
 
 // Launches of few planes run a plane's fields in blocks of their own, FB
@@ -833,15 +862,14 @@ template <bool MULTI>
 static void launch_inverse_build(const Grid& g, const PhysArgs& a, cudaStream_t st) {
   const int fb = (g.tcminb == 4 || g.tcminb == 5 || g.tcminb == 8) ? 1 : 2;
   const dim3 grid(g.Q, a.ninst, inverse_groups(g, a, fb));
-  const bool cfl = a.cfl_check != 0;
-  const size_t s2 = phys_tc_smem_bytes(g, cfl, 2), s1 = phys_tc_smem_bytes(g, cfl, 1);
+  auto s = [&](int fb, int minb) { return phys_tc_smem_chunked(g, fb, minb); };
   using RT = SizesRT;
   switch (g.tcminb) {
-    case 3: k_phys_inverse_tc<MULTI, 3, 2, 256, RT><<<grid, 256, s2, st>>>(g, a); break;
-    case 4: k_phys_inverse_tc<MULTI, 4, 1, 128, RT><<<grid, 128, s1, st>>>(g, a); break;
-    case 5: k_phys_inverse_tc<MULTI, 5, 1, 128, RT><<<grid, 128, s1, st>>>(g, a); break;
-    case 8: k_phys_inverse_tc<MULTI, 3, 1, 192, RT><<<grid, 192, s1, st>>>(g, a); break;
-    default: k_phys_inverse_tc<MULTI, 2, 2, 256, RT><<<grid, 256, s2, st>>>(g, a); break;
+    case 3: k_phys_inverse_tc<MULTI, 3, 2, 256, RT><<<grid, 256, s(2, 3), st>>>(g, a); break;
+    case 4: k_phys_inverse_tc<MULTI, 4, 1, 128, RT><<<grid, 128, s(1, 4), st>>>(g, a); break;
+    case 5: k_phys_inverse_tc<MULTI, 5, 1, 128, RT><<<grid, 128, s(1, 5), st>>>(g, a); break;
+    case 8: k_phys_inverse_tc<MULTI, 3, 1, 192, RT><<<grid, 192, s(1, 3), st>>>(g, a); break;
+    default: k_phys_inverse_tc<MULTI, 2, 2, 256, RT><<<grid, 256, s(2, 2), st>>>(g, a); break;
   }
 }
 
@@ -862,15 +890,14 @@ static bool inverse_ct_build(int b) { return b == 6 || b == 7 || b >= 9; }
 template <class S>
 static void launch_inverse_ct(const Grid& g, const PhysArgs& a, cudaStream_t st) {
   const dim3 grid(g.Q, a.ninst, inverse_groups(g, a, g.tcminb == 7 ? 2 : 1));
-  const bool cfl = a.cfl_check != 0;
-  const size_t s1 = phys_tc_smem_bytes(g, cfl, 1);
+  const size_t s1 = phys_tc_smem_bytes(g, 1);
   switch (g.tcminb) {
     case 6: k_phys_inverse_tc<false, 4, 1, 128, S><<<grid, 128, s1, st>>>(g, a); break;
     case 9: k_phys_inverse_tc<false, 3, 1, 192, S><<<grid, 192, s1, st>>>(g, a); break;
     case 10: k_phys_inverse_tc<false, 5, 1, 128, S><<<grid, 128, s1, st>>>(g, a); break;
     case 11: k_phys_inverse_tc<false, 4, 1, 192, S><<<grid, 192, s1, st>>>(g, a); break;
     case 12: k_phys_inverse_tc<false, 3, 1, 256, S><<<grid, 256, s1, st>>>(g, a); break;
-    default: k_phys_inverse_tc<false, 2, 2, 256, S><<<grid, 256, phys_tc_smem_bytes(g, cfl, 2), st>>>(g, a); break;
+    default: k_phys_inverse_tc<false, 2, 2, 256, S><<<grid, 256, phys_tc_smem_bytes(g, 2), st>>>(g, a); break;
   }
 }
 
