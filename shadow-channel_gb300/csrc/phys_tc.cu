@@ -496,6 +496,13 @@ __global__ void __launch_bounds__(kThreads) k_cfl(const __grid_constant__ Grid g
 // ---------------------------------------------------------------------------
 
 static constexpr int kPB = 3;  // products computed per pass over the plane
+// threads of the one-plane build with run-time sizes for batches of one grid,
+// whose blocks are large and two to an SM: 24 warps instead of 16 cover more of
+// the latency that binds it (12 instances at 48x97x48 forward 0.947 -> 0.893 ms,
+// 4 adjoint 0.618 -> 0.592).  The other builds keep 256: one component a block
+// is slower with 384 (8 of 16x33x16 30 -> 34 us), several grids no faster (the
+// register limit spills more there).
+static constexpr int kWideThreads = 384;
 
 // shared memory of a products block: pb product planes, x-stage digits of
 // xch columns (a chunk), z-stage digits, exponents (px is even: a plane is
@@ -535,11 +542,11 @@ size_t fwd_tc_smem_bytes(const Grid& g, int pb, int xch) { return fwd_tc_smem_n(
 // modes 0/1 write H slots 0..2, modes 2/3 fold each component into the
 // output slots (assemble_stage).  Same outputs as k_products_fwd /
 // k_products_adj.
-// S: the sizes (SizesRT, or SizesCT for a specialised grid); MINB blocks
-// per SM (the register budget; with MINB > 2 the x stage runs in the chunks
+// S: the sizes (SizesRT, or SizesCT for a specialised grid); NTHR threads, MINB
+// blocks per SM (the register budget; with MINB > 2 the x stage runs in the chunks
 // that let MINB blocks share an SM)
-template <bool MULTI, int PB, class S, int MINB = 2>
-__global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_constant__ Grid g0, ProdArgs a, int mode) {
+template <bool MULTI, int PB, class S, int MINB = 2, int NTHR = kThreads>
+__global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constant__ Grid g0, ProdArgs a, int mode) {
   const int inst = blockIdx.y, y = blockIdx.x;
   CHN_INSTANCE_GRID(g0, a.grids, inst);
   const S gsz(g);
@@ -574,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
   const int* __restrict__ AxE = mode == 3 ? g.tcFXUE : g.tcFXE;
   const uint4* __restrict__ Az = reinterpret_cast<const uint4*>(g.tcFZ);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
-  constexpr int nwarp = kThreads >> 5;
+  constexpr int nwarp = NTHR >> 5;
   // this block's components: all of them, or one of gridDim.z groups
   const int nall = mode >= 2 ? 6 : 3, qper = (nall + gridDim.z - 1) / gridDim.z, qbeg = blockIdx.z * qper;
   const int ncomp = min(nall, qbeg + qper);
@@ -588,10 +595,10 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     if (c == 0) {
       // ---- products of components q .. q+2 (each field loaded once per
       // point), row exponents (one column per zp)
-      for (int i = threadIdx.x; i < pb * exs; i += kThreads) exx3[i] = 0;
+      for (int i = threadIdx.x; i < pb * exs; i += NTHR) exx3[i] = 0;
       __syncthreads();
       const int nc = min(pb, ncomp - q);
-      FlatRC rc(threadIdx.x, kThreads, gsz.px());
+      FlatRC rc(threadIdx.x, NTHR, gsz.px());
       auto point = [&](int i) {
         double v[PB];
 #pragma unroll
@@ -606,10 +613,10 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
         }
       };
       if constexpr (std::is_same<S, SizesRT>::value) {
-        for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += kThreads, rc.next()) point(i);
+        for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += NTHR, rc.next()) point(i);
       } else {
 #pragma unroll 3
-        for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += kThreads, rc.next()) point(i);
+        for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += NTHR, rc.next()) point(i);
       }
       __syncthreads();
     }
@@ -617,11 +624,11 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     // into the staging region (Y row zp lies below stage row zp, 16 X < 8 px
     // bytes per row, so a chunk's outputs only cover rows already digitised)
     // (the z stage's column exponents are cleared for this component first)
-    for (int i = threadIdx.x; i < gsz.X(); i += kThreads) exz[i] = 0;
+    for (int i = threadIdx.x; i < gsz.X(); i += NTHR) exz[i] = 0;
     for (int zc = 0; zc < d.pzp; zc += XCH) {
       const int nch = min(XCH, d.pzp - zc);
-      FlatRC rcx(threadIdx.x, kThreads, d.KTxc * 8);
-      for (int i = threadIdx.x; i < nch * (d.KTxc * 8); i += kThreads, rcx.next()) {
+      FlatRC rcx(threadIdx.x, NTHR, d.KTxc * 8);
+      for (int i = threadIdx.x; i < nch * (d.KTxc * 8); i += NTHR, rcx.next()) {
         const int n = zc + rcx.r;
         fwd_x_digits(d, stage + (size_t)n * gsz.px(), 2 * rcx.c, n < gsz.pz(), exx[min(n, gsz.pz() - 1)] - 1022,
                      reinterpret_cast<uint32_t*>(dig + (size_t)rcx.r * d.KSx), xstride / 2);
@@ -656,8 +663,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     // ---- z stage inputs: columns kx (Re, Im of Y[zp][kx] interleaved)
     {
       uint32_t* dw = reinterpret_cast<uint32_t*>(dig);
-      FlatRC rc(threadIdx.x, kThreads, d.KTzc * 8);
-      for (int i = threadIdx.x; i < d.Xp * (d.KTzc * 8); i += kThreads, rc.next()) {
+      FlatRC rc(threadIdx.x, NTHR, d.KTzc * 8);
+      for (int i = threadIdx.x; i < d.Xp * (d.KTzc * 8); i += NTHR, rc.next()) {
         const int n = rc.r, zp = rc.c;
         longlong2 u = make_longlong2(0, 0), v = u;
         if (n < gsz.X() && zp < d.pzh) {
@@ -701,8 +708,8 @@ __global__ void __launch_bounds__(kThreads, MINB) k_products_tc(const __grid_con
     }
     __syncthreads();
     // ---- outputs (the (kk, kx) -> thread map is the same for every q)
-    FlatRC rco(threadIdx.x, kThreads, gsz.X());
-    for (int i = threadIdx.x; i < d.Kk * gsz.X(); i += kThreads, rco.next()) {
+    FlatRC rco(threadIdx.x, NTHR, gsz.X());
+    for (int i = threadIdx.x; i < d.Kk * gsz.X(); i += NTHR, rco.next()) {
       const int kk = rco.r, x = rco.c;
       const int z = kk < gsz.Nz() / 2 ? kk : kk + 1;
       if (mode < 2) H[(((size_t)z * 5 + q) * gsz.Q() + y) * gsz.X() + x] = Fb[i];
@@ -773,7 +780,7 @@ static void launch_products_sizes(const Grid& g, const ProdArgs& a, int mode, cu
     else k_products_tc<false, kPB, S><<<grid, kThreads, sm, st>>>(g, a, mode);
   } else {
     if (M && a.grids) k_products_tc<true, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
-    else k_products_tc<false, 1, S><<<grid, kThreads, sm, st>>>(g, a, mode);
+    else k_products_tc<false, 1, S, 2, M ? kWideThreads : kThreads><<<grid, M ? kWideThreads : kThreads, sm, st>>>(g, a, mode);
   }
 }
 
@@ -944,6 +951,7 @@ void prepare_phys_tc(int optin) {
   allow_max_smem(k_products_tc<false, kPB, RT>, optin);
   allow_max_smem(k_products_tc<true, kPB, RT>, optin);
   allow_max_smem(k_products_tc<false, 1, RT>, optin);
+  allow_max_smem(k_products_tc<false, 1, RT, 2, kWideThreads>, optin);
   allow_max_smem(k_products_tc<true, 1, RT>, optin);
   allow_max_smem(k_products_tc<false, kPB, Sizes32>, optin);
   allow_max_smem(k_products_tc<false, 2, SizesRT, 3>, optin);

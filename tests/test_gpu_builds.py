@@ -15,6 +15,8 @@ exact adjoint.  The grids sit where a build begins or ends:
   lengths with remainders, 60x33x48 (two k-tiles per digit sum);
 - components in blocks of their own (one trajectory at 32x65x32) and together
   (20x17x18, 20 trajectories: three product planes per pass);
+- 48x33x48, 10 trajectories: the inverse's x stage in chunks, one product plane
+  a pass in the wider blocks;
 - planes that do not fit one block: 128x33x64, and 128x33x54 (odd).
 
 Both evaluate the same step to rounding.  The oracle built with and without
@@ -38,7 +40,7 @@ TOL = [(33, (5e-12, 1e-11, 3e-11)), (67, (1.8e-11, 3e-11, 5.6e-11)), (131, (8.6e
        (172, (7.8e-9, 7.8e-9, 6.2e-9))]
 CASES = [(12, 18, 6, 1, 2), (12, 19, 6, 1, 2), (20, 67, 6, 2, 2), (12, 131, 6, 1, 2), (12, 171, 6, 1, 1),
          (20, 33, 16, 12, 2), (20, 17, 18, 20, 2), (32, 65, 32, 1, 1), (60, 33, 48, 1, 1),
-         (128, 33, 64, 1, 1), (128, 33, 54, 2, 1)]
+         (48, 33, 48, 10, 1), (128, 33, 64, 1, 1), (128, 33, 54, 2, 1)]
 
 
 def _step(cc, Nx, Ny, Nz, nseg, ntan, ref):
