@@ -2642,6 +2642,11 @@ int c_multi_init(int n, const int* Nx, const int* Ny, const int* Nz, const doubl
     gmax.tci = std::min(gmax.tci, g.tci);
     gmax.tcf = std::min(gmax.tcf, g.tcf);
   }
+  // an even padded z length's digits, split in two classes, can take a k-tile
+  // more than those of the next odd length: a mixed batch is sized as even
+  bool even = false;
+  for (int i = 0; i < n; ++i) even |= m->tabs[i].g.pz % 2 == 0;
+  if (even) gmax.pz += gmax.pz % 2;
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);

@@ -90,3 +90,36 @@ def test_builds_match_the_fp64_kernels(case):
             assert not np.array_equal(a, b)   # two builds' roundings, not one's
         for s in range(a.shape[0]):
             assert np.linalg.norm(a[s] - b[s]) <= tol * np.linalg.norm(b[s])
+
+
+def test_uneven_batch_of_odd_and_even_padded_lengths():
+    """3 Nz/2 = 21 beside 18, whose z-stage digits need a k-tile more: each
+    instance against itself alone."""
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    from channel import c_channel as cc
+    grids = [(12, 17, 14), (12, 17, 12), (12, 17, 14)]
+    i3 = lambda j: (ctypes.c_int * 3)(*[g[j] for g in grids])
+    d3 = lambda v: (ctypes.c_double * 3)(v, v, v)
+    states = [[O.synthetic_state(*g, seed=k + i, laminar=k == 0) for i, g in enumerate(grids)] for k in (0, 10, 20)]
+    C, IC, AC = (np.concatenate([x.ravel() for x in xs]) for xs in states)
+    inh = (ctypes.c_int * 1)(1)
+    assert cc.lib.c_multi_init(3, i3(0), i3(1), i3(2), d3(2 * np.pi), d3(np.pi), d3(2000.0), d3(2.0), d3(0.004), 1, 1,
+                               0) == 0, cc.c_last_error_message()
+    try:
+        assert cc.lib.c_multi_forward(0, 1, C.ctypes.data, IC.ctypes.data, inh) == 0, cc.c_last_error_message()
+        assert cc.lib.c_multi_adjoint(1, 0, AC.ctypes.data, 1.0) == 0, cc.c_last_error_message()
+    finally:
+        cc.lib.c_multi_destroy()
+    off = 0
+    for i, g in enumerate(grids):
+        c, ic, ac = (states[k][i].copy() for k in range(3))
+        assert cc.c_init(*g, 2 * np.pi, np.pi, 2000.0, 2.0, 0.004, 1) == 0, cc.c_last_error_message()
+        cc.c_primal(0, c)
+        cc.c_tangent(0, 1, ic, 1)
+        cc.c_adjoint(1, 0, ac, 0, 1.0)
+        assert cc.c_last_error() == 0, cc.c_last_error_message()
+        cc.c_destroy()
+        for a, b, tol in zip((C, IC, AC), (c, ic, ac), TOL[0][1]):
+            assert np.linalg.norm(a[off:off + b.size] - b.ravel()) <= tol * np.linalg.norm(b)
+        off += c.size
