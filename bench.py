@@ -204,7 +204,7 @@ def products_fwd_flops(ninst, g):
 
 
 def tc_inverse_mma_flops(ninst, g, nfields=6):
-    """bf16 tensor-core flop of one k_phys_inverse_tc launch: per pair of
+    """16-bit tensor-core flop of one k_phys_inverse_tc launch: per pair of
     fields the radix-2 z-stage GEMM (pz rows x 2 (Nz-1) x 2X, the even and
     odd modes' k-tiles) and x-stage GEMM (px/2 rows x 2X x 2 pz) in m16n8k16
     tiles, each tile 28 digit-pair MMAs."""
@@ -221,13 +221,18 @@ def tc_inverse_mma_flops(ninst, g, nfields=6):
 
 
 def tc_products_mma_flops(ninst, g, ncomp=3):
-    """bf16 tensor-core flop of one k_products_tc launch: per component an
-    x-stage GEMM (2X x px x pz) and a z-stage GEMM (2 (Nz-1) x 2 pz x X) in
+    """Tensor-core flop of one k_products_tc launch: per component the radix-2
+    x-stage GEMM (even and odd kx, 2 rows each, x px/2 x pz) and z-stage GEMM
+    (the kept modes of even and odd index, 2 rows each, x 2 pz/2 x X) in
     m16n8k16 tiles of 28 digit-pair MMAs."""
     X, Nz = g["Nx"] // 2, g["Nz"]
     pz, px, Q = 3 * Nz // 2, 3 * g["Nx"] // 2, 3 * g["Ny"] // 2
     t = lambda n, d: (n + d - 1) // d
-    per = 28 * (t(2 * X, 16) * t(px, 16) * t(pz, 8) + t(2 * (Nz - 1), 16) * t(2 * pz, 16) * t(X, 8))
+    h = Nz // 2
+    nzE, nzO = ((Nz - 1, 0) if pz % 2 else ((h + 1) // 2 + (h - 1) // 2, h // 2 + h // 2))
+    kz = 2 * pz if pz % 2 else pz
+    per = 28 * ((t(2 * ((X + 1) // 2), 16) + t(2 * (X // 2), 16)) * t(px // 2, 16) * t(pz, 8)
+                + (t(2 * nzE, 16) + t(2 * nzO, 16)) * t(kz, 16) * t(X, 8))
     return ninst * Q * ncomp * per * 4096.0
 
 

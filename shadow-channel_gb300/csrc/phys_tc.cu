@@ -1,7 +1,7 @@
 // The inverse 3/2-padded transforms (channel/pass1.c:42-114,
 // channel/spec2phys.c:39-76) as exact digit GEMMs on the tensor cores.
 //
-// One block per (instance, plane y), two fields per pass:
+// One block per (instance, plane y), one or two fields per pass:
 //   z stage   Z[m][x] = sum_kz F[kz][x] exp(+2 pi i m zp(kz)/pz) over the
 //             Nz - 1 kept rows, one column per (field, x);
 //   x stage   P[m][xp] = Re Z[m][0] + 2 sum_{0<j<X} Re(Z[m][j] exp(+2 pi i j xp/px))
@@ -20,7 +20,7 @@
 // The DFT matrices hold the FFT's own twiddle doubles; operands are base-256
 // digits with exact FP32 level sums (tc_common.cuh), so each output is the
 // (faithfully) rounded value of the exact sum of the 56-bit operands.  The
-// intermediate Z is rounded to FP64 in shared memory between the stages.  Same outputs,
+// intermediate Z stays a folded 64-bit sum in shared memory between the stages.  Same outputs,
 // CFL check and status bits as k_phys_inverse.
 #include <algorithm>
 #include <cmath>
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
       // from; the exponent of each value into its x-stage column (fl, m) (not
       // the imaginary part of the kx = 0 bin, which c2r ignores)
       const int NT = (nfb * gsz.X() + 7) / 8;
-      const size_t dstride = (size_t)((d.NZ + 7) / 8 * 8) * d.KSz;  // bf16 between digits
+      const size_t dstride = (size_t)((d.NZ + 7) / 8 * 8) * d.KSz;  // fp16 between digits
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long TE[4], TO[4];

@@ -227,7 +227,7 @@ struct SolveSmem {
 // parameter kTile, which stands for the file's 16 inside them.
 
 // digits of one quadrature input for the tensor-core quadrature:
-// [7][2 kTile columns][KS] bf16 + kTile exponents
+// [7][2 kTile columns][KS] fp16 + kTile exponents
 __host__ __device__ inline size_t solve_tc_kstride(const Grid& g) { return (size_t)((g.Q + 15) / 16) * 16 + 8; }
 
 // the FP64 quadrature's parity-combined inputs only where it runs (g.tc = 0)

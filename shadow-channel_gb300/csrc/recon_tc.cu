@@ -5,18 +5,16 @@
 //   v = Q alpha, Q' alpha, Q'' alpha, g = R beta, R' beta   (Q planes each),
 // followed by the K-algebra that mixes them into u, w, du/dy, dw/dy.  On
 // GB300 the FP64 pipe (1.2 TFLOP/s) bounds the direct form; here each
-// contraction runs as a bf16 tensor-core GEMM on integer digits:
+// contraction runs as an fp16 tensor-core GEMM on integer digits:
 //   - every basis row (plane y) and every coefficient column is scaled by a
 //     power of two into an integer of 56 significant bits, written as seven
 //     balanced base-256 digits (the top digit in [-256, 256], the others in
-//     [-128, 127]); digits are exact in bf16;
+//     [-128, 127]); digits are exact in fp16;
 //   - digit products of level l = i + k accumulate in FP32 through
-//     mma.sync m16n8k16 (bf16 inputs, FP32 accumulator).  With K <= 112
-//     terms a level's partial sums stay below 2^24, so FP32 holds them
-//     exactly;
+//     mma.sync m16n8k16 (fp16 inputs, FP32 accumulator), exactly, in chunks
+//     of two k-tiles (append_digit_table checks each table);
 //   - levels l < 7 are kept (the rest lie below 2^-56 of the operands'
-//     scale), recombined exactly in 64-bit integers and rounded once to FP64
-//     by one fma.
+//     scale), folded into one 64-bit integer and rounded once to FP64.
 // Only the rounding and the K-algebra use the FP64 pipe.  Results agree with the FP64
 // contraction to its own rounding.
 #include <cuda_bf16.h>
@@ -173,7 +171,7 @@ bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std
 // device
 // ---------------------------------------------------------------------------
 
-__host__ __device__ inline int recon_tc_kstride(int KT) { return KT * 16 + 8; }  // bf16 per digit row (padded)
+__host__ __device__ inline int recon_tc_kstride(int KT) { return KT * 16 + 8; }  // fp16 per digit row (padded)
 
 // tile: kx columns per block (16 or 8)
 size_t recon_tc_smem_bytes(const Grid& g, int tile) {

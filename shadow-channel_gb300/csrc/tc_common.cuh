@@ -1,4 +1,4 @@
-// Exact FP64 contractions on the bf16 tensor cores (shared by the
+// Exact FP64 contractions on the 16-bit tensor cores (shared by the
 // reconstruction, recon_tc.cu, and the quadratures of the implicit solve,
 // recon_solve.cu).
 //
