@@ -2787,6 +2787,10 @@ double c_batch_kernel_ms(int which, int reps) {
   int zero = 0;
   cudaMemcpyAsync(w.step, &zero, sizeof(int), cudaMemcpyHostToDevice, e.st);
   cudaMemsetAsync(w.status, 0, sizeof(uint32_t) * w.nseg, e.st);
+  // the primal's fields as the sweeps read them: from the cache where they are
+  // (Pp then holds none: products of zeros, whose sums' roundings take the
+  // slow way, and a solve of them)
+  const Batch<const double> prim = w.cached(0, 1) ? cbd(w.Pc, w.cstride) : cbd(w.Pp, w.psz);
   auto launch = [&]() -> cudaError_t {
     switch (which) {
       case 0: {
@@ -2816,7 +2820,7 @@ double c_batch_kernel_ms(int which, int reps) {
         ap.grids = w.gdev;
         ap.tmp = w.Zt;
         ap.tmp_inst = w.zt_inst;
-        ap.Pp = cbd(w.Pp, w.psz);
+        ap.Pp = prim;
         ap.pdiv = w.ntan;
         ap.Pt = cbd(w.Pt, w.psz);
         ap.H = mb(w.Ut, w.usz);
@@ -2846,7 +2850,7 @@ double c_batch_kernel_ms(int which, int reps) {
         ap.grids = w.gdev;
         ap.tmp = w.Zt;
         ap.tmp_inst = w.zt_inst;
-        ap.Pp = cbd(w.Pp, w.psz);
+        ap.Pp = prim;
         ap.pdiv = 1;
         ap.Pt = cbd(w.Pl, w.psz);
         ap.H = mb(w.Up, w.usz);
