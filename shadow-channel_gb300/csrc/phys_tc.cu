@@ -300,6 +300,13 @@ __device__ __forceinline__ void plane_cfl(const Grid& g, const PhysArgs& a, cons
   }
 }
 
+// The even modes' rests wait for the odd modes' tile packed in the run-time-size
+// builds, whose registers are fewest (48x33x48, 192 threads at 3 blocks:
+// 88 bytes spilled instead of 184); the compiled sizes lose by it (192 instances
+// of 32x65x32 2.86 -> 2.90 ms)
+template <class S>
+static constexpr bool kPackRests = std::is_same<S, SizesRT>::value;
+
 // FB fields per pass, NTHR threads, MINB blocks per SM (the register
 // budget), S the sizes (SizesRT, or SizesCT for a specialised grid)
 template <bool MULTI, int MINB, int FB, int NTHR, class S>
@@ -383,7 +390,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
     __syncthreads();
     {
       // rows Re Z[m], Im Z[m] for m < pzh; E + O -> Z[m], E - O -> Z[m + pzh],
-      // kept as the folded 64-bit sums (scale 2^zsum_exp(column): the rows of
+      // kept as 64-bit sums, rounded to kFoldShift's unit (scale 2^zsum_exp(column): the rows of
       // this table share one exponent) that the x stage takes its digits
       // from; the exponent of each value into its x-stage column (fl, m) (not
       // the imaginary part of the kx = 0 bin, which c2r ignores)
@@ -392,8 +399,10 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long TE[4], TO[4];
-        tc_tile_range(Az, mt, d.KTz, 0, d.KTzE, chunk, dig, d.KSz, dstride, nt * 8, lane, TE);
-        tc_tile_range(Az, mt, d.KTz, d.KTzE, d.KTz, chunk, dig, d.KSz, dstride, nt * 8, lane, TO);
+        uint32_t RE[4] = {kFoldHalf, kFoldHalf, kFoldHalf, kFoldHalf}, RO[4] = {0, 0, 0, 0};
+        tc_tile_range(Az, mt, d.KTz, 0, d.KTzE, chunk, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
+        const Rests<kPackRests<S>> rE(RE);
+        tc_tile_range(Az, mt, d.KTz, d.KTzE, d.KTz, chunk, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int row = mt * 16 + gq + 8 * (r >> 1), col = nt * 8 + 2 * t + (r & 1);
@@ -404,14 +413,18 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
           int fl = 0, x = col;  // col = fl X + x, fl < FB
           while (x >= gsz.X()) { x -= gsz.X(); ++fl; }
           const bool counts = !(im && x == 0);
-          const long long tp = TE[r] + TO[r];
+          long long t;
+          uint32_t rest;
+          sum_plus(TE[r], rE[r], TO[r], RO[r], t, rest);
+          const long long tp = sum_whole(t, rest);
           longlong2& zp = Zs[((size_t)fl * gsz.pz() + m) * gsz.X() + x];
           if (im) zp.y = tp;
           else zp.x = tp;
           const int ep = zsum_field(tp, ce);
           if (counts && ep > 0) atomicMax(&exx[fl * gsz.pz() + m], ep);
           if (d.Rz == 2) {
-            const long long tm = TE[r] - TO[r];
+            sum_minus(TE[r], rE[r], TO[r], RO[r], t, rest);
+            const long long tm = sum_whole(t, rest);
             longlong2& zm = Zs[((size_t)fl * gsz.pz() + m + d.pzh) * gsz.X() + x];
             if (im) zm.y = tm;
             else zm.x = tm;
@@ -458,8 +471,10 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
         for (int item = warp; item < d.MTx * NT; item += nwarp) {
           const int mt = item / NT, nt = item - mt * NT;
           long long TE[4], TO[4];
-          tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE);
-          tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO);
+          uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
+          tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE, RE);
+          const Rests<kPackRests<S>> rE(RE);
+          tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO, RO);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const int xp = mt * 16 + gq + 8 * (r >> 1), col = n0 + nt * 8 + 2 * t + (r & 1);
@@ -468,8 +483,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
             while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
             const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + kFoldShift;
             double* Pr = P + ((size_t)(f0 + fl) * gsz.Q() + y) * plane + (size_t)m * gsz.px();
-            Pr[xp] = round_sum(TE[r] + TO[r], e, nonfinite);
-            if (d.Rx == 2) Pr[xp + d.pxh] = round_sum(TE[r] - TO[r], e, nonfinite);
+            Pr[xp] = round_plus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+            if (d.Rx == 2) Pr[xp + d.pxh] = round_minus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
           }
         }
       }
@@ -638,7 +653,9 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
       for (int item = warp; item < d.MTx * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
-        tc_tile(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, xstride, nt * 8, lane, T);
+        uint32_t R[4] = {kFoldHalf, kFoldHalf, kFoldHalf, kFoldHalf};  // (kept as T alone)
+        tc_tile(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, xstride, nt * 8, lane, T,
+                R);
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
           FwdRow row;
@@ -689,7 +706,9 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
-        tc_tile(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, zstride, nt * 8, lane, T);
+        uint32_t R[4] = {0, 0, 0, 0};
+        tc_tile(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, zstride, nt * 8, lane, T,
+                R);
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
           FwdRow row;
@@ -701,7 +720,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
             const int kx = nt * 8 + 2 * t + c2;
             if (kx >= gsz.X()) continue;
             reinterpret_cast<double*>(Fb + (size_t)kk * gsz.X() + kx)[row.part] =
-                round_sum(T[2 * rr + c2], er + col_exp(exz[kx]));
+                round_sum(T[2 * rr + c2], R[2 * rr + c2], er + col_exp(exz[kx]));
           }
         }
       }

@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
     const bool zwarp = 32 * q < t.ncz;
     const int nz = 32 * q + lane;
     const int rows_grp = t.NpZ / kT5Groups;  // a multiple of 4
-    // fold the even sums into the Z buffer's slot of the first output they feed
+    // fold the even sums into the Z buffer's slots of the two outputs they feed (t, r)
     if (zwarp) {
       for (int r0 = grp * rows_grp; r0 < (grp + 1) * rows_grp; r0 += 4) {
         float lv[kDig][4];
@@ -392,7 +392,11 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             for (int l = 0; l < kDig; ++l) c[l] = lv[l][j];
             const bool im = r >= d.pzh;
             const int m = im ? r - d.pzh : r;
-            reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x])[im ? 1 : 0] = fold_levels(c);
+            long long tE = 0;
+            uint32_t rE = kFoldHalf;
+            fold_levels(c, tE, rE);
+            reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x])[im ? 1 : 0] = tE;
+            reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x])[im ? 1 : 0] = rE;
           }
         }
       }
@@ -429,7 +433,15 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             const int m = im ? r - d.pzh : r;
             long long* sp_ = reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x]) + (im ? 1 : 0);
             long long* sm_ = reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x]) + (im ? 1 : 0);
-            const long long tE = *sp_, tO = fold_levels(c), tp = tE + tO, tq = tE - tO;
+            const long long tE = *sp_;
+            const uint32_t rE = (uint32_t)*sm_;
+            long long tO = 0, tv = 0;
+            uint32_t rO = 0, rest = 0;
+            fold_levels(c, tO, rO);
+            sum_plus(tE, rE, tO, rO, tv, rest);
+            const long long tp = sum_whole(tv, rest);
+            sum_minus(tE, rE, tO, rO, tv, rest);
+            const long long tq = sum_whole(tv, rest);
             *sp_ = tp;
             *sm_ = tq;
             if (!(im && x == 0)) {  // c2r ignores the imaginary part of the kx = 0 bin
@@ -504,10 +516,13 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
                 cE[l] = lvE[l][j];
                 cO[l] = lvO[l][j];
               }
-              const long long tE = fold_levels(cE), tO = fold_levels(cO);
+              long long tE = 0, tO = 0;
+              uint32_t rE = 0, rO = 0;
+              fold_levels(cE, tE, rE);
+              fold_levels(cO, tO, rO);
               const int e = g.tcXE[xp] + col_exp(ecol) - 64 + kFoldShift;
-              stage[(size_t)nl * t.stage_ld + xp] = round_sum(tE + tO, e, nonfinite);
-              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = round_sum(tE - tO, e, nonfinite);
+              stage[(size_t)nl * t.stage_ld + xp] = round_plus(tE, rE, tO, rO, e, nonfinite);
+              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = round_minus(tE, rE, tO, rO, e, nonfinite);
             }
           }
         }

@@ -90,16 +90,21 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_inv_tc(const __grid_constant_
   for (int item = warp; item < d.MTz * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long TE[4], TO[4];
-    tc_tile_range<true>(Az, mt, d.KTz, 0, d.KTzE, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TE);
-    tc_tile_range<true>(Az, mt, d.KTz, d.KTzE, d.KTz, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TO);
+    uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
+    tc_tile_range<true>(Az, mt, d.KTz, 0, d.KTzE, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
+    const Rests<true> rE(RE);
+    tc_tile_range<true>(Az, mt, d.KTz, d.KTzE, d.KTz, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
       if (row >= 2 * d.pzh || n >= nx) continue;
       const int e = kZRowExp + col_exp(exz[n]) - 64 + kFoldShift;
       const int im = row >= d.pzh, m = im ? row - d.pzh : row;
-      reinterpret_cast<double*>(Tp + (size_t)m * g.X + x0 + n)[im] = round_sum(TE[r] + TO[r], e);
-      if (d.Rz == 2) reinterpret_cast<double*>(Tp + (size_t)(m + d.pzh) * g.X + x0 + n)[im] = round_sum(TE[r] - TO[r], e);
+      bool bad = false;
+      reinterpret_cast<double*>(Tp + (size_t)m * g.X + x0 + n)[im] = round_plus(TE[r], rE[r], TO[r], RO[r], e, bad);
+      if (d.Rz == 2)
+        reinterpret_cast<double*>(Tp + (size_t)(m + d.pzh) * g.X + x0 + n)[im] =
+            round_minus(TE[r], rE[r], TO[r], RO[r], e, bad);
     }
   }
 }
@@ -161,15 +166,17 @@ __global__ void __launch_bounds__(kThreads, 3) k_x_inv_tc(const __grid_constant_
   for (int item = warp; item < d.MTx * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long TE[4], TO[4];
-    tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TE);
-    tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TO);
+    uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
+    tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TE, RE);
+    const Rests<true> rE(RE);
+    tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int xp = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
       if (xp >= d.pxh || n >= nm) continue;
       const int e = g.tcXE[xp] + col_exp(exx[n]) - 64 + kFoldShift;
-      Pm[(size_t)n * g.px + xp] = round_sum(TE[r] + TO[r], e, nonfinite);
-      if (d.Rx == 2) Pm[(size_t)n * g.px + xp + d.pxh] = round_sum(TE[r] - TO[r], e, nonfinite);
+      Pm[(size_t)n * g.px + xp] = round_plus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+      if (d.Rx == 2) Pm[(size_t)n * g.px + xp + d.pxh] = round_minus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
     }
   }
   if (nonfinite && a.status) atomicOr(&a.status[inst / a.sdiv], ST_NONFINITE);
@@ -231,7 +238,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant_
   for (int item = warp; item < d.MTx * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
-    tc_tile<true>(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, dstride, nt * 8, lane, S);
+    uint32_t R[4] = {0, 0, 0, 0};
+    tc_tile<true>(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, dstride, nt * 8, lane, S, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       FwdRow row;
@@ -241,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant_
       for (int c = 0; c < 2; ++c) {
         const int n = nt * 8 + 2 * t + c;
         if (n >= nz) continue;
-        reinterpret_cast<double*>(Tp + (size_t)n * g.X + kx)[row.part] = round_sum(S[2 * rr + c], er + col_exp(exx[n]));
+        reinterpret_cast<double*>(Tp + (size_t)n * g.X + kx)[row.part] = round_sum(S[2 * rr + c], R[2 * rr + c], er + col_exp(exx[n]));
       }
     }
   }
@@ -303,7 +311,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_fwd_tc(const __grid_constant_
   for (int item = warp; item < d.MTz * NT; item += kWarps) {
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
-    tc_tile<true>(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, dstride, nt * 8, lane, S);
+    uint32_t R[4] = {0, 0, 0, 0};
+    tc_tile<true>(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, dstride, nt * 8, lane, S, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       FwdRow row;
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_fwd_tc(const __grid_constant_
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int n = nt * 8 + 2 * t + c;
-        if (n < nx) reinterpret_cast<double*>(out + n)[row.part] = round_sum(S[2 * rr + c], er + col_exp(exz[n]));
+        if (n < nx) reinterpret_cast<double*>(out + n)[row.part] = round_sum(S[2 * rr + c], R[2 * rr + c], er + col_exp(exz[n]));
       }
     }
   }

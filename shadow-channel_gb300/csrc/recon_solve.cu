@@ -523,13 +523,15 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
       const int col = nt * 4 + t;
       const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kFoldShift;
       long long T[4];
-      tc_tile<true>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T);
+      uint32_t R[4] = {0, 0, 0, 0};
+      tc_tile<true>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
+                    R);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = mt * 16 + gq + 8 * rr;
         if (row >= N || col >= nx) continue;
         const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol;
-        const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
+        const cpx val = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
         cpx& f = F[row * kTile + col];
         if (first) {
           f = val;

@@ -14,7 +14,7 @@
 //     mma.sync m16n8k16 (fp16 inputs, FP32 accumulator), exactly, in chunks
 //     of two k-tiles (append_digit_table checks each table);
 //   - levels l < 7 are kept (the rest lie below 2^-56 of the operands'
-//     scale), folded into one 64-bit integer and rounded once to FP64.
+//     scale), folded exactly (digit_sum.cuh) and rounded once to FP64.
 // Only the rounding and the K-algebra use the FP64 pipe.  Results agree with the FP64
 // contraction to its own rounding.
 #include <cuda_bf16.h>
@@ -309,16 +309,17 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
       const int KTb = ((cls == 0 ? gsz.D() : gsz.R()) + 15) / 16;
       const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kFoldShift;
       long long T[4];
+      uint32_t R[4] = {0, 0, 0, 0};
       tc_tile_range<(MINB <= 2)>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
                                  dig + (size_t)cls * kDig * (2 * TILE) * KS, KS, (size_t)(2 * TILE) * KS, nt * 8, lane,
-                                 T);
+                                 T, R);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int y = mt * 16 + gq + 8 * rr;
         if (y >= gsz.Q() || col >= nx) continue;
         const bool mean = meancol && col == 0;
         const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol;
-        const cpx val = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
+        const cpx val = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
         const int x = x0 + col;
         cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
         const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
@@ -419,12 +420,13 @@ __global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Gr
       const int b = grp == 0 ? (part ? 3 : 1) : (grp == 1 ? (part ? 4 : 2) : 0), cls = b < 3 ? 0 : 1;
       const uint4* next = part + 1 < nparts ? table(item, 1) : (nxt < nit ? table(nxt, 0) : nullptr);
       long long T[4];
-      tc_tile_stream(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T);
+      uint32_t R[4] = {0, 0, 0, 0};
+      tc_tile_stream(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
       const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kFoldShift;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
-        const cpx v = {round_sum(T[2 * rr], e), round_sum(T[2 * rr + 1], e)};
+        const cpx v = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
         if (part) val[1][rr] = v;
         else val[0][rr] = v;
       }

@@ -10,6 +10,7 @@
 // floating-point association (this file is compiled without FMA
 // contraction), so they agree with the reference's bit for bit;
 // tests/test_product_setup.py checks that on the CPU.
+#include "digit_sum.cuh"
 #include "setup.h"
 
 #include <cmath>
@@ -377,4 +378,40 @@ extern "C" int c_setup_tc_table(int Nx, int Ny, int Nz, double Lx, double Lz, do
   if (frag) std::memcpy(frag, f[sel].data(), sizeof(uint32_t) * f[sel].size());
   if (ex) std::memcpy(ex, e[sel].data(), sizeof(int) * e[sel].size());
   return 0;
+}
+
+// The digit GEMMs' sums (digit_sum.cuh) on the host, for tests: the level sums
+// [chunks][7] of one or of two contractions (nb = 0: none) folded as the
+// kernels fold them, from the rest `first` on, then a (op 0), a + b (1) or a - b (2).
+// out: t, r, the word that is rounded and its shift; returns t's unit's bits,
+// -1 where the two forms of the fold differ.
+extern "C" int c_setup_digit_sum(const int* a, int na, const int* b, int nb, int op, int first, long long* out) {
+  auto fold = [](const int* lv, int n, uint32_t r0, long long& t, uint32_t& r) {
+    long long ti = 0;
+    uint32_t ri = r0;
+    t = 0;
+    r = r0;
+    for (int c = 0; c < n; ++c) {
+      int v[chn::kDig];
+      uint32_t bits[chn::kDig];
+      for (int l = 0; l < chn::kDig; ++l) {
+        v[l] = lv[c * chn::kDig + l];
+        bits[l] = chn::kAccBits + (l == chn::kDig - 1 ? r : 0u) + (uint32_t)v[l];
+      }
+      chn::fold_bits(bits, t, r);
+      chn::fold_ints(v, ti, ri);
+    }
+    return t == ti && r == ri;
+  };
+  long long ta, tb;
+  uint32_t ra, rb;
+  if (!fold(a, na, (uint32_t)first, ta, ra) || !fold(b, nb, 0u, tb, rb)) return -1;
+  if (op == 1) chn::sum_plus(ta, ra, tb, rb, ta, ra);
+  if (op == 2) chn::sum_minus(ta, ra, tb, rb, ta, ra);
+  int up;
+  out[0] = ta;
+  out[1] = ra;
+  out[2] = chn::sum_word(ta, ra, up);
+  out[3] = up;
+  return chn::kFoldShift;
 }

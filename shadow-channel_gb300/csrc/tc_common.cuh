@@ -8,16 +8,14 @@
 // in the bf16 of the tcgen05 kernel).  Digit products of level l = i + k
 // accumulate in FP32 through mma.sync m16n8k16, exactly, in chunks of at most
 // two or three k-tiles.  Levels l < 7 are kept (the rest lie below 2^-56 of the
-// operands' scale), folded into one 64-bit integer per output (to 2^-56 of
-// that scale, a sixteenth of what the dropped levels leave) and rounded once
-// to FP64.
+// operands' scale), folded exactly (digit_sum.cuh) and rounded once to FP64.
 //
 // What bounds these tiles is the work around the products: the digits, the
 // folds and the roundings.  Start values that make a level's integer readable
 // from the accumulator's bit pattern, levels combined in pairs in 32 bits, one
-// 64-bit sum instead of two and a rounding without a normalising shift take a
-// fold and rounding from about 45 instructions to 20, the packed fp16 digits
-// those of a pair of values from 39 to 17.
+// 64-bit sum and a byte instead of two 64-bit sums and a rounding without a
+// normalising shift take a fold and rounding from about 45 instructions to 30,
+// the packed fp16 digits those of a pair of values from 39 to 17.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -28,10 +26,9 @@
 #include <vector>
 
 #include "chn_common.cuh"
+#include "digit_sum.cuh"
 
 namespace chn {
-
-static constexpr int kDig = 7;      // base-256 digits per operand
 
 inline uint16_t bf16_bits_of_int(int d) {
   const float f = (float)d;  // |d| <= 256: exact in bf16, low 16 bits zero
@@ -60,26 +57,12 @@ inline uint16_t half_bits_of_bf16_digit(uint16_t b) {
   return r.x;
 }
 
-// Level accumulators start at 1.5 * 2^23 instead of 0: while a level sum
-// stays within +-2^22 the FP32 accumulator is 1.5 * 2^23 + sum exactly and
-// its bit pattern is kAccBits + sum, so the integer comes out without a
-// float-to-integer conversion.  The first product of a level takes the start
-// value as its C operand.  Level 6 starts 2^(kFoldShift - 1) higher, which
-// rounds the fold's shift to nearest.
-static constexpr uint32_t kAccBits = 0x4B400000u;
-// the folded sums' unit: 2^kFoldShift of level 6's
-static constexpr int kFoldShift = 8;
 // k-tiles per accumulation chunk: append_digit_table finds the most for which
 // every level sum stays within +-2^22 whatever the data (a digit of a table
 // averages 64 of 128 at most, so two k-tiles have a margin of two; three do
 // for most tables)
 static constexpr int kChunkKT = 2;     // the Legendre tables (FP64 kernels where a table allows fewer)
 static constexpr int kMaxChunkKT = 3;  // the transforms': Grid::tcch
-static constexpr long long kLevelMax = (1LL << 22) - (1LL << kFoldShift);
-
-__device__ __forceinline__ float acc_start(int l) {
-  return __uint_as_float(kAccBits + (l == kDig - 1 ? (1u << (kFoldShift - 1)) : 0u));
-}
 
 __device__ __forceinline__ void mma_f16_16816(float* d, const uint4& a, uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -142,12 +125,14 @@ __device__ __forceinline__ int sum_bits(long long t) {
   return 64 - __clzll((long long)a);
 }
 
-// t * 2^e, rounded once: one FP64 conversion, the power of two added to the
-// exponent field.  Zeros, results outside the normal range and NaN columns
-// (e >= kNanExp / 2) take the multiplications below; bad is set for results
-// that are not finite.
-__device__ __forceinline__ double round_sum(long long t, int e, bool& bad) {
-  const double v = (double)t;
+// the sum (t, r) (digit_sum.cuh) * 2^e, e that of t's unit, rounded once: one
+// FP64 conversion, the power of two added to the exponent field.  Zeros,
+// results outside the normal range and NaN columns (e >= kNanExp / 2) take the
+// multiplications below; bad is set for results that are not finite.
+__device__ __forceinline__ double round_sum(long long t, uint32_t r, int e, bool& bad) {
+  int up;
+  const double v = (double)sum_word(t, r, up);
+  e -= up;
   const int hi = __double2hiint(v);
   const int ef = hi & 0x7FF00000;
   if (ef != 0 && (unsigned)((ef >> 20) + e - 1) < 2046u) return __hiloint2double(hi + (e << 20), __double2loint(v));
@@ -158,14 +143,48 @@ __device__ __forceinline__ double round_sum(long long t, int e, bool& bad) {
   const int h = e >> 1;
   const double f0 = __hiloint2double((min(max(h, -1022), 1023) + 1023) << 20, 0);
   const double f1 = __hiloint2double((min(max(e - h, -1022), 1023) + 1023) << 20, 0);
-  const double r = v * f0 * f1;
-  bad |= exp_field(r) == 0x7FF;
-  return r;
+  const double y = v * f0 * f1;
+  bad |= exp_field(y) == 0x7FF;
+  return y;
 }
 
-__device__ __forceinline__ double round_sum(long long t, int e) {
+__device__ __forceinline__ double round_sum(long long t, uint32_t r, int e) {
   bool bad = false;
-  return round_sum(t, e, bad);
+  return round_sum(t, r, e, bad);
+}
+
+// the four rests of a tile that wait while the warp runs its next one, PACK: as
+// bytes of one register
+template <bool PACK>
+struct Rests {
+  uint32_t v[PACK ? 1 : 4];
+  __device__ __forceinline__ explicit Rests(const uint32_t (&R)[4]) {
+    static_assert(kFoldShift == 8, "a byte each");
+    if constexpr (PACK) {
+      v[0] = __byte_perm(__byte_perm(R[0], R[1], 0x0040), __byte_perm(R[2], R[3], 0x0040), 0x5410);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] = R[r];
+    }
+  }
+  __device__ __forceinline__ uint32_t operator[](int r) const {
+    if constexpr (PACK) return __byte_perm(v[0], 0, 0x4440 + r);
+    else return v[r];
+  }
+};
+
+// of the sum and of the difference of two sums
+__device__ __forceinline__ double round_plus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
+  long long t;
+  uint32_t r;
+  sum_plus(ta, ra, tb, rb, t, r);
+  return round_sum(t, r, e, bad);
+}
+__device__ __forceinline__ double round_minus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
+  long long t;
+  uint32_t r;
+  sum_minus(ta, ra, tb, rb, t, r);
+  return round_sum(t, r, e, bad);
 }
 
 // x is neither infinite nor NaN (integer test on the exponent field)
@@ -231,34 +250,21 @@ __device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t
   }
 }
 
-// Folds the level sums of one mma accumulator element (acc[l][r], levels
-// 0..6, started at acc_start) into t in units of 2^kFoldShift of level 6:
-// adjacent levels combine in 32 bits (|l + 256 l'| < 2^31), so a fold is seven
-// integer instructions.  The start values' bit patterns stay in: kFoldBias
-// per fold.
-__device__ __forceinline__ long long fold_raw(const float (&acc)[kDig][4], int r) {
-  auto bits = [&](int l) { return __float_as_uint(acc[l][r]); };
-  const uint32_t u56 = bits(6) + (bits(5) << 8), u34 = bits(4) + (bits(3) << 8), u12 = bits(2) + (bits(1) << 8);
-  unsigned long long t = u56 >> kFoldShift;
-  t += (unsigned long long)u34 * (1u << (16 - kFoldShift));
-  t += (unsigned long long)u12 * (1u << (32 - kFoldShift));
-  t += (unsigned long long)bits(0) << (48 - kFoldShift);
-  return (long long)t;
+// the level sums of one mma accumulator element (acc[l][i], levels 0..6)
+// folded into (t, r)
+__device__ __forceinline__ void fold_acc(const float (&acc)[kDig][4], int i, long long& t, uint32_t& r) {
+  uint32_t b[kDig];
+#pragma unroll
+  for (int l = 0; l < kDig; ++l) b[l] = __float_as_uint(acc[l][i]);
+  fold_bits(b, t, r);
 }
 
-constexpr uint32_t kPairBits = kAccBits + (kAccBits << 8);  // of two combined start values (mod 2^32)
-constexpr unsigned long long kFoldBias =
-    (unsigned long long)(kPairBits >> kFoldShift) + ((unsigned long long)kPairBits << (16 - kFoldShift)) +
-    ((unsigned long long)kPairBits << (32 - kFoldShift)) + ((unsigned long long)kAccBits << (48 - kFoldShift));
-
-// the same fold of seven exact integer level sums (the tcgen05 kernel)
-__device__ __forceinline__ long long fold_levels(const float (&lv)[kDig]) {
+// of seven exact level sums (the tcgen05 kernel)
+__device__ __forceinline__ void fold_levels(const float (&lv)[kDig], long long& t, uint32_t& r) {
   int v[kDig];
 #pragma unroll
   for (int l = 0; l < kDig; ++l) v[l] = __float2int_rn(lv[l]);
-  const int p56 = v[6] + v[5] * 256 + (1 << (kFoldShift - 1)), p34 = v[4] + v[3] * 256, p12 = v[2] + v[1] * 256;
-  return (long long)(p56 >> kFoldShift) + (long long)p34 * (1LL << (16 - kFoldShift)) +
-         (long long)p12 * (1LL << (32 - kFoldShift)) + (long long)v[0] * (1LL << (48 - kFoldShift));
+  fold_ints(v, t, r);
 }
 
 // lane's ldmatrix address of the digits of the eight columns from n0
@@ -271,6 +277,7 @@ __device__ __forceinline__ uint32_t tc_row_addr(const uint16_t* dig, size_t KS, 
 
 // the 28 digit products of one k-tile (table fragments af, digits at row;
 // dst2 bytes between digit pairs), `first` of a chunk: on fresh accumulators
+// (level 6: on acc's)
 __device__ __forceinline__ void tc_ktile(const uint4 (&af)[kDig], uint32_t row, uint32_t dst2, float (&acc)[kDig][4],
                                          bool first) {
   uint32_t b0[kDig], b1[kDig];
@@ -281,7 +288,8 @@ __device__ __forceinline__ void tc_ktile(const uint4 (&af)[kDig], uint32_t row, 
   for (int i = 0; i < kDig; ++i)
 #pragma unroll
     for (int k = 0; k < kDig - i; ++k) {
-      if (first && i == 0) mma_f16_16816_from(acc[k], af[i], b0[k], b1[k], acc_start(k));
+      if (first && i == 0 && k < kDig - 1)
+        mma_f16_16816_from(acc[k], af[i], b0[k], b1[k], __uint_as_float(kAccBits));
       else mma_f16_16816(acc[i + k], af[i], b0[k], b1[k]);
     }
 }
@@ -291,19 +299,25 @@ __device__ __forceinline__ void tc_load_frags(uint4 (&af)[kDig], const uint4* __
   for (int i = 0; i < kDig; ++i) af[i] = __ldg(A + i * 32);
 }
 
+// level 6 of a chunk's accumulators: what the chunk before left of the sums
+__device__ __forceinline__ void acc_begin(float (&acc)[kDig][4], const uint32_t (&R)[4]) {
+#pragma unroll
+  for (int r = 0; r < 4; ++r) acc[kDig - 1][r] = __uint_as_float(kAccBits + R[r]);
+}
+
 static constexpr int kFragStep = kDig * 32;  // uint4 between the k-tiles of a table
 
 // One exact digit GEMM tile of a fixed table A (fragment order
 // [mt][KT][7][32][4]) against the smem digits of the eight columns from n0,
 // over the k-tiles [k0, k1): exact level sums per chunk of at most `chunk`
-// k-tiles, folded into one 64-bit integer per accumulator element.  The sum is
-// t 2^(e_row + e_col - 64 + kFoldShift) for operands scaled to 56-bit
-// integers; an empty range gives zeros.  PF: the table fragments of k-tile
+// k-tiles, folded into (T, R) per accumulator element (R on entry: added to the
+// sum).  The sum is t 2^(e_row + e_col - 64 + kFoldShift) and R a fraction of
+// it, for operands scaled to 56-bit integers; an empty range gives T = 0.  PF: the table fragments of k-tile
 // kt + 1 are loaded while kt's products run (tables that live in L2).
 template <bool PF = false>
 __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int mt, int KT, int k0, int k1, int chunk,
                                               const uint16_t* dig, size_t KS, size_t dstride, int n0, int lane,
-                                              long long (&T)[4]) {
+                                              long long (&T)[4], uint32_t (&R)[4]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) T[r] = 0;
   const uint4* Am = A + (size_t)mt * KT * kFragStep + lane;
@@ -313,6 +327,7 @@ __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int m
   if (PF && k0 < k1) tc_load_frags(an, Am + (size_t)k0 * kFragStep);
   for (int kc = k0; kc < k1; kc += chunk) {
     float acc[kDig][4];
+    acc_begin(acc, R);
     const int kend = min(k1, kc + chunk);
     auto tile = [&](int kt, bool first) {
       uint4 af[kDig];
@@ -328,14 +343,15 @@ __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int m
     tile(kc, true);
     for (int kt = kc + 1; kt < kend; ++kt) tile(kt, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) T[r] += fold_raw(acc, r) - (long long)kFoldBias;
+    for (int r = 0; r < 4; ++r) fold_acc(acc, r, T[r], R[r]);
   }
 }
 
 template <bool PF = false>
 __device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
-                                        size_t KS, size_t dstride, int n0, int lane, long long (&T)[4]) {
-  tc_tile_range<PF>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T);
+                                        size_t KS, size_t dstride, int n0, int lane, long long (&T)[4],
+                                        uint32_t (&R)[4]) {
+  tc_tile_range<PF>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T, R);
 }
 
 // The same whole tile as one of a sequence that a warp runs with few others
@@ -351,12 +367,13 @@ __device__ __forceinline__ void tc_stream_start(FragPair& pf, const uint4* __res
   tc_load_frags(pf.f[1], Am + kFragStep);
 }
 __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __restrict__ Am, const uint4* __restrict__ An,
-                                               int KT, uint32_t base, uint32_t dst2, long long (&T)[4]) {
+                                               int KT, uint32_t base, uint32_t dst2, long long (&T)[4], uint32_t (&R)[4]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) T[r] = 0;
   if (An == nullptr) An = Am;  // the last tile: loads that nothing uses
   for (int kc = 0; kc < KT; kc += kChunkKT) {
     float acc[kDig][4];
+    acc_begin(acc, R);
     auto tile = [&](int kt, bool first) {
       uint4 af[kDig];
 #pragma unroll
@@ -372,7 +389,7 @@ __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __rest
     tile(kc, true);
     if (kc + 1 < KT) tile(kc + 1, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) T[r] += fold_raw(acc, r) - (long long)kFoldBias;
+    for (int r = 0; r < 4; ++r) fold_acc(acc, r, T[r], R[r]);
   }
 }
 
