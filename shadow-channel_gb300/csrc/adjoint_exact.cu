@@ -394,16 +394,16 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
   for (int item = warp; item < MTn * NT; item += blockDim.x >> 5) {
     const int mt = item / NT, nt = item - mt * NT;
     const int col = nt * 4 + t;
-    const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kFoldShift;
+    const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
     long long sums[4];
     uint32_t R[4] = {0, 0, 0, 0};
-    tc_tile(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
+    tc_tile<false, kLongFoldShift>(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const int row = mt * 16 + gq + 8 * rr;
       if (row >= N || col >= nx) continue;
       const int e = TE[(size_t)b * gsz.R() + row] + ecol;
-      const cpx val = {round_sum(sums[2 * rr], R[2 * rr], e), round_sum(sums[2 * rr + 1], R[2 * rr + 1], e)};
+      const cpx val = {round_sum<kLongFoldShift>(sums[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(sums[2 * rr + 1], R[2 * rr + 1], e)};
       comb(row, col, val);
     }
   }
@@ -563,14 +563,14 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const uint16_t* d = b < 2 ? dA : dB;
-      const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + kFoldShift;
+      const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + kLongFoldShift;
       long long sums[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
+      tc_tile<false, kLongFoldShift>(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int y = min(mt * 16 + gq + 8 * (r >> 1), gsz.Q() - 1);
-        v[b][r] = round_sum(sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + ecol);
+        v[b][r] = round_sum<kLongFoldShift>(sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + ecol);
       }
     }
 #pragma unroll
@@ -646,14 +646,14 @@ __device__ __forceinline__ void quad_T_few(const Grid& g, const S& gsz, int z, i
       const int cls = b < 2 ? 0 : 1, nm = mt + NTHR / 32;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_stream(pf, table(mt, b), b < 2 ? table(mt, b + 1) : (nm < MTq ? table(nm, 0) : nullptr), KTr,
+      tc_tile_stream<kLongFoldShift>(pf, table(mt, b), b < 2 ? table(mt, b + 1) : (nm < MTq ? table(nm, 0) : nullptr), KTr,
                      tc_row_addr(s.dig + (size_t)cls * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
                      (uint32_t)(4 * NC * KS), T, R);
-      const int ecol = col_exp(exc[cls * TT + t]) - 64 + kFoldShift;
+      const int ecol = col_exp(exc[cls * TT + t]) - 64 + kLongFoldShift;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int e = g.tcWTE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
-        v[b][rr] = cpx{round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
+        v[b][rr] = cpx{round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
       }
     }
 #pragma unroll

@@ -170,7 +170,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   if (!T.up(qs, &a) || !T.up(rs, &b)) return false;
   T.luQs = const_cast<double*>(a);
   T.luRs = const_cast<double*>(b);
-  bool tc_ok = false, tct_ok = false;
+  bool tc_ok = false, tct_ok = false, long_inv = false, long_fwd = false;
   {
     std::vector<uint32_t> frag, wfrag;
     std::vector<int> ex, wex;
@@ -184,13 +184,13 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
       return false;
     std::vector<uint32_t> zf, xf;
     std::vector<int> ze, xe, zm;
-    const int ci = build_phys_tc_tables(h, zf, ze, xf, xe, zm);
+    const int ci = build_phys_tc_tables(h, zf, ze, xf, xe, zm, long_inv);
     if (!T.up_digits(zf, &g.tcZ) || !T.up(ze, &g.tcZE) || !T.up_digits(xf, &g.tcX) || !T.up(xe, &g.tcXE) ||
         !T.up(zm, &g.tcZM))
       return false;
     std::vector<uint32_t> fxf, fzf, fuf;
     std::vector<int> fxe, fze, fue;
-    tct_ok = ci >= kChunkKT && build_fwd_split_tables(h, fxf, fxe, fzf, fze, fuf, fue) >= kChunkKT;
+    tct_ok = ci >= kChunkKT && build_fwd_split_tables(h, fxf, fxe, fzf, fze, fuf, fue, long_fwd) >= kChunkKT;
     g.tcch = ci;
     if (!T.up_digits(fxf, &g.tcFX) || !T.up(fxe, &g.tcFXE) || !T.up_digits(fzf, &g.tcFZ) || !T.up(fze, &g.tcFZE) ||
         !T.up_digits(fuf, &g.tcFXU) || !T.up(fue, &g.tcFXUE))
@@ -214,12 +214,14 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // reconstruction and quadratures on the tensor cores unless CHN_RECON_FP64=1 (or it does not fit)
   const char* fp64 = getenv("CHN_RECON_FP64");
   g.tc = (tc_ok && !(fp64 && fp64[0] == '1') && recon_tc_smem_bytes(g) + 4096 <= (size_t)optin) ? 1 : 0;
-  // inverse transforms on the tensor cores unless CHN_TRANSFORMS_FP64=1 (or they do not fit)
+  // inverse transforms on the tensor cores unless CHN_TRANSFORMS_FP64=1 (or they
+  // do not fit; a plane long and narrow enough for one block, Nx or Nz past 130,
+  // whose sums between the stages would lose bits takes the split passes)
   const char* tfp64 = getenv("CHN_TRANSFORMS_FP64");
-  g.tci = (tct_ok && !(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
+  g.tci = (tct_ok && !long_inv && !(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
   g.fwdpb = 3;
   g.fxch = 8;
-  g.tcf = (tct_ok && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
+  g.tcf = (tct_ok && !long_fwd && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
   // and as split tensor-core passes where a plane does not fit one block
   g.tcs = (tct_ok && !(tfp64 && tfp64[0] == '1') && !(force && force[0] == '1') && phys_tcs_fits(g, optin)) ? 1 : 0;
   // the kernels' builds compiled for the grid's sizes where it has them

@@ -120,15 +120,16 @@ bool phys_tc_matrices(const HostTables& h, std::vector<double>& Az, std::vector<
 }
 
 int build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std::vector<int>& zex,
-                          std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap) {
+                         std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap, bool& long_rows) {
+  long_rows = false;
   std::vector<double> Az, Ax;
   int zrows = 0, Kz = 0, xrows = 0, Kx = 0;
   if (!phys_tc_matrices(h, Az, Ax, zmap, zrows, Kz, xrows, Kx)) return 0;
   zfrag.clear(); zex.clear(); xfrag.clear(); xex.clear();
   // one table per stage with both classes in its K: a row's exponent covers
   // its even and odd parts, so their integer sums add exactly
-  const int cz = append_digit_table(Az.data(), zrows, Kz, (zrows + 15) / 16, Kz / 16, zfrag, zex);
-  const int cx = append_digit_table(Ax.data(), xrows, Kx, (xrows + 15) / 16, Kx / 16, xfrag, xex);
+  const int cz = append_digit_table(Az.data(), zrows, Kz, (zrows + 15) / 16, Kz / 16, zfrag, zex, 256, &long_rows);
+  const int cx = append_digit_table(Ax.data(), xrows, Kx, (xrows + 15) / 16, Kx / 16, xfrag, xex, 256, &long_rows);
   for (int e : zex)
     if (e != kZRowExp) return 0;  // (every row holds a 1: exp(0) of kz = 0)
   return std::min(cz, cx);
@@ -179,8 +180,9 @@ int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::
 // chunk the tables allow.
 int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
                            std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
-                           std::vector<int>& uex) {
+                           std::vector<int>& uex, bool& long_rows) {
   const int pz = h.pz, px = h.px, Nz = h.Nz, X = h.X;
+  long_rows = false;
   const FwdTcDims d = fwd_tc_dims_n(Nz, X, pz, px);
   const double norm = 1.0 / ((3. * h.Nx / 2.) * (3. * h.Nz / 2.));
   xfrag.clear(); xex.clear(); zfrag.clear(); zex.clear(); ufrag.clear(); uex.clear();
@@ -196,8 +198,8 @@ int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, st
           Ax[(size_t)(2 * e + part) * d.pxh + xp] = h.twx[2 * idx + part] * norm;
         }
       }
-    chunk = std::min(chunk, append_digit_table(Ax.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, xfrag, xex, 512));
-    chunk = std::min(chunk, append_digit_table(Au.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, ufrag, uex, 512));
+    chunk = std::min(chunk, append_digit_table(Ax.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, xfrag, xex, 512, &long_rows));
+    chunk = std::min(chunk, append_digit_table(Au.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, ufrag, uex, 512, &long_rows));
   }
   for (int c = 0; c < d.Rz; ++c) {
     std::vector<int> kk;
@@ -216,7 +218,7 @@ int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, st
         Az[(size_t)(2 * e + 1) * K + 2 * zp + 1] = cs;
       }
     }
-    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, 512));
+    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, 512, &long_rows));
   }
   return chunk;
 }
@@ -416,15 +418,15 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
           long long t;
           uint32_t rest;
           sum_plus(TE[r], rE[r], TO[r], RO[r], t, rest);
-          const long long tp = sum_whole(t, rest);
+          const long long tp = sum_whole<kFoldShift>(t, rest);
           longlong2& zp = Zs[((size_t)fl * gsz.pz() + m) * gsz.X() + x];
           if (im) zp.y = tp;
           else zp.x = tp;
           const int ep = zsum_field(tp, ce);
           if (counts && ep > 0) atomicMax(&exx[fl * gsz.pz() + m], ep);
           if (d.Rz == 2) {
-            sum_minus(TE[r], rE[r], TO[r], RO[r], t, rest);
-            const long long tm = sum_whole(t, rest);
+            sum_minus<kFoldShift>(TE[r], rE[r], TO[r], RO[r], t, rest);
+            const long long tm = sum_whole<kFoldShift>(t, rest);
             longlong2& zm = Zs[((size_t)fl * gsz.pz() + m + d.pzh) * gsz.X() + x];
             if (im) zm.y = tm;
             else zm.x = tm;

@@ -439,9 +439,9 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             uint32_t rO = 0, rest = 0;
             fold_levels(c, tO, rO);
             sum_plus(tE, rE, tO, rO, tv, rest);
-            const long long tp = sum_whole(tv, rest);
-            sum_minus(tE, rE, tO, rO, tv, rest);
-            const long long tq = sum_whole(tv, rest);
+            const long long tp = sum_whole<kFoldShift>(tv, rest);
+            sum_minus<kFoldShift>(tE, rE, tO, rO, tv, rest);
+            const long long tq = sum_whole<kFoldShift>(tv, rest);
             *sp_ = tp;
             *sm_ = tq;
             if (!(im && x == 0)) {  // c2r ignores the imaginary part of the kx = 0 bin

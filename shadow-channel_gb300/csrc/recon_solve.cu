@@ -521,17 +521,17 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
     for (int item = warp; item < MTn * NT; item += NTHR >> 5) {
       const int mt = item / NT, nt = item - mt * NT;
       const int col = nt * 4 + t;
-      const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kFoldShift;
+      const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile<true>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
+      tc_tile<true, kLongFoldShift>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
                     R);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = mt * 16 + gq + 8 * rr;
         if (row >= N || col >= nx) continue;
         const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol;
-        const cpx val = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
         cpx& f = F[row * kTile + col];
         if (first) {
           f = val;

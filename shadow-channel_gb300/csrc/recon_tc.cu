@@ -42,10 +42,10 @@ static constexpr int kReconRegs = 8;  // coefficient rows a thread keeps in regi
 // ---------------------------------------------------------------------------
 
 // the exponent of a row of K entries: |row| < 2^e, and the sum of the row's
-// 56-bit integers below 127 * 2^56, so that a folded sum over the whole row
-// fits 64 bits (only rows of more than 127 entries can need the second); top:
-// the largest top digit of the data, 256, or 512 for the sums and differences
-// of two 56-bit integers (half the row's sum then)
+// 56-bit integers at most kLongRowSum * 2^56, so that a folded sum over the whole
+// row fits 64 bits (only rows of more than 506 entries can need the second);
+// top: the largest top digit of the data, 256, or 512 for the sums and
+// differences of two 56-bit integers (half the row's sum then)
 int digit_row_exponent(const double* row, int K, int top) {
   double mx = 0.0, sum = 0.0;
   for (int j = 0; j < K; ++j) {
@@ -54,12 +54,12 @@ int digit_row_exponent(const double* row, int K, int top) {
   }
   int e = 0;
   std::frexp(mx, &e);
-  while (std::ldexp(sum, -e) >= 126.5 * 256 / top) ++e;
+  while (std::ldexp(sum, -e) >= kLongRowSum * 256 / top) ++e;
   return e;
 }
 
 int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
-                        std::vector<int>& ex, int top) {
+                        std::vector<int>& ex, int top, bool* long_rows) {
   const size_t base = frag.size();
   frag.resize(base + (size_t)MT * KT * kDig * 32 * 4, 0u);
   const size_t ebase = ex.size();
@@ -72,6 +72,9 @@ int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::ve
     if (mx == 0.0) continue;
     const int e = digit_row_exponent(&M[(size_t)y * K], K, top);  // |M[y][j]| < 2^e
     ex[ebase + y] = e;
+    double sum = 0.0;
+    for (int j = 0; j < K; ++j) sum += std::fabs(M[(size_t)y * K + j]);
+    if (long_rows && std::ldexp(sum, -e) >= kRowSum * 256 / top) *long_rows = true;
     for (int j = 0; j < K; ++j) {
       const long long x = std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e));
       digits56(x, &dig[((size_t)y * (KT * 16) + j) * kDig]);
@@ -307,10 +310,10 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
     for (int ob = 0; ob < 5; ++ob) {
       const int b = order[ob], cls = b < 3 ? 0 : 1;
       const int KTb = ((cls == 0 ? gsz.D() : gsz.R()) + 15) / 16;
-      const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kFoldShift;
+      const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kLongFoldShift;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_range<(MINB <= 2)>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
+      tc_tile_range<(MINB <= 2), kLongFoldShift>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
                                  dig + (size_t)cls * kDig * (2 * TILE) * KS, KS, (size_t)(2 * TILE) * KS, nt * 8, lane,
                                  T, R);
 #pragma unroll
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
         if (y >= gsz.Q() || col >= nx) continue;
         const bool mean = meancol && col == 0;
         const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol;
-        const cpx val = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
         const int x = x0 + col;
         cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
         const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
@@ -421,12 +424,12 @@ __global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Gr
       const uint4* next = part + 1 < nparts ? table(item, 1) : (nxt < nit ? table(nxt, 0) : nullptr);
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_stream(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
-      const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kFoldShift;
+      tc_tile_stream<kLongFoldShift>(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
+      const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kLongFoldShift;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
-        const cpx v = {round_sum(T[2 * rr], R[2 * rr], e), round_sum(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const cpx v = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
         if (part) val[1][rr] = v;
         else val[0][rr] = v;
       }

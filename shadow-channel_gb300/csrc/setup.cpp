@@ -350,18 +350,18 @@ extern "C" int c_setup_tc_table(int Nx, int Ny, int Nz, double Lx, double Lz, do
   if (!sizes || !chn::build_tables(Nx, Ny, Nz, Lx, Lz, Re, flux, dt, t, &err)) return -1;
   std::vector<uint32_t> f[3];
   std::vector<int> e[3], m;
-  bool ok = false;
+  bool ok = false, lr = false;
   int sel = 0;
   switch (which) {
     case 0: case 1: ok = chn::build_recon_tc_tables(t, f[0], e[0], f[1], e[1]); sel = which; break;
-    case 2: case 3: ok = chn::build_phys_tc_tables(t, f[0], e[0], f[1], e[1], m); sel = which - 2; break;
+    case 2: case 3: ok = chn::build_phys_tc_tables(t, f[0], e[0], f[1], e[1], m, lr); sel = which - 2; break;
     case 4: case 5: case 6: ok = chn::build_fwd_tc_tables(t, f[0], e[0], f[1], e[1], f[2], e[2]); sel = which - 4; break;
     case 7: case 8: ok = chn::build_adj_tc_tables(t, f[0], e[0], f[1], e[1]); sel = which - 7; break;
     case 9: case 10: {
       // the tcgen05 inverse's stacked tables (bytes as 32-bit words) with the
       // row exponents of the mma.sync tables they share
       std::vector<uint8_t> zt, xt;
-      ok = chn::build_phys_tc5_tables(t, zt, xt) && chn::build_phys_tc_tables(t, f[2], e[0], f[2], e[1], m);
+      ok = chn::build_phys_tc5_tables(t, zt, xt) && chn::build_phys_tc_tables(t, f[2], e[0], f[2], e[1], m, lr);
       const std::vector<uint8_t>& b = which == 9 ? zt : xt;
       f[which - 9].assign(b.size() / 4, 0u);
       if (!b.empty()) std::memcpy(f[which - 9].data(), b.data(), b.size());
@@ -383,9 +383,10 @@ extern "C" int c_setup_tc_table(int Nx, int Ny, int Nz, double Lx, double Lz, do
 // The digit GEMMs' sums (digit_sum.cuh) on the host, for tests: the level sums
 // [chunks][7] of one or of two contractions (nb = 0: none) folded as the
 // kernels fold them, from the rest `first` on, then a (op 0), a + b (1) or a - b (2).
-// out: t, r, the word that is rounded and its shift; returns t's unit's bits,
-// -1 where the two forms of the fold differ.
-extern "C" int c_setup_digit_sum(const int* a, int na, const int* b, int nb, int op, int first, long long* out) {
+// out: t, r, the word that is rounded and its shift; -1 where the two forms of
+// the fold differ.
+template <int FS>
+static int digit_sum(const int* a, int na, const int* b, int nb, int op, int first, long long* out) {
   auto fold = [](const int* lv, int n, uint32_t r0, long long& t, uint32_t& r) {
     long long ti = 0;
     uint32_t ri = r0;
@@ -398,8 +399,8 @@ extern "C" int c_setup_digit_sum(const int* a, int na, const int* b, int nb, int
         v[l] = lv[c * chn::kDig + l];
         bits[l] = chn::kAccBits + (l == chn::kDig - 1 ? r : 0u) + (uint32_t)v[l];
       }
-      chn::fold_bits(bits, t, r);
-      chn::fold_ints(v, ti, ri);
+      chn::fold_bits<FS>(bits, t, r);
+      chn::fold_ints<FS>(v, ti, ri);
     }
     return t == ti && r == ri;
   };
@@ -407,11 +408,18 @@ extern "C" int c_setup_digit_sum(const int* a, int na, const int* b, int nb, int
   uint32_t ra, rb;
   if (!fold(a, na, (uint32_t)first, ta, ra) || !fold(b, nb, 0u, tb, rb)) return -1;
   if (op == 1) chn::sum_plus(ta, ra, tb, rb, ta, ra);
-  if (op == 2) chn::sum_minus(ta, ra, tb, rb, ta, ra);
+  if (op == 2) chn::sum_minus<FS>(ta, ra, tb, rb, ta, ra);
   int up;
   out[0] = ta;
   out[1] = ra;
-  out[2] = chn::sum_word(ta, ra, up);
+  out[2] = chn::sum_word<FS>(ta, ra, up);
   out[3] = up;
-  return chn::kFoldShift;
+  return 0;
+}
+
+extern "C" int c_setup_digit_sum(int shift, const int* a, int na, const int* b, int nb, int op, int first,
+                                 long long* out) {
+  if (shift == chn::kFoldShift) return digit_sum<chn::kFoldShift>(a, na, b, nb, op, first, out);
+  if (shift == chn::kLongFoldShift) return digit_sum<chn::kLongFoldShift>(a, na, b, nb, op, first, out);
+  return -2;
 }

@@ -44,15 +44,16 @@ bool build_recon_tc_tables(const HostTables& h, std::vector<uint32_t>& frag, std
                            std::vector<uint32_t>& wfrag, std::vector<int>& wex);
 bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std::vector<int>& btex,
                          std::vector<uint32_t>& wtfrag, std::vector<int>& wtex);
-// DFT matrices of the inverse z and x transforms as digit tables (phys_tc.cu)
+// DFT matrices of the inverse z and x transforms as digit tables (phys_tc.cu);
+// long_rows: rows that the sums kept between two stages have no room for (kRowSum)
 int build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std::vector<int>& zex,
-                          std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap);
+                          std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap, bool& long_rows);
 // the same matrices' digit tables as tcgen05 B operands (phys_tc5.cu)
 bool build_phys_tc5_tables(const HostTables& h, std::vector<uint8_t>& zt, std::vector<uint8_t>& xt);
 // DFT matrices of the forward x and z transforms as digit tables (phys_tc.cu)
 int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
                            std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
-                           std::vector<int>& uex);
+                           std::vector<int>& uex, bool& long_rows);
 int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
                          std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
                          std::vector<int>& uex);

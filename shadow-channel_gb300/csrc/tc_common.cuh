@@ -129,9 +129,10 @@ __device__ __forceinline__ int sum_bits(long long t) {
 // FP64 conversion, the power of two added to the exponent field.  Zeros,
 // results outside the normal range and NaN columns (e >= kNanExp / 2) take the
 // multiplications below; bad is set for results that are not finite.
+template <int FS = kFoldShift>
 __device__ __forceinline__ double round_sum(long long t, uint32_t r, int e, bool& bad) {
   int up;
-  const double v = (double)sum_word(t, r, up);
+  const double v = (double)sum_word<FS>(t, r, up);
   e -= up;
   const int hi = __double2hiint(v);
   const int ef = hi & 0x7FF00000;
@@ -148,43 +149,50 @@ __device__ __forceinline__ double round_sum(long long t, uint32_t r, int e, bool
   return y;
 }
 
+template <int FS = kFoldShift>
 __device__ __forceinline__ double round_sum(long long t, uint32_t r, int e) {
   bool bad = false;
-  return round_sum(t, r, e, bad);
+  return round_sum<FS>(t, r, e, bad);
 }
 
 // the four rests of a tile that wait while the warp runs its next one, PACK: as
-// bytes of one register
-template <bool PACK>
+// bytes of one register, or (FS 10) halves of two
+template <bool PACK, int FS = kFoldShift>
 struct Rests {
-  uint32_t v[PACK ? 1 : 4];
+  static constexpr int kPer = PACK ? (FS == 8 ? 4 : 2) : 1;
+  uint32_t v[4 / kPer];
   __device__ __forceinline__ explicit Rests(const uint32_t (&R)[4]) {
-    static_assert(kFoldShift == 8, "a byte each");
-    if constexpr (PACK) {
+    if constexpr (kPer == 4) {
       v[0] = __byte_perm(__byte_perm(R[0], R[1], 0x0040), __byte_perm(R[2], R[3], 0x0040), 0x5410);
+    } else if constexpr (kPer == 2) {
+      v[0] = __byte_perm(R[0], R[1], 0x5410);
+      v[1] = __byte_perm(R[2], R[3], 0x5410);
     } else {
 #pragma unroll
       for (int r = 0; r < 4; ++r) v[r] = R[r];
     }
   }
   __device__ __forceinline__ uint32_t operator[](int r) const {
-    if constexpr (PACK) return __byte_perm(v[0], 0, 0x4440 + r);
+    if constexpr (kPer == 4) return __byte_perm(v[0], 0, 0x4440 + r);
+    else if constexpr (kPer == 2) return __byte_perm(v[r >> 1], 0, r & 1 ? 0x4432 : 0x4410);
     else return v[r];
   }
 };
 
 // of the sum and of the difference of two sums
+template <int FS = kFoldShift>
 __device__ __forceinline__ double round_plus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
   long long t;
   uint32_t r;
   sum_plus(ta, ra, tb, rb, t, r);
-  return round_sum(t, r, e, bad);
+  return round_sum<FS>(t, r, e, bad);
 }
+template <int FS = kFoldShift>
 __device__ __forceinline__ double round_minus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
   long long t;
   uint32_t r;
-  sum_minus(ta, ra, tb, rb, t, r);
-  return round_sum(t, r, e, bad);
+  sum_minus<FS>(ta, ra, tb, rb, t, r);
+  return round_sum<FS>(t, r, e, bad);
 }
 
 // x is neither infinite nor NaN (integer test on the exponent field)
@@ -252,11 +260,12 @@ __device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t
 
 // the level sums of one mma accumulator element (acc[l][i], levels 0..6)
 // folded into (t, r)
+template <int FS>
 __device__ __forceinline__ void fold_acc(const float (&acc)[kDig][4], int i, long long& t, uint32_t& r) {
   uint32_t b[kDig];
 #pragma unroll
   for (int l = 0; l < kDig; ++l) b[l] = __float_as_uint(acc[l][i]);
-  fold_bits(b, t, r);
+  fold_bits<FS>(b, t, r);
 }
 
 // of seven exact level sums (the tcgen05 kernel)
@@ -264,7 +273,7 @@ __device__ __forceinline__ void fold_levels(const float (&lv)[kDig], long long& 
   int v[kDig];
 #pragma unroll
   for (int l = 0; l < kDig; ++l) v[l] = __float2int_rn(lv[l]);
-  fold_ints(v, t, r);
+  fold_ints<kFoldShift>(v, t, r);
 }
 
 // lane's ldmatrix address of the digits of the eight columns from n0
@@ -311,10 +320,10 @@ static constexpr int kFragStep = kDig * 32;  // uint4 between the k-tiles of a t
 // [mt][KT][7][32][4]) against the smem digits of the eight columns from n0,
 // over the k-tiles [k0, k1): exact level sums per chunk of at most `chunk`
 // k-tiles, folded into (T, R) per accumulator element (R on entry: added to the
-// sum).  The sum is t 2^(e_row + e_col - 64 + kFoldShift) and R a fraction of
+// sum).  The sum is t 2^(e_row + e_col - 64 + FS) and R a fraction of
 // it, for operands scaled to 56-bit integers; an empty range gives T = 0.  PF: the table fragments of k-tile
 // kt + 1 are loaded while kt's products run (tables that live in L2).
-template <bool PF = false>
+template <bool PF = false, int FS = kFoldShift>
 __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int mt, int KT, int k0, int k1, int chunk,
                                               const uint16_t* dig, size_t KS, size_t dstride, int n0, int lane,
                                               long long (&T)[4], uint32_t (&R)[4]) {
@@ -343,15 +352,15 @@ __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int m
     tile(kc, true);
     for (int kt = kc + 1; kt < kend; ++kt) tile(kt, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fold_acc(acc, r, T[r], R[r]);
+    for (int r = 0; r < 4; ++r) fold_acc<FS>(acc, r, T[r], R[r]);
   }
 }
 
-template <bool PF = false>
+template <bool PF = false, int FS = kFoldShift>
 __device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
                                         size_t KS, size_t dstride, int n0, int lane, long long (&T)[4],
                                         uint32_t (&R)[4]) {
-  tc_tile_range<PF>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T, R);
+  tc_tile_range<PF, FS>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T, R);
 }
 
 // The same whole tile as one of a sequence that a warp runs with few others
@@ -366,6 +375,7 @@ __device__ __forceinline__ void tc_stream_start(FragPair& pf, const uint4* __res
   tc_load_frags(pf.f[0], Am);
   tc_load_frags(pf.f[1], Am + kFragStep);
 }
+template <int FS>
 __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __restrict__ Am, const uint4* __restrict__ An,
                                                int KT, uint32_t base, uint32_t dst2, long long (&T)[4], uint32_t (&R)[4]) {
 #pragma unroll
@@ -389,7 +399,7 @@ __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __rest
     tile(kc, true);
     if (kc + 1 < KT) tile(kc + 1, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fold_acc(acc, r, T[r], R[r]);
+    for (int r = 0; r < 4; ++r) fold_acc<FS>(acc, r, T[r], R[r]);
   }
 }
 
@@ -398,8 +408,9 @@ int digit_row_exponent(const double* row, int K, int top = 256);
 
 // host: digit table of a row-major matrix M[rows][K] in mma A-fragment order
 // [MT][KT][7][32 lanes][4] (appended to frag), row exponents appended to ex;
-// returns the k-tiles per chunk its level sums allow (0: none)
+// returns the k-tiles per chunk its level sums allow (0: none).  long_rows: set
+// where a row's sum needs kLongFoldShift
 int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
-                        std::vector<int>& ex, int top = 256);
+                       std::vector<int>& ex, int top = 256, bool* long_rows = nullptr);
 
 }  // namespace chn
