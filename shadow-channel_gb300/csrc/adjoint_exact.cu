@@ -159,8 +159,8 @@ struct SolveTSmem {
 // bytes of the tensor-core digits: Recon^T's [7][32][Q pad] (+ exponents),
 // Quad^T's two [7][32][R pad] (+ exponents)
 __host__ __device__ inline size_t solveT_tc_bytes(const Grid& g) {
-  const size_t rq = (size_t)kDig * 32 * ((g.Q + 15) / 16 * 16 + 8) * 2 + kTile * sizeof(int);
-  const size_t qt = (size_t)2 * kDig * 32 * ((g.R + 15) / 16 * 16 + 8) * 2 + 2 * kTile * sizeof(int);
+  const size_t rq = (size_t)kDig * 32 * ((g.Q + 15) / 16 * 16 + 8) * 2 + (kTile + 1) * sizeof(int);
+  const size_t qt = (size_t)2 * kDig * 32 * ((g.R + 15) / 16 * 16 + 8) * 2 + (2 * kTile + 1) * sizeof(int);
   return rq > qt ? rq : qt;
 }
 
@@ -180,7 +180,7 @@ static size_t solveT_smem_bytes(const Grid& g) {
 __host__ __device__ inline size_t solveT_few_dig_bytes(const Grid& g, int tile) {
   const size_t rt = (size_t)5 * kDig * 2 * tile * ((g.Q + 15) / 16 * 16 + 8) * 2;
   const size_t qt = (size_t)2 * kDig * 2 * tile * ((g.R + 15) / 16 * 16 + 8) * 2;
-  return ((rt > qt ? rt : qt) + 5 * tile * sizeof(int) + 15) / 16 * 16;
+  return ((rt > qt ? rt : qt) + (5 * tile + 2) * sizeof(int) + 15) / 16 * 16;
 }
 static size_t solveT_few_smem_bytes(const Grid& g, int tile) {
   return solveT_few_dig_bytes(g, tile) + (size_t)tile * (3 * g.R + g.D) * sizeof(cpx) +
@@ -216,10 +216,9 @@ __device__ inline SolveTSmem carve_solveT(const Grid& g, unsigned char* base) {
 }
 
 // the mean line's: R^T (u + i w) and R'^T (du + i dw), both real lines (its
-// imaginary parts never reach the fields); a non-finite one makes the input NaN
+// imaginary parts never reach the fields); a non-finite one makes its line NaN
 __device__ __forceinline__ cpx recon_T_mean_input(const cpx& u, const cpx& w) {
-  const bool bad = exp_field(u.im) == 0x7FF || exp_field(w.im) == 0x7FF;
-  return cpx{bad ? u.im + w.im : u.re, w.re};
+  return cpx{exp_field(u.im) == 0x7FF ? u.im : u.re, exp_field(w.im) == 0x7FF ? w.im : w.re};
 }
 
 // Recon^T of the velocity cotangent of columns x0.. (the mean line: recon_T_mean_input):
@@ -339,53 +338,58 @@ static constexpr int kTRegs = 8;  // plane inputs a thread keeps in registers (Q
 // comb(row, col, v) for rows < N and columns col < nx of the contraction of
 // table b (row-major [rows][Q] digits: [b][ceil(R/16)][KT][7][32][4], row
 // exponents TE[b * R + row]) with the per-column plane inputs in(y, col)
-// (Re and Im as two GEMM columns sharing the column exponent)
+// (Re and Im as two GEMM columns sharing the column exponent; meancol: column 0
+// is the (0, 0) line's, an exponent each)
 template <class S, typename In, typename Comb>
 __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __restrict__ T, const int* __restrict__ TE,
-                                   int b, int N, int nx, In input, Comb comb, uint16_t* dig, int* exc) {
+                                   int b, int N, int nx, bool meancol, In input, Comb comb, uint16_t* dig, int* exc) {
   const int KT = (gsz.Q() + 15) / 16, MTw = (gsz.R() + 15) / 16;
   const size_t KS = (size_t)KT * 16 + 8;
-  for (int i = threadIdx.x; i < kTile; i += blockDim.x) exc[i] = 0;
+  for (int i = threadIdx.x; i < kTile + 1; i += blockDim.x) exc[i] = 0;
+  auto own = [&](int col) { return meancol && col == 0; };
   __syncthreads();
   if (KT <= kTRegs && blockDim.x == 16 * kTile) {
     const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
     auto plane = [&](int k) { return y0 + 32 * (k >> 1) + (k & 1); };  // plane pairs, as quad_rhs_tc
     cpx vin[kTRegs];
-    int emax = 0;
+    int emax = 0, eim = 0;
 #pragma unroll
     for (int k = 0; k < kTRegs; ++k) {
       const int y = plane(k);
       vin[k] = (y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
-      emax = max(emax, max(exp_field(vin[k].re), exp_field(vin[k].im)));
+      column_exponents(vin[k], own(col), emax, eim);
     }
     if (emax) atomicMax(&exc[col], emax);
+    if (eim) atomicMax(&exc[kTile], eim);
     __syncthreads();
-    const int ex = exc[col] - 1022;
+    const int ex = exc[col] - 1022, exi = own(col) ? exc[kTile] - 1022 : ex;
 #pragma unroll
     for (int k = 0; k < kTRegs; k += 2) {
       const int y = plane(k);
       if (y >= KT * 16) break;
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
       digits_pair(scaled56(vin[k].re, ex), scaled56(vin[k + 1].re, ex), d, 16 * KS);
-      digits_pair(scaled56(vin[k].im, ex), scaled56(vin[k + 1].im, ex), d + KS / 2, 16 * KS);
+      digits_pair(scaled56(vin[k].im, exi), scaled56(vin[k + 1].im, exi), d + KS / 2, 16 * KS);
     }
   } else {
     for (int i = threadIdx.x; i < gsz.Q() * kTile; i += blockDim.x) {
       const int y = i / kTile, col = i - y * kTile;
       if (col >= nx) continue;
       const cpx v = input(y, col);
-      const int e = max(exp_field(v.re), exp_field(v.im));
+      int e = 0, eim = 0;
+      column_exponents(v, own(col), e, eim);
       if (e) atomicMax(&exc[col], e);
+      if (eim) atomicMax(&exc[kTile], eim);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < KT * 8 * kTile; i += blockDim.x) {
       const int y = 2 * (i / kTile), col = i % kTile;
       const cpx v0 = (y < gsz.Q() && col < nx) ? input(y, col) : cpx{0.0, 0.0};
       const cpx v1 = (y + 1 < gsz.Q() && col < nx) ? input(y + 1, col) : cpx{0.0, 0.0};
-      const int ex = exc[col] - 1022;
+      const int ex = exc[col] - 1022, exi = own(col) ? exc[kTile] - 1022 : ex;
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
       digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, 16 * KS);
-      digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, 16 * KS);
+      digits_pair(scaled56(v0.im, exi), scaled56(v1.im, exi), d + KS / 2, 16 * KS);
     }
   }
   __syncthreads();
@@ -395,6 +399,7 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
     const int mt = item / NT, nt = item - mt * NT;
     const int col = nt * 4 + t;
     const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
+    const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + kLongFoldShift : ecol;
     long long sums[4];
     uint32_t R[4] = {0, 0, 0, 0};
     tc_tile<false, kLongFoldShift>(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
@@ -402,8 +407,9 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
     for (int rr = 0; rr < 2; ++rr) {
       const int row = mt * 16 + gq + 8 * rr;
       if (row >= N || col >= nx) continue;
-      const int e = TE[(size_t)b * gsz.R() + row] + ecol;
-      const cpx val = {round_sum<kLongFoldShift>(sums[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(sums[2 * rr + 1], R[2 * rr + 1], e)};
+      const int e = TE[(size_t)b * gsz.R() + row];
+      const cpx val = {round_sum<kLongFoldShift>(sums[2 * rr], R[2 * rr], e + ecol),
+                       round_sum<kLongFoldShift>(sums[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
       comb(row, col, val);
     }
   }
@@ -437,11 +443,11 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
   };
   // alpha_bar = Q^T v_bar - Q'^T Xp_bar + Q''^T dx_bar -> s.Fa
   contract_planes_tc(
-      g, gsz, T, g.tcBTE, 0, gsz.D(), nx,
+      g, gsz, T, g.tcBTE, 0, gsz.D(), nx, false,
       [&](int y, int col) { return col < xfirst ? cpx{0.0, 0.0} : at(1, y, col); },
       [&](int row, int col, cpx v) { s.Fa[row * kTile + col] = v; }, dig, exc);
   contract_planes_tc(
-      g, gsz, T, g.tcBTE, 1, gsz.D(), nx,
+      g, gsz, T, g.tcBTE, 1, gsz.D(), nx, false,
       [&](int y, int col) {
         if (col < xfirst) return cpx{0.0, 0.0};
         double ax, az;
@@ -456,7 +462,7 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
       },
       dig, exc);
   contract_planes_tc(
-      g, gsz, T, g.tcBTE, 2, gsz.D(), nx,
+      g, gsz, T, g.tcBTE, 2, gsz.D(), nx, false,
       [&](int y, int col) {
         if (col < xfirst) return cpx{0.0, 0.0};
         double ax, az;
@@ -472,7 +478,7 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
       dig, exc);
   // beta_bar = R^T Zp_bar + R'^T dz_bar -> s.Fb
   contract_planes_tc(
-      g, gsz, T, g.tcBTE, 3, gsz.R(), nx,
+      g, gsz, T, g.tcBTE, 3, gsz.R(), nx, xfirst == 1,
       [&](int y, int col) {
         if (col < xfirst) return recon_T_mean_input(at(0, y, col), at(2, y, col));
         double ax, az;
@@ -482,7 +488,7 @@ __device__ void recon_T_tc(const Grid& g, const S& gsz, const cpx* __restrict__ 
       },
       [&](int row, int col, cpx v) { s.Fb[row * kTile + col] = v; }, dig, exc);
   contract_planes_tc(
-      g, gsz, T, g.tcBTE, 4, gsz.R(), nx,
+      g, gsz, T, g.tcBTE, 4, gsz.R(), nx, xfirst == 1,
       [&](int y, int col) {
         if (col < xfirst) return recon_T_mean_input(at(3, y, col), at(4, y, col));
         double ax, az;
@@ -525,16 +531,19 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
   const size_t KS = (size_t)KTr * 16 + 8;
   uint16_t* dA = reinterpret_cast<uint16_t*>(s.hc);             // [7][32][KS] digits of Fa
   uint16_t* dB = dA + (size_t)kDig * 32 * KS;                    // digits of Fb
-  int* exa = reinterpret_cast<int*>(dB + (size_t)kDig * 32 * KS);  // [2][kTile] column exponents
-  for (int i = threadIdx.x; i < 2 * kTile; i += blockDim.x) exa[i] = 0;
+  int* exa = reinterpret_cast<int*>(dB + (size_t)kDig * 32 * KS);  // [2][kTile] column exponents, mean's Im
+  auto own = [&](bool fb, int col) { return fb && col < xfirst; };
+  for (int i = threadIdx.x; i < 2 * kTile + 1; i += blockDim.x) exa[i] = 0;
   __syncthreads();
   for (int i = threadIdx.x; i < (gsz.D() + gsz.R()) * kTile; i += blockDim.x) {
     const bool fb = i >= gsz.D() * kTile;
     const int j = fb ? i - gsz.D() * kTile : i, row = j / kTile, col = j - row * kTile;
     if (col >= nx || (col < xfirst && !fb)) continue;
     const cpx v = (fb ? s.Fb : s.Fa)[row * kTile + col];
-    const int e = max(exp_field(v.re), exp_field(v.im));
+    int e = 0, eim = 0;
+    column_exponents(v, own(fb, col), e, eim);
     if (e) atomicMax(&exa[(fb ? kTile : 0) + col], e);
+    if (eim) atomicMax(&exa[2 * kTile], eim);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < 2 * KTr * 8 * kTile; i += blockDim.x) {
@@ -545,10 +554,10 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
       return (r < N && col < nx && (col >= xfirst || fb)) ? (fb ? s.Fb : s.Fa)[r * kTile + col] : cpx{0.0, 0.0};
     };
     const cpx v0 = at(row), v1 = at(row + 1);
-    const int ex = exa[(fb ? kTile : 0) + col] - 1022;
+    const int ex = exa[(fb ? kTile : 0) + col] - 1022, exi = own(fb, col) ? exa[2 * kTile] - 1022 : ex;
     uint32_t* d = reinterpret_cast<uint32_t*>((fb ? dB : dA) + (size_t)(2 * col) * KS + row);
     digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, 16 * KS);
-    digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, 16 * KS);
+    digits_pair(scaled56(v0.im, exi), scaled56(v1.im, exi), d + KS / 2, 16 * KS);
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
@@ -564,13 +573,14 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
     for (int b = 0; b < 3; ++b) {
       const uint16_t* d = b < 2 ? dA : dB;
       const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + kLongFoldShift;
+      const int ecoli = own(b == 2, col) ? col_exp(exa[2 * kTile]) - 64 + kLongFoldShift : ecol;
       long long sums[4];
       uint32_t R[4] = {0, 0, 0, 0};
       tc_tile<false, kLongFoldShift>(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int y = min(mt * 16 + gq + 8 * (r >> 1), gsz.Q() - 1);
-        v[b][r] = round_sum<kLongFoldShift>(sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + ecol);
+        v[b][r] = round_sum<kLongFoldShift>(sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + (r & 1 ? ecoli : ecol));
       }
     }
 #pragma unroll
@@ -598,37 +608,38 @@ __device__ __forceinline__ void quad_T_few(const Grid& g, const S& gsz, int z, i
   constexpr int TT = 4, NTHR = 256, NC = 2 * TT;
   const int KTr = (gsz.R() + 15) / 16, MTq = (gsz.Q() + 15) / 16;
   const size_t KS = (size_t)KTr * 16 + 8;
-  int* exc = reinterpret_cast<int*>(s.dig + (size_t)2 * kDig * NC * KS);  // [2][TT]
-  if (threadIdx.x < 2 * TT) exc[threadIdx.x] = 0;
+  int* exc = reinterpret_cast<int*>(s.dig + (size_t)2 * kDig * NC * KS);  // [2][TT], mean's Im
+  if (threadIdx.x < 2 * TT + 1) exc[threadIdx.x] = 0;
   __syncthreads();
   {
     // threads [0, 128) take Fa, the rest Fb; row pairs 2 (t / TT) + 64 k
     const int cls = threadIdx.x >> 7, col = threadIdx.x % TT, j0 = 2 * ((threadIdx.x & 127) / TT);
     const int N = cls ? gsz.R() : gsz.D();
     const cpx* F = cls ? s.Fb : s.Fa;
-    const bool on = col < nx && (col >= xfirst || cls);
+    const bool on = col < nx && (col >= xfirst || cls), own = cls && col < xfirst;
     cpx v[KP][2];
-    int e = 0;
+    int e = 0, eim = 0;
 #pragma unroll
     for (int k = 0; k < KP; ++k)
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         const int j = j0 + p + 64 * k;
         v[k][p] = (on && j < N) ? F[j * TT + col] : cpx{0.0, 0.0};
-        e = max(e, max(exp_field(v[k][p].re), exp_field(v[k][p].im)));
+        column_exponents(v[k][p], own, e, eim);
       }
 #pragma unroll
     for (int o = 16; o >= TT; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
     if ((threadIdx.x & 31) < TT) atomicMax(&exc[cls * TT + col], e);
+    if (eim) atomicMax(&exc[2 * TT], eim);
     __syncthreads();
-    const int ex = exc[cls * TT + col] - 1022;
+    const int ex = exc[cls * TT + col] - 1022, exi = own ? exc[2 * TT] - 1022 : ex;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
       const int j = j0 + 64 * k;
       if (j >= KTr * 16) break;
       uint32_t* d = reinterpret_cast<uint32_t*>(s.dig + ((size_t)cls * kDig * NC + 2 * col) * KS + j);
       digits_pair(scaled56(v[k][0].re, ex), scaled56(v[k][1].re, ex), d, NC * KS / 2);
-      digits_pair(scaled56(v[k][0].im, ex), scaled56(v[k][1].im, ex), d + KS / 2, NC * KS / 2);
+      digits_pair(scaled56(v[k][0].im, exi), scaled56(v[k][1].im, exi), d + KS / 2, NC * KS / 2);
     }
   }
   __syncthreads();
@@ -650,10 +661,12 @@ __device__ __forceinline__ void quad_T_few(const Grid& g, const S& gsz, int z, i
                      tc_row_addr(s.dig + (size_t)cls * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
                      (uint32_t)(4 * NC * KS), T, R);
       const int ecol = col_exp(exc[cls * TT + t]) - 64 + kLongFoldShift;
+      const int ecoli = cls && t < xfirst ? col_exp(exc[2 * TT]) - 64 + kLongFoldShift : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
-        const int e = g.tcWTE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
-        v[b][rr] = cpx{round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const int e = g.tcWTE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)];
+        v[b][rr] = cpx{round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
+                       round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
       }
     }
 #pragma unroll
@@ -677,7 +690,7 @@ __device__ __forceinline__ void recon_T_few(const Grid& g, const S& gsz, const c
   const cpx* Uc = Ub + (size_t)z * 5 * cs + x;
   const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
   few_contract<TT, NTHR, KP>(
-      gsz, g.tcBT, g.tcBTE, true, nx, s.dig,
+      gsz, g.tcBT, g.tcBTE, true, nx, xfirst == 1, s.dig,
       [&](int y, cpx (&o)[5]) {
         const cpx* b = Uc + (size_t)y * gsz.X();
         if (col < xfirst) {

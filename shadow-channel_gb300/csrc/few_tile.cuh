@@ -80,11 +80,12 @@ __device__ __forceinline__ void chain_sweep(int M, int steps, int l, bool on, do
 // third of a sum.  One pass of loads and three barriers for all inputs; a warp
 // per 16 rows of Fa or of Fb runs its tables' k-tiles as one stream with two
 // in flight.  Quadratures at 32x65x32, one instance: 62k -> 20k cycles a block
-// for the forward inputs.  dig: (all ? 5 : 3) inputs' digits and exponents; KP: plane pairs
+// for the forward inputs.  meancol: column 0 of inputs 3 and 4 is the (0, 0)
+// line's.  dig: (all ? 5 : 3) inputs' digits and exponents; KP: plane pairs
 // a thread holds (Q <= KP 2 NTHR / kTile).  Waits for the block's staged copies.
 template <int kTile, int NTHR, int KP, class S, class Load, class Table, class Comb>
 __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __restrict__ Wt, const int* __restrict__ WE,
-                                             bool all, int nx, uint16_t* dig, Load load, Table wq, Comb comb, cpx* Fa,
+                                             bool all, int nx, bool meancol, uint16_t* dig, Load load, Table wq, Comb comb, cpx* Fa,
                                              cpx* Fb) {
   static_assert(kTile == 4, "one 8-column digit tile");
   constexpr int NC = 2 * kTile;
@@ -92,14 +93,15 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
   const size_t KS = (size_t)KT * 16 + 8;
   const int nin = all ? 5 : 3;
   auto slot_of = [&](int q) { return all ? q : (q == 3 ? 2 : q); };
-  int* exc = reinterpret_cast<int*>(dig + (size_t)nin * kDig * NC * KS);  // [nin][kTile]
-  for (int i = threadIdx.x; i < nin * kTile; i += NTHR) exc[i] = 0;
+  int* exc = reinterpret_cast<int*>(dig + (size_t)nin * kDig * NC * KS);  // [nin][kTile], mean's Im [2]
+  const int own0 = nin * kTile - 3;  // the slot of input q's mean Im: own0 + q
+  for (int i = threadIdx.x; i < nin * kTile + 2; i += NTHR) exc[i] = 0;
   __syncthreads();
   const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
   constexpr int kStep = 2 * (NTHR / kTile);
   cpx v[KP][2][5];
   {
-    int e[5] = {0, 0, 0, 0, 0};
+    int e[5] = {0, 0, 0, 0, 0}, eim[5] = {0, 0, 0, 0, 0};
 #pragma unroll
     for (int k = 0; k < KP; ++k)
 #pragma unroll
@@ -109,7 +111,7 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
         for (int q = 0; q < 5; ++q) v[k][p][q] = cpx{0.0, 0.0};
         if (y < gsz.Q() && col < nx) load(y, v[k][p]);
 #pragma unroll
-        for (int q = 0; q < 5; ++q) e[q] = max(e[q], max(exp_field(v[k][p][q].re), exp_field(v[k][p][q].im)));
+        for (int q = 0; q < 5; ++q) column_exponents(v[k][p][q], q >= 3 && meancol && col == 0, e[q], eim[q]);
       }
     // lanes of a column lie kTile apart
 #pragma unroll
@@ -118,6 +120,7 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
 #pragma unroll
       for (int o = 16; o >= kTile; o >>= 1) e[q] = max(e[q], __shfl_xor_sync(0xffffffffu, e[q], o));
       if ((threadIdx.x & 31) < kTile) atomicMax(&exc[slot_of(q) * kTile + col], e[q]);
+      if (q >= 3 && eim[q]) atomicMax(&exc[own0 + q], eim[q]);
     }
   }
   __syncthreads();
@@ -125,13 +128,14 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
   for (int q = 0; q < 5; ++q) {
     if (!all && (q == 2 || q == 4)) continue;
     const int ex = exc[slot_of(q) * kTile + col] - 1022;
+    const int exi = q >= 3 && meancol && col == 0 ? exc[own0 + q] - 1022 : ex;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
       const int y = y0 + k * kStep;
       if (y >= KT * 16) break;
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)slot_of(q) * kDig * NC + 2 * col) * KS + y);
       digits_pair(scaled56(v[k][0][q].re, ex), scaled56(v[k][1][q].re, ex), d, NC * KS / 2);
-      digits_pair(scaled56(v[k][0][q].im, ex), scaled56(v[k][1][q].im, ex), d + KS / 2, NC * KS / 2);
+      digits_pair(scaled56(v[k][0][q].im, exi), scaled56(v[k][1][q].im, exi), d + KS / 2, NC * KS / 2);
     }
   }
   asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -153,11 +157,13 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
                      tc_row_addr(dig + (size_t)slot_of(q) * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
                      (uint32_t)(4 * NC * KS), T, R);
       const int ecol = col_exp(exc[slot_of(q) * kTile + t]) - 64 + kLongFoldShift;
+      const int ecoli = q >= 3 && meancol && t == 0 ? col_exp(exc[own0 + q]) - 64 + kLongFoldShift : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = min(mt * 16 + gq + 8 * rr, N - 1);
-        const int e = WE[(size_t)wq(q) * gsz.R() + row] + ecol;
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const int e = WE[(size_t)wq(q) * gsz.R() + row];
+        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         f[rr] = q == q0 ? val : comb(q, f[rr], val);
       }
     }

@@ -227,7 +227,7 @@ struct SolveSmem {
 // parameter kTile, which stands for the file's 16 inside them.
 
 // digits of one quadrature input for the tensor-core quadrature:
-// [7][2 kTile columns][KS] fp16 + kTile exponents
+// [7][2 kTile columns][KS] fp16 + kTile exponents and the mean line's second
 __host__ __device__ inline size_t solve_tc_kstride(const Grid& g) { return (size_t)((g.Q + 15) / 16) * 16 + 8; }
 
 // the FP64 quadrature's parity-combined inputs only where it runs (g.tc = 0)
@@ -235,7 +235,7 @@ template <int kTile>
 __host__ __device__ inline size_t solve_hc_elems(const Grid& g) {
   size_t hc = g.tc ? 0 : (size_t)g.Qh * kTile * 6, r = 2 * (size_t)g.R * kTile;
   const size_t tc =
-      ((size_t)kDig * 2 * kTile * solve_tc_kstride(g) * 2 + kTile * sizeof(int) + sizeof(cpx) - 1) / sizeof(cpx);
+      ((size_t)kDig * 2 * kTile * solve_tc_kstride(g) * 2 + (kTile + 1) * sizeof(int) + sizeof(cpx) - 1) / sizeof(cpx);
   if (r > hc) hc = r;
   return tc > hc ? tc : hc;
 }
@@ -268,7 +268,7 @@ __device__ inline SolveSmem carve_solve(const Grid& g, unsigned char* base) {
 // The FEW build's plan: digits of the 3 inputs (5 for the adjoint), right-
 // hand sides, F, the tile's factors
 __host__ __device__ inline size_t solve_few_dig_bytes(const Grid& g, int tile, bool adj) {
-  return ((size_t)(adj ? 5 : 3) * kDig * 2 * tile * solve_tc_kstride(g) * 2 + 5 * tile * sizeof(int) + 15) / 16 * 16;
+  return ((size_t)(adj ? 5 : 3) * kDig * 2 * tile * solve_tc_kstride(g) * 2 + (5 * tile + 2) * sizeof(int) + 15) / 16 * 16;
 }
 inline size_t solve_few_smem_bytes(const Grid& g, int tile, bool adj) {
   return solve_few_dig_bytes(g, tile, adj) + (size_t)tile * (3 * g.R + g.D) * sizeof(cpx) +
@@ -439,7 +439,8 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
   const int KT = (gsz.Q() + 15) / 16, MTw = (gsz.R() + 15) / 16;
   const size_t KS = (size_t)((gsz.Q() + 15) / 16) * 16 + 8;  // solve_tc_kstride
   uint16_t* dig = reinterpret_cast<uint16_t*>(s.hc);             // [7][NC][KS]
-  int* exc = reinterpret_cast<int*>(dig + (size_t)kDig * NC * KS);  // [kTile]
+  int* exc = reinterpret_cast<int*>(dig + (size_t)kDig * NC * KS);  // [kTile], mean's Im
+  const bool meancol = z == 0 && x0 == 0;
   const double kz = g.Kz[z];
   const size_t cs = (size_t)gsz.Q() * gsz.X();
   const cpx* Hz_ = H + (size_t)z * 5 * cs;  // slot c at Hz_ + c*cs + y*X + x
@@ -470,7 +471,8 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
     const int N = toA ? gsz.D() : gsz.R();
     cpx* F = toA ? s.Fa : s.Fb;
     const bool first = (q == 0 || q == 3);
-    for (int i = threadIdx.x; i < kTile; i += NTHR) exc[i] = 0;
+    for (int i = threadIdx.x; i < kTile + 1; i += NTHR) exc[i] = 0;
+    auto own = [&](int col) { return meancol && q >= 3 && col == 0; };
     __syncthreads();
     if (KT <= kQuadRegs && NTHR == 16 * kTile) {
       // thread t holds column t % kTile and the plane pairs 2 (t / kTile) +
@@ -479,41 +481,44 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
       const int col = threadIdx.x % kTile, y0 = 2 * (threadIdx.x / kTile);
       auto plane = [&](int k) { return y0 + 32 * (k >> 1) + (k & 1); };
       cpx vin[kQuadRegs];
-      int emax = 0;
+      int emax = 0, eim = 0;
 #pragma unroll
       for (int k = 0; k < kQuadRegs; ++k) {
         const int y = plane(k);
         vin[k] = (y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
-        emax = max(emax, max(exp_field(vin[k].re), exp_field(vin[k].im)));
+        column_exponents(vin[k], own(col), emax, eim);
       }
       if (emax) atomicMax(&exc[col], emax);
+      if (eim) atomicMax(&exc[kTile], eim);
       __syncthreads();
-      const int ex = exc[col] - 1022;
+      const int ex = exc[col] - 1022, exi = own(col) ? exc[kTile] - 1022 : ex;
 #pragma unroll
       for (int k = 0; k < kQuadRegs; k += 2) {
         const int y = plane(k);
         if (y >= KT * 16) break;
         uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
         digits_pair(scaled56(vin[k].re, ex), scaled56(vin[k + 1].re, ex), d, kTile * KS);
-        digits_pair(scaled56(vin[k].im, ex), scaled56(vin[k + 1].im, ex), d + KS / 2, kTile * KS);
+        digits_pair(scaled56(vin[k].im, exi), scaled56(vin[k + 1].im, exi), d + KS / 2, kTile * KS);
       }
     } else {
       for (int i = threadIdx.x; i < gsz.Q() * kTile; i += NTHR) {
         const int y = i / kTile, col = i - y * kTile;
         if (col >= nx) continue;
         const cpx v = input(q, y, col);
-        const int e = max(exp_field(v.re), exp_field(v.im));
+        int e = 0, eim = 0;
+        column_exponents(v, own(col), e, eim);
         if (e) atomicMax(&exc[col], e);
+        if (eim) atomicMax(&exc[kTile], eim);
       }
       __syncthreads();
       for (int i = threadIdx.x; i < KT * 8 * kTile; i += NTHR) {
         const int y = 2 * (i / kTile), col = i % kTile;
         const cpx v0 = (y < gsz.Q() && col < nx) ? input(q, y, col) : cpx{0.0, 0.0};
         const cpx v1 = (y + 1 < gsz.Q() && col < nx) ? input(q, y + 1, col) : cpx{0.0, 0.0};
-        const int ex = exc[col] - 1022;
+        const int ex = exc[col] - 1022, exi = own(col) ? exc[kTile] - 1022 : ex;
         uint32_t* d = reinterpret_cast<uint32_t*>(dig + (size_t)(2 * col) * KS + y);
         digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, kTile * KS);
-        digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, kTile * KS);
+        digits_pair(scaled56(v0.im, exi), scaled56(v1.im, exi), d + KS / 2, kTile * KS);
       }
     }
     __syncthreads();
@@ -522,6 +527,7 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
       const int mt = item / NT, nt = item - mt * NT;
       const int col = nt * 4 + t;
       const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
+      const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + kLongFoldShift : ecol;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
       tc_tile<true, kLongFoldShift>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
@@ -530,8 +536,9 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
       for (int rr = 0; rr < 2; ++rr) {
         const int row = mt * 16 + gq + 8 * rr;
         if (row >= N || col >= nx) continue;
-        const int e = g.tcWE[(size_t)w * gsz.R() + row] + ecol;
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const int e = g.tcWE[(size_t)w * gsz.R() + row];
+        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         cpx& f = F[row * kTile + col];
         if (first) {
           f = val;
@@ -562,7 +569,7 @@ __device__ void quad_rhs_few(const Grid& g, const S& gsz, const cpx* __restrict_
   const int lx = x0 + min((int)(threadIdx.x & 3), nx - 1);
   const double k2 = g.K2[(size_t)z * gsz.X() + lx];  // of this lane's output column
   few_contract<kTile, NTHR, KP>(
-      gsz, g.tcW, g.tcWE, adj, nx, s.dig,
+      gsz, g.tcW, g.tcWE, adj, nx, z == 0 && x0 == 0, s.dig,
       [&](int y, cpx (&o)[5]) {
         const cpx* b = Hc + (size_t)y * gsz.X();
         const cpx hz = b[0], hx = b[cs];

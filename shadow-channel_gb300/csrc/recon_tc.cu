@@ -179,7 +179,7 @@ __host__ __device__ inline int recon_tc_kstride(int KT) { return KT * 16 + 8; } 
 // tile: kx columns per block (16 or 8)
 size_t recon_tc_smem_bytes(const Grid& g, int tile) {
   const int KT = (g.R + 15) / 16;
-  return (size_t)2 * kDig * (2 * tile) * recon_tc_kstride(KT) * sizeof(uint16_t) + 2 * tile * sizeof(int);
+  return (size_t)2 * kDig * (2 * tile) * recon_tc_kstride(KT) * sizeof(uint16_t) + (2 * tile + 1) * sizeof(int);
 }
 
 size_t recon_tc_smem_bytes(const Grid& g) { return recon_tc_smem_bytes(g, kTile); }
@@ -188,12 +188,10 @@ size_t recon_tc_smem_bytes(const Grid& g) { return recon_tc_smem_bytes(g, kTile)
 // du = R' a, v = 0, w = R b, dw = R' b with a, b the real parts of alpha and
 // beta (a complex-to-real transform ignores the imaginary parts).  Its two
 // systems are Re and Im of the beta class's column 0: the contractions with R
-// and R' give (u, w) and (du, dw).  A non-finite imaginary part makes the
-// column NaN.
-__device__ __forceinline__ cpx mean_coefficients(const cpx& al, const cpx& be, int& e) {
-  e = max(e, max(exp_field(al.re), exp_field(be.re)));
-  if (exp_field(al.im) == 0x7FF || exp_field(be.im) == 0x7FF) e = 0x7FF;
-  return cpx{al.re, be.re};
+// and R' give (u, w) and (du, dw).  A non-finite imaginary part makes its
+// system's column NaN.
+__device__ __forceinline__ cpx mean_coefficients(const cpx& al, const cpx& be) {
+  return cpx{exp_field(al.im) == 0x7FF ? al.im : al.re, exp_field(be.im) == 0x7FF ? be.im : be.re};
 }
 
 // u, w and du/dy, dw/dy of a column from f = -Q' alpha, g = R beta and Q''
@@ -226,23 +224,27 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
   const bool meancol = (z == 0 && x0 == 0);  // column 0 of this tile is the mean mode
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* dig = reinterpret_cast<uint16_t*>(smem);  // [cls][digit][n 2 TILE][KS]
-  int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * (2 * TILE) * KS * sizeof(uint16_t));  // [cls][TILE]
+  int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * (2 * TILE) * KS * sizeof(uint16_t));  // [cls][TILE], mean's Im
   const cpx* __restrict__ C = a.C.at(inst);
   if (a.slot.stride) C += (long long)a.slot.slot() * a.slot.stride;
-  // coefficient (class, row, column), its exponent field joined into e
-  auto cval = [&](int cls, int j, int col, int& e) -> cpx {
+  auto mean_slot = [&](int cls, int col) { return meancol && cls == 1 && col == 0; };
+  auto im_slot = [&](int cls, int col) { return mean_slot(cls, col) ? 2 * TILE : cls * TILE + col; };
+  // coefficient (class, row, column), its exponent fields joined into e, eim
+  auto cval = [&](int cls, int j, int col, int& e, int& eim) -> cpx {
     const int K = cls == 0 ? gsz.D() : gsz.R();
     if (j >= K || col >= nx) return cpx{0.0, 0.0};
     const cpx* p = C + (((size_t)z * 2 + cls) * gsz.R() + j) * gsz.X() + x0 + col;
     if (meancol && col == 0) {
       if (cls == 0) return cpx{0.0, 0.0};
-      return mean_coefficients(*(p - (size_t)gsz.R() * gsz.X()), *p, e);
+      const cpx v = mean_coefficients(*(p - (size_t)gsz.R() * gsz.X()), *p);
+      column_exponents(v, true, e, eim);
+      return v;
     }
-    e = max(e, max(exp_field(p->re), exp_field(p->im)));
+    column_exponents(*p, false, e, eim);
     return *p;
   };
   // column exponents: |c| < 2^exc over the column's real and imaginary parts
-  for (int i = threadIdx.x; i < 2 * TILE; i += NTHR) exc[i] = 0;
+  for (int i = threadIdx.x; i < 2 * TILE + 1; i += NTHR) exc[i] = 0;
   __syncthreads();
   const int nent = 2 * (KT * 16) * TILE;
   if (KT <= kReconRegs && NTHR == 16 * TILE) {
@@ -253,46 +255,48 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
     const int col = threadIdx.x % TILE, j0 = 2 * (threadIdx.x / TILE);
     auto row = [&](int k) { return j0 + 32 * (k >> 1) + (k & 1); };
     cpx vin[2][kReconRegs];
-    int emax[2] = {0, 0};
+    int emax[2] = {0, 0}, eim = 0;
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls)
 #pragma unroll
       for (int k = 0; k < kReconRegs; ++k) {
-        vin[cls][k] = k < (KT + 1) / 2 * 2 ? cval(cls, row(k), col, emax[cls]) : cpx{0.0, 0.0};
+        vin[cls][k] = k < (KT + 1) / 2 * 2 ? cval(cls, row(k), col, emax[cls], eim) : cpx{0.0, 0.0};
       }
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls)
       if (emax[cls]) atomicMax(&exc[cls * TILE + col], emax[cls]);
+    if (eim) atomicMax(&exc[2 * TILE], eim);
     __syncthreads();
 #pragma unroll
     for (int cls = 0; cls < 2; ++cls) {
-      const int ex = exc[cls * TILE + col] - 1022;
+      const int ex = exc[cls * TILE + col] - 1022, exi = exc[im_slot(cls, col)] - 1022;
 #pragma unroll
       for (int k = 0; k < kReconRegs; k += 2) {
         if (k >= KT || row(k) >= KT * 16) break;
         // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
         uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col) * KS + row(k));
         digits_pair(scaled56(vin[cls][k].re, ex), scaled56(vin[cls][k + 1].re, ex), d, (size_t)TILE * KS);
-        digits_pair(scaled56(vin[cls][k].im, ex), scaled56(vin[cls][k + 1].im, ex), d + KS / 2, (size_t)TILE * KS);
+        digits_pair(scaled56(vin[cls][k].im, exi), scaled56(vin[cls][k + 1].im, exi), d + KS / 2, (size_t)TILE * KS);
       }
     }
   } else {
     for (int i = threadIdx.x; i < nent; i += NTHR) {
       const int cls = i / ((KT * 16) * TILE), r = i - cls * (KT * 16) * TILE, j = r / TILE, col = r - j * TILE;
-      int e = 0;
-      cval(cls, j, col, e);
+      int e = 0, eim = 0;
+      cval(cls, j, col, e, eim);
       if (e) atomicMax(&exc[cls * TILE + col], e);
+      if (eim) atomicMax(&exc[2 * TILE], eim);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < nent / 2; i += NTHR) {
       const int cls = i / ((KT * 8) * TILE), r = i - cls * (KT * 8) * TILE, j = 2 * (r / TILE), col = r % TILE;
-      int e = 0;
-      const cpx v0 = cval(cls, j, col, e), v1 = cval(cls, j + 1, col, e);
-      const int ex = exc[cls * TILE + col] - 1022;
+      int e = 0, eim = 0;
+      const cpx v0 = cval(cls, j, col, e, eim), v1 = cval(cls, j + 1, col, e, eim);
+      const int ex = exc[cls * TILE + col] - 1022, exi = exc[im_slot(cls, col)] - 1022;
       // digit q of column n at dig[((cls * 7 + q) * 2 TILE + n) * KS + j]
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * (2 * TILE) + 2 * col) * KS + j);
       digits_pair(scaled56(v0.re, ex), scaled56(v1.re, ex), d, (size_t)TILE * KS);
-      digits_pair(scaled56(v0.im, ex), scaled56(v1.im, ex), d + KS / 2, (size_t)TILE * KS);
+      digits_pair(scaled56(v0.im, exi), scaled56(v1.im, exi), d + KS / 2, (size_t)TILE * KS);
     }
   }
   __syncthreads();
@@ -311,6 +315,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
       const int b = order[ob], cls = b < 3 ? 0 : 1;
       const int KTb = ((cls == 0 ? gsz.D() : gsz.R()) + 15) / 16;
       const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kLongFoldShift;
+      const int ecoli = col_exp(exc[im_slot(cls, col)]) - 64 + kLongFoldShift;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
       tc_tile_range<(MINB <= 2), kLongFoldShift>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
@@ -321,8 +326,9 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
         const int y = mt * 16 + gq + 8 * rr;
         if (y >= gsz.Q() || col >= nx) continue;
         const bool mean = meancol && col == 0;
-        const int e = g.tcE[(size_t)b * gsz.Q() + y] + ecol;
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const int e = g.tcE[(size_t)b * gsz.Q() + y];
+        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         const int x = x0 + col;
         cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
         const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
@@ -365,38 +371,39 @@ __global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Gr
   const int KT = (gsz.R() + 15) / 16, KS = recon_tc_kstride(KT), MT = (gsz.Q() + 15) / 16;
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* dig = reinterpret_cast<uint16_t*>(smem);  // [cls][digit][n 2 TILE][KS]
-  int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * NC * KS * sizeof(uint16_t));  // [cls][TILE]
-  if (threadIdx.x < 2 * TILE) exc[threadIdx.x] = 0;
+  int* exc = reinterpret_cast<int*>(smem + (size_t)2 * kDig * NC * KS * sizeof(uint16_t));  // [cls][TILE], mean's Im
+  if (threadIdx.x < 2 * TILE + 1) exc[threadIdx.x] = 0;
   __syncthreads();
   {
     // threads [0, 128) the alpha rows, the rest the beta ones; row pairs 2 (t / TILE) + 64 k
     const int cls = threadIdx.x >> 7, col = threadIdx.x % TILE, j0 = 2 * ((threadIdx.x & 127) / TILE);
     const int K = cls == 0 ? gsz.D() : gsz.R();
-    const bool mean = meancol && col == 0, on = col < nx && !(mean && cls == 0);
+    const bool mean = meancol && col == 0, on = col < nx && !(mean && cls == 0), own = mean && cls == 1;
     const cpx* src = C + ((size_t)(z * 2 + cls) * gsz.R()) * gsz.X() + x0 + col;
     cpx v[KP][2];
-    int e = 0;
+    int e = 0, eim = 0;
 #pragma unroll
     for (int k = 0; k < KP; ++k)
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
         const int j = j0 + p + 64 * k;
         v[k][p] = (on && j < K) ? src[(size_t)j * gsz.X()] : cpx{0.0, 0.0};
-        if (mean && on && j < K) v[k][p] = mean_coefficients(src[((ptrdiff_t)j - gsz.R()) * gsz.X()], v[k][p], e);
-        else e = max(e, max(exp_field(v[k][p].re), exp_field(v[k][p].im)));
+        if (mean && on && j < K) v[k][p] = mean_coefficients(src[((ptrdiff_t)j - gsz.R()) * gsz.X()], v[k][p]);
+        column_exponents(v[k][p], own, e, eim);
       }
 #pragma unroll
     for (int o = 16; o >= TILE; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
     if ((threadIdx.x & 31) < TILE) atomicMax(&exc[cls * TILE + col], e);
+    if (eim) atomicMax(&exc[2 * TILE], eim);
     __syncthreads();
-    const int ex = exc[cls * TILE + col] - 1022;
+    const int ex = exc[cls * TILE + col] - 1022, exi = own ? exc[2 * TILE] - 1022 : ex;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
       const int j = j0 + 64 * k;
       if (j >= KT * 16) break;
       uint32_t* d = reinterpret_cast<uint32_t*>(dig + ((size_t)cls * kDig * NC + 2 * col) * KS + j);
       digits_pair(scaled56(v[k][0].re, ex), scaled56(v[k][1].re, ex), d, (size_t)NC * KS / 2);
-      digits_pair(scaled56(v[k][0].im, ex), scaled56(v[k][1].im, ex), d + KS / 2, (size_t)NC * KS / 2);
+      digits_pair(scaled56(v[k][0].im, exi), scaled56(v[k][1].im, exi), d + KS / 2, (size_t)NC * KS / 2);
     }
   }
   __syncthreads();
@@ -426,10 +433,12 @@ __global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Gr
       uint32_t R[4] = {0, 0, 0, 0};
       tc_tile_stream<kLongFoldShift>(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
       const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kLongFoldShift;
+      const int ecoli = meancol && cls == 1 && t == 0 ? col_exp(exc[2 * TILE]) - 64 + kLongFoldShift : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
-        const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)] + ecol;
-        const cpx v = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e), round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e)};
+        const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)];
+        const cpx v = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
+                       round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         if (part) val[1][rr] = v;
         else val[0][rr] = v;
       }

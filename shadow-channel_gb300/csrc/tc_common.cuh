@@ -100,6 +100,15 @@ __device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >
 static constexpr int kNanExp = 1 << 20;
 __device__ __forceinline__ int col_exp(int ce) { return ce == 0x7FF ? kNanExp : ce - 1022; }
 
+// The (0, 0) line's two real systems (u and w) run as Re and Im of one column of
+// a contraction.  They are independent, w often far below u, so each has an
+// exponent of its own (eim where `mean`).
+__device__ __forceinline__ void column_exponents(const cpx& v, bool mean, int& e, int& eim) {
+  const int im = exp_field(v.im);
+  e = max(e, max(exp_field(v.re), mean ? 0 : im));
+  if (mean) eim = max(eim, im);
+}
+
 // v * 2^(56 - ex) as an integer, rounded half away from zero, from the bit
 // pattern (integer ops only); ex bounds the column: |v| < 2^ex
 __device__ __forceinline__ long long scaled56(double v, int ex) {

@@ -6,10 +6,21 @@ tensor-core passes and agree with the FP64 kernels to rounding.  The oracle buil
 and without FMA contraction differs by at most (primal, tangent, adjoint)
 3.3e-13, 4.0e-13, 3.4e-13 there; the one-step parity tolerances 5e-12, 1e-11,
 3e-11 hold.
+
+A flow without spanwise variation whose spanwise velocity is 1e-10 of the
+streamwise one: w and the wall-normal vorticity, odd under spanwise reflection,
+keep their own relative accuracy through a step, in every build (the (0, 0)
+line's u and w are two columns of one contraction, with an exponent each).  The
+odd part alone (beta of kz = 0) is compared; the oracle built with and without
+FMA contraction differs in it by 7.5e-13, 6.3e-13, 8.8e-13 and (exact adjoint)
+1.3e-13, and the parity tolerances hold for it too.
 """
+import os
+
 import numpy as np
 import pytest
 
+import oracle as O
 from conftest import has_gpu
 from test_gpu_builds import _step
 
@@ -21,6 +32,62 @@ def test_long_transforms_match_the_fp64_kernels(case):
     if not has_gpu():
         pytest.skip("no CUDA device")
     from channel import c_channel as cc
-    for a, b, tol in zip(_step(cc, *case, False), _step(cc, *case, True), (5e-12, 1e-11, 3e-11, 3e-11)):
+    for a, b, tol in zip(_step(cc, *case, False), _step(cc, *case, True), PARITY):
         for s in range(a.shape[0]):
             assert np.linalg.norm(a[s] - b[s]) <= tol * np.linalg.norm(b[s])
+
+
+ODD_GRID = (16, 33, 16)
+PARITY = (5e-12, 1e-11, 3e-11, 3e-11)  # primal, tangent, adjoint, exact adjoint
+KNOBS = ("CHN_RECON_FP64", "CHN_TRANSFORMS_FP64", "CHN_SOLVE_TILE", "CHN_RECON_BUILD", "CHN_AUTOTUNE")
+
+
+def odd_state(seed, laminar):
+    Nx, Ny, Nz = ODD_GRID
+    C = O.synthetic_state(Nx, Ny, Nz, seed=seed, laminar=laminar)
+    C[1:] = 0.0
+    rng = np.random.default_rng(seed)
+    line = rng.standard_normal((2, 6)) * 0.1
+    C[0, 0, :6, 0] += line[0]
+    C[0, 1, :6, 0] += line[1]
+    C[0, 1] *= 1e-10
+    return C
+
+
+def odd_part(C):
+    return C[0, 1]
+
+
+def odd_step(cc, env):
+    old = {k: os.environ.pop(k, None) for k in KNOBS}
+    os.environ.update({"CHN_AUTOTUNE": "0", **env})
+    try:
+        assert cc.c_init(*ODD_GRID, 2 * np.pi, np.pi, 2000.0, 2.0, 0.004, 1) == 0, cc.c_last_error_message()
+        C, IC, AC = odd_state(1, True), odd_state(2, False), odd_state(3, False)
+        AX, flow = AC.copy(), np.zeros((3, 3 * ODD_GRID[0] // 2, cc.c_qpts(), 3 * ODD_GRID[2] // 2))
+        cc.c_spec2phys(C.copy(), flow)
+        cc.c_primal(0, C)
+        cc.c_tangent(0, 1, IC, 0)
+        cc.c_adjoint(1, 0, AC, 0, 0.0)
+        cc.c_adjoint_exact(1, 0, AX)
+        assert cc.c_last_error() == 0, cc.c_last_error_message()
+        cc.c_destroy()
+        return flow[2], [odd_part(x) for x in (C, IC, AC, AX)]
+    finally:
+        for k, v in old.items():
+            os.environ.pop(k, None)
+            if v is not None:
+                os.environ[k] = v
+
+
+@pytest.mark.parametrize("tile,recon", [(None, None), ("16", "0"), ("8", "1"), ("8/128", "2")])
+def test_a_small_spanwise_part_keeps_its_digits(tile, recon):
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    from channel import c_channel as cc
+    env = {"CHN_SOLVE_TILE": tile, "CHN_RECON_BUILD": recon} if tile else {}
+    w, tc = odd_step(cc, env)
+    w0, ref = odd_step(cc, {"CHN_RECON_FP64": "1", "CHN_TRANSFORMS_FP64": "1"})
+    assert np.abs(w - w0).max() <= 1e-14 * np.abs(w0).max()  # as test_gpu_recon_tc.py, of its own scale
+    for a, b, tol in zip(tc, ref, PARITY):
+        assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
