@@ -1101,15 +1101,16 @@ cudaError_t launch_solve_T(const Grid& g, const SolveTArgs& a, cudaStream_t st) 
   if (solveT_few(g, a)) {
     const dim3 grid(g.Nz * ((g.X + 3) / 4), a.ninst);
     const size_t sm = solveT_few_smem_bytes(g, 4);
-    if (sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
-    else if (sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
+    const bool fx = (g.fixed & FIXED_SOLVE) != 0;  // the solve's fixed-size choice covers its transpose
+    if (fx && sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
+    else if (fx && sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
     else if (g.Q <= 128 && g.R <= 64) k_solve_T<false, SizesRT, 4, 1><<<grid, kThreads, sm, st>>>(g, a);
     else k_solve_T<false, SizesRT, 4, 2><<<grid, kThreads, sm, st>>>(g, a);
     return cudaGetLastError();
   }
   const dim3 grid(g.Nz * ((g.X + kTile - 1) / kTile), a.ninst);
   const size_t sm = solveT_smem_bytes(g);
-  const bool fx = (g.fixed & FIXED_SOLVE) && !a.grids;  // the solve's fixed-size choice covers its transpose
+  const bool fx = (g.fixed & FIXED_SOLVE) && !a.grids;
   if (a.grids) k_solve_T<true, SizesRT><<<grid, kThreads, sm, st>>>(g, a);
   else if (fx && sizes_match<Sizes32>(g)) k_solve_T<false, Sizes32><<<grid, kThreads, sm, st>>>(g, a);
   else if (fx && sizes_match<Sizes16>(g)) k_solve_T<false, Sizes16><<<grid, kThreads, sm, st>>>(g, a);

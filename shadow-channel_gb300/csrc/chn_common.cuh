@@ -149,6 +149,8 @@ struct Grid {
   int adjpb;  // product planes per pass of the adjoint product modes (1 or 3; autotuned)
   int prodb;  // products build, bit 0 forward, bit 1 adjoint: 0 = the plan above, 1 = two planes per pass at 3 blocks per SM
               // (single-grid batches; autotuned)
+  int pfixed;  // CHN_PRODUCTS_BUILD (bits 0, 1) or CHN_ADJ_PRODUCTS_PER_PASS (bit 1) asked for a build of the
+               // forward / adjoint products: none of one component a block in its place
   // kernels that run their build compiled for the grid's sizes (32x65x32,
   // 16x33x16): FIXED_* bits of sizes.cuh (autotuned; the same results)
   int fixed;

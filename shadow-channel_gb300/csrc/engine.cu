@@ -245,6 +245,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // 1 (two planes per pass at 3 blocks per SM); CHN_PRODUCTS_BUILD fixes it
   const char* pbe = getenv("CHN_PRODUCTS_BUILD");
   g.prodb = (pbe && pbe[0] == '1' && pbe[1] == 0) ? 3 : 0;
+  g.pfixed = (pbe && pbe[0]) ? 3 : ((apb && apb[0]) ? 2 : 0);
   // the solve's block tile: 8 until the autotuner has timed both (a single
   // trajectory past the few-block builds: 128x129x128 0.80 -> 0.53 ms, 64x65x64
   // 0.073 -> 0.064; 16 columns leave the last wave of blocks half empty);

@@ -815,13 +815,14 @@ static void launch_products_b3(const Grid& g, const ProdArgs& a, int mode, cudaS
 }
 
 // The products' launches of few planes likewise: one component per block, the
-// adjoint modes through the scratch array and k_assemble.  Forward modes up to
+// adjoint modes through the scratch array and k_assemble (unless a switch asked
+// for a build of the others).  Forward modes up to
 // 3 planes per SM (one instance at 32x65x32 40 -> 25 us), adjoint modes up to 2
 // (76 -> 41); alone they gain up to 4 and 3 (8 of 16x33x16 39 -> 31, 64 -> 53),
 // but not beside the tangents' launches (the limits below: inverse_groups).
 int products_groups(const Grid& g, const ProdArgs& a, int mode) {
   const long long planes = (long long)g.Q * a.ninst;
-  if (a.grids) return 1;
+  if (a.grids || (g.pfixed & (mode < 2 ? 1 : 2))) return 1;
   if (mode < 2) return planes <= 3 * 152 ? 3 : 1;
   return planes <= 2 * 152 && a.tmp && a.ninst <= a.tmp_inst ? 6 : 1;
 }
@@ -835,8 +836,9 @@ cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaS
     const dim3 grid(g.Q, a.ninst, groups);
     const int xch = g.fxch < d.pzp ? g.fxch : d.pzp;
     const size_t sm = fwd_tc_smem_bytes(g, 1, xch);
-    if (xch == d.pzp && sizes_match<Sizes32>(g)) k_products_tc<false, 1, Sizes32><<<grid, kThreads, sm, st>>>(g, a, mode);
-    else if (xch == d.pzp && sizes_match<Sizes16>(g)) k_products_tc<false, 1, Sizes16><<<grid, kThreads, sm, st>>>(g, a, mode);
+    const bool fx = (g.fixed & FIXED_PRODUCTS) && xch == d.pzp;
+    if (fx && sizes_match<Sizes32>(g)) k_products_tc<false, 1, Sizes32><<<grid, kThreads, sm, st>>>(g, a, mode);
+    else if (fx && sizes_match<Sizes16>(g)) k_products_tc<false, 1, Sizes16><<<grid, kThreads, sm, st>>>(g, a, mode);
     else k_products_tc<false, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
     if (mode >= 2) launch_assemble(g, a, mode == 3, 0, a.ninst, st);
     return cudaGetLastError();

@@ -979,8 +979,9 @@ cudaError_t launch_solve(const Grid& g, const SolveArgs& a, cudaStream_t st) {
   if (solve_few(g, a)) {
     const dim3 grid(g.Nz * ((g.X + 3) / 4), a.ninst);
     const size_t sm = solve_few_smem_bytes(g, 4, a.adjoint != 0);
-    if (g.Q <= 128 && sizes_match<Sizes32>(g)) k_solve<false, 4, Sizes32, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
-    else if (g.Q <= 128 && sizes_match<Sizes16>(g)) k_solve<false, 4, Sizes16, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
+    const bool fx = (g.fixed & FIXED_SOLVE) != 0;
+    if (fx && sizes_match<Sizes32>(g)) k_solve<false, 4, Sizes32, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
+    else if (fx && sizes_match<Sizes16>(g)) k_solve<false, 4, Sizes16, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
     else if (g.Q <= 128) k_solve<false, 4, SizesRT, 256, 1, 1><<<grid, 256, sm, st>>>(g, a);
     else k_solve<false, 4, SizesRT, 256, 1, 2><<<grid, 256, sm, st>>>(g, a);
     return cudaGetLastError();

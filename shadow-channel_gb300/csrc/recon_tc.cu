@@ -488,8 +488,9 @@ cudaError_t launch_recon_tc(const Grid& g, const ReconArgs& a, cudaStream_t st) 
   if (!a.grids && !g.rfixed && g.R > 16 && g.R <= 128 && (long long)ntf * a.ninst <= kFewTiles) {
     const dim3 grid(ntf, a.ninst);
     const size_t sm = recon_tc_smem_bytes(g, 4);
-    if (sizes_match<Sizes32>(g)) k_recon_few<Sizes32, 1><<<grid, 256, sm, st>>>(g, a);
-    else if (sizes_match<Sizes16>(g)) k_recon_few<Sizes16, 1><<<grid, 256, sm, st>>>(g, a);
+    const bool fx = (g.fixed & FIXED_RECON) != 0;
+    if (fx && sizes_match<Sizes32>(g)) k_recon_few<Sizes32, 1><<<grid, 256, sm, st>>>(g, a);
+    else if (fx && sizes_match<Sizes16>(g)) k_recon_few<Sizes16, 1><<<grid, 256, sm, st>>>(g, a);
     else if (g.R <= 64) k_recon_few<SizesRT, 1><<<grid, 256, sm, st>>>(g, a);
     else k_recon_few<SizesRT, 2><<<grid, 256, sm, st>>>(g, a);
     return cudaGetLastError();
