@@ -14,6 +14,11 @@ line's u and w are two columns of one contraction, with an exponent each).  The
 odd part alone (beta of kz = 0) is compared; the oracle built with and without
 FMA contraction differs in it by 7.5e-13, 6.3e-13, 8.8e-13 and (exact adjoint)
 1.3e-13, and the parity tolerances hold for it too.
+
+The adjoint's two product passes as concurrent branches, which only launches of
+more than two planes an SM are (4 of 32x65x32, 7 of 16x33x16, 3 of 48x97x48),
+and products of one component a block, which launches of fewer are, give the
+bits of the passes in turn and of whole planes a block.
 """
 import os
 
@@ -22,6 +27,7 @@ import pytest
 
 import oracle as O
 from conftest import has_gpu
+import test_gpu_variants as V
 from test_gpu_builds import _step
 
 pytestmark = pytest.mark.gpu
@@ -91,3 +97,24 @@ def test_a_small_spanwise_part_keeps_its_digits(tile, recon):
     assert np.abs(w - w0).max() <= 1e-14 * np.abs(w0).max()  # as test_gpu_recon_tc.py, of its own scale
     for a, b, tol in zip(tc, ref, PARITY):
         assert np.linalg.norm(a - b) <= tol * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("gi,nseg,cache", [(0, 4, "1"), (0, 4, "0"), (2, 7, "1"), (2, 7, "0"), (1, 3, "1")])
+def test_concurrent_adjoint_passes_give_the_same_bits(monkeypatch, gi, nseg, cache):
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    from channel import c_channel as cc
+    monkeypatch.setattr(V, "NSEG", nseg)
+    assert 3 * V.GRIDS[gi][1] // 2 * nseg > 2 * 152
+    env = {"CHN_AUTOTUNE": "0", "CHN_NO_FIELD_CACHE": "1" if cache == "0" else "0"}
+    runs = [V._sweeps(cc, V.GRIDS[gi], {**env, "CHN_CONCURRENT_CHAINS": c})[0] for c in "01"]
+    V._same(*runs)
+
+
+@pytest.mark.parametrize("gi", [0, 1, 2])
+def test_products_of_one_component_a_block_give_the_same_bits(gi):
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    from channel import c_channel as cc
+    runs = [V._sweeps(cc, V.GRIDS[gi], {"CHN_AUTOTUNE": "0", **env})[0] for env in ({}, {"CHN_PRODUCTS_BUILD": "0"})]
+    V._same(*runs)
