@@ -83,6 +83,24 @@ CHN_HD void sum_minus(long long ta, uint32_t ra, long long tb, uint32_t rb, long
 template <int FS>
 CHN_HD long long sum_whole(long long t, uint32_t r) { return t + (r >> FS); }
 
+// bits of |t|: |t| < 2^n (0 for t = 0)
+CHN_HD int sum_bits(long long t) {
+  const unsigned long long a = (unsigned long long)(t < 0 ? -t : t);
+#ifdef __CUDA_ARCH__
+  return 64 - __clzll((long long)a);
+#else
+  return a ? 64 - __builtin_clzll(a) : 0;
+#endif
+}
+
+// exponent field of t 2^e, a sum of columns with the largest field ce: at least
+// 1 for what is not zero; 0x7FF (a column that comes out NaN) past FP64's range and where ce is
+CHN_HD int sum_field(long long t, int e, int ce) {
+  if (ce == 0x7FF) return 0x7FF;
+  const int f = sum_bits(t) + e + 1022;
+  return t == 0 ? 0 : (f < 1 ? 1 : (f > 0x7FF ? 0x7FF : f));
+}
+
 // The sum as one 64-bit integer whose conversion to FP64 rounds it correctly:
 // (t 2^FS + r) = x 2^(FS - up), exactly (FS 10: cut
 // to four units of level 6) while |t| < 2^54; from there on an FP64 value ends two bits or

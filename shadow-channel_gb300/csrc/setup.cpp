@@ -423,3 +423,6 @@ extern "C" int c_setup_digit_sum(int shift, const int* a, int na, const int* b, 
   if (shift == chn::kLongFoldShift) return digit_sum<chn::kLongFoldShift>(a, na, b, nb, op, first, out);
   return -2;
 }
+
+// the exponent field of a kept sum t 2^e from a column with the largest field ce
+extern "C" int c_setup_sum_field(long long t, int e, int ce) { return chn::sum_field(t, e, ce); }

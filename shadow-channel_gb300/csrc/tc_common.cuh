@@ -127,13 +127,6 @@ __device__ __forceinline__ long long scaled_sum(long long t, int s) {
   return t << min(-s, 63);
 }
 
-// bits of |t|: |t| < 2^n (0 for t = 0; one's complement of a negative t,
-// which at most loses the step to an exact power of two)
-__device__ __forceinline__ int sum_bits(long long t) {
-  const unsigned long long a = (unsigned long long)(t < 0 ? -t : t);
-  return 64 - __clzll((long long)a);
-}
-
 // the sum (t, r) (digit_sum.cuh) * 2^e, e that of t's unit, rounded once: one
 // FP64 conversion, the power of two added to the exponent field.  Zeros,
 // results outside the normal range and NaN columns (e >= kNanExp / 2) take the

@@ -8,6 +8,10 @@ off.  The word that is converted to FP64 has to give that sum correctly
 rounded, for one contraction and for the sum and difference of two (s = 8), or
 cut to four units first (s = 10, which has room for long rows).
 
+A sum that is kept between a transform's stages gives its column an exponent
+field: that of a NaN past FP64's range (a larger number would pass for a finite
+one, and hide a NaN beside it).
+
 A table's row exponents have to be those of its entries, whatever the row's
 length: a larger one gives away table bits.
 """
@@ -125,3 +129,12 @@ def test_legendre_row_exponents(lib, ny):
 def test_long_transforms_have_tables(lib, nz):
     """the inverse z stage: rows of 2 (Nz - 1) entries of at most 1"""
     assert (tables(lib, (8, 17, nz), 2) == 1).all()
+
+
+@pytest.mark.parametrize("t,e,ce,field", [
+    (0, 900, 1023, 0), (1, 0, 1023, 1023), (-1, 0, 1023, 1023), (2 ** 40, 0, 1023, 1063), (3, -1100, 5, 1),
+    (1, 1023, 2046, 2046), (1, 1024, 2046, 0x7FF), (2 ** 60, 972, 2046, 0x7FF), (-2 ** 60, 1030, 2046, 0x7FF),
+    (7, 0, 0x7FF, 0x7FF), (0, 0, 0x7FF, 0x7FF)])
+def test_exponent_field_of_a_kept_sum(lib, t, e, ce, field):
+    lib.c_setup_sum_field.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    assert lib.c_setup_sum_field(t, e, ce) == field
