@@ -398,18 +398,18 @@ __device__ void contract_planes_tc(const Grid& g, const S& gsz, const uint4* __r
   for (int item = warp; item < MTn * NT; item += blockDim.x >> 5) {
     const int mt = item / NT, nt = item - mt * NT;
     const int col = nt * 4 + t;
-    const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
-    const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + kLongFoldShift : ecol;
+    const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + LongFold().shift();
+    const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + LongFold().shift() : ecol;
     long long sums[4];
     uint32_t R[4] = {0, 0, 0, 0};
-    tc_tile<false, kLongFoldShift>(T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
+    tc_tile(LongFold(), T + (size_t)b * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       const int row = mt * 16 + gq + 8 * rr;
       if (row >= N || col >= nx) continue;
       const int e = TE[(size_t)b * gsz.R() + row];
-      const cpx val = {round_sum<kLongFoldShift>(sums[2 * rr], R[2 * rr], e + ecol),
-                       round_sum<kLongFoldShift>(sums[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+      const cpx val = {round_sum(LongFold(), sums[2 * rr], R[2 * rr], e + ecol),
+                       round_sum(LongFold(), sums[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
       comb(row, col, val);
     }
   }
@@ -572,15 +572,15 @@ __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, in
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const uint16_t* d = b < 2 ? dA : dB;
-      const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + kLongFoldShift;
-      const int ecoli = own(b == 2, col) ? col_exp(exa[2 * kTile]) - 64 + kLongFoldShift : ecol;
+      const int ecol = col_exp(exa[(b < 2 ? 0 : kTile) + min(col, kTile - 1)]) - 64 + LongFold().shift();
+      const int ecoli = own(b == 2, col) ? col_exp(exa[2 * kTile]) - 64 + LongFold().shift() : ecol;
       long long sums[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile<false, kLongFoldShift>(W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
+      tc_tile(LongFold(), W + (size_t)b * MTq * KTr * kDig * 32, mt, KTr, kChunkKT, d, KS, (size_t)32 * KS, nt * 8, lane, sums, R);
 #pragma unroll
       for (int r = 0; r < 4; ++r) {
         const int y = min(mt * 16 + gq + 8 * (r >> 1), gsz.Q() - 1);
-        v[b][r] = round_sum<kLongFoldShift>(sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + (r & 1 ? ecoli : ecol));
+        v[b][r] = round_sum(LongFold(), sums[r], R[r], g.tcWTE[(size_t)b * gsz.Q() + y] + (r & 1 ? ecoli : ecol));
       }
     }
 #pragma unroll
@@ -657,16 +657,16 @@ __device__ __forceinline__ void quad_T_few(const Grid& g, const S& gsz, int z, i
       const int cls = b < 2 ? 0 : 1, nm = mt + NTHR / 32;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_stream<kLongFoldShift>(pf, table(mt, b), b < 2 ? table(mt, b + 1) : (nm < MTq ? table(nm, 0) : nullptr), KTr,
+      tc_tile_stream(LongFold(), pf, table(mt, b), b < 2 ? table(mt, b + 1) : (nm < MTq ? table(nm, 0) : nullptr), KTr,
                      tc_row_addr(s.dig + (size_t)cls * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
                      (uint32_t)(4 * NC * KS), T, R);
-      const int ecol = col_exp(exc[cls * TT + t]) - 64 + kLongFoldShift;
-      const int ecoli = cls && t < xfirst ? col_exp(exc[2 * TT]) - 64 + kLongFoldShift : ecol;
+      const int ecol = col_exp(exc[cls * TT + t]) - 64 + LongFold().shift();
+      const int ecoli = cls && t < xfirst ? col_exp(exc[2 * TT]) - 64 + LongFold().shift() : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int e = g.tcWTE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)];
-        v[b][rr] = cpx{round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
-                       round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+        v[b][rr] = cpx{round_sum(LongFold(), T[2 * rr], R[2 * rr], e + ecol),
+                       round_sum(LongFold(), T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
       }
     }
 #pragma unroll

@@ -144,6 +144,7 @@ struct Grid {
   const uint32_t* tcFZ;
   const int* tcFZE;
   int tcf;
+  int tcfl;   // the forward tables have rows too long for Fold's sums (digit_sum.cuh)
   int fwdpb;  // product planes per pass of the forward modes (3, or 1 where 3 leave no room for two blocks)
   int fxch;   // x-stage columns per chunk of the forward products (a multiple of 8; all where they fit)
   int adjpb;  // product planes per pass of the adjoint product modes (1 or 3; autotuned)

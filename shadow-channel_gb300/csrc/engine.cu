@@ -191,6 +191,13 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
     std::vector<uint32_t> fxf, fzf, fuf;
     std::vector<int> fxe, fze, fue;
     tct_ok = ci >= kChunkKT && build_fwd_split_tables(h, fxf, fxe, fzf, fze, fuf, fue, long_fwd) >= kChunkKT;
+    // from Nz = 196 on the inverse's rows are too long for the sums kept between
+    // its stages.  Planes of that length fit one block of the FFT kernels, or
+    // are not accepted, and batches are faster there than as DFTs: inverse and
+    // products of 32 instances of 8x17x200 1.03 / 0.59 ms, 2.47 / 1.23 as split
+    // tensor-core passes, the products 1.00 in one-block ones
+    tct_ok = tct_ok && !long_inv;
+    g.tcfl = long_fwd ? 1 : 0;
     g.tcch = ci;
     if (!T.up_digits(fxf, &g.tcFX) || !T.up(fxe, &g.tcFXE) || !T.up_digits(fzf, &g.tcFZ) || !T.up(fze, &g.tcFZE) ||
         !T.up_digits(fuf, &g.tcFXU) || !T.up(fue, &g.tcFXUE))
@@ -214,14 +221,12 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // reconstruction and quadratures on the tensor cores unless CHN_RECON_FP64=1 (or it does not fit)
   const char* fp64 = getenv("CHN_RECON_FP64");
   g.tc = (tc_ok && !(fp64 && fp64[0] == '1') && recon_tc_smem_bytes(g) + 4096 <= (size_t)optin) ? 1 : 0;
-  // inverse transforms on the tensor cores unless CHN_TRANSFORMS_FP64=1 (or they
-  // do not fit; a plane long and narrow enough for one block, Nx or Nz past 130,
-  // whose sums between the stages would lose bits takes the split passes)
+  // inverse transforms on the tensor cores unless CHN_TRANSFORMS_FP64=1 (or they do not fit)
   const char* tfp64 = getenv("CHN_TRANSFORMS_FP64");
-  g.tci = (tct_ok && !long_inv && !(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
+  g.tci = (tct_ok && !(tfp64 && tfp64[0] == '1') && phys_tc_fits(g, optin)) ? 1 : 0;
   g.fwdpb = 3;
   g.fxch = 8;
-  g.tcf = (tct_ok && !long_fwd && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
+  g.tcf = (tct_ok && !(tfp64 && tfp64[0] == '1') && fwd_tc_plan(g, optin, g.fwdpb, g.fxch)) ? 1 : 0;
   // and as split tensor-core passes where a plane does not fit one block
   g.tcs = (tct_ok && !(tfp64 && tfp64[0] == '1') && !(force && force[0] == '1') && phys_tcs_fits(g, optin)) ? 1 : 0;
   // the kernels' builds compiled for the grid's sizes where it has them
@@ -2644,6 +2649,7 @@ int c_multi_init(int n, const int* Nx, const int* Ny, const int* Nz, const doubl
     gmax.tc = std::min(gmax.tc, g.tc);
     gmax.tci = std::min(gmax.tci, g.tci);
     gmax.tcf = std::min(gmax.tcf, g.tcf);
+    gmax.tcfl = std::max(gmax.tcfl, g.tcfl);
   }
   // an even padded z length's digits, split in two classes, can take a k-tile
   // more than those of the next odd length: a mixed batch is sized as even

@@ -153,17 +153,17 @@ __device__ __forceinline__ void few_contract(const S& gsz, const uint32_t* __res
     for (int q = q0; q < q1; ++q) {
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_stream<kLongFoldShift>(pf, table(q), q + 1 < q1 ? table(q + 1) : nullptr, KT,
+      tc_tile_stream(LongFold(), pf, table(q), q + 1 < q1 ? table(q + 1) : nullptr, KT,
                      tc_row_addr(dig + (size_t)slot_of(q) * kDig * NC * KS, KS, (size_t)NC * KS, 0, lane),
                      (uint32_t)(4 * NC * KS), T, R);
-      const int ecol = col_exp(exc[slot_of(q) * kTile + t]) - 64 + kLongFoldShift;
-      const int ecoli = q >= 3 && meancol && t == 0 ? col_exp(exc[own0 + q]) - 64 + kLongFoldShift : ecol;
+      const int ecol = col_exp(exc[slot_of(q) * kTile + t]) - 64 + LongFold().shift();
+      const int ecoli = q >= 3 && meancol && t == 0 ? col_exp(exc[own0 + q]) - 64 + LongFold().shift() : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = min(mt * 16 + gq + 8 * rr, N - 1);
         const int e = WE[(size_t)wq(q) * gsz.R() + row];
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
-                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+        const cpx val = {round_sum(LongFold(), T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum(LongFold(), T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         f[rr] = q == q0 ? val : comb(q, f[rr], val);
       }
     }

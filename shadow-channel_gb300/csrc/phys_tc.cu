@@ -218,7 +218,9 @@ int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, st
         Az[(size_t)(2 * e + 1) * K + 2 * zp + 1] = cs;
       }
     }
-    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, 512, &long_rows));
+    // (an odd length's inputs are no sums: 56 bits)
+    const int top = d.Rz == 2 ? 512 : 256;
+    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, top, &long_rows));
   }
   return chunk;
 }
@@ -344,6 +346,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
   constexpr int nwarp = NTHR >> 5;
   const int Kk = gsz.Nz() - 1;  // kept kz rows
   const int chunk = gsz.tcch();
+  const auto fold = gsz.fold();
   bool nonfinite = false;
   // this block's fields: all of them, or one of gridDim.z groups
   const int fper = (a.nfields + gridDim.z - 1) / gridDim.z, fbeg = blockIdx.z * fper;
@@ -392,7 +395,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
     __syncthreads();
     {
       // rows Re Z[m], Im Z[m] for m < pzh; E + O -> Z[m], E - O -> Z[m + pzh],
-      // kept as 64-bit sums, rounded to kFoldShift's unit (scale 2^zsum_exp(column): the rows of
+      // kept as 64-bit sums, rounded to their unit (scale 2^zsum_exp(column): the rows of
       // this table share one exponent) that the x stage takes its digits
       // from; the exponent of each value into its x-stage column (fl, m) (not
       // the imaginary part of the kx = 0 bin, which c2r ignores)
@@ -401,10 +404,11 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
       for (int item = warp; item < d.MTz * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long TE[4], TO[4];
-        uint32_t RE[4] = {kFoldHalf, kFoldHalf, kFoldHalf, kFoldHalf}, RO[4] = {0, 0, 0, 0};
-        tc_tile_range(Az, mt, d.KTz, 0, d.KTzE, chunk, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
-        const Rests<kPackRests<S>> rE(RE);
-        tc_tile_range(Az, mt, d.KTz, d.KTzE, d.KTz, chunk, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
+        const uint32_t h = fold_half(fold);
+        uint32_t RE[4] = {h, h, h, h}, RO[4] = {0, 0, 0, 0};
+        tc_tile_range(fold, Az, mt, d.KTz, 0, d.KTzE, chunk, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
+        const Rests<kPackRests<S>, Fold> rE(RE);
+        tc_tile_range(fold, Az, mt, d.KTz, d.KTzE, d.KTz, chunk, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const int row = mt * 16 + gq + 8 * (r >> 1), col = nt * 8 + 2 * t + (r & 1);
@@ -418,19 +422,19 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
           long long t;
           uint32_t rest;
           sum_plus(TE[r], rE[r], TO[r], RO[r], t, rest);
-          const long long tp = sum_whole<kFoldShift>(t, rest);
+          const long long tp = sum_whole(fold, t, rest);
           longlong2& zp = Zs[((size_t)fl * gsz.pz() + m) * gsz.X() + x];
           if (im) zp.y = tp;
           else zp.x = tp;
-          const int ep = zsum_field(tp, ce);
+          const int ep = zsum_field(tp, ce, fold.shift());
           if (counts && ep > 0) atomicMax(&exx[fl * gsz.pz() + m], ep);
           if (d.Rz == 2) {
-            sum_minus<kFoldShift>(TE[r], rE[r], TO[r], RO[r], t, rest);
-            const long long tm = sum_whole<kFoldShift>(t, rest);
+            sum_minus(fold, TE[r], rE[r], TO[r], RO[r], t, rest);
+            const long long tm = sum_whole(fold, t, rest);
             longlong2& zm = Zs[((size_t)fl * gsz.pz() + m + d.pzh) * gsz.X() + x];
             if (im) zm.y = tm;
             else zm.x = tm;
-            const int em = zsum_field(tm, ce);
+            const int em = zsum_field(tm, ce, fold.shift());
             if (counts && em > 0) atomicMax(&exx[fl * gsz.pz() + m + d.pzh], em);
           }
         }
@@ -456,7 +460,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
             if (j == 0) v.y = 0;
             int fl = 0, m = n;  // n = fl pz + m
             while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
-            const int s = exx[n] - 1078 - zsum_exp(exz[fl * gsz.X() + j]);
+            const int s = exx[n] - 1078 - zsum_exp(exz[fl * gsz.X() + j], fold.shift());
             v.x = scaled_sum(v.x, s);
             v.y = scaled_sum(v.y, s);
           }
@@ -474,19 +478,19 @@ __global__ void __launch_bounds__(NTHR, MINB) k_phys_inverse_tc(const __grid_con
           const int mt = item / NT, nt = item - mt * NT;
           long long TE[4], TO[4];
           uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
-          tc_tile_range(Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE, RE);
-          const Rests<kPackRests<S>> rE(RE);
-          tc_tile_range(Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO, RO);
+          tc_tile_range(fold, Ax, mt, d.KTx, 0, d.KTxE, chunk, dig, d.KSx, xstride, nt * 8, lane, TE, RE);
+          const Rests<kPackRests<S>, Fold> rE(RE);
+          tc_tile_range(fold, Ax, mt, d.KTx, d.KTxE, d.KTx, chunk, dig, d.KSx, xstride, nt * 8, lane, TO, RO);
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const int xp = mt * 16 + gq + 8 * (r >> 1), col = n0 + nt * 8 + 2 * t + (r & 1);
             if (xp >= d.pxh || col >= ncx) continue;
             int fl = 0, m = col;  // col = fl pz + m, fl < FB
             while (m >= gsz.pz()) { m -= gsz.pz(); ++fl; }
-            const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + kFoldShift;
+            const int e = g.tcXE[xp] + col_exp(exx[col]) - 64 + fold.shift();
             double* Pr = P + ((size_t)(f0 + fl) * gsz.Q() + y) * plane + (size_t)m * gsz.px();
-            Pr[xp] = round_plus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
-            if (d.Rx == 2) Pr[xp + d.pxh] = round_minus(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+            Pr[xp] = round_plus(fold, TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+            if (d.Rx == 2) Pr[xp + d.pxh] = round_minus(fold, TE[r], rE[r], TO[r], RO[r], e, nonfinite);
           }
         }
       }
@@ -580,7 +584,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
   // the plan's (Grid::fxch, a multiple of 8)
   int XCH = d.pzp;
   if constexpr (MINB > 2) XCH = fwd_tc_xch_n(gsz.Nz(), gsz.X(), gsz.pz(), gsz.px(), PB, MINB);
-  else if constexpr (std::is_same<S, SizesRT>::value) XCH = min(g.fxch, d.pzp);
+  else if constexpr (kRunTimeSizes<S>) XCH = min(g.fxch, d.pzp);
   {
     const size_t dx = (size_t)kDig * XCH * d.KSx * 2, dz = (size_t)kDig * d.Xp * d.KSz * 2;
     p += ((dx > dz ? dx : dz) + 15) / 16 * 16;
@@ -599,6 +603,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
   const uint4* __restrict__ Az = reinterpret_cast<const uint4*>(g.tcFZ);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, t = lane & 3;
   constexpr int nwarp = NTHR >> 5;
+  const auto fold = gsz.fold();
   // this block's components: all of them, or one of gridDim.z groups
   const int nall = mode >= 2 ? 6 : 3, qper = (nall + gridDim.z - 1) / gridDim.z, qbeg = blockIdx.z * qper;
   const int ncomp = min(nall, qbeg + qper);
@@ -629,7 +634,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
           if (e) atomicMax(&exx3[cc * exs + row], e);
         }
       };
-      if constexpr (std::is_same<S, SizesRT>::value) {
+      if constexpr (kRunTimeSizes<S>) {
         for (int i = threadIdx.x; i < gsz.pz() * gsz.px(); i += NTHR, rc.next()) point(i);
       } else {
 #pragma unroll 3
@@ -655,8 +660,9 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
       for (int item = warp; item < d.MTx * NT; item += nwarp) {
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
-        uint32_t R[4] = {kFoldHalf, kFoldHalf, kFoldHalf, kFoldHalf};  // (kept as T alone)
-        tc_tile(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, xstride, nt * 8, lane, T,
+        const uint32_t h = fold_half(fold);
+        uint32_t R[4] = {h, h, h, h};  // (kept as T alone)
+        tc_tile(fold, Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, xstride, nt * 8, lane, T,
                 R);
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
@@ -672,7 +678,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
             longlong2& yv = Yb[(size_t)zp * gsz.X() + kx];
             if (row.part) yv.y = tv;
             else yv.x = tv;
-            ef = max(ef, sum_field(tv, er + ysum_exp(exx[zp]), exx[zp]));
+            ef = max(ef, sum_field(tv, er + ysum_exp(exx[zp], fold.shift()), exx[zp]));
           }
           if (ef > 0) atomicMax(&exz[kx], ef);
         }
@@ -690,7 +696,7 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
           const int2 er = *reinterpret_cast<const int2*>(AxE + 2 * ((n & 1) * d.nxE + (n >> 1)));
           auto input = [&](int z) {
             longlong2 w = Yb[(size_t)z * gsz.X() + n];
-            const int s = exz[n] - 1078 - ysum_exp(exx[z]);
+            const int s = exz[n] - 1078 - ysum_exp(exx[z], fold.shift());
             w.x = scaled_sum(w.x, s - er.x);
             w.y = scaled_sum(w.y, s - er.y);
             return w;
@@ -709,20 +715,20 @@ __global__ void __launch_bounds__(NTHR, MINB) k_products_tc(const __grid_constan
         const int mt = item / NT, nt = item - mt * NT;
         long long T[4];
         uint32_t R[4] = {0, 0, 0, 0};
-        tc_tile(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, zstride, nt * 8, lane, T,
+        tc_tile(fold, Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, zstride, nt * 8, lane, T,
                 R);
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
           FwdRow row;
           if (!fwd_row(mt, gq + 8 * rr, d.MTzE, d.nzE, d.nzO, row)) continue;
-          const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + kFoldShift;
+          const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + fold.shift();
           const int kk = fwd_z_mode(gsz.Nz(), d.Rz, row.cls, row.e);
 #pragma unroll
           for (int c2 = 0; c2 < 2; ++c2) {
             const int kx = nt * 8 + 2 * t + c2;
             if (kx >= gsz.X()) continue;
             reinterpret_cast<double*>(Fb + (size_t)kk * gsz.X() + kx)[row.part] =
-                round_sum(T[2 * rr + c2], R[2 * rr + c2], er + col_exp(exz[kx]));
+                round_sum(fold, T[2 * rr + c2], R[2 * rr + c2], er + col_exp(exz[kx]));
           }
         }
       }
@@ -792,15 +798,16 @@ bool fwd_tc_fits(const Grid& g, int optin) {
 template <class S>
 static void launch_products_sizes(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st) {
   const FwdTcDims d = fwd_tc_dims(g);
-  const int xch = std::is_same<S, SizesRT>::value ? (g.fxch < d.pzp ? g.fxch : d.pzp) : d.pzp;
+  const int xch = kRunTimeSizes<S> ? (g.fxch < d.pzp ? g.fxch : d.pzp) : d.pzp;
   const size_t sm = fwd_tc_smem_bytes(g, products_per_pass(g, mode), xch);
   const dim3 grid(g.Q, a.ninst);
-  constexpr bool M = std::is_same<S, SizesRT>::value;  // only the run-time sizes serve uneven batches
+  constexpr bool M = kRunTimeSizes<S>;  // only the run-time sizes serve uneven batches
+  using RunTime = std::conditional_t<M, S, SizesRT>;
   if (products_per_pass(g, mode) == kPB) {
-    if (M && a.grids) k_products_tc<true, kPB, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
+    if (M && a.grids) k_products_tc<true, kPB, RunTime><<<grid, kThreads, sm, st>>>(g, a, mode);
     else k_products_tc<false, kPB, S><<<grid, kThreads, sm, st>>>(g, a, mode);
   } else {
-    if (M && a.grids) k_products_tc<true, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
+    if (M && a.grids) k_products_tc<true, 1, RunTime><<<grid, kThreads, sm, st>>>(g, a, mode);
     else k_products_tc<false, 1, S, 2, M ? kWideThreads : kThreads><<<grid, M ? kWideThreads : kThreads, sm, st>>>(g, a, mode);
   }
 }
@@ -839,6 +846,7 @@ cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaS
     const bool fx = (g.fixed & FIXED_PRODUCTS) && xch == d.pzp;
     if (fx && sizes_match<Sizes32>(g)) k_products_tc<false, 1, Sizes32><<<grid, kThreads, sm, st>>>(g, a, mode);
     else if (fx && sizes_match<Sizes16>(g)) k_products_tc<false, 1, Sizes16><<<grid, kThreads, sm, st>>>(g, a, mode);
+    else if (g.tcfl) k_products_tc<false, 1, SizesLong><<<grid, kThreads, sm, st>>>(g, a, mode);
     else k_products_tc<false, 1, SizesRT><<<grid, kThreads, sm, st>>>(g, a, mode);
     if (mode >= 2) launch_assemble(g, a, mode == 3, 0, a.ninst, st);
     return cudaGetLastError();
@@ -847,12 +855,14 @@ cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaS
     const bool fx = (g.fixed & FIXED_PRODUCTS) != 0;
     if (fx && sizes_match<Sizes32>(g)) launch_products_b3<Sizes32>(g, a, mode, st);
     else if (fx && sizes_match<Sizes16>(g)) launch_products_b3<Sizes16>(g, a, mode, st);
+    else if (g.tcfl) launch_products_b3<SizesLong>(g, a, mode, st);
     else launch_products_b3<SizesRT>(g, a, mode, st);
     return cudaGetLastError();
   }
   const bool fx = (g.fixed & FIXED_PRODUCTS) && !a.grids && g.fxch >= fwd_tc_dims(g).pzp;
   if (fx && sizes_match<Sizes32>(g)) launch_products_sizes<Sizes32>(g, a, mode, st);
   else if (fx && sizes_match<Sizes16>(g)) launch_products_sizes<Sizes16>(g, a, mode, st);
+  else if (g.tcfl) launch_products_sizes<SizesLong>(g, a, mode, st);
   else launch_products_sizes<SizesRT>(g, a, mode, st);
   return cudaGetLastError();
 }
@@ -976,6 +986,12 @@ void prepare_phys_tc(int optin) {
   allow_max_smem(k_products_tc<false, 1, RT>, optin);
   allow_max_smem(k_products_tc<false, 1, RT, 2, kWideThreads>, optin);
   allow_max_smem(k_products_tc<true, 1, RT>, optin);
+  allow_max_smem(k_products_tc<false, kPB, SizesLong>, optin);
+  allow_max_smem(k_products_tc<true, kPB, SizesLong>, optin);
+  allow_max_smem(k_products_tc<false, 1, SizesLong>, optin);
+  allow_max_smem(k_products_tc<false, 1, SizesLong, 2, kWideThreads>, optin);
+  allow_max_smem(k_products_tc<true, 1, SizesLong>, optin);
+  allow_max_smem(k_products_tc<false, 2, SizesLong, 3>, optin);
   allow_max_smem(k_products_tc<false, kPB, Sizes32>, optin);
   allow_max_smem(k_products_tc<false, 2, SizesRT, 3>, optin);
   allow_max_smem(k_products_tc<false, 2, Sizes32, 3>, optin);

@@ -62,15 +62,15 @@ __host__ __device__ inline PhysTcDims phys_tc_dims(const Grid& g, int fb = kFB) 
   return phys_tc_dims_n(g.Nz, g.pz, g.px, g.X, fb);
 }
 
-// the folded sums t of the z stage (every row of its table has the exponent
-// kZRowExp) of a column whose largest input exponent field is ce: the value is
-// t 2^zsum_exp(ce); zsum_field: its exponent field (<= 0 for zeros; 0x7FF where
+// the folded sums t (unit 2^fs) of the z stage (every row of its table has the
+// exponent kZRowExp) of a column whose largest input exponent field is ce: the
+// value is t 2^zsum_exp(ce); zsum_field: its exponent field (<= 0 for zeros; 0x7FF where
 // the column held an infinity or a NaN)
 static constexpr int kZRowExp = 1;
-__device__ __forceinline__ int zsum_exp(int ce) { return kZRowExp + ce - 1022 - 64 + kFoldShift; }
-__device__ __forceinline__ int zsum_field(long long t, int ce) { return sum_field(t, zsum_exp(ce), ce); }
+__device__ __forceinline__ int zsum_exp(int ce, int fs) { return kZRowExp + ce - 1022 - 64 + fs; }
+__device__ __forceinline__ int zsum_field(long long t, int ce, int fs) { return sum_field(t, zsum_exp(ce, fs), ce); }
 // of the forward x stage, without its row's exponent
-__device__ __forceinline__ int ysum_exp(int ce) { return ce - 1022 - 64 + kFoldShift; }
+__device__ __forceinline__ int ysum_exp(int ce, int fs) { return ce - 1022 - 64 + fs; }
 
 // Dimensions of the forward transforms as digit GEMMs, the x stage (px is even)
 // and for an even pz the z stage split radix-2 (decimation in frequency: the even outputs are the

@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             const bool im = r >= d.pzh;
             const int m = im ? r - d.pzh : r;
             long long tE = 0;
-            uint32_t rE = kFoldHalf;
+            uint32_t rE = fold_half(Fold());
             fold_levels(c, tE, rE);
             reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m) * g.X + x])[im ? 1 : 0] = tE;
             reinterpret_cast<long long*>(&Zb[((size_t)f * g.pz + m + d.pzh) * g.X + x])[im ? 1 : 0] = rE;
@@ -439,13 +439,13 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
             uint32_t rO = 0, rest = 0;
             fold_levels(c, tO, rO);
             sum_plus(tE, rE, tO, rO, tv, rest);
-            const long long tp = sum_whole<kFoldShift>(tv, rest);
-            sum_minus<kFoldShift>(tE, rE, tO, rO, tv, rest);
-            const long long tq = sum_whole<kFoldShift>(tv, rest);
+            const long long tp = sum_whole(Fold(), tv, rest);
+            sum_minus(Fold(), tE, rE, tO, rO, tv, rest);
+            const long long tq = sum_whole(Fold(), tv, rest);
             *sp_ = tp;
             *sm_ = tq;
             if (!(im && x == 0)) {  // c2r ignores the imaginary part of the kx = 0 bin
-              const int ep = zsum_field(tp, ez), em = zsum_field(tq, ez);
+              const int ep = zsum_field(tp, ez, Fold().shift()), em = zsum_field(tq, ez, Fold().shift());
               if (ep > 0) atomicMax(&exx[f * g.pz + m], ep);
               if (em > 0) atomicMax(&exx[f * g.pz + m + d.pzh], em);
             }
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
         if (nl < nct && j >= 0) {
           v = reinterpret_cast<const longlong2*>(Zb)[(size_t)n * g.X + j];
           if (j == 0) v.y = 0;
-          const int s = exx[n] - 1078 - zsum_exp(exz[n / g.pz * g.X + j]);
+          const int s = exx[n] - 1078 - zsum_exp(exz[n / g.pz * g.X + j], Fold().shift());
           v.x = scaled_sum(v.x, s);
           v.y = scaled_sum(v.y, s);
         }
@@ -520,9 +520,9 @@ __global__ void __launch_bounds__(kT5Threads, 1) k_phys_inverse_tc5(const __grid
               uint32_t rE = 0, rO = 0;
               fold_levels(cE, tE, rE);
               fold_levels(cO, tO, rO);
-              const int e = g.tcXE[xp] + col_exp(ecol) - 64 + kFoldShift;
-              stage[(size_t)nl * t.stage_ld + xp] = round_plus(tE, rE, tO, rO, e, nonfinite);
-              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = round_minus(tE, rE, tO, rO, e, nonfinite);
+              const int e = g.tcXE[xp] + col_exp(ecol) - 64 + Fold().shift();
+              stage[(size_t)nl * t.stage_ld + xp] = round_plus(Fold(), tE, rE, tO, rO, e, nonfinite);
+              stage[(size_t)nl * t.stage_ld + xp + d.pxh] = round_minus(Fold(), tE, rE, tO, rO, e, nonfinite);
             }
           }
         }

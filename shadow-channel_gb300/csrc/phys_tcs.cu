@@ -91,20 +91,20 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_inv_tc(const __grid_constant_
     const int mt = item / NT, nt = item - mt * NT;
     long long TE[4], TO[4];
     uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
-    tc_tile_range<true, kLongFoldShift>(Az, mt, d.KTz, 0, d.KTzE, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
-    const Rests<true, kLongFoldShift> rE(RE);
-    tc_tile_range<true, kLongFoldShift>(Az, mt, d.KTz, d.KTzE, d.KTz, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
+    tc_tile_range<true>(LongFold(), Az, mt, d.KTz, 0, d.KTzE, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TE, RE);
+    const Rests<true, LongFold> rE(RE);
+    tc_tile_range<true>(LongFold(), Az, mt, d.KTz, d.KTzE, d.KTz, g.tcch, dig, d.KSz, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int row = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
       if (row >= 2 * d.pzh || n >= nx) continue;
-      const int e = kZRowExp + col_exp(exz[n]) - 64 + kLongFoldShift;
+      const int e = kZRowExp + col_exp(exz[n]) - 64 + LongFold().shift();
       const int im = row >= d.pzh, m = im ? row - d.pzh : row;
       bool bad = false;
-      reinterpret_cast<double*>(Tp + (size_t)m * g.X + x0 + n)[im] = round_plus<kLongFoldShift>(TE[r], rE[r], TO[r], RO[r], e, bad);
+      reinterpret_cast<double*>(Tp + (size_t)m * g.X + x0 + n)[im] = round_plus(LongFold(), TE[r], rE[r], TO[r], RO[r], e, bad);
       if (d.Rz == 2)
         reinterpret_cast<double*>(Tp + (size_t)(m + d.pzh) * g.X + x0 + n)[im] =
-            round_minus<kLongFoldShift>(TE[r], rE[r], TO[r], RO[r], e, bad);
+            round_minus(LongFold(), TE[r], rE[r], TO[r], RO[r], e, bad);
     }
   }
 }
@@ -167,16 +167,16 @@ __global__ void __launch_bounds__(kThreads, 3) k_x_inv_tc(const __grid_constant_
     const int mt = item / NT, nt = item - mt * NT;
     long long TE[4], TO[4];
     uint32_t RE[4] = {0, 0, 0, 0}, RO[4] = {0, 0, 0, 0};
-    tc_tile_range<false, kLongFoldShift>(Ax, mt, d.KTx, 0, d.KTxE, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TE, RE);
-    const Rests<true, kLongFoldShift> rE(RE);
-    tc_tile_range<false, kLongFoldShift>(Ax, mt, d.KTx, d.KTxE, d.KTx, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TO, RO);
+    tc_tile_range(LongFold(), Ax, mt, d.KTx, 0, d.KTxE, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TE, RE);
+    const Rests<true, LongFold> rE(RE);
+    tc_tile_range(LongFold(), Ax, mt, d.KTx, d.KTxE, d.KTx, g.tcch, dig, d.KSx, dstride, nt * 8, lane, TO, RO);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int xp = mt * 16 + gq + 8 * (r >> 1), n = nt * 8 + 2 * t + (r & 1);
       if (xp >= d.pxh || n >= nm) continue;
-      const int e = g.tcXE[xp] + col_exp(exx[n]) - 64 + kLongFoldShift;
-      Pm[(size_t)n * g.px + xp] = round_plus<kLongFoldShift>(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
-      if (d.Rx == 2) Pm[(size_t)n * g.px + xp + d.pxh] = round_minus<kLongFoldShift>(TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+      const int e = g.tcXE[xp] + col_exp(exx[n]) - 64 + LongFold().shift();
+      Pm[(size_t)n * g.px + xp] = round_plus(LongFold(), TE[r], rE[r], TO[r], RO[r], e, nonfinite);
+      if (d.Rx == 2) Pm[(size_t)n * g.px + xp + d.pxh] = round_minus(LongFold(), TE[r], rE[r], TO[r], RO[r], e, nonfinite);
     }
   }
   if (nonfinite && a.status) atomicOr(&a.status[inst / a.sdiv], ST_NONFINITE);
@@ -239,17 +239,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_x_fwd_tc(const __grid_constant_
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
     uint32_t R[4] = {0, 0, 0, 0};
-    tc_tile<true, kLongFoldShift>(Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, dstride, nt * 8, lane, S, R);
+    tc_tile<true>(LongFold(), Ax, mt, d.KTxc, kChunkKT, dig + (mt >= d.MTxE ? d.KTxc * 16 : 0), d.KSx, dstride, nt * 8, lane, S, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       FwdRow row;
       if (!fwd_row(mt, gq + 8 * rr, d.MTxE, d.nxE, d.nxO, row)) continue;
-      const int kx = 2 * row.e + row.cls, er = AxE[2 * (row.cls * d.nxE + row.e) + row.part] - 64 + kLongFoldShift;
+      const int kx = 2 * row.e + row.cls, er = AxE[2 * (row.cls * d.nxE + row.e) + row.part] - 64 + LongFold().shift();
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int n = nt * 8 + 2 * t + c;
         if (n >= nz) continue;
-        reinterpret_cast<double*>(Tp + (size_t)n * g.X + kx)[row.part] = round_sum<kLongFoldShift>(S[2 * rr + c], R[2 * rr + c], er + col_exp(exx[n]));
+        reinterpret_cast<double*>(Tp + (size_t)n * g.X + kx)[row.part] = round_sum(LongFold(), S[2 * rr + c], R[2 * rr + c], er + col_exp(exx[n]));
       }
     }
   }
@@ -312,18 +312,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_z_fwd_tc(const __grid_constant_
     const int mt = item / NT, nt = item - mt * NT;
     long long S[4];
     uint32_t R[4] = {0, 0, 0, 0};
-    tc_tile<true, kLongFoldShift>(Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, dstride, nt * 8, lane, S, R);
+    tc_tile<true>(LongFold(), Az, mt, d.KTzc, kChunkKT, dig + (mt >= d.MTzE ? d.KTzc * 16 : 0), d.KSz, dstride, nt * 8, lane, S, R);
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
       FwdRow row;
       if (!fwd_row(mt, gq + 8 * rr, d.MTzE, d.nzE, d.nzO, row)) continue;
-      const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + kLongFoldShift;
+      const int er = g.tcFZE[2 * (row.cls * d.nzE + row.e) + row.part] - 64 + LongFold().shift();
       const int kk = fwd_z_mode(g.Nz, d.Rz, row.cls, row.e), z = kk < g.Nz / 2 ? kk : kk + 1;
       cpx* out = mode < 2 ? H + (((size_t)z * 5 + q) * g.Q + y) * g.X + x0 : Tc + (size_t)kk * g.X;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         const int n = nt * 8 + 2 * t + c;
-        if (n < nx) reinterpret_cast<double*>(out + n)[row.part] = round_sum<kLongFoldShift>(S[2 * rr + c], R[2 * rr + c], er + col_exp(exz[n]));
+        if (n < nx) reinterpret_cast<double*>(out + n)[row.part] = round_sum(LongFold(), S[2 * rr + c], R[2 * rr + c], er + col_exp(exz[n]));
       }
     }
   }

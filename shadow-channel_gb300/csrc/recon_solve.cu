@@ -526,19 +526,19 @@ __device__ void quad_rhs_tc(const Grid& g, const S& gsz, const cpx* __restrict__
     for (int item = warp; item < MTn * NT; item += NTHR >> 5) {
       const int mt = item / NT, nt = item - mt * NT;
       const int col = nt * 4 + t;
-      const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + kLongFoldShift;
-      const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + kLongFoldShift : ecol;
+      const int ecol = col_exp(exc[min(col, kTile - 1)]) - 64 + LongFold().shift();
+      const int ecoli = own(col) ? col_exp(exc[kTile]) - 64 + LongFold().shift() : ecol;
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile<true, kLongFoldShift>(W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
+      tc_tile<true>(LongFold(), W + (size_t)w * MTw * KT * kDig * 32, mt, KT, kChunkKT, dig, KS, (size_t)NC * KS, nt * 8, lane, T,
                     R);
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int row = mt * 16 + gq + 8 * rr;
         if (row >= N || col >= nx) continue;
         const int e = g.tcWE[(size_t)w * gsz.R() + row];
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
-                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+        const cpx val = {round_sum(LongFold(), T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum(LongFold(), T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         cpx& f = F[row * kTile + col];
         if (first) {
           f = val;

@@ -314,11 +314,11 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
     for (int ob = 0; ob < 5; ++ob) {
       const int b = order[ob], cls = b < 3 ? 0 : 1;
       const int KTb = ((cls == 0 ? gsz.D() : gsz.R()) + 15) / 16;
-      const int ecol = col_exp(exc[cls * TILE + col]) - 64 + kLongFoldShift;
-      const int ecoli = col_exp(exc[im_slot(cls, col)]) - 64 + kLongFoldShift;
+      const int ecol = col_exp(exc[cls * TILE + col]) - 64 + LongFold().shift();
+      const int ecoli = col_exp(exc[im_slot(cls, col)]) - 64 + LongFold().shift();
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_range<(MINB <= 2), kLongFoldShift>(A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
+      tc_tile_range<(MINB <= 2)>(LongFold(), A + (size_t)b * MT * KT * kDig * 32, mt, KT, 0, KTb, kChunkKT,
                                  dig + (size_t)cls * kDig * (2 * TILE) * KS, KS, (size_t)(2 * TILE) * KS, nt * 8, lane,
                                  T, R);
 #pragma unroll
@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(NTHR, MINB) k_recon_tc(const __grid_constant__
         if (y >= gsz.Q() || col >= nx) continue;
         const bool mean = meancol && col == 0;
         const int e = g.tcE[(size_t)b * gsz.Q() + y];
-        const cpx val = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
-                         round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+        const cpx val = {round_sum(LongFold(), T[2 * rr], R[2 * rr], e + ecol),
+                         round_sum(LongFold(), T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         const int x = x0 + col;
         cpx* out = U + ((size_t)z * 5 * gsz.Q() + y) * gsz.X() + x;
         const double ax = g.kxK2[(size_t)z * gsz.X() + x], az = g.kzK2[(size_t)z * gsz.X() + x];
@@ -431,14 +431,14 @@ __global__ void __launch_bounds__(256, 1) k_recon_few(const __grid_constant__ Gr
       const uint4* next = part + 1 < nparts ? table(item, 1) : (nxt < nit ? table(nxt, 0) : nullptr);
       long long T[4];
       uint32_t R[4] = {0, 0, 0, 0};
-      tc_tile_stream<kLongFoldShift>(pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
-      const int ecol = col_exp(exc[cls * TILE + t]) - 64 + kLongFoldShift;
-      const int ecoli = meancol && cls == 1 && t == 0 ? col_exp(exc[2 * TILE]) - 64 + kLongFoldShift : ecol;
+      tc_tile_stream(LongFold(), pf, table(item, part), next, KT, base0 + cls * cls_bytes, (uint32_t)(4 * NC * KS), T, R);
+      const int ecol = col_exp(exc[cls * TILE + t]) - 64 + LongFold().shift();
+      const int ecoli = meancol && cls == 1 && t == 0 ? col_exp(exc[2 * TILE]) - 64 + LongFold().shift() : ecol;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const int e = g.tcE[(size_t)b * gsz.Q() + min(mt * 16 + gq + 8 * rr, gsz.Q() - 1)];
-        const cpx v = {round_sum<kLongFoldShift>(T[2 * rr], R[2 * rr], e + ecol),
-                       round_sum<kLongFoldShift>(T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
+        const cpx v = {round_sum(LongFold(), T[2 * rr], R[2 * rr], e + ecol),
+                       round_sum(LongFold(), T[2 * rr + 1], R[2 * rr + 1], e + ecoli)};
         if (part) val[1][rr] = v;
         else val[0][rr] = v;
       }

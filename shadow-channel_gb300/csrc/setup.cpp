@@ -385,9 +385,9 @@ extern "C" int c_setup_tc_table(int Nx, int Ny, int Nz, double Lx, double Lz, do
 // kernels fold them, from the rest `first` on, then a (op 0), a + b (1) or a - b (2).
 // out: t, r, the word that is rounded and its shift; -1 where the two forms of
 // the fold differ.
-template <int FS>
-static int digit_sum(const int* a, int na, const int* b, int nb, int op, int first, long long* out) {
-  auto fold = [](const int* lv, int n, uint32_t r0, long long& t, uint32_t& r) {
+template <class F>
+static int digit_sum(F f, const int* a, int na, const int* b, int nb, int op, int first, long long* out) {
+  auto fold = [&](const int* lv, int n, uint32_t r0, long long& t, uint32_t& r) {
     long long ti = 0;
     uint32_t ri = r0;
     t = 0;
@@ -399,8 +399,8 @@ static int digit_sum(const int* a, int na, const int* b, int nb, int op, int fir
         v[l] = lv[c * chn::kDig + l];
         bits[l] = chn::kAccBits + (l == chn::kDig - 1 ? r : 0u) + (uint32_t)v[l];
       }
-      chn::fold_bits<FS>(bits, t, r);
-      chn::fold_ints<FS>(v, ti, ri);
+      chn::fold_bits(f, bits, t, r);
+      chn::fold_ints(f, v, ti, ri);
     }
     return t == ti && r == ri;
   };
@@ -408,21 +408,37 @@ static int digit_sum(const int* a, int na, const int* b, int nb, int op, int fir
   uint32_t ra, rb;
   if (!fold(a, na, (uint32_t)first, ta, ra) || !fold(b, nb, 0u, tb, rb)) return -1;
   if (op == 1) chn::sum_plus(ta, ra, tb, rb, ta, ra);
-  if (op == 2) chn::sum_minus<FS>(ta, ra, tb, rb, ta, ra);
+  if (op == 2) chn::sum_minus(f, ta, ra, tb, rb, ta, ra);
   int up;
   out[0] = ta;
   out[1] = ra;
-  out[2] = chn::sum_word<FS>(ta, ra, up);
+  out[2] = chn::sum_word(f, ta, ra, up);
   out[3] = up;
   return 0;
 }
 
 extern "C" int c_setup_digit_sum(int shift, const int* a, int na, const int* b, int nb, int op, int first,
                                  long long* out) {
-  if (shift == chn::kFoldShift) return digit_sum<chn::kFoldShift>(a, na, b, nb, op, first, out);
-  if (shift == chn::kLongFoldShift) return digit_sum<chn::kLongFoldShift>(a, na, b, nb, op, first, out);
+  if (shift == chn::Fold().shift()) return digit_sum(chn::Fold(), a, na, b, nb, op, first, out);
+  if (shift == chn::LongFold().shift()) return digit_sum(chn::LongFold(), a, na, b, nb, op, first, out);
   return -2;
 }
 
 // the exponent field of a kept sum t 2^e from a column with the largest field ce
 extern "C" int c_setup_sum_field(long long t, int e, int ce) { return chn::sum_field(t, e, ce); }
+
+// of a grid's transform tables: k-tiles per chunk of the inverse and the forward
+// ones, and whether their rows are long (kRowSum)
+extern "C" int c_setup_transform_rows(int Nx, int Ny, int Nz, int* out) {
+  chn::HostTables t;
+  const char* err = nullptr;
+  if (!chn::build_tables(Nx, Ny, Nz, 6.0, 3.0, 2000.0, 2.0, 0.01, t, &err)) return -1;
+  std::vector<uint32_t> f[3];
+  std::vector<int> e[3], m;
+  bool li = false, lf = false;
+  out[0] = chn::build_phys_tc_tables(t, f[0], e[0], f[1], e[1], m, li);
+  out[1] = chn::build_fwd_split_tables(t, f[0], e[0], f[1], e[1], f[2], e[2], lf);
+  out[2] = li;
+  out[3] = lf;
+  return 0;
+}

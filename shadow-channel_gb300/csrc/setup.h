@@ -45,7 +45,7 @@ bool build_recon_tc_tables(const HostTables& h, std::vector<uint32_t>& frag, std
 bool build_adj_tc_tables(const HostTables& h, std::vector<uint32_t>& btfrag, std::vector<int>& btex,
                          std::vector<uint32_t>& wtfrag, std::vector<int>& wtex);
 // DFT matrices of the inverse z and x transforms as digit tables (phys_tc.cu);
-// long_rows: rows that the sums kept between two stages have no room for (kRowSum)
+// long_rows: some rows need LongFold's sums
 int build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std::vector<int>& zex,
                           std::vector<uint32_t>& xfrag, std::vector<int>& xex, std::vector<int>& zmap, bool& long_rows);
 // the same matrices' digit tables as tcgen05 B operands (phys_tc5.cu)

@@ -3,7 +3,10 @@
 // arithmetic; loops over known extents unroll and index arithmetic folds).
 #pragma once
 
+#include <type_traits>
+
 #include "chn_common.cuh"
+#include "digit_sum.cuh"
 
 namespace chn {
 
@@ -20,7 +23,16 @@ struct SizesRT {
   __device__ int R() const { return g.R; }
   __device__ int D() const { return g.D; }
   __device__ int tcch() const { return g.tcch; }
+  __device__ static constexpr Fold fold() { return Fold(); }
 };
+
+// the same for the one-block forward transforms of grids with long rows (Grid::tcfl)
+struct SizesLong : SizesRT {
+  using SizesRT::SizesRT;
+  __device__ static constexpr LongFold fold() { return LongFold(); }
+};
+template <class S>
+static constexpr bool kRunTimeSizes = std::is_base_of<SizesRT, S>::value;
 
 // the sizes of an NX x NY x NZ grid (Nx, Ny, Nz as in c_init)
 template <int NX, int NY, int NZ>
@@ -35,12 +47,13 @@ struct SizesCT {
   __host__ __device__ static constexpr int R() { return NY - 2; }
   __host__ __device__ static constexpr int D() { return NY - 4; }
   __host__ __device__ static constexpr int tcch() { return 3; }
+  __host__ __device__ static constexpr Fold fold() { return Fold(); }
 };
 
 template <class S>
 __host__ __device__ inline bool sizes_match(const Grid& g) {
   return g.Nz == S::Nz() && g.X == S::X() && g.pz == S::pz() && g.px == S::px() && g.Q == S::Q() &&
-         g.Qh == S::Qh() && g.R == S::R() && g.D == S::D() && g.tcch >= S::tcch();
+         g.Qh == S::Qh() && g.R == S::R() && g.D == S::D() && g.tcch >= S::tcch() && !g.tcfl;
 }
 
 // the grids with specialised builds

@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "chn_common.cuh"
@@ -131,10 +132,10 @@ __device__ __forceinline__ long long scaled_sum(long long t, int s) {
 // FP64 conversion, the power of two added to the exponent field.  Zeros,
 // results outside the normal range and NaN columns (e >= kNanExp / 2) take the
 // multiplications below; bad is set for results that are not finite.
-template <int FS = kFoldShift>
-__device__ __forceinline__ double round_sum(long long t, uint32_t r, int e, bool& bad) {
+template <class F>
+__device__ __forceinline__ double round_sum(F f, long long t, uint32_t r, int e, bool& bad) {
   int up;
-  const double v = (double)sum_word<FS>(t, r, up);
+  const double v = (double)sum_word(f, t, r, up);
   e -= up;
   const int hi = __double2hiint(v);
   const int ef = hi & 0x7FF00000;
@@ -151,17 +152,17 @@ __device__ __forceinline__ double round_sum(long long t, uint32_t r, int e, bool
   return y;
 }
 
-template <int FS = kFoldShift>
-__device__ __forceinline__ double round_sum(long long t, uint32_t r, int e) {
+template <class F>
+__device__ __forceinline__ double round_sum(F f, long long t, uint32_t r, int e) {
   bool bad = false;
-  return round_sum<FS>(t, r, e, bad);
+  return round_sum(f, t, r, e, bad);
 }
 
 // the four rests of a tile that wait while the warp runs its next one, PACK: as
-// bytes of one register, or (FS 10) halves of two
-template <bool PACK, int FS = kFoldShift>
+// bytes of one register, or (LongFold) halves of two
+template <bool PACK, class F>
 struct Rests {
-  static constexpr int kPer = PACK ? (FS == 8 ? 4 : 2) : 1;
+  static constexpr int kPer = PACK ? (std::is_same<F, Fold>::value ? 4 : 2) : 1;
   uint32_t v[4 / kPer];
   __device__ __forceinline__ explicit Rests(const uint32_t (&R)[4]) {
     if constexpr (kPer == 4) {
@@ -182,19 +183,19 @@ struct Rests {
 };
 
 // of the sum and of the difference of two sums
-template <int FS = kFoldShift>
-__device__ __forceinline__ double round_plus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
+template <class F>
+__device__ __forceinline__ double round_plus(F f, long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
   long long t;
   uint32_t r;
   sum_plus(ta, ra, tb, rb, t, r);
-  return round_sum<FS>(t, r, e, bad);
+  return round_sum(f, t, r, e, bad);
 }
-template <int FS = kFoldShift>
-__device__ __forceinline__ double round_minus(long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
+template <class F>
+__device__ __forceinline__ double round_minus(F f, long long ta, uint32_t ra, long long tb, uint32_t rb, int e, bool& bad) {
   long long t;
   uint32_t r;
-  sum_minus<FS>(ta, ra, tb, rb, t, r);
-  return round_sum<FS>(t, r, e, bad);
+  sum_minus(f, ta, ra, tb, rb, t, r);
+  return round_sum(f, t, r, e, bad);
 }
 
 // x is neither infinite nor NaN (integer test on the exponent field)
@@ -262,12 +263,12 @@ __device__ __forceinline__ void digits_pair(long long x0, long long x1, uint32_t
 
 // the level sums of one mma accumulator element (acc[l][i], levels 0..6)
 // folded into (t, r)
-template <int FS>
-__device__ __forceinline__ void fold_acc(const float (&acc)[kDig][4], int i, long long& t, uint32_t& r) {
+template <class F>
+__device__ __forceinline__ void fold_acc(F f, const float (&acc)[kDig][4], int i, long long& t, uint32_t& r) {
   uint32_t b[kDig];
 #pragma unroll
   for (int l = 0; l < kDig; ++l) b[l] = __float_as_uint(acc[l][i]);
-  fold_bits<FS>(b, t, r);
+  fold_bits(f, b, t, r);
 }
 
 // of seven exact level sums (the tcgen05 kernel)
@@ -275,7 +276,7 @@ __device__ __forceinline__ void fold_levels(const float (&lv)[kDig], long long& 
   int v[kDig];
 #pragma unroll
   for (int l = 0; l < kDig; ++l) v[l] = __float2int_rn(lv[l]);
-  fold_ints<kFoldShift>(v, t, r);
+  fold_ints(Fold(), v, t, r);
 }
 
 // lane's ldmatrix address of the digits of the eight columns from n0
@@ -322,11 +323,11 @@ static constexpr int kFragStep = kDig * 32;  // uint4 between the k-tiles of a t
 // [mt][KT][7][32][4]) against the smem digits of the eight columns from n0,
 // over the k-tiles [k0, k1): exact level sums per chunk of at most `chunk`
 // k-tiles, folded into (T, R) per accumulator element (R on entry: added to the
-// sum).  The sum is t 2^(e_row + e_col - 64 + FS) and R a fraction of
+// sum).  The sum is t 2^(e_row + e_col - 64 + fs) and R a fraction of
 // it, for operands scaled to 56-bit integers; an empty range gives T = 0.  PF: the table fragments of k-tile
 // kt + 1 are loaded while kt's products run (tables that live in L2).
-template <bool PF = false, int FS = kFoldShift>
-__device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int mt, int KT, int k0, int k1, int chunk,
+template <bool PF = false, class F>
+__device__ __forceinline__ void tc_tile_range(F f, const uint4* __restrict__ A, int mt, int KT, int k0, int k1, int chunk,
                                               const uint16_t* dig, size_t KS, size_t dstride, int n0, int lane,
                                               long long (&T)[4], uint32_t (&R)[4]) {
 #pragma unroll
@@ -354,15 +355,15 @@ __device__ __forceinline__ void tc_tile_range(const uint4* __restrict__ A, int m
     tile(kc, true);
     for (int kt = kc + 1; kt < kend; ++kt) tile(kt, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fold_acc<FS>(acc, r, T[r], R[r]);
+    for (int r = 0; r < 4; ++r) fold_acc(f, acc, r, T[r], R[r]);
   }
 }
 
-template <bool PF = false, int FS = kFoldShift>
-__device__ __forceinline__ void tc_tile(const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
+template <bool PF = false, class F>
+__device__ __forceinline__ void tc_tile(F f, const uint4* __restrict__ A, int mt, int KT, int chunk, const uint16_t* dig,
                                         size_t KS, size_t dstride, int n0, int lane, long long (&T)[4],
                                         uint32_t (&R)[4]) {
-  tc_tile_range<PF, FS>(A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T, R);
+  tc_tile_range<PF>(f, A, mt, KT, 0, KT, chunk, dig, KS, dstride, n0, lane, T, R);
 }
 
 // The same whole tile as one of a sequence that a warp runs with few others
@@ -377,8 +378,8 @@ __device__ __forceinline__ void tc_stream_start(FragPair& pf, const uint4* __res
   tc_load_frags(pf.f[0], Am);
   tc_load_frags(pf.f[1], Am + kFragStep);
 }
-template <int FS>
-__device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __restrict__ Am, const uint4* __restrict__ An,
+template <class F>
+__device__ __forceinline__ void tc_tile_stream(F f, FragPair& pf, const uint4* __restrict__ Am, const uint4* __restrict__ An,
                                                int KT, uint32_t base, uint32_t dst2, long long (&T)[4], uint32_t (&R)[4]) {
 #pragma unroll
   for (int r = 0; r < 4; ++r) T[r] = 0;
@@ -401,7 +402,7 @@ __device__ __forceinline__ void tc_tile_stream(FragPair& pf, const uint4* __rest
     tile(kc, true);
     if (kc + 1 < KT) tile(kc + 1, false);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) fold_acc<FS>(acc, r, T[r], R[r]);
+    for (int r = 0; r < 4; ++r) fold_acc(f, acc, r, T[r], R[r]);
   }
 }
 
@@ -411,7 +412,7 @@ int digit_row_exponent(const double* row, int K, int top = 256);
 // host: digit table of a row-major matrix M[rows][K] in mma A-fragment order
 // [MT][KT][7][32 lanes][4] (appended to frag), row exponents appended to ex;
 // returns the k-tiles per chunk its level sums allow (0: none).  long_rows: set
-// where a row's sum needs kLongFoldShift
+// where a row's sum needs LongFold
 int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::vector<uint32_t>& frag,
                        std::vector<int>& ex, int top = 256, bool* long_rows = nullptr);
 

@@ -138,3 +138,15 @@ def test_long_transforms_have_tables(lib, nz):
 def test_exponent_field_of_a_kept_sum(lib, t, e, ce, field):
     lib.c_setup_sum_field.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
     assert lib.c_setup_sum_field(t, e, ce) == field
+
+
+@pytest.mark.parametrize("nx,nz,inverse,forward", [
+    (16, 16, 0, 0), (32, 32, 0, 0), (48, 48, 0, 0), (24, 98, 0, 0), (12, 126, 0, 0), (8, 128, 0, 0), (84, 8, 0, 0), (128, 8, 0, 1),
+    (8, 144, 0, 1), (144, 8, 0, 1), (8, 200, 1, 1)])
+def test_which_transforms_have_long_rows(lib, nx, nz, inverse, forward):
+    """(odd padded lengths, whose forward inputs are no sums of two, take twice
+    the length)"""
+    out = (ctypes.c_int * 4)()
+    assert lib.c_setup_transform_rows(nx, 9, nz, out) == 0
+    assert out[0] >= 2 and out[1] >= 2
+    assert (out[2], out[3]) == (inverse, forward)

@@ -1,11 +1,11 @@
 """Calls whose kernels a rule picks, against the kernels of another rule.
 
-Long transforms (144x17x8, 8x17x200): planes that fit one block, whose tables'
-rows have no room in the sums kept between two stages, run the split
-tensor-core passes and agree with the FP64 kernels to rounding.  The oracle built with
-and without FMA contraction differs by at most (primal, tangent, adjoint)
-3.3e-13, 4.0e-13, 3.4e-13 there; the one-step parity tolerances 5e-12, 1e-11,
-3e-11 hold.
+Long transforms: 144x17x8 and 8x17x144, whose forward tables' rows have no room in
+the sums that other grids keep between the stages, run the one-block products
+with coarser ones, 8x17x200 the FFT kernels.  They agree with the FP64 kernels to
+rounding (the oracle built with and without FMA contraction differs by at most
+3.3e-13, 4.0e-13, 3.4e-13 in primal, tangent and adjoint there; the one-step parity
+tolerances hold), and the products' builds with one another bit for bit.
 
 A flow without spanwise variation whose spanwise velocity is 1e-10 of the
 streamwise one: w and the wall-normal vorticity, odd under spanwise reflection,
@@ -33,7 +33,7 @@ from test_gpu_builds import _step
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 200, 1, 2)], ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 144, 1, 2), (8, 17, 200, 1, 2)], ids=lambda c: "x".join(map(str, c)))
 def test_long_transforms_match_the_fp64_kernels(case):
     if not has_gpu():
         pytest.skip("no CUDA device")
@@ -118,3 +118,15 @@ def test_products_of_one_component_a_block_give_the_same_bits(gi):
     from channel import c_channel as cc
     runs = [V._sweeps(cc, V.GRIDS[gi], {"CHN_AUTOTUNE": "0", **env})[0] for env in ({}, {"CHN_PRODUCTS_BUILD": "0"})]
     V._same(*runs)
+
+
+@pytest.mark.parametrize("grid", [(144, 17, 8), (8, 17, 144)], ids=str)
+def test_products_builds_of_long_transforms_give_the_same_bits(grid):
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    from channel import c_channel as cc
+    args = (*grid, 2 * np.pi, np.pi, 2000.0, 2.0, 0.004, 2)
+    runs = [V._sweeps(cc, args, {"CHN_AUTOTUNE": "0", **env})[0] for env in
+            ({}, {"CHN_PRODUCTS_BUILD": "0"}, {"CHN_PRODUCTS_BUILD": "1"}, {"CHN_ADJ_PRODUCTS_PER_PASS": "3"})]
+    for r in runs[1:]:
+        V._same(runs[0], r)
