@@ -2651,18 +2651,26 @@ int c_multi_init(int n, const int* Nx, const int* Ny, const int* Nz, const doubl
     gmax.tcf = std::min(gmax.tcf, g.tcf);
     gmax.tcfl = std::max(gmax.tcfl, g.tcfl);
   }
-  // an even padded z length's digits, split in two classes, can take a k-tile
-  // more than those of the next odd length: a mixed batch is sized as even
-  bool even = false;
-  for (int i = 0; i < n; ++i) even |= m->tabs[i].g.pz % 2 == 0;
-  if (even) gmax.pz += gmax.pz % 2;
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const char* force = getenv("CHN_SPLIT_TRANSFORMS");
+  // an even padded z length's digits, split in two classes, can take a k-tile
+  // more than those of the next odd length: a batch whose largest length is odd
+  // is sized for the next even one where an instance needs that (sized so
+  // throughout, 98 beside any other grid lost the tensor-core transforms, and
+  // some lengths the one-block ones)
+  const int tci = gmax.tci, tcf = gmax.tcf, pz = gmax.pz;
+  for (int even = 0; even < 2; ++even) {
+    gmax.pz = pz + (even ? pz % 2 : 0);
+    gmax.tci = tci && phys_tc_fits(gmax, optin) ? 1 : 0;
+    gmax.tcf = tcf && fwd_tc_plan(gmax, optin, gmax.fwdpb, gmax.fxch) ? 1 : 0;
+    bool covered = true;
+    for (int i = 0; i < n; ++i) covered &= phys_tc_covers(gmax, m->tabs[i].g);
+    if (covered) break;
+  }
+  if (!gmax.tci && !gmax.tcf) gmax.pz = pz;
   gmax.split = (!fused_transforms_fit(gmax, optin) || (force && force[0] == '1')) ? 1 : 0;
-  if (!phys_tc_fits(gmax, optin)) gmax.tci = 0;
-  if (!fwd_tc_plan(gmax, optin, gmax.fwdpb, gmax.fxch)) gmax.tcf = 0;
   if (solve_smem_limit(gmax) > (size_t)optin) {
     set_error(1, "c_multi_init: the largest grid needs more shared memory than the device has");
     c_multi_destroy();

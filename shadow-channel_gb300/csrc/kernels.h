@@ -170,6 +170,8 @@ int tc5_take_error();
 // products + forward transforms as digit GEMMs (mode 0 primal, 1 tangent, 2 adjoint, 3 exact transpose)
 cudaError_t launch_products_tc(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st);
 bool fwd_tc_fits(const Grid& g, int optin);
+// whether an uneven batch's launches, sized for gmax, hold instances of grid g
+bool phys_tc_covers(const Grid& gmax, const Grid& g);
 // the same transforms as z and x passes through PhysArgs::tmp / ProdArgs::tmp, for
 // planes that do not fit one block (phys_tcs.cu; single-grid launches)
 bool phys_tcs_fits(const Grid& g, int optin);

@@ -795,6 +795,19 @@ bool fwd_tc_fits(const Grid& g, int optin) {
   return fwd_tc_plan(g, optin, pb, xch);
 }
 
+bool phys_tc_covers(const Grid& gmax, const Grid& g) {
+  if (gmax.tci)
+    for (int fb = 1; fb <= kFB; ++fb)
+      for (int minb = 2; minb <= 5; ++minb)
+        if (phys_tc_smem_bytes(g, fb, 8) > phys_tc_smem_chunked(gmax, fb, minb)) return false;
+  if (gmax.tcf)
+    for (int pb : {1, gmax.fwdpb}) {
+      auto bytes = [&](const Grid& a) { return fwd_tc_smem_bytes(a, pb, std::min(gmax.fxch, fwd_tc_dims(a).pzp)); };
+      if (bytes(g) > bytes(gmax)) return false;
+    }
+  return true;
+}
+
 template <class S>
 static void launch_products_sizes(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st) {
   const FwdTcDims d = fwd_tc_dims(g);

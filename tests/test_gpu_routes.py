@@ -19,7 +19,15 @@ The adjoint's two product passes as concurrent branches, which only launches of
 more than two planes an SM are (4 of 32x65x32, 7 of 16x33x16, 3 of 48x97x48),
 and products of one component a block, which launches of fewer are, give the
 bits of the passes in turn and of whole planes a block.
+
+Uneven batches whose largest padded z length is odd: 147 beside 18 (24x17x98 and
+20x17x12) keeps the tensor-core transforms, 21 beside 18 (12x17x14 and 20x17x12)
+is sized for an instance that needs more shared memory than the largest, 216 x
+12 beside 18 (144x17x8, long rows) takes the coarser sums for all.  Each
+instance against itself alone; the oracle's two builds differ by at most
+3.9e-13 there.
 """
+import ctypes
 import os
 
 import numpy as np
@@ -32,8 +40,11 @@ from test_gpu_builds import _step
 
 pytestmark = pytest.mark.gpu
 
+PARITY = (5e-12, 1e-11, 3e-11, 3e-11)  # primal, tangent, adjoint, exact adjoint
 
-@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 144, 1, 2), (8, 17, 200, 1, 2)], ids=lambda c: "x".join(map(str, c)))
+
+@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 144, 1, 2), (8, 17, 200, 1, 2)],
+                         ids=lambda c: "x".join(map(str, c)))
 def test_long_transforms_match_the_fp64_kernels(case):
     if not has_gpu():
         pytest.skip("no CUDA device")
@@ -44,7 +55,6 @@ def test_long_transforms_match_the_fp64_kernels(case):
 
 
 ODD_GRID = (16, 33, 16)
-PARITY = (5e-12, 1e-11, 3e-11, 3e-11)  # primal, tangent, adjoint, exact adjoint
 KNOBS = ("CHN_RECON_FP64", "CHN_TRANSFORMS_FP64", "CHN_SOLVE_TILE", "CHN_RECON_BUILD", "CHN_AUTOTUNE")
 
 
@@ -130,3 +140,44 @@ def test_products_builds_of_long_transforms_give_the_same_bits(grid):
             ({}, {"CHN_PRODUCTS_BUILD": "0"}, {"CHN_PRODUCTS_BUILD": "1"}, {"CHN_ADJ_PRODUCTS_PER_PASS": "3"})]
     for r in runs[1:]:
         V._same(runs[0], r)
+@pytest.mark.parametrize("grids", [[(24, 17, 98), (20, 17, 12)], [(20, 17, 12), (12, 17, 14), (20, 17, 12)],
+                                   [(144, 17, 8), (20, 17, 12)]], ids=str)
+def test_uneven_batches(grids):
+    if not has_gpu():
+        pytest.skip("no CUDA device")
+    import torch
+    from channel import c_channel as cc
+    from torch.profiler import ProfilerActivity, profile
+    n = len(grids)
+    i3 = lambda j: (ctypes.c_int * n)(*[g[j] for g in grids])
+    d3 = lambda v: (ctypes.c_double * n)(*[v] * n)
+    states = [[O.synthetic_state(*g, seed=k + i, laminar=k == 0) for i, g in enumerate(grids)] for k in (0, 10, 20)]
+    C, IC, AC = (np.concatenate([x.ravel() for x in xs]) for xs in states)
+    inh = (ctypes.c_int * 1)(1)
+    os.environ["CHN_SWEEP_GRAPHS"] = "0"
+    try:
+        assert cc.lib.c_multi_init(n, i3(0), i3(1), i3(2), d3(2 * np.pi), d3(np.pi), d3(2000.0), d3(2.0), d3(0.004), 1,
+                                   1, 0) == 0, cc.c_last_error_message()
+        with profile(activities=[ProfilerActivity.CUDA]):
+            torch.zeros(8, device="cuda").add_(1)
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            assert cc.lib.c_multi_forward(0, 1, C.ctypes.data, IC.ctypes.data, inh) == 0, cc.c_last_error_message()
+            assert cc.lib.c_multi_adjoint(1, 0, AC.ctypes.data, 1.0) == 0, cc.c_last_error_message()
+    finally:
+        os.environ.pop("CHN_SWEEP_GRAPHS", None)
+        cc.lib.c_multi_destroy()
+    names = {e.name for e in prof.events() if "chn::" in e.name}
+    if names:
+        assert any("k_phys_inverse_tc<" in k for k in names) and any("k_products_tc<" in k for k in names)
+    off = 0
+    for i, g in enumerate(grids):
+        c, ic, ac = (states[k][i].copy() for k in range(3))
+        assert cc.c_init(*g, 2 * np.pi, np.pi, 2000.0, 2.0, 0.004, 1) == 0, cc.c_last_error_message()
+        cc.c_primal(0, c)
+        cc.c_tangent(0, 1, ic, 1)
+        cc.c_adjoint(1, 0, ac, 0, 1.0)
+        assert cc.c_last_error() == 0, cc.c_last_error_message()
+        cc.c_destroy()
+        for a, b, tol in zip((C, IC, AC), (c, ic, ac), PARITY):
+            assert np.linalg.norm(a[off:off + b.size] - b.ravel()) <= tol * np.linalg.norm(b)
+        off += c.size
