@@ -126,6 +126,7 @@ struct Grid {
   const int* tcZM;
   int tci;
   int tcs;     // the transforms that do not fit one block's tensor-core kernel as split tensor-core passes (phys_tcs.cu)
+  int fused;   // a plane fits one block of the FFT kernels
   int tcch;    // k-tiles per accumulation chunk of the transforms' tables (tc_common.cuh; 2 or 3)
   int tcminb;  // build of the tensor-core inverse (2..5: fields per pass, threads, blocks per SM; autotuned)
   // the same inverse on the fifth-generation tensor cores (phys_tc5.cu,

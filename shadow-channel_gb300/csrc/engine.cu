@@ -210,7 +210,8 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   const char* force = getenv("CHN_SPLIT_TRANSFORMS");
   g.general = (radix234_only(g.pz) && radix234_only(g.px)) ? 0 : 1;
-  g.split = (!fused_transforms_fit(g, optin) || (force && force[0] == '1')) ? 1 : 0;
+  g.fused = fused_transforms_fit(g, optin) ? 1 : 0;
+  g.split = (!g.fused || (force && force[0] == '1')) ? 1 : 0;
   g.tvar = 0;
   const char* var = getenv("CHN_SPLIT_VARIANT");  // with CHN_SPLIT_TRANSFORMS=1: this variant
   if (force && force[0] == '1' && var) g.tvar = atoi(var);
@@ -1160,7 +1161,9 @@ static bool autotune_transforms(Engine& e, Work& w) {
   const char* force = getenv("CHN_SPLIT_TRANSFORMS");
   if (force && force[0] == '1') return true;
   Grid& g = e.T.g;
-  if (g.tcs && !w.gdev && !(g.tci && g.tcf)) return true;  // (no choice among the split tensor-core passes)
+  const int nt = w.nseg * (w.ntan > 0 ? w.ntan : 1);
+  // (no choice among the split tensor-core passes)
+  if (g.tcs && !w.gdev && !(g.tci && g.tcf) && (g.tci || split_tc_inverse(g, nt))) return true;
   int dev = 0, optin = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
@@ -1194,7 +1197,6 @@ static bool autotune_transforms(Engine& e, Work& w) {
       if (split_variant_fits(v, g, optin)) cands.push_back({1, v, g.tcminb, 0, 0.f});
   }
   if (cands.size() < 2 || !w.Zt) return true;
-  const int nt = w.nseg * (w.ntan > 0 ? w.ntan : 1);
   auto enqueue = [&]() -> bool {
     PhysArgs p{};
     p.U = cb(w.Ut, w.usz);

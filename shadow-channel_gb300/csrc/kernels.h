@@ -175,6 +175,8 @@ bool phys_tc_covers(const Grid& gmax, const Grid& g);
 // the same transforms as z and x passes through PhysArgs::tmp / ProdArgs::tmp, for
 // planes that do not fit one block (phys_tcs.cu; single-grid launches)
 bool phys_tcs_fits(const Grid& g, int optin);
+// whether an inverse launch of ninst instances takes them (Grid::tcs)
+bool split_tc_inverse(const Grid& g, int ninst);
 cudaError_t launch_phys_inverse_tcs(const Grid& g, const PhysArgs& a, cudaStream_t st);
 cudaError_t launch_products_tcs(const Grid& g, const ProdArgs& a, int mode, cudaStream_t st);
 // pieces the two share: the CFL check from the written fields, the adjoint

@@ -353,7 +353,7 @@ cudaError_t launch_phys_inverse(const Grid& g, const PhysArgs& a, cudaStream_t s
   // the autotuner's choice among the bit-identical FFT variants)
   if (g.tc5 && !a.grids) return launch_phys_inverse_tc5(g, a, st);  // fits every nfields once 6 fit
   if (g.tci) return launch_phys_inverse_tc(g, a, st);
-  if (g.tcs && !a.grids && a.tmp && a.tmp_inst > 0) return launch_phys_inverse_tcs(g, a, st);
+  if (g.tcs && !a.grids && a.tmp && a.tmp_inst > 0 && split_tc_inverse(g, a.ninst)) return launch_phys_inverse_tcs(g, a, st);
   if (g.split) return kSplit[split_index(g)].inverse(g, a, st);
   const size_t sm = phys_smem_bytes(g, a.cfl_check != 0);
   CHN_LAUNCH_FUSED(k_phys_inverse, dim3(g.Q, a.ninst), sm, st, g, a);

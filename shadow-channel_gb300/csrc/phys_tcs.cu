@@ -338,6 +338,21 @@ bool phys_tcs_fits(const Grid& g, int optin) {
   return z_inv_smem(g) <= room && x_inv_smem(g) <= room && x_fwd_smem(g) <= room && z_fwd_smem(g) <= room;
 }
 
+// Narrow planes that fit one block of the FFT kernels (X <= 8 from about Nz = 112
+// on) fill few of a z pass's 16 columns, and their DFTs' work grows with Nz^2: batches
+// of them run the FFTs.  A launch of few planes, one FFT block each, leaves the
+// chip idle and takes the passes.  Inverse of instances of 4x17x128, FFTs against
+// passes: 2 (50 planes) 0.049 / 0.066 ms, 64 0.374 / 1.85; 8x17x128: 2 0.087 /
+// 0.066, 4 0.102 / 0.121, 64 0.78 / 1.91; 12x17x128: 4 (100 planes) 0.124 / 0.126,
+// 32 0.78 / 1.01; 16x33x128 (X = 8, radix 2 and 3): 8 0.562 / 0.519, 32 1.88 /
+// 1.98; 16x17x112 (radix 7): 32 1.11 / 0.93; 20x17x108: 32 1.41 / 1.16.
+bool split_tc_inverse(const Grid& g, int ninst) {
+  const long long planes = (long long)g.Q * ninst;
+  if (!g.fused || g.X > 8) return true;
+  if (g.X == 8) return g.general || planes <= 3 * 152;
+  return planes <= 16 * g.X;
+}
+
 cudaError_t launch_phys_inverse_tcs(const Grid& g, const PhysArgs& a, cudaStream_t st) {
   const int cap = a.tmp_inst * 6 / a.nfields;
   for (int i0 = 0; i0 < a.ninst; i0 += cap) {

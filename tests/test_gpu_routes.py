@@ -43,7 +43,7 @@ pytestmark = pytest.mark.gpu
 PARITY = (5e-12, 1e-11, 3e-11, 3e-11)  # primal, tangent, adjoint, exact adjoint
 
 
-@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 144, 1, 2), (8, 17, 200, 1, 2)],
+@pytest.mark.parametrize("case", [(144, 17, 8, 1, 2), (8, 17, 144, 1, 2), (8, 17, 144, 4, 2), (8, 17, 200, 1, 2)],
                          ids=lambda c: "x".join(map(str, c)))
 def test_long_transforms_match_the_fp64_kernels(case):
     if not has_gpu():

@@ -5,6 +5,9 @@ A launch of few blocks has builds of its own (a component or field per block,
 sizes in or out there as well; CHN_PRODUCTS_BUILD, CHN_ADJ_PRODUCTS_PER_PASS, CHN_SOLVE_TILE
 and CHN_RECON_BUILD ask for a build of the others and get it.  The kernels that
 ran are read by name from the CUDA activity record.
+
+So are those that a rule on sizes picks: the inverse of planes of few kx columns
+(8x17x128) runs the FFTs in batches, the split tensor-core passes where planes are few.
 """
 import ctypes
 import os
@@ -98,3 +101,12 @@ def test_products(grid, env):
 def test_tiles(env, gone):
     assert any(re.search(gone, n) for n in kernels(GRIDS[1], {}))
     assert not any(re.search(gone, n) for n in kernels(GRIDS[1], env))
+
+
+@pytest.mark.parametrize("grid,nseg,kernel", [((8, 17, 128), 1, "k_z_inv_tc"), ((8, 17, 128), 8, "k_phys_inverse"),
+                                              ((20, 17, 108), 20, "k_z_inv_tc")], ids=str)
+def test_inverse_of_narrow_planes(grid, nseg, kernel):
+    names = kernels(grid, {}, nseg)
+    inverse = {k for k in ("k_z_inv_tc", "k_phys_inverse", "k_phys_inverse_tc", "k_tz_inv")
+               if any(re.search(rf"\b{k}\b", n) for n in names)}
+    assert inverse == {kernel}
