@@ -137,16 +137,16 @@ int build_phys_tc_tables(const HostTables& h, std::vector<uint32_t>& zfrag, std:
 
 // forward transforms (channel/pass1.c:312-339): x stage Y[zp][kx] =
 // norm sum_xp p[zp][xp] exp(-2 pi i kx xp/px) for kx < X (rows 2kx, 2kx+1 =
-// Re, Im; the 1/(px pz) scaling folded in; the exact transpose's products
-// take an unscaled copy), z stage F[kz][kx] = sum_zp
-// Y[zp][kx] exp(-2 pi i zp(kz) zp/pz) for the Nz - 1 kept rows (rows 2kk,
+// Re, Im; the 1/(px pz) scaling folded in, Ax; the exact transpose's products
+// take an unscaled copy, Au), z stage F[kz][kx] = sum_zp
+// Y[zp][kx] exp(-2 pi i zp(kz) zp/pz) for the Nz - 1 kept rows (Az: rows 2kk,
 // 2kk+1; K = 2 pz with Re, Im of Y interleaved)
-int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
-                         std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
-                         std::vector<int>& uex) {
+static void fwd_tc_matrices(const HostTables& h, std::vector<double>& Ax, std::vector<double>& Au, std::vector<double>& Az) {
   const int pz = h.pz, px = h.px, Nz = h.Nz, X = h.X, Kk = Nz - 1;
   const double norm = 1.0 / ((3. * h.Nx / 2.) * (3. * h.Nz / 2.));
-  std::vector<double> Ax((size_t)2 * X * px, 0.0), Au((size_t)2 * X * px, 0.0), Az((size_t)2 * Kk * 2 * pz, 0.0);
+  Ax.assign((size_t)2 * X * px, 0.0);
+  Au.assign((size_t)2 * X * px, 0.0);
+  Az.assign((size_t)2 * Kk * 2 * pz, 0.0);
   for (int kx = 0; kx < X; ++kx)
     for (int xp = 0; xp < px; ++xp) {
       const int idx = (int)(((long long)kx * xp) % px);
@@ -166,6 +166,16 @@ int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::
       Az[(size_t)(2 * kk + 1) * 2 * pz + 2 * zp + 1] = c;
     }
   }
+}
+
+// the matrices as whole tables (c_setup_tc_table: they show what the split
+// tables below take their rows from)
+int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
+                        std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
+                        std::vector<int>& uex) {
+  const int pz = h.pz, px = h.px, X = h.X, Kk = h.Nz - 1;
+  std::vector<double> Ax, Au, Az;
+  fwd_tc_matrices(h, Ax, Au, Az);
   xfrag.clear(); xex.clear(); zfrag.clear(); zex.clear(); ufrag.clear(); uex.clear();
   const int cx = append_digit_table(Ax.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, xfrag, xex);
   const int cu = append_digit_table(Au.data(), 2 * X, px, (2 * X + 15) / 16, (px + 15) / 16, ufrag, uex);
@@ -181,46 +191,34 @@ int build_fwd_tc_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::
 int build_fwd_split_tables(const HostTables& h, std::vector<uint32_t>& xfrag, std::vector<int>& xex,
                            std::vector<uint32_t>& zfrag, std::vector<int>& zex, std::vector<uint32_t>& ufrag,
                            std::vector<int>& uex, bool& long_rows) {
-  const int pz = h.pz, px = h.px, Nz = h.Nz, X = h.X;
+  const int pz = h.pz, px = h.px, Nz = h.Nz;
   long_rows = false;
-  const FwdTcDims d = fwd_tc_dims_n(Nz, X, pz, px);
-  const double norm = 1.0 / ((3. * h.Nx / 2.) * (3. * h.Nz / 2.));
+  const FwdTcDims d = fwd_tc_dims_n(Nz, h.X, pz, px);
+  std::vector<double> Ax, Au, Az, C;
+  fwd_tc_matrices(h, Ax, Au, Az);
   xfrag.clear(); xex.clear(); zfrag.clear(); zex.clear(); ufrag.clear(); uex.clear();
   int chunk = kMaxChunkKT;
+  // outputs (of M's row pairs of ld words) of one class over its first K words
+  auto add = [&](const std::vector<double>& M, int ld, const std::vector<int>& out, int K, int KT, int top,
+                 std::vector<uint32_t>& frag, std::vector<int>& ex) {
+    const int rows = 2 * (int)out.size();
+    C.resize((size_t)rows * K);
+    for (int r = 0; r < rows; ++r)
+      std::copy_n(&M[(size_t)(2 * out[r / 2] + r % 2) * ld], K, &C[(size_t)r * K]);
+    chunk = std::min(chunk, append_digit_table(C.data(), rows, K, (rows + 15) / 16, KT, frag, ex, top, &long_rows));
+  };
   for (int c = 0; c < 2; ++c) {
-    const int n = c ? d.nxO : d.nxE;
-    std::vector<double> Ax((size_t)2 * n * d.pxh), Au((size_t)2 * n * d.pxh);
-    for (int e = 0; e < n; ++e)
-      for (int xp = 0; xp < d.pxh; ++xp) {
-        const int idx = (int)(((long long)(2 * e + c) * xp) % px);
-        for (int part = 0; part < 2; ++part) {  // cos, -sin
-          Au[(size_t)(2 * e + part) * d.pxh + xp] = h.twx[2 * idx + part];
-          Ax[(size_t)(2 * e + part) * d.pxh + xp] = h.twx[2 * idx + part] * norm;
-        }
-      }
-    chunk = std::min(chunk, append_digit_table(Ax.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, xfrag, xex, 512, &long_rows));
-    chunk = std::min(chunk, append_digit_table(Au.data(), 2 * n, d.pxh, (2 * n + 15) / 16, d.KTxc, ufrag, uex, 512, &long_rows));
+    std::vector<int> kx;
+    for (int e = 0; e < (c ? d.nxO : d.nxE); ++e) kx.push_back(2 * e + c);
+    add(Ax, px, kx, d.pxh, d.KTxc, 512, xfrag, xex);
+    add(Au, px, kx, d.pxh, d.KTxc, 512, ufrag, uex);
   }
   for (int c = 0; c < d.Rz; ++c) {
     std::vector<int> kk;
     z_class_modes(Nz, pz, c, kk);
-    const int n = (int)kk.size(), K = 2 * d.pzh;
-    if (n != (c ? d.nzO : d.nzE)) return 0;
-    std::vector<double> Az((size_t)2 * n * K);
-    for (int e = 0; e < n; ++e) {
-      const int zo = kk[e] < Nz / 2 ? kk[e] : kk[e] + 1 + Nz / 2;  // padded output row
-      for (int zp = 0; zp < d.pzh; ++zp) {
-        const int idx = (int)(((long long)zo * zp) % pz);
-        const double cs = h.twz[2 * idx], ms = h.twz[2 * idx + 1];  // cos, -sin
-        Az[(size_t)(2 * e) * K + 2 * zp] = cs;
-        Az[(size_t)(2 * e) * K + 2 * zp + 1] = -ms;
-        Az[(size_t)(2 * e + 1) * K + 2 * zp] = ms;
-        Az[(size_t)(2 * e + 1) * K + 2 * zp + 1] = cs;
-      }
-    }
+    if ((int)kk.size() != (c ? d.nzO : d.nzE)) return 0;
     // (an odd length's inputs are no sums: 56 bits)
-    const int top = d.Rz == 2 ? 512 : 256;
-    chunk = std::min(chunk, append_digit_table(Az.data(), 2 * n, K, (2 * n + 15) / 16, d.KTzc, zfrag, zex, top, &long_rows));
+    add(Az, 2 * pz, kk, 2 * d.pzh, d.KTzc, d.Rz == 2 ? 512 : 256, zfrag, zex);
   }
   return chunk;
 }

@@ -356,6 +356,10 @@ extern "C" int c_setup_tc_table(int Nx, int Ny, int Nz, double Lx, double Lz, do
     case 0: case 1: ok = chn::build_recon_tc_tables(t, f[0], e[0], f[1], e[1]); sel = which; break;
     case 2: case 3: ok = chn::build_phys_tc_tables(t, f[0], e[0], f[1], e[1], m, lr); sel = which - 2; break;
     case 4: case 5: case 6: ok = chn::build_fwd_tc_tables(t, f[0], e[0], f[1], e[1], f[2], e[2]); sel = which - 4; break;
+    case 11: case 12: case 13:  // as the kernels take them: x, z, unscaled x
+      ok = chn::build_fwd_split_tables(t, f[0], e[0], f[1], e[1], f[2], e[2], lr);
+      sel = which - 11;
+      break;
     case 7: case 8: ok = chn::build_adj_tc_tables(t, f[0], e[0], f[1], e[1]); sel = which - 7; break;
     case 9: case 10: {
       // the tcgen05 inverse's stacked tables (bytes as 32-bit words) with the
