@@ -524,7 +524,8 @@ __device__ __forceinline__ void quad_T_mean(double scl, const cpx& rb, cpx* out,
 // H_bar = Quad^T(F_bar) on the tensor cores for the columns [0, nx):
 // per plane y the contractions over the modes pa = Qpw^T Fa, qa = Qw^T Fa,
 // rb = Rw^T Fb as GEMMs (rows: planes), then the combination of the FP64
-// loop in k_solve_T (the mean column keeps that loop)
+// loop in k_solve_T (the mean column, whose two lines are Re and Im of Fb's
+// column 0: quad_T_mean)
 template <class S>
 __device__ void quad_T_tc(const Grid& g, const S& gsz, int z, int x0, int nx, int xfirst, SolveTSmem& s, cpx* __restrict__ Hb) {
   const int KTr = (gsz.R() + 15) / 16, MTq = (gsz.Q() + 15) / 16;

@@ -239,7 +239,7 @@ static bool build_device_tables(DevTables& T, int Nx, int Ny, int Nz, double Lx,
   // the inverse's build (phys_tc.cu) until a batch's autotuner has timed
   // them: one field per block, compiled for the grid's sizes where it has
   // them;
-  // CHN_INVERSE_BUILD=2..7 fixes it (and skips that timing)
+  // CHN_INVERSE_BUILD=2..12 fixes it (and skips that timing)
   const char* ib = getenv("CHN_INVERSE_BUILD");
   const int ibv = ib ? atoi(ib) : 0;
   g.tcminb = (ibv >= 2 && ibv <= 12) ? ibv : (spec ? 11 : 4);

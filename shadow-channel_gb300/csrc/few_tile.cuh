@@ -32,7 +32,7 @@ __device__ __forceinline__ void stage_factors(const Grid& g, const S& gsz, size_
 
 // One sweep over the M rows of an elimination chain by a group of NL lanes
 // (NL: the band's reach), rows ascending or (DOWN) descending.  An FP64 warp
-// instruction occupies its scheduler's FP64 unit for some 70 cycles however
+// instruction occupies its scheduler's FP64 unit for some 64 cycles however
 // few lanes are active, so a lane per chain waits for every multiply-add of
 // every row (279 a chain of the alpha band at 32x65x32: 23k cycles); here lane
 // l of the group owns the rows congruent to l, a row's result goes to the

@@ -593,7 +593,9 @@ static int s_t5_optin = 0;
 bool phys_tc5_fits(const Grid& g, int nf, int optin) {
   if (g.pz % 2 || g.px % 2 || nf < 1) return false;
   const T5Dims t = t5_dims(g, nf);
-  // (every class of modes in one chunk of the mma.sync kernel: the same folds)
+  // (every class of modes within the k-tiles for which the tables bound the
+  // level sums: one fold a class.  Where the rest fits, a class has at most
+  // three k-tiles, which every such table allows)
   const PhysTcDims& d = t.d;
   if (max(max(d.KTzE, d.KTz - d.KTzE), max(d.KTxE, d.KTx - d.KTxE)) > g.tcch) return false;
   return t.ncz <= 128 && 7 * t.NpZ <= kT5Cols && 7 * t.NpX <= kT5XO && t5_smem_bytes(t) <= (size_t)optin;
