@@ -76,7 +76,7 @@ __device__ __forceinline__ int ysum_exp(int ce, int fs) { return ce - 1022 - 64 
 // and for an even pz the z stage split radix-2 (decimation in frequency: the even outputs are the
 // transform of a[n] + a[n + N/2], the odd ones of a[n] - a[n + N/2], exact on
 // the 56-bit integers; half the digit products and table bytes: 32x65x32, 256
-// products' instances 2.91 -> 2.78 ms, 128x129x128, one, 1.21 -> 0.87).  Class c of a
+// products' instances 2.91 -> 2.78 ms over zero primal fields, 128x129x128, one, 1.21 -> 0.87).  Class c of a
 // stage: its row tiles from MT?E on (c = 1), its digits KT?c k-tiles on.
 struct FwdTcDims {
   int Rz, pxh, pzh;                     // radix of the z stage's split, inputs per class

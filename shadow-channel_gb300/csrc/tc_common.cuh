@@ -14,7 +14,8 @@
 // folds and the roundings.  Start values that make a level's integer readable
 // from the accumulator's bit pattern, levels combined in pairs in 32 bits, one
 // 64-bit sum and a byte instead of two 64-bit sums and a rounding without a
-// normalising shift take a fold and rounding from about 45 instructions to 30,
+// normalising shift take a fold and rounding from about 45 instructions to 40
+// (30 without the rest, whose price digit_sum.cuh gives),
 // the packed fp16 digits those of a pair of values from 39 to 17.
 #pragma once
 
