@@ -70,31 +70,44 @@ int append_digit_table(const double* M, int rows, int K, int MT, int KT, std::ve
     double mx = 0.0;
     for (int j = 0; j < K; ++j) mx = std::fmax(mx, std::fabs(M[(size_t)y * K + j]));
     if (mx == 0.0) continue;
-    const int e = digit_row_exponent(&M[(size_t)y * K], K, top);  // |M[y][j]| < 2^e
-    ex[ebase + y] = e;
+    int e = digit_row_exponent(&M[(size_t)y * K], K, top);  // |M[y][j]| < 2^e
     double sum = 0.0;
     for (int j = 0; j < K; ++j) sum += std::fabs(M[(size_t)y * K + j]);
-    if (long_rows && std::ldexp(sum, -e) >= kRowSum * 256 / top) *long_rows = true;
-    for (int j = 0; j < K; ++j) {
-      const long long x = std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e));
-      digits56(x, &dig[((size_t)y * (KT * 16) + j) * kDig]);
-    }
-    // the largest level sum any data digits (|d_0| <= top, the others <= 128)
-    // can reach over `chunk` consecutive k-tiles
-    for (int kt = 0; kt < KT && chunk > 0; ++kt) {
-      const int k1 = std::min(std::min(kt + chunk, KT) * 16, K);
-      long long used = 0;  // sum |digit i| of the window, i ascending
-      for (int l = 0; l < kDig; ++l) {
-        long long last = 0;
-        for (int j = kt * 16; j < k1; ++j) last += std::abs(dig[((size_t)y * (KT * 16) + j) * kDig + l]);
-        if (used * 128 + last * top > kLevelMax) {
-          --chunk;
-          --kt;  // this window again, one k-tile narrower
-          break;
-        }
-        used += last;
+    auto is_long = [&] { return std::ldexp(sum, -e) >= kRowSum * 256 / top; };
+    // The largest level sum any data digits (|d_0| <= top, the others <= 128)
+    // can reach over `chunk` consecutive k-tiles sets the chunk.  Equal entries
+    // (the kx = 0 row) have equal digits, which can all be large: a long row
+    // that would not allow kChunkKT gives up a bit and takes other digits (Nx = 100,
+    // Nz = 20, which ran the FFTs otherwise, at half the speed).
+    auto row_chunk = [&](int chunk) {
+      for (int j = 0; j < K; ++j) {
+        const long long x = std::llround(std::ldexp(M[(size_t)y * K + j], 56 - e));
+        digits56(x, &dig[((size_t)y * (KT * 16) + j) * kDig]);
       }
+      for (int kt = 0; kt < KT && chunk > 0; ++kt) {
+        const int k1 = std::min(std::min(kt + chunk, KT) * 16, K);
+        long long used = 0;  // sum |digit i| of the window, i ascending
+        for (int l = 0; l < kDig; ++l) {
+          long long last = 0;
+          for (int j = kt * 16; j < k1; ++j) last += std::abs(dig[((size_t)y * (KT * 16) + j) * kDig + l]);
+          if (used * 128 + last * top > kLevelMax) {
+            --chunk;
+            --kt;  // this window again, one k-tile narrower
+            break;
+          }
+          used += last;
+        }
+      }
+      return chunk;
+    };
+    int c = row_chunk(chunk);
+    while (c < kChunkKT && chunk >= kChunkKT && is_long()) {
+      ++e;
+      c = row_chunk(chunk);
     }
+    chunk = c;
+    ex[ebase + y] = e;
+    if (long_rows && is_long()) *long_rows = true;
   }
   auto at = [&](int y, int k, int i) -> uint16_t {
     if (y >= rows || k >= K) return 0;
